@@ -57,6 +57,8 @@ SIGNATURES = {
                                                 c_ptr]),
     "exact_act_quantized_backward_f16": (c_int, [c_int, c_ptr, c_ptr, c_i64, c_f32, c_ptr, c_ptr]),
     "exact_spmm_f16": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_int, c_ptr, c_ptr]),
+    "exact_spmm_f16_planned": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_i64, c_int, c_ptr, c_i64, c_ptr,
+                                       c_i64, c_ptr, c_ptr]),
     "exact_rows_scale_colsum_workspace_bytes": (c_i64, [c_i64]),
     "exact_rows_scale_colsum": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_ptr, c_i64, c_i64, c_ptr, c_ptr, c_i64, c_ptr]),
     "exact_bn_backward_workspace_bytes": (c_i64, [c_i64]),
@@ -282,9 +284,10 @@ class KernelTimer:
         return out
 
 
-def invoke(name, nbytes, *args, device=None, **extra):
+def invoke(name, nbytes, *args, device=None, label=None, **extra):
     """Call entry point `name` on the device its tensor arguments live on (made current for the call, with
-    that device's current stream); count it as one kernel launch; raise on a non-zero return code."""
+    that device's current stream); count it as one kernel launch; raise on a non-zero return code.  `label`: the
+    name the timer files the call under, when several entry points do one thing."""
     global LAUNCHES
     import torch
     fn = getattr(load(), name)
@@ -300,7 +303,7 @@ def invoke(name, nbytes, *args, device=None, **extra):
         stream = torch.cuda.current_stream(dev).cuda_stream
         args = tuple(stream if a is STREAM else a for a in args)
         if TIMER is not None:
-            rc = TIMER.bracket(name, nbytes, lambda: fn(*args), extra)
+            rc = TIMER.bracket(label or name, nbytes, lambda: fn(*args), extra)
         else:
             rc = fn(*args)
     if HOST_CLOCK is not None:

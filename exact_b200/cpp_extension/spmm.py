@@ -68,6 +68,17 @@ def row_order(rowptr):
     return per["row_order"]
 
 
+def longest_rows(rowptr, threshold):
+    """The rows with more than `threshold` edges, longest first (int32), or None; cached per row-pointer tensor."""
+    per = _plans_of(rowptr)
+    key = ("longest", threshold)
+    if key not in per:
+        deg = rowptr[1:] - rowptr[:-1]
+        n = int((deg > threshold).sum())
+        per[key] = row_order(rowptr)[:n] if n else None
+    return per[key]
+
+
 def _spmm(rowptr, col, value, mat, reduce, regroup=False, route=None):
     """spmm.cc:12-18 -> spmm_cuda.cu:106-170.  `regroup`: the caller accepts a regrouped per-row fp32 sum
     (narrow operands then gather several edges per load instruction).  `route` = (shard, col0, ldd, addresses):
@@ -98,8 +109,19 @@ def _spmm(rowptr, col, value, mat, reduce, regroup=False, route=None):
         out = torch.empty((M, K), dtype=torch.float16, device=mat.device)
         ib = 4 if col.dtype == torch.int32 else 8
         nnz = col.numel()
-        _lib.invoke("exact_spmm_f16", nnz * (2 * K + ib) + 2 * M * K, _lib.ptr(rowptr), _lib.ptr(col), ib, _lib.ptr(value),
-                    _lib.ptr(mat), M, K, _lib.REDUCE[reduce], _lib.ptr(out), _lib.stream_ptr())
+        ldm = (K + 7) // 8 * 8
+        if ldm != K:     # rows in whole 16-byte pieces: the copy is read and written once, the gathers nnz / N times
+            padded = torch.empty((mat.size(0), ldm), dtype=torch.float16, device=mat.device)
+            padded[:, :K].copy_(mat)
+            mat = padded
+        # Four times the fp32 kernel's bound: a row's sum cannot be cut, and up to about a thousand edges the warp that
+        # walks it costs less than the two that chain it (171 us with 1,024, 189 with 512, 215 with 2,048 at 2.5 M edges x 256)
+        thr = 4 * int(config.spmm_long_row)
+        hubs = longest_rows(rowptr, thr) if thr > 0 else None
+        _lib.invoke("exact_spmm_f16_planned", nnz * (2 * K + ib) + 2 * M * K, _lib.ptr(rowptr), _lib.ptr(col), ib,
+                    _lib.ptr(value), _lib.ptr(mat), ldm, M, K, _lib.REDUCE[reduce], _lib.ptr(row_order(rowptr)), thr,
+                    _lib.ptr(hubs), 0 if hubs is None else hubs.numel(), _lib.ptr(out), _lib.stream_ptr(),
+                    label="exact_spmm_f16")
         return out
     if value is not None:
         value = value.detach().to(torch.float32).contiguous()

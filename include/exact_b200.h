@@ -292,10 +292,19 @@ EXACT_API int exact_bn_backward_from_packed(const float* grad_out, int64_t N, in
  * cast the operands to fp16, exact/exact/ops.py:260, 313): term = half(value[e] * mat[col[e], c]) (the bare operand
  * without values), result = half(result + term) in CSR order, mean = half(result / half(max(count, 1))); every
  * Half (op) Half an fp32 operation on the widened values.  value (or NULL), mat [N, K], out [M, K]: fp16 bit
- * patterns.  Rounding after every edge makes the order part of the result: one warp sums a row in CSR order
- * whatever its length. */
+ * patterns.  Rounding after every edge makes the order part of the result: a row is one chain of adds in CSR
+ * order whatever its length. */
 EXACT_API int exact_spmm_f16(const void* rowptr, const void* col, int idx_bytes, const void* value, const void* mat,
                              int64_t M, int64_t K, int reduce, void* out, void* stream);
+
+/* exact_spmm_f16 with a plan of the adjacency's rows: operand rows of pitch `ldm` elements (when ldm is a multiple of 8
+ * and mat 16-byte aligned, the columns K .. ldm - 1 are read and ignored), `row_order` (or NULL) the order in which the
+ * rows are taken, `long_row` the n_long rows with more than `long_threshold` edges, longest first (their sums run on
+ * warps of their own, still one chain in CSR order).  Same bits as exact_spmm_f16. */
+EXACT_API int exact_spmm_f16_planned(const void* rowptr, const void* col, int idx_bytes, const void* value, const void* mat,
+                                     int64_t ldm, int64_t M, int64_t K, int reduce, const int32_t* row_order,
+                                     int64_t long_threshold, const int32_t* long_row, int64_t n_long, void* out,
+                                     void* stream);
 
 /* exact_spmm_split with the second exchange folded into it (no counterpart in the reference): instead of a local
  * [M, K] result followed by exact_rows_scatter, every output row r is stored, by the warp that summed it,
