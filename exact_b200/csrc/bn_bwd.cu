@@ -8,7 +8,7 @@
 // reconstruction never exists, and the backward moves 12 N D bytes instead of 24 N D.
 //
 //   pass 1  bn_bwd_sums_kernel      per column d: sum_n g[n, d] and sum_n g[n, d] (x[n, d] - mean[d]); every CTA
-//                                   writes its partial sums, bn_bwd_finish_kernel adds them in CTA order (no float
+//                                   writes its partial sums, bn_bwd_finish_kernel adds them in a fixed order (no float
 //                                   atomics: results are run-to-run identical) and forms
 //                                   grad_bias = sum g, grad_weight = invstd * sum g (x - mean);
 //   pass 2  bn_bwd_apply_kernel     training: grad_in = (g - sum_g / N - (x - mean) * invstd^2 * sum_gx / N) * invstd * w
@@ -19,6 +19,7 @@
 // is a 16-byte piece of a row.
 #include "exact_b200.h"
 #include "common.cuh"
+#include "partial_sums.cuh"
 
 namespace exb {
 
@@ -159,15 +160,14 @@ __global__ void __launch_bounds__(kBnThreads) bn_bwd_kernel(const __grid_constan
   }
 }
 
-__global__ void bn_bwd_finish_kernel(const float* __restrict__ partial, int n_partial, int D, const float* __restrict__ invstd,
-                                     float* __restrict__ sums, float* __restrict__ grad_weight, float* __restrict__ grad_bias) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= D) return;
-  float a = 0.f, b = 0.f;
-  for (int i = 0; i < n_partial; i++) {
-    a = __fadd_rn(a, partial[(long long)i * 2 * D + d]);
-    b = __fadd_rn(b, partial[(long long)i * 2 * D + D + d]);
-  }
+__global__ void __launch_bounds__(32 * kSumSlices) bn_bwd_finish_kernel(
+    const float* __restrict__ partial, int n_partial, int D, const float* __restrict__ invstd, float* __restrict__ sums,
+    float* __restrict__ grad_weight, float* __restrict__ grad_bias) {
+  __shared__ float s_part[kSumSlices][33];
+  const int d = blockIdx.x * 32 + threadIdx.x;
+  const float a = sum_partials(partial + d, 2LL * D, n_partial, d < D, s_part);
+  const float b = sum_partials(partial + D + d, 2LL * D, n_partial, d < D, s_part);
+  if (threadIdx.y != 0 || d >= D) return;
   sums[d] = a;
   sums[D + d] = b;
   if (grad_bias) grad_bias[d] = a;
@@ -232,7 +232,7 @@ int exact_bn_backward_from_packed(const float* grad_out, int64_t N, int64_t D, c
   if (need_sums) {
     EXB_BN_SWITCH(false)
     EXB_CUDA_OK(cudaGetLastError());
-    bn_bwd_finish_kernel<<<(unsigned)((D + 127) / 128), 128, 0, st>>>(p.partial, grid, (int)D, invstd, p.sums, grad_weight,
+    bn_bwd_finish_kernel<<<(unsigned)((D + 31) / 32), dim3(32, kSumSlices), 0, st>>>(p.partial, grid, (int)D, invstd, p.sums, grad_weight,
                                                                      grad_bias);
     EXB_CUDA_OK(cudaGetLastError());
   }

@@ -4,10 +4,11 @@
 //                                           (A_mean^T g = A^T (D^-1 g), spmm.cc:128-137), zero-padded to Kout columns
 // The framework's own route is a broadcast multiply (a non-vectorised element-wise kernel, split in two above
 // 2 GB: 1.64 ms at 2,449,029 x 256) and a two-stage column reduction (0.58 ms); this kernel reads g once with
-// 16-byte accesses.  Column sums are added in a fixed order (per-CTA partial rows, then CTA order): results are
+// 16-byte accesses.  Column sums are added in a fixed order (per-CTA partial rows, then those): results are
 // run-to-run identical.  A thread owns VEC adjacent columns and walks down the rows.
 #include "exact_b200.h"
 #include "common.cuh"
+#include "partial_sums.cuh"
 
 namespace exb {
 
@@ -88,13 +89,12 @@ __global__ void __launch_bounds__(kRowOpsThreads) rows_scale_colsum_kernel(const
   }
 }
 
-__global__ void rows_colsum_finish_kernel(const float* __restrict__ partial, int n_partial, int K, int Kout,
-                                          float* __restrict__ colsum) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= K) return;
-  float a = 0.f;
-  for (int i = 0; i < n_partial; i++) a = __fadd_rn(a, partial[(long long)i * Kout + c]);
-  colsum[c] = a;
+__global__ void __launch_bounds__(32 * kSumSlices) rows_colsum_finish_kernel(const float* __restrict__ partial, int n_partial,
+                                                                             int K, int Kout, float* __restrict__ colsum) {
+  __shared__ float s_part[kSumSlices][33];
+  const int c = blockIdx.x * 32 + threadIdx.x;
+  const float a = sum_partials(partial + c, Kout, n_partial, c < K, s_part);
+  if (threadIdx.y == 0 && c < K) colsum[c] = a;
 }
 
 }  // namespace exb
@@ -140,7 +140,7 @@ int exact_rows_scale_colsum(const float* g, int64_t n, int64_t K, int64_t ldg, c
   else rows_scale_colsum_kernel<1><<<grid, kRowOpsThreads, 0, st>>>(p);
   EXB_CUDA_OK(cudaGetLastError());
   if (colsum != nullptr) {
-    rows_colsum_finish_kernel<<<(unsigned)((K + 127) / 128), 128, 0, st>>>(p.partial, grid, (int)K, (int)Kout, colsum);
+    rows_colsum_finish_kernel<<<(unsigned)((K + 31) / 32), dim3(32, kSumSlices), 0, st>>>(p.partial, grid, (int)K, (int)Kout, colsum);
     EXB_CUDA_OK(cudaGetLastError());
   }
   return EXB_OK;

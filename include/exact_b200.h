@@ -423,8 +423,9 @@ EXACT_API int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t
  *   g [N, O] fp32, 16-byte aligned, O % 4 == 0, O <= 256; other shapes return code 3 (the caller unpacks and
  *   uses a library GEMM).  tf32 inputs, fp32 accumulation: about 5e-4 relative.
  *   workspace: exact_grad_weight_workspace_bytes(O, pad16(k0) + pad16(k1), SM count) bytes, 256-byte aligned:
- *   its first int32 is the status word (see exact_rp_quantize_pack), the rest holds one partial result per CTA,
- *   added in CTA order by a second kernel (the result does not depend on timing). */
+ *   its first int32 is the status word (see exact_rp_quantize_pack), the rest holds one partial result per CTA (of at
+ *   most 256 columns: more are multiplied in passes), added in a fixed order by a second kernel (the result does not
+ *   depend on timing). */
 EXACT_API int64_t exact_grad_weight_workspace_bytes(int64_t O, int64_t k_total_padded, int max_ctas);
 EXACT_API int exact_grad_weight_from_packed(const float* g, int64_t N, int64_t O, const uint8_t* packed0,
                                             const uint16_t* scale0, const uint16_t* min0, int64_t k0,
