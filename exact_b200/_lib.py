@@ -1,12 +1,19 @@
-"""ctypes binding of libexact_b200.so -- the only route from Python to the CUDA kernels.
+"""Binding of libexact_b200.so -- the only route from Python to the CUDA kernels.
+
+Two ways lead to the same C ABI: native() is the C++ host path on torch tensors that the hot ops and layers take, load()
+the ctypes handle for everything else (row shards, comparison switches, tests).
 
 There is no CPU or eager-PyTorch fallback: if the library is missing or a call fails, an exception
 is raised.
 """
 import ctypes
-import time
+import importlib.machinery
+import importlib.util
 import os
+import sys
 import threading
+import time
+import types
 
 from . import _build
 
@@ -126,6 +133,24 @@ def load():
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The C++ host path (csrc/native*.cpp), bound to the library load() uses.  Raises if it has not been built."""
+    global _native
+    if _native is None:
+        load()
+        if not os.path.exists(_build.NATIVE):
+            raise ExactB200Error(f"{_build.NATIVE} not found: build it with `python -m exact_b200._build`")
+        loader = importlib.machinery.ExtensionFileLoader("_native", _build.NATIVE)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_native", _build.NATIVE, loader=loader))
+        loader.exec_module(mod)
+        mod.bind(os.path.abspath(lib_path()), ExactB200Error)
+        _native = mod
+    return _native
+
+
 def check(rc, what):
     if rc != 0:
         msg = load().exact_last_error()
@@ -190,7 +215,8 @@ def check_status(device=None, force=False):
     caller synchronises anyway (reading the loss, the end of a step); without launches to check it is free."""
     import torch
     dev = torch.cuda.current_device() if device is None else torch.device(device).index
-    if not (force or STATUS_PENDING.get(dev)):
+    pending = _native is not None and _native.take_status_pending(dev)
+    if not (force or pending or STATUS_PENDING.get(dev)):
         return
     lib = load()
     word = c_int(0)
@@ -203,44 +229,59 @@ def check_status(device=None, force=False):
     raise_for_status(word.value)
 
 
-_POLLS = {}   # device index -> (pinned int32 tensor, event) of the status copy in flight
-
-
 def poll_status(device=None):
     """check_status without a synchronisation: looks at the copy of the status word enqueued by the previous
     poll (if it has arrived) and enqueues the next one behind the work launched so far.  A training loop that
     polls once per step learns of an abandoned kernel one step late and never waits for the GPU."""
     import torch
     dev = torch.cuda.current_device() if device is None else torch.device(device).index
-    lib = load()
-    prev = _POLLS.get(dev)
-    word = 0
-    if prev is not None:
-        pinned, event = prev
-        if not event.query():
-            return            # still in flight: look again at the next poll
-        word = int(pinned[0])
-    else:
-        pinned = torch.zeros(1, dtype=torch.int32).pin_memory()
-    if word == 0 and not STATUS_PENDING.get(dev):
-        _POLLS.pop(dev, None)
-        return
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev)
-        if word != 0:
-            check(lib.exact_clear_status(stream.cuda_stream), "exact_clear_status")
-        check(lib.exact_status_async(pinned.data_ptr(), stream.cuda_stream), "exact_status_async")
-        event = torch.cuda.Event()
-        event.record(stream)
-    STATUS_PENDING[dev] = False
-    _POLLS[dev] = (pinned, event)
-    raise_for_status(word)
+    word = native().poll_status(dev, bool(STATUS_PENDING.get(dev)))
+    if word >= 0:
+        STATUS_PENDING[dev] = False
+        raise_for_status(word)
 
 
 # ---- launch accounting and optional per-kernel CUDA-event timing ----------------------------------
-LAUNCHES = 0      # kernels of this library launched so far (each kernel-launching entry point = 1)
-TIMER = None      # a KernelTimer while a benchmark wants per-kernel device times
-HOST_CLOCK = None  # [ns, calls] while a benchmark wants the host time spent inside invoke() (binding + C entry point)
+# LAUNCHES     kernels of this library launched so far (each kernel-launching entry point = 1)
+# TIMER        a KernelTimer while a benchmark wants per-kernel device times
+# HOST_CLOCK   [ns, calls] while a benchmark wants the host time spent inside the binding and the C entry points
+# are properties of this module (below): the C++ host path keeps its own share of each.
+_launches = 0
+_timer = None
+_clock = None
+
+
+class _Module(types.ModuleType):
+    @property
+    def LAUNCHES(self):
+        return _launches + (_native.launches() if _native is not None else 0)
+
+    @property
+    def TIMER(self):
+        return _timer
+
+    @TIMER.setter
+    def TIMER(self, timer):
+        global _timer
+        _timer = timer
+        if _native is not None or timer is not None:
+            native().set_timing(timer is not None)
+
+    @property
+    def HOST_CLOCK(self):
+        if _clock is None or _native is None:
+            return _clock
+        return [_clock[0] + _native.host_ns(), _clock[1] + _native.host_calls()]
+
+    @HOST_CLOCK.setter
+    def HOST_CLOCK(self, clock):
+        global _clock
+        _clock = clock
+        if _native is not None or clock is not None:
+            native().set_clock(clock is not None)
+
+
+sys.modules[__name__].__class__ = _Module
 
 
 LIBRARY_CALLS = {}   # name -> calls: dense work of the path handed to a library kernel (torch) instead of this library's
@@ -260,6 +301,7 @@ class KernelTimer:
 
     def __init__(self):
         self.records = {}
+        self.native = {}    # what summary() has taken from the C++ host path
 
     def bracket(self, name, nbytes, thunk, extra=None):
         import torch
@@ -275,20 +317,31 @@ class KernelTimer:
         import torch
         torch.cuda.synchronize()
         out = {}
+        for name, ms, nbytes, l2_bytes, edge_columns, flops in native().take_calls():
+            r = self.native.setdefault(name, {"launches": 0, "ms": 0.0, "bytes": 0})
+            r["launches"] += 1
+            r["ms"] += ms
+            r["bytes"] += nbytes
+            for key, v in (("l2_bytes", l2_bytes), ("edge_columns", edge_columns), ("flops", flops)):
+                if v >= 0:
+                    r[key] = r.get(key, 0) + v
         for name, recs in self.records.items():
             ms = [r[0].elapsed_time(r[1]) for r in recs]
             out[name] = {"launches": len(recs), "ms": sum(ms), "bytes": sum(r[2] for r in recs)}
             for key in ("l2_bytes", "flops", "edge_columns"):
                 if any(key in r[3] for r in recs):
                     out[name][key] = sum(r[3].get(key, r[2] if key == "l2_bytes" else 0) for r in recs)
+        for name, r in self.native.items():
+            have = out.setdefault(name, {})
+            for key, v in r.items():
+                have[key] = have.get(key, 0) + v
         return out
 
 
-def invoke(name, nbytes, *args, device=None, label=None, **extra):
+def invoke(name, nbytes, *args, device=None, **extra):
     """Call entry point `name` on the device its tensor arguments live on (made current for the call, with
-    that device's current stream); count it as one kernel launch; raise on a non-zero return code.  `label`: the
-    name the timer files the call under, when several entry points do one thing."""
-    global LAUNCHES
+    that device's current stream); count it as one kernel launch; raise on a non-zero return code."""
+    global _launches
     import torch
     fn = getattr(load(), name)
     noted = getattr(_tls, "devices", None) or set()
@@ -297,18 +350,18 @@ def invoke(name, nbytes, *args, device=None, label=None, **extra):
         noted = noted | {torch.device(device).index if torch.device(device).index is not None
                          else torch.cuda.current_device()}
     dev = resolve_device(noted, torch.cuda.current_device())
-    LAUNCHES += 1
-    t0 = time.perf_counter_ns() if HOST_CLOCK is not None else 0
+    _launches += 1
+    t0 = time.perf_counter_ns() if _clock is not None else 0
     with torch.cuda.device(dev):
         stream = torch.cuda.current_stream(dev).cuda_stream
         args = tuple(stream if a is STREAM else a for a in args)
-        if TIMER is not None:
-            rc = TIMER.bracket(label or name, nbytes, lambda: fn(*args), extra)
+        if _timer is not None:
+            rc = _timer.bracket(name, nbytes, lambda: fn(*args), extra)
         else:
             rc = fn(*args)
-    if HOST_CLOCK is not None:
-        HOST_CLOCK[0] += time.perf_counter_ns() - t0
-        HOST_CLOCK[1] += 1
+    if _clock is not None:
+        _clock[0] += time.perf_counter_ns() - t0
+        _clock[1] += 1
     check(rc, name)
     if name in STATUS_CALLS:
         STATUS_PENDING[dev] = True

@@ -125,6 +125,23 @@ class QuantizationConfig:
         # benchmark use it to hash the packed streams); None: no call.
         self.quantized_hook = None
 
+    def native_layers(self):
+        """Whether nothing is set that the layers' C++ nodes do not do: comparison switches, parking in host memory, the
+        simulation mode and per-tensor hooks run in the Python nodes."""
+        return (self.compress_activation and self.stochastic and not self.simulate and not self.swap
+                and self.quantized_hook is None and self.empty_cache_threshold is None and not self.check_device_status
+                and self.grad_weight_in_projected_space and self.skip_dead_saves and self.linear_tensor_core
+                and self.grad_weight_tensor_core)
+
+    def kept_columns(self, width):
+        """Columns of a saved activation after the random projection (ops.py:142); 0 without one."""
+        return int(self.kept_frac * width + 0.999) if self.kept_frac < 1.0 else 0
+
+    def take_offsets(self, n):
+        off = self._offset
+        self._offset += n
+        return off
+
     def manual_seed(self, seed):
         self.seed = int(seed)
         self._offset = 0

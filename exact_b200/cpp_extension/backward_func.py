@@ -34,36 +34,9 @@ def linear_forward(a, weight, bias=None, a2=None, weight2=None, out=None, accumu
         if out is not None:
             return out.add_(r) if accumulate else out.copy_(r)
         return r
-    lib = _lib.load()
-    M, K = a.shape
-    N = weight.size(0)
-    a = _rows16(a)
-    w = weight if weight.stride(1) == 1 else weight.contiguous()
-    K2 = 0
-    if a2 is not None:
-        K2 = a2.size(1)
-        a2 = _rows16(a2)
-        w2 = weight2 if weight2.stride(1) == 1 else weight2.contiguous()
-    if bias is not None:
-        bias = bias.contiguous()
-    if out is None:
-        out = torch.empty((M, N), dtype=torch.float32, device=a.device)
-        accumulate = False
-    assert out.shape == (M, N) and out.stride(1) == 1
-    for n0 in range(0, N, 256):
-        n1 = min(N, n0 + 256)
-        ws = torch.empty(int(lib.exact_linear_workspace_bytes(n1 - n0, K, K2)), dtype=torch.uint8, device=a.device)
-        wb, cb = w[n0:n1], out[:, n0:n1]
-        nbytes = 4 * (M * (K + K2) + (n1 - n0) * (K + K2) + M * (n1 - n0) * (2 if accumulate else 1))
-        _lib.invoke("exact_linear_forward", nbytes, _lib.ptr(a), M, K, a.stride(0), _lib.ptr(wb), wb.stride(0),
-                    _lib.ptr(a2) if K2 else None, K2, a2.stride(0) if K2 else 0,
-                    _lib.ptr(w2[n0:n1]) if K2 else None, w2.stride(0) if K2 else 0, n1 - n0,
-                    _lib.ptr(bias[n0:n1]) if bias is not None else None, 1 if accumulate else 0, _lib.ptr(ws),
-                    _lib.ptr(cb), out.stride(0), _lib.stream_ptr(), flops=6.0 * M * (K + K2) * (n1 - n0))
-        if config.check_device_status:
-            status = int(ws[:4].view(torch.int32).item())
-            if status != 0:
-                raise _lib.ExactB200Error(f"linear_forward: device status {status} (a bounded on-chip wait expired)")
+    out = _lib.native().linear(a, weight, bias, a2, weight2, out, accumulate)
+    if config.check_device_status:
+        _lib.check_status(a.device, force=True)
     return out
 
 
@@ -96,39 +69,16 @@ def grad_weight_supported(g, k0, k1, bits):
             and g.is_contiguous() and (g.data_ptr() % 16 == 0 or O % 4 != 0))
 
 
-_SM_COUNT = {}
-
-
 def grad_weight_from_packed(g, q0, k0, q1=None, k1=0):
     """(g^T Xq0 [O, k0], g^T Xq1 [O, k1] or None) for packed activations q = (packed, bits, scale_bf16, min_bf16)
     of N rows: backward_func.cc:87 with the dequantisation of ops.py:164 folded in, one pass over g."""
-    lib = _lib.load()
-    N, O_true = g.shape
-    if O_true % 4:
-        gp = g.new_zeros((N, (O_true + 3) // 4 * 4))
-        gp[:, :O_true].copy_(g)
-        g = gp
-    N, O = g.shape
-    bits = q0[1]
-    k0pad = (k0 + 15) // 16 * 16
-    kpad = k0pad + ((k1 + 15) // 16 * 16 if q1 is not None else 0)
-    dev = g.device
-    sms = _SM_COUNT.get(dev.index)
-    if sms is None:
-        sms = _SM_COUNT[dev.index] = torch.cuda.get_device_properties(dev).multi_processor_count
-    ws_bytes = int(lib.exact_grad_weight_workspace_bytes(O, kpad, sms))
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-    out = torch.empty((O, kpad), dtype=torch.float32, device=dev)
-    nbytes = 4 * N * O + (N * (k0 + (k1 if q1 is not None else 0)) * bits) // 8 + 4 * N * (2 if q1 is not None else 1)
-    _lib.invoke("exact_grad_weight_from_packed", nbytes, _lib.ptr(g), N, O, _lib.ptr(q0[0]), _lib.ptr(q0[2]), _lib.ptr(q0[3]),
-                k0, _lib.ptr(q1[0]) if q1 is not None else None, _lib.ptr(q1[2]) if q1 is not None else None,
-                _lib.ptr(q1[3]) if q1 is not None else None, k1 if q1 is not None else 0, bits, _lib.ptr(ws), ws_bytes,
-                _lib.ptr(out), kpad, _lib.stream_ptr(), flops=2.0 * N * O * kpad)
+    q1 = (None, None, None, None) if q1 is None else q1
+    k1 = k1 if q1[0] is not None else 0
+    out = _lib.native().grad_weight(g, q0[1], q0[0], q0[2], q0[3], k0, q1[0], q1[2], q1[3], k1)
     if config.check_device_status:
-        status = int(ws[:4].view(torch.int32).item())
-        if status != 0:
-            raise _lib.ExactB200Error(f"grad_weight_from_packed: device status {status} (a bounded on-chip wait expired)")
-    return out[:O_true, :k0], (out[:O_true, k0pad:k0pad + k1] if q1 is not None else None)
+        _lib.check_status(g.device, force=True)
+    k0pad = (k0 + 15) // 16 * 16
+    return out[:, :k0], (out[:, k0pad:k0pad + k1] if k1 else None)
 
 
 def linear_backward(grad_output, input, weight, bias=None, need_grad_input=True):
@@ -168,27 +118,11 @@ def batch_norm_backward_from_packed(grad_out, quantized, weight, running_mean, r
     both of its passes: the column sums and the element-wise pass read the packed bytes and the bf16 row
     statistics, the [N, D] reconstruction is never written.  Returns (grad_input, grad_weight, grad_bias)."""
     q_input, q_bits, q_scale, q_min = quantized
-    g = grad_out.contiguous()
-    N, D = g.shape
     if train:
         mean, invstd = save_mean, save_invstd
     else:
         mean, invstd = running_mean, torch.rsqrt(running_var + eps)
-    mean, invstd = mean.to(torch.float32).contiguous(), invstd.to(torch.float32).contiguous()
-    w = None if weight is None else weight.detach().to(torch.float32).contiguous()
-    lib = _lib.load()
-    ws_bytes = int(lib.exact_bn_backward_workspace_bytes(D))
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=g.device)
-    grad_input = torch.empty_like(g) if output_mask[0] else None
-    grad_weight = torch.empty(D, dtype=torch.float32, device=g.device) if output_mask[1] else None
-    grad_bias = torch.empty(D, dtype=torch.float32, device=g.device) if output_mask[2] else None
-    wpt = 8 // q_bits
-    nbytes = (2 if (grad_input is not None and (train or grad_weight is not None or grad_bias is not None)) else 1) * (
-        N * D * 4 + (N + wpt - 1) // wpt * D + 4 * N) + (N * D * 4 if grad_input is not None else 0)
-    _lib.invoke("exact_bn_backward_from_packed", nbytes, _lib.ptr(g), N, D, _lib.ptr(q_input), q_bits, _lib.ptr(q_scale),
-                _lib.ptr(q_min), _lib.ptr(w), _lib.ptr(mean), _lib.ptr(invstd), 1 if train else 0, _lib.ptr(ws), ws_bytes,
-                _lib.ptr(grad_input), _lib.ptr(grad_weight), _lib.ptr(grad_bias), _lib.stream_ptr())
-    return grad_input, grad_weight, grad_bias
+    return _lib.native().bn_backward(grad_out, q_input, q_scale, q_min, q_bits, weight, mean, invstd, train, *output_mask)
 
 
 def rows_scale_colsum(g, rowscale=None, want_scaled=False, want_colsum=True, pad_to=4):
@@ -196,21 +130,12 @@ def rows_scale_colsum(g, rowscale=None, want_scaled=False, want_colsum=True, pad
     g.sum(0) or None): the operand D^-1 g of the transposed mean aggregation (spmm.cc:128-137) and the bias gradient
     (backward_func.cc:88-90).  Small or non-fp32 inputs take the framework's ops."""
     N, K = g.shape
-    if not (g.is_cuda and g.dtype == torch.float32 and g.dim() == 2 and g.stride(1) == 1 and N >= 1024):
+    if not (g.is_cuda and g.dtype == torch.float32 and g.dim() == 2 and g.stride(1) == 1 and N >= 1024 and pad_to == 4):
         scaled = None
         if want_scaled:
             scaled = g.new_zeros((N, (K + pad_to - 1) // pad_to * pad_to))
             scaled[:, :K] = g if rowscale is None else g * rowscale.unsqueeze(1)
         return scaled, (g.sum(0) if want_colsum else None)
-    lib = _lib.load()
-    Kout = (K + pad_to - 1) // pad_to * pad_to if want_scaled else K
-    out = torch.empty((N, Kout), dtype=torch.float32, device=g.device) if want_scaled else None
-    colsum = torch.empty(K, dtype=torch.float32, device=g.device) if want_colsum else None
-    ws_bytes = int(lib.exact_rows_scale_colsum_workspace_bytes(Kout)) if want_colsum else 0
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=g.device) if want_colsum else None
     if rowscale is not None:
         rowscale = rowscale.to(torch.float32).contiguous()
-    nbytes = 4 * N * K + (4 * N * Kout if want_scaled else 0)
-    _lib.invoke("exact_rows_scale_colsum", nbytes, _lib.ptr(g), N, K, g.stride(0), _lib.ptr(rowscale), _lib.ptr(out), Kout,
-                Kout, _lib.ptr(colsum), _lib.ptr(ws), ws_bytes, _lib.stream_ptr())
-    return out, colsum
+    return _lib.native().rows_scale_colsum(g, rowscale, want_scaled, want_colsum)

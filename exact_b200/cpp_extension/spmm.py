@@ -68,14 +68,15 @@ def row_order(rowptr):
     return per["row_order"]
 
 
-def longest_rows(rowptr, threshold):
-    """The rows with more than `threshold` edges, longest first (int32), or None; cached per row-pointer tensor."""
+def native_plan(rowptr):
+    """The plans of the rows for the C++ host path (made there when a call first needs them); one per row-pointer tensor."""
+    thr = int(config.spmm_long_row)
     per = _plans_of(rowptr)
-    key = ("longest", threshold)
+    key = ("native", thr)
     if key not in per:
-        deg = rowptr[1:] - rowptr[:-1]
-        n = int((deg > threshold).sum())
-        per[key] = row_order(rowptr)[:n] if n else None
+        # fp16: four times the fp32 kernel's bound.  A row's sum cannot be cut, and up to about a thousand edges the warp that
+        # walks it costs less than the two that chain it (171 us with 1,024, 189 with 512, 215 with 2,048 at 2.5 M edges x 256)
+        per[key] = _lib.native().make_plan(thr, 4 * thr)
     return per[key]
 
 
@@ -99,35 +100,14 @@ def _spmm(rowptr, col, value, mat, reduce, regroup=False, route=None):
     mat = mat.contiguous()
     rowptr = rowptr.contiguous()
     col = col.contiguous()
+    if route is None:
+        return _lib.native().spmm(rowptr, col, native_plan(rowptr), value, mat, _lib.REDUCE[reduce] == 1)
     if mat.dtype == torch.float16:
-        # the reference's half instantiation (spmm_cuda.cu:142): every step rounded to half, rows in CSR order
-        if route is not None:
-            raise RuntimeError("fp16 operands have no routed output")
-        if value is not None:
-            value = value.detach().to(torch.float16).contiguous()
-        M, K = rowptr.numel() - 1, mat.size(1)
-        out = torch.empty((M, K), dtype=torch.float16, device=mat.device)
-        ib = 4 if col.dtype == torch.int32 else 8
-        nnz = col.numel()
-        ldm = (K + 7) // 8 * 8
-        if ldm != K:     # rows in whole 16-byte pieces: the copy is read and written once, the gathers nnz / N times
-            padded = torch.empty((mat.size(0), ldm), dtype=torch.float16, device=mat.device)
-            padded[:, :K].copy_(mat)
-            mat = padded
-        # Four times the fp32 kernel's bound: a row's sum cannot be cut, and up to about a thousand edges the warp that
-        # walks it costs less than the two that chain it (171 us with 1,024, 189 with 512, 215 with 2,048 at 2.5 M edges x 256)
-        thr = 4 * int(config.spmm_long_row)
-        hubs = longest_rows(rowptr, thr) if thr > 0 else None
-        _lib.invoke("exact_spmm_f16_planned", nnz * (2 * K + ib) + 2 * M * K, _lib.ptr(rowptr), _lib.ptr(col), ib,
-                    _lib.ptr(value), _lib.ptr(mat), ldm, M, K, _lib.REDUCE[reduce], _lib.ptr(row_order(rowptr)), thr,
-                    _lib.ptr(hubs), 0 if hubs is None else hubs.numel(), _lib.ptr(out), _lib.stream_ptr(),
-                    label="exact_spmm_f16")
-        return out
+        raise RuntimeError("fp16 operands have no routed output")
     if value is not None:
         value = value.detach().to(torch.float32).contiguous()
     M = rowptr.numel() - 1
     K = mat.size(1)
-    out = torch.empty((M, K), dtype=mat.dtype, device=mat.device) if route is None else None
     ib = 4 if col.dtype == torch.int32 else 8
     nnz = col.numel()
     index_bytes = nnz * (ib + (4 if value is not None else 0)) + (M + 1) * ib
@@ -138,35 +118,20 @@ def _spmm(rowptr, col, value, mat, reduce, regroup=False, route=None):
     thr = int(config.spmm_long_row)
     plan = long_row_plan(rowptr, thr, col) if thr > 0 else None
     red = _lib.REDUCE[reduce] | (REGROUP if regroup else 0)
-    narrow = K <= 64 and K % 4 == 0 and M > 0
-    if route is None and narrow:
-        route = (M, 0, K, [out.data_ptr()])   # the same entry point, one local destination: it takes a row order
-    if route is not None:
-        shard, col0, ldd, addresses = route
-        arr = (ctypes.c_void_p * len(addresses))(*addresses)
-        order = row_order(rowptr) if narrow else None
-        none = {"item_row": None, "item_begin": None, "item_end": None, "item_slot": None, "n_items": 0,
-                "long_row": None, "long_item_ptr": None, "n_long": 0}
-        pl = plan if plan is not None else none
-        scratch = torch.empty((pl["n_items"], K), dtype=torch.float32, device=mat.device) if plan is not None else None
-        _lib.invoke("exact_spmm_split_routed", nbytes, _lib.ptr(rowptr), _lib.ptr(col), ib, _lib.ptr(value),
-                    _lib.ptr(mat), M, K, red, thr if plan is not None else 0, _lib.ptr(pl["item_row"]),
-                    _lib.ptr(pl["item_begin"]), _lib.ptr(pl["item_end"]), _lib.ptr(pl["item_slot"]), pl["n_items"],
-                    _lib.ptr(pl["long_row"]), _lib.ptr(pl["long_item_ptr"]), pl["n_long"], _lib.ptr(scratch),
-                    _lib.ptr(order), shard, col0, ldd, arr, len(addresses), _lib.stream_ptr(), device=mat.device,
-                    l2_bytes=l2_bytes, edge_columns=nnz * K)
-        return out
-    if plan is None:
-        _lib.invoke("exact_spmm", nbytes, _lib.ptr(rowptr), _lib.ptr(col), ib, _lib.ptr(value), _lib.ptr(mat), M, K,
-                    red, _lib.ptr(out), _lib.stream_ptr(), l2_bytes=l2_bytes, edge_columns=nnz * K)
-    else:
-        scratch = torch.empty((plan["n_items"], K), dtype=torch.float32, device=mat.device)
-        _lib.invoke("exact_spmm_split", nbytes, _lib.ptr(rowptr), _lib.ptr(col), ib, _lib.ptr(value), _lib.ptr(mat),
-                    M, K, red, thr, _lib.ptr(plan["item_row"]), _lib.ptr(plan["item_begin"]),
-                    _lib.ptr(plan["item_end"]), _lib.ptr(plan["item_slot"]), plan["n_items"], _lib.ptr(plan["long_row"]),
-                    _lib.ptr(plan["long_item_ptr"]), plan["n_long"], _lib.ptr(scratch), _lib.ptr(out),
-                    _lib.stream_ptr(), l2_bytes=l2_bytes, edge_columns=nnz * K)
-    return out
+    shard, col0, ldd, addresses = route
+    arr = (ctypes.c_void_p * len(addresses))(*addresses)
+    order = row_order(rowptr) if K <= 64 and K % 4 == 0 and M > 0 else None
+    none = {"item_row": None, "item_begin": None, "item_end": None, "item_slot": None, "n_items": 0,
+            "long_row": None, "long_item_ptr": None, "n_long": 0}
+    pl = plan if plan is not None else none
+    scratch = torch.empty((pl["n_items"], K), dtype=torch.float32, device=mat.device) if plan is not None else None
+    _lib.invoke("exact_spmm_split_routed", nbytes, _lib.ptr(rowptr), _lib.ptr(col), ib, _lib.ptr(value),
+                _lib.ptr(mat), M, K, red, thr if plan is not None else 0, _lib.ptr(pl["item_row"]),
+                _lib.ptr(pl["item_begin"]), _lib.ptr(pl["item_end"]), _lib.ptr(pl["item_slot"]), pl["n_items"],
+                _lib.ptr(pl["long_row"]), _lib.ptr(pl["long_item_ptr"]), pl["n_long"], _lib.ptr(scratch),
+                _lib.ptr(order), shard, col0, ldd, arr, len(addresses), _lib.stream_ptr(), device=mat.device,
+                l2_bytes=l2_bytes, edge_columns=nnz * K)
+    return None
 
 
 def spmm_sum_fw(row, rowptr, col, value, colptr, csr2csc, mat):

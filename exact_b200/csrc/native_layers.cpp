@@ -1,0 +1,303 @@
+// See native_layers.h.  Each node keeps the tensors the reference's nodes keep (ops.py:128-178, 257-371; layers.py:123-178,
+// 215-265), compressed; what they are made of runs in C++ from the first check to the last launch.
+#include "native_layers.h"
+
+#include <ATen/ThreadLocalState.h>
+
+namespace exb {
+
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+
+namespace {
+
+// Library ops inside a node: no autograd bookkeeping, and no autocast (the node has cast what it casts).
+struct Plain {
+  at::AutoDispatchBelowADInplaceOrView below;
+  c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA)};
+};
+
+template <class T>
+c10::intrusive_ptr<T> state_of(AutogradContext* ctx) {
+  auto it = ctx->saved_data.find("s");
+  if (it == ctx->saved_data.end())
+    throw std::runtime_error("the compressed activations of this layer were released by an earlier backward pass");
+  auto s = c10::static_intrusive_pointer_cast<T>(it->second.toCapsule());
+  ctx->saved_data.clear();   // freed when the backward is done, as `del ctx.saved` does
+  return s;
+}
+
+struct Compressed {
+  Packed q;
+  Tensor R;            // [D, k] of a projected activation
+  int64_t width = 0;   // columns of the packed activation
+};
+
+// (input2rp ->) quantize_activation (ops.py:142-149).  Uses one offset, two with a projection.
+Compressed compress(const Tensor& x, const Saving& how, uint64_t offset) {
+  Compressed c;
+  if (how.kept == 0) {
+    c.q = quantize_pack(x, how.bits, {}, how.seed, offset, how.row_offset);
+    c.width = x.size(1);
+    return c;
+  }
+  c.width = how.kept;
+  c.R = rademacher(x.size(1), how.kept, how.seed, offset, x);
+  if (x.scalar_type() == at::kFloat && how.fused && rp_supported(x.size(1), how.kept)) {
+    c.q = rp_quantize_pack(x, c.R, how.bits, how.seed, offset + 1, how.row_offset);
+    return c;
+  }
+  Tensor y;
+  if (x.scalar_type() == at::kFloat) {
+    y = linear(x, c.R.t(), {}, {}, {}, {}, false);
+  } else {
+    c.R = c.R.to(x.scalar_type());
+    y = at::matmul(x, c.R);
+  }
+  c.q = quantize_pack(y, how.bits, {}, how.seed, offset + 1, how.row_offset);
+  return c;
+}
+
+// g^T x_hat for a saved activation: [O, in_features].
+Tensor weight_grad(const Tensor& g, const Compressed& c, int64_t bits, int64_t N) {
+  Tensor G;
+  if (g.scalar_type() == at::kFloat && g.size(1) <= 256) {
+    G = grad_weight(g.contiguous(), bits, c.q, c.width, nullptr, 0).narrow(1, 0, c.width);
+  } else {
+    G = at::mm(g.t(), unpack(c.q.codes, bits, c.q.scale, c.q.mn, N, c.width));
+  }
+  return c.R.defined() ? at::mm(G, c.R.t()) : G.contiguous();
+}
+
+}  // namespace
+
+// ---- activations --------------------------------------------------------------------------------------
+struct ActNode : Function<ActNode> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t op, double param, const OptTensor& uniforms, int64_t seed,
+                        int64_t offset, int64_t index_offset) {
+    auto [out, mask] = act_forward(op, x, param, uniforms, (uint64_t)seed, (uint64_t)offset, index_offset);
+    ctx->save_for_backward({mask});
+    ctx->saved_data["op"] = op;
+    ctx->saved_data["param"] = param;
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    Plain plain;
+    Tensor g = act_backward(ctx->saved_data["op"].toInt(), grads[0], ctx->get_saved_variables()[0],
+                            ctx->saved_data["param"].toDouble());
+    return {g, {}, {}, {}, {}, {}, {}};
+  }
+};
+
+Tensor act_node(const Tensor& x, int64_t op, double param, const OptTensor& uniforms, uint64_t seed, uint64_t offset,
+                int64_t index_offset) {
+  return ActNode::apply(x, op, param, uniforms, (int64_t)seed, (int64_t)offset, index_offset);
+}
+
+// ---- GCN: A (x W^T) + b ---------------------------------------------------------------------------------
+struct GcnState : torch::CustomClassHolder {
+  c10::intrusive_ptr<Graph> graph;
+  Saving how;
+  Compressed x;
+  Tensor w;            // as used by the products (half under autocast)
+  bool has_bias, half;
+  int64_t rows;
+};
+
+struct GcnNode : Function<GcnNode> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x_, const Tensor& w_, const OptTensor& b,
+                        const c10::intrusive_ptr<GcnState>& s) {
+    const Graph& g = *s->graph;
+    Tensor x = x_.contiguous(), w = w_.detach();
+    Tensor out;
+    if (s->half) {
+      // autocast: the quantised ops cast to half (ops.py:130, 260), the products are the library's half GEMMs
+      x = x.to(at::kHalf);
+      w = w.to(at::kHalf);
+      s->x = compress(x, s->how, s->how.offset);
+      out = spmm(g.fw, g.fw.value, at::linear(x, w), false);
+      if (b) out = out + *b;                 // half + float: float, as the promotion of the reference's add gives
+    } else {
+      s->x = compress(x, s->how, s->how.offset);
+      if (x.size(1) < w.size(0) && x.size(1) % 4 == 0) {
+        // fewer columns in than out: A (x W^T) = (A x) W^T gathers the narrower operand
+        out = linear(spmm(g.fw, g.fw.value, x, false), w, b, {}, {}, {}, false);
+      } else {
+        out = spmm(g.fw, g.fw.value, linear(x, w, {}, {}, {}, {}, false), false);
+        if (b) out.add_(*b);
+      }
+    }
+    s->w = w;
+    s->rows = x.size(0);
+    s->has_bias = b.has_value();
+    ctx->saved_data["s"] = c10::IValue::make_capsule(s);
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    Plain plain;
+    auto s = state_of<GcnState>(ctx);
+    const Graph& gr = *s->graph;
+    const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
+    Tensor g = grads[0].contiguous(), gb, gw, gx;
+    const int64_t O = g.size(1);
+    if (s->half) {
+      if (s->has_bias) gb = std::get<1>(rows_scale_colsum(g.to(at::kFloat), {}, false, true));
+      if (need_x || need_w) {
+        const Tensor gh = spmm(gr.bw, gr.bw.value, g.to(at::kHalf), false);
+        if (need_w) gw = weight_grad(gh, s->x, s->how.bits, s->rows).to(at::kFloat);
+        if (need_x) gx = at::mm(gh, s->w).to(at::kFloat);
+      }
+      return {gx, gw, gb, {}};
+    }
+    if (O % 4) {
+      // whole 16-byte column groups for the gather, the bias gradient on the way
+      auto [padded, sum] = rows_scale_colsum(g, {}, true, s->has_bias);
+      g = padded;
+      gb = sum;
+    } else if (s->has_bias) {
+      gb = std::get<1>(rows_scale_colsum(g, {}, false, true));
+    }
+    if (need_x || need_w) {
+      const Tensor gh = spmm(gr.bw, gr.bw.value, g, false);
+      if (need_w) {
+        gw = weight_grad(gh, s->x, s->how.bits, s->rows);
+        if (O % 4) gw = gw.narrow(0, 0, O);
+      }
+      if (need_x) gx = linear(gh.narrow(1, 0, O), s->w.t(), {}, {}, {}, {}, false);
+    }
+    return {gx, gw, gb, {}};
+  }
+};
+
+Tensor gcn_node(const Tensor& x, const Tensor& w, const OptTensor& b, const c10::intrusive_ptr<Graph>& graph, const Saving& how,
+                bool half) {
+  auto s = c10::make_intrusive<GcnState>();
+  s->graph = graph;
+  s->how = how;
+  s->half = half;
+  c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA)};
+  return GcnNode::apply(x, w, b, s);
+}
+
+// ---- GraphSAGE: reduce(A, x) W_l^T + b (+ x W_r^T) -------------------------------------------------------
+// The compressed tensors are those of the reference's nodes (x once, shared by the aggregation and lin_r; reduce(A, x) for
+// lin_l), drawn in the same order; results differ by fp32 reassociation only.
+struct SageState : torch::CustomClassHolder {
+  c10::intrusive_ptr<Graph> graph;
+  Saving how;
+  Compressed x, agg;
+  Tensor w_l, w_r;
+  bool mean, has_bias, gradient_first, projected_first;
+  int64_t rows;
+};
+
+struct SageNode : Function<SageNode> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x_, const Tensor& w_l_, const OptTensor& b, const OptTensor& w_r_,
+                        const c10::intrusive_ptr<SageState>& s) {
+    const Graph& g = *s->graph;
+    const Tensor x = x_.contiguous(), w_l = w_l_.detach();
+    const int64_t out_f = w_l.size(0), in_f = w_l.size(1);
+    OptTensor w_r;
+    if (w_r_) w_r = w_r_->detach();
+    s->w_l = w_l;
+    if (w_r) s->w_r = *w_r;
+    s->rows = x.size(0);
+    s->has_bias = b.has_value();
+    uint64_t offset = s->how.offset;
+    s->x = compress(x, s->how, offset);       // without lin_r nothing reads it; the noise stays that of the separate nodes
+    if (!w_r) s->x = Compressed();
+    offset += s->how.kept ? 2 : 1;
+    const int64_t k = s->how.kept, kp = (k + 3) / 4 * 4, op = (out_f + 3) / 4 * 4;
+    Tensor out;
+    if (s->projected_first && k && kp + op < in_f) {
+      // Few outputs: reduce(A, x) R = reduce(A, x R) and reduce(A, x) W_l^T = reduce(A, x W_l^T), so the SpMM works on
+      // k + out_features columns and its result holds what lin_l saves (ops.py:142-149) and lin_l's output.
+      s->agg.R = rademacher(in_f, k, s->how.seed, offset, x);
+      s->agg.width = k;
+      Tensor wcat = at::zeros({kp + op, in_f}, w_l.options());
+      wcat.narrow(0, 0, k).copy_(s->agg.R.t());
+      wcat.narrow(0, kp, out_f).copy_(w_l);
+      const Tensor t = spmm(g.fw, g.fw.value, linear(x, wcat, {}, {}, {}, {}, false), s->mean);
+      s->agg.q = quantize_pack(t.narrow(1, 0, k).contiguous(), s->how.bits, {}, s->how.seed, offset + 1, s->how.row_offset);
+      out = t.narrow(1, kp, out_f).contiguous();
+      if (b) out.add_(*b);
+      if (w_r) linear(x, *w_r, {}, {}, {}, out, true);
+    } else {
+      const Tensor agg = spmm(g.fw, g.fw.value, x, s->mean);
+      s->agg = compress(agg, s->how, offset);
+      OptTensor a2;
+      if (w_r) a2 = x;
+      out = linear(agg, w_l, b, a2, w_r, {}, false);
+    }
+    ctx->saved_data["s"] = c10::IValue::make_capsule(s);
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    Plain plain;
+    auto s = state_of<SageState>(ctx);
+    const Graph& gr = *s->graph;
+    const bool need_x = ctx->needs_input_grad(0), has_r = s->w_r.defined();
+    Tensor g = grads[0].contiguous(), gx, gl, gb, gwr;
+    const int64_t O = g.size(1), in_f = s->w_l.size(1), k = s->agg.width;
+    const bool aggregate_g = need_x && s->gradient_first && O <= in_f;
+    const bool by_degree = s->mean && gr.inv_degree.has_value();
+    // One pass over g: D^-1 g (zero-padded to whole column groups), the operand of the transposed mean, and the bias
+    // gradient g.sum(0) (backward_func.cc:88-90).
+    Tensor scaled;
+    if (aggregate_g && (by_degree || O % 4)) {
+      auto [sc, sum] = rows_scale_colsum(g, by_degree ? gr.inv_degree : OptTensor(), true, s->has_bias);
+      scaled = sc;
+      gb = sum;
+    } else if (s->has_bias) {
+      gb = std::get<1>(rows_scale_colsum(g, {}, false, true));
+    }
+    if (O % 4) g = at::constant_pad_nd(g, {0, 4 - O % 4});   // rows in 16-byte pieces for the products below
+    // both weight gradients in one pass over g: g^T [Xq_agg | Xq_x], then the two small transposed projections
+    if (O <= 256) {
+      const int64_t k0pad = (k + 15) / 16 * 16;
+      const Tensor G = grad_weight(g, s->how.bits, s->agg.q, k, has_r ? &s->x.q : nullptr, has_r ? s->x.width : 0).narrow(0, 0, O);
+      gl = G.narrow(1, 0, k);
+      if (has_r) gwr = G.narrow(1, k0pad, s->x.width);
+      gl = s->agg.R.defined() ? at::mm(gl, s->agg.R.t()) : gl.contiguous();
+      if (has_r) gwr = s->x.R.defined() ? at::mm(gwr, s->x.R.t()) : gwr.contiguous();
+    } else {
+      gl = weight_grad(g, s->agg, s->how.bits, s->rows).narrow(0, 0, O);
+      if (has_r) gwr = weight_grad(g, s->x, s->how.bits, s->rows).narrow(0, 0, O);
+    }
+    if (need_x) {
+      const Tensor g_true = g.narrow(1, 0, O);
+      OptTensor a2, w2;
+      if (has_r) {
+        a2 = g_true;
+        w2 = s->w_r.t();
+      }
+      if (aggregate_g) {
+        // A^T (D^-1 g) reads no edge weights; with edge values, or a sum, the transposed structure's weights apply
+        const Tensor t = spmm(gr.bw, by_degree ? OptTensor() : gr.bw.value, scaled.defined() ? scaled : g, false);
+        gx = linear(t.narrow(1, 0, O), s->w_l.t(), {}, a2, w2, {}, false);
+      } else {
+        Tensor y = linear(g_true, s->w_l.t(), {}, {}, {}, {}, false);
+        if (by_degree) y.mul_(gr.inv_degree->unsqueeze(1));   // the transposed structure carries no weights of the mean
+        gx = spmm(gr.bw, gr.bw.value, y, false);
+        if (has_r) linear(g_true, s->w_r.t(), {}, {}, {}, gx, true);
+      }
+    }
+    return {gx, gl, gb, gwr, {}};
+  }
+};
+
+Tensor sage_node(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const OptTensor& w_r,
+                 const c10::intrusive_ptr<Graph>& graph, bool mean, const Saving& how, bool projected_first,
+                 bool gradient_first) {
+  auto s = c10::make_intrusive<SageState>();
+  s->graph = graph;
+  s->how = how;
+  s->mean = mean;
+  s->projected_first = projected_first;
+  s->gradient_first = gradient_first;
+  return SageNode::apply(x, w_l, b_l, w_r, s);
+}
+
+}  // namespace exb

@@ -1,0 +1,304 @@
+// Python bindings of the native ops and layers: METH_FASTCALL functions whose argument conversions are derived from the
+// C++ signatures.
+#include <Python.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <dlfcn.h>
+
+#include "native_layers.h"
+
+namespace exb {
+namespace {
+
+PyObject* g_library_error = nullptr;   // exact_b200.ExactB200Error
+
+// ---- Python -> C++ ------------------------------------------------------------------------------------
+const Tensor& tensor_of(PyObject* o) {
+  if (!THPVariable_Check(o)) throw std::runtime_error("expected a tensor, got " + std::string(Py_TYPE(o)->tp_name));
+  return THPVariable_Unpack(o);
+}
+template <class T>
+struct Arg;
+template <>
+struct Arg<Tensor> {
+  static const Tensor& get(PyObject* o) { return tensor_of(o); }
+};
+template <>
+struct Arg<OptTensor> {
+  static OptTensor get(PyObject* o) { return o == Py_None ? OptTensor() : OptTensor(tensor_of(o)); }
+};
+template <>
+struct Arg<int64_t> {
+  static int64_t get(PyObject* o) {
+    const int64_t v = PyLong_AsLongLong(o);
+    if (v == -1 && PyErr_Occurred()) throw python_error();
+    return v;
+  }
+};
+template <>
+struct Arg<uint64_t> {
+  static uint64_t get(PyObject* o) {
+    const uint64_t v = PyLong_AsUnsignedLongLongMask(o);
+    if (v == (uint64_t)-1 && PyErr_Occurred()) throw python_error();
+    return v;
+  }
+};
+template <>
+struct Arg<double> {
+  static double get(PyObject* o) {
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1.0 && PyErr_Occurred()) throw python_error();
+    return v;
+  }
+};
+template <>
+struct Arg<bool> {
+  static bool get(PyObject* o) { return PyObject_IsTrue(o) == 1; }
+};
+template <class T>
+struct Capsule;   // name of a C++ object that travels as a capsule
+template <>
+struct Capsule<PlanPtr> { static constexpr const char* name = "exact_b200.RowPlan"; };
+template <>
+struct Capsule<c10::intrusive_ptr<Graph>> { static constexpr const char* name = "exact_b200.Graph"; };
+template <class T>
+T& capsule_of(PyObject* o) {
+  void* p = PyCapsule_GetPointer(o, Capsule<T>::name);
+  if (p == nullptr) throw python_error();
+  return *static_cast<T*>(p);
+}
+template <class T>
+PyObject* make_capsule(T value) {
+  return PyCapsule_New(new T(std::move(value)), Capsule<T>::name,
+                       [](PyObject* o) { delete static_cast<T*>(PyCapsule_GetPointer(o, Capsule<T>::name)); });
+}
+template <>
+struct Arg<PlanPtr> {
+  static const PlanPtr& get(PyObject* o) { return capsule_of<PlanPtr>(o); }
+};
+template <>
+struct Arg<c10::intrusive_ptr<Graph>> {
+  static const c10::intrusive_ptr<Graph>& get(PyObject* o) { return capsule_of<c10::intrusive_ptr<Graph>>(o); }
+};
+
+// ---- C++ -> Python ------------------------------------------------------------------------------------
+PyObject* to_py(const Tensor& t) {
+  if (!t.defined()) Py_RETURN_NONE;
+  return THPVariable_Wrap(t);
+}
+PyObject* to_py(int64_t v) { return PyLong_FromLongLong(v); }
+PyObject* to_py(bool v) { return PyBool_FromLong(v); }
+PyObject* to_py(PyObject* o) { return o; }
+PyObject* tuple_of(std::initializer_list<const Tensor*> ts) {
+  PyObject* r = PyTuple_New((Py_ssize_t)ts.size());
+  Py_ssize_t i = 0;
+  for (const Tensor* t : ts) PyTuple_SET_ITEM(r, i++, to_py(*t));
+  return r;
+}
+PyObject* to_py(const Packed& q) { return tuple_of({&q.codes, &q.scale, &q.mn}); }
+PyObject* to_py(const std::tuple<Tensor, Tensor>& t) { return tuple_of({&std::get<0>(t), &std::get<1>(t)}); }
+
+PyObject* to_py(const std::tuple<Tensor, Tensor, Tensor>& t) { return tuple_of({&std::get<0>(t), &std::get<1>(t), &std::get<2>(t)}); }
+
+template <class F>
+struct Fast;
+template <class R, class... A>
+struct Fast<R (*)(A...)> {
+  template <R (*fn)(A...), size_t... I>
+  static PyObject* run(PyObject* const* args, std::index_sequence<I...>) {
+    return to_py(fn(Arg<std::decay_t<A>>::get(args[I])...));
+  }
+  template <R (*fn)(A...)>
+  static PyObject* call(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    try {
+      if (n != (Py_ssize_t)sizeof...(A))
+        throw std::runtime_error("expected " + std::to_string(sizeof...(A)) + " arguments, got " + std::to_string(n));
+      return run<fn>(args, std::index_sequence_for<A...>());
+    } catch (const LibraryError& e) {
+      PyErr_SetString(g_library_error ? g_library_error : PyExc_RuntimeError, e.what());
+      return nullptr;
+    }
+    END_HANDLE_TH_ERRORS
+  }
+};
+#define EXB_METHOD(name, fn) \
+  { name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&Fast<decltype(&fn)>::call<&fn>)), METH_FASTCALL, nullptr }
+
+// ---- functions with shapes of their own ------------------------------------------------------------------
+int64_t launches() { return acct.launches.load(); }
+bool set_timing(bool on) {
+  const bool was = acct.timing.exchange(on);
+  if (on) {
+    std::lock_guard<std::mutex> lock(acct.mu);
+    for (TimedCall& c : acct.calls) {
+      cudaEventDestroy(c.begin);
+      cudaEventDestroy(c.end);
+    }
+    acct.calls.clear();
+  }
+  return was;
+}
+// [(name, ms, bytes, l2_bytes, edge_columns, flops)] of the calls since the last set_timing(True) or take_calls().
+// The caller has synchronised.
+PyObject* take_calls() {
+  std::vector<TimedCall> calls;
+  {
+    std::lock_guard<std::mutex> lock(acct.mu);
+    calls.swap(acct.calls);
+  }
+  PyObject* list = PyList_New(0);
+  for (TimedCall& c : calls) {
+    float ms = 0;
+    cudaEventElapsedTime(&ms, c.begin, c.end);
+    cudaEventDestroy(c.begin);
+    cudaEventDestroy(c.end);
+    PyObject* t = Py_BuildValue("(sdLLLd)", c.name, (double)ms, (long long)c.bytes, (long long)c.l2_bytes, (long long)c.edge_columns,
+                                c.flops);
+    PyList_Append(list, t);
+    Py_DECREF(t);
+  }
+  return list;
+}
+bool set_clock(bool on) {
+  acct.host_ns = 0;
+  acct.host_calls = 0;
+  return acct.clock.exchange(on);
+}
+int64_t host_ns() { return acct.host_ns.load(); }
+int64_t host_calls() { return acct.host_calls.load(); }
+// whether kernels with bounded waits ran on the device since the last call
+bool take_status_pending(int64_t device) {
+  const uint64_t bit = 1ull << (device & 63);
+  return (acct.status_pending.fetch_and(~bit) & bit) != 0;
+}
+
+// _lib.poll_status: a copy of the library's status word is enqueued behind the work launched so far, the next call looks at
+// it if it has arrived.  `also_pending`: launches outside this module are to be looked at.  Returns the word
+// (0: nothing to report, -1: the last copy is still in flight).
+int64_t poll_status(int64_t device, bool also_pending) {
+  struct Poll {
+    int* word = nullptr;      // pinned
+    cudaEvent_t event = nullptr;
+    bool in_flight = false;
+  };
+  static std::mutex mu;
+  static Poll polls[64];
+  if (device < 0 || device >= 64) throw std::runtime_error("poll_status: device out of range");
+  std::lock_guard<std::mutex> lock(mu);
+  Poll& p = polls[device];
+  int word = 0;
+  if (p.in_flight) {
+    if (cudaEventQuery(p.event) != cudaSuccess) {
+      cudaGetLastError();     // not ready: look again at the next poll
+      return -1;
+    }
+    word = *p.word;
+    p.in_flight = false;
+  }
+  const bool pending = take_status_pending(device) || also_pending;
+  if (word == 0 && !pending) return 0;
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+  const cudaStream_t st = c10::cuda::getCurrentCUDAStream().stream();
+  if (p.word == nullptr) {
+    if (cudaHostAlloc(reinterpret_cast<void**>(&p.word), sizeof(int), cudaHostAllocPortable) != cudaSuccess ||
+        cudaEventCreateWithFlags(&p.event, cudaEventDisableTiming) != cudaSuccess)
+      throw LibraryError("poll_status: no pinned memory or event");
+  }
+  int rc = word != 0 ? lib.exact_clear_status(st) : 0;
+  if (rc == 0) rc = lib.exact_status_async(p.word, st);
+  if (rc != 0) library_failure("poll_status", rc);
+  cudaEventRecord(p.event, st);
+  p.in_flight = true;
+  return word;
+}
+
+PyObject* make_plan(int64_t threshold, int64_t threshold_f16) {
+  auto a = std::make_shared<RowPlan>();
+  a->threshold = threshold;
+  a->threshold_f16 = threshold_f16;
+  return make_capsule(PlanPtr(std::move(a)));
+}
+PyObject* make_graph(const Tensor& rowptr, const Tensor& col, const OptTensor& value, const PlanPtr& plan, const Tensor& t_rowptr,
+                     const Tensor& t_col, const OptTensor& t_value, const PlanPtr& t_plan, const OptTensor& inv_degree) {
+  auto g = c10::make_intrusive<Graph>();
+  g->fw = Csr{rowptr, col, value, plan};
+  g->bw = Csr{t_rowptr, t_col, t_value, t_plan};
+  g->inv_degree = inv_degree;
+  return make_capsule(std::move(g));
+}
+Tensor spmm_op(const Tensor& rowptr, const Tensor& col, const PlanPtr& plan, const OptTensor& value, const Tensor& mat, bool mean) {
+  return spmm(rowptr, col, *plan, value, mat, mean);
+}
+PyObject* rp_quantize_pack_op(const Tensor& x, const Tensor& R, int64_t bits, uint64_t seed, uint64_t offset, int64_t row_offset,
+                              bool want_projection) {
+  Tensor y;
+  const Packed q = rp_quantize_pack(x, R, bits, seed, offset, row_offset, want_projection ? &y : nullptr);
+  return want_projection ? tuple_of({&q.codes, &q.scale, &q.mn, &y}) : to_py(q);
+}
+std::tuple<Tensor, Tensor, Tensor> bn_backward_op(const Tensor& g, const Tensor& codes, const Tensor& scale, const Tensor& mn,
+                                                  int64_t bits, const OptTensor& weight, const Tensor& mean, const Tensor& invstd,
+                                                  bool train, bool want_input, bool want_weight, bool want_bias) {
+  return bn_backward(g, Packed{codes, scale, mn}, bits, weight, mean, invstd, train, want_input, want_weight, want_bias);
+}
+Tensor grad_weight_op(const Tensor& g, int64_t bits, const Tensor& p0, const Tensor& s0, const Tensor& m0, int64_t k0,
+                      const OptTensor& p1, const OptTensor& s1, const OptTensor& m1, int64_t k1) {
+  const Packed q0{p0, s0, m0};
+  if (!p1) return grad_weight(g, bits, q0, k0, nullptr, 0);
+  const Packed q1{*p1, *s1, *m1};
+  return grad_weight(g, bits, q0, k0, &q1, k1);
+}
+Tensor gcn_op(const Tensor& x, const Tensor& w, const OptTensor& b, const c10::intrusive_ptr<Graph>& graph, int64_t bits,
+              int64_t kept, uint64_t seed, uint64_t offset, int64_t row_offset, bool fused, bool half) {
+  return gcn_node(x, w, b, graph, Saving{bits, kept, seed, offset, row_offset, fused}, half);
+}
+Tensor sage_op(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const OptTensor& w_r,
+               const c10::intrusive_ptr<Graph>& graph, bool mean, int64_t bits, int64_t kept, uint64_t seed, uint64_t offset,
+               int64_t row_offset, bool fused, bool projected_first, bool gradient_first) {
+  return sage_node(x, w_l, b_l, w_r, graph, mean, Saving{bits, kept, seed, offset, row_offset, fused}, projected_first,
+                   gradient_first);
+}
+
+// bind(path of libexact_b200.so, ExactB200Error)
+PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 2) {
+    PyErr_SetString(PyExc_TypeError, "bind(path, error type)");
+    return nullptr;
+  }
+  const char* path = PyUnicode_AsUTF8(args[0]);
+  if (path == nullptr) return nullptr;
+  void* h = dlopen(path, RTLD_NOW | RTLD_LOCAL);
+  if (h == nullptr) {
+    PyErr_SetString(PyExc_OSError, dlerror());
+    return nullptr;
+  }
+#define EXB_RESOLVE(name)                                                          \
+  lib.name = reinterpret_cast<decltype(lib.name)>(dlsym(h, #name));                \
+  if (lib.name == nullptr) {                                                       \
+    PyErr_SetString(PyExc_AttributeError, "the library does not export " #name);   \
+    return nullptr;                                                                \
+  }
+  EXB_FUNCTIONS(EXB_RESOLVE)
+#undef EXB_RESOLVE
+  Py_XDECREF(g_library_error);
+  Py_INCREF(args[1]);
+  g_library_error = args[1];
+  Py_RETURN_NONE;
+}
+
+PyMethodDef methods[] = {
+    {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&bind)), METH_FASTCALL, nullptr},
+    EXB_METHOD("launches", launches), EXB_METHOD("set_timing", set_timing), EXB_METHOD("take_calls", take_calls),
+    EXB_METHOD("set_clock", set_clock), EXB_METHOD("host_ns", host_ns), EXB_METHOD("host_calls", host_calls),
+    EXB_METHOD("take_status_pending", take_status_pending), EXB_METHOD("poll_status", poll_status), EXB_METHOD("make_plan", make_plan), EXB_METHOD("make_graph", make_graph),
+    EXB_METHOD("quantize_pack", quantize_pack), EXB_METHOD("unpack", unpack), EXB_METHOD("rademacher", rademacher),
+    EXB_METHOD("rp_quantize_pack", rp_quantize_pack_op), EXB_METHOD("bn_backward", bn_backward_op), EXB_METHOD("linear", linear), EXB_METHOD("grad_weight", grad_weight_op),
+    EXB_METHOD("rows_scale_colsum", rows_scale_colsum), EXB_METHOD("spmm", spmm_op), EXB_METHOD("act", act_node),
+    EXB_METHOD("gcn", gcn_op), EXB_METHOD("sage", sage_op), {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+}  // namespace exb
+
+PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&exb::module); }

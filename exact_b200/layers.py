@@ -9,6 +9,7 @@ import torch.nn.functional as F
 from torch import Tensor
 from torch.nn import Parameter
 
+from . import _lib
 from .conf import config
 from .cpp_extension import quantization as ext_quantization
 from .ops import project_and_quantize, qbatch_norm, qlinear
@@ -239,6 +240,12 @@ class QGCNConv(GCNConv):
 
     def forward(self, x, edge_index, edge_weight=None):
         adj_t = self._norm(edge_index)
+        if self.training and config.native_layers() and self._native_takes(adj_t, x):
+            # linear, aggregation and bias as one autograd node; the same compressed tensor and noise as the nodes below
+            st, kept = adj_t.storage, config.kept_columns(x.size(1))
+            return _lib.native().gcn(x, self.weight, self.bias, st.native_graph("sum"), config.activation_compression_bits[0],
+                                     kept, config.seed, config.take_offsets(2 if kept else 1), config.row_offset,
+                                     config.fused_rp, torch.is_autocast_enabled("cuda"))
         if self.training:
             # layers.py:252 passes lin_scheme in the `randmat` slot; the call is equivalent to this one.
             x = qlinear.apply(x, self.weight, None, None, None, self.lin_scheme, True)
@@ -248,6 +255,14 @@ class QGCNConv(GCNConv):
         if self.bias is not None:
             out = out + self.bias
         return out
+
+    def _native_takes(self, adj_t, x):
+        """One GPU's graph without a gradient to its edge values, summed, with enough rows for the tensor-core kernels."""
+        if not isinstance(adj_t, SparseTensor) or self.msg_and_aggr_func.reduce != "sum":
+            return False
+        value = adj_t.storage._value
+        return (x.is_cuda and x.dim() == 2 and x.size(0) >= 1024 and (value is None or not value.requires_grad)
+                and (x.dtype == torch.float32 or torch.is_autocast_enabled("cuda")) and self.weight.dtype == torch.float32)
 
     def message_and_aggregate(self, adj_t, x):
         return self.msg_and_aggr_func(adj_t, x)
@@ -277,6 +292,14 @@ class QSAGEConv(SAGEConv):
         else:
             l_eq_r = False
         if l_eq_r and self.training and not self.normalize and sage_layer_applies(edge_index):
+            if config.native_layers() and self._native_takes(edge_index, x[0]):
+                kept = config.kept_columns(x[0].size(1))
+                return _lib.native().sage(x[0], self.lin_l.weight, self.lin_l.bias,
+                                          self.lin_r.weight if self.root_weight else None,
+                                          edge_index.storage.native_graph(self.msg_and_aggr_func.reduce),
+                                          self.msg_and_aggr_func.reduce == "mean", config.activation_compression_bits[0], kept,
+                                          config.seed, config.take_offsets(4 if kept else 2), config.row_offset, config.fused_rp,
+                                          config.aggregate_projected_first, config.aggregate_gradient_first)
             return qsage_layer.apply(edge_index, x[0], self.lin_l.weight, self.lin_l.bias,
                                      self.lin_r.weight if self.root_weight else None,
                                      self.msg_and_aggr_func.reduce, self.scheme, self.lin_l.scheme)
@@ -292,6 +315,10 @@ class QSAGEConv(SAGEConv):
         if self.normalize:
             out = F.normalize(out, p=2.0, dim=-1)
         return out
+
+    def _native_takes(self, adj_t, x):
+        return (isinstance(adj_t, SparseTensor) and self.msg_and_aggr_func.reduce in ("sum", "mean") and x.is_cuda
+                and x.dim() == 2 and x.size(0) >= 1024 and x.dtype == torch.float32 and self.lin_l.weight.dtype == torch.float32)
 
     def message_and_aggregate(self, adj_t, x, quantized=None, randmat=None):
         return self.msg_and_aggr_func(adj_t, x[0], quantized=quantized, randmat=randmat)

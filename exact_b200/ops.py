@@ -112,9 +112,9 @@ def dequantize_activation(quantized, q_input_shape):
 def _rademacher(rows, cols, device, dtype, seed=None, offset=None):
     """R[D,k] = +-1/sqrt(k) (ops.py:112-114).  The signs come from Philox keyed by (config.seed, offset)
     instead of torch's global CUDA generator, so every rank of a row-sharded run draws the same R."""
-    out = torch.empty((rows, cols), dtype=torch.float32, device=device)
     seed = config.seed if seed is None else seed
     offset = config.next_offset() if offset is None else offset
+    out = torch.empty((rows, cols), dtype=torch.float32, device=device)
     _lib.invoke("exact_rademacher", rows * cols * 4, seed, offset, rows, cols, _lib.ptr(out), _lib.stream_ptr())
     return out if dtype == torch.float32 else out.to(dtype)
 

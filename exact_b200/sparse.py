@@ -85,6 +85,33 @@ class SparseStorage:
         return out
 
 
+    def native_graph(self, reduce):
+        """The adjacency with its transpose and row plans for the layers' C++ nodes (_lib.native()), cached."""
+        from . import _lib
+        from .conf import config
+        from .cpp_extension.spmm import native_plan
+        key = ("native", reduce, config.spmm_long_row)
+        version = None if self._value is None else self._value._version
+        hit = self._t_cache.get(key)
+        if hit is not None and hit[0] == version:
+            return hit[1]
+        t_ptr, t_row, t_w = self.transposed("sum" if self._value is None else reduce)
+        inv = self.inverse_rowcount() if reduce == "mean" and self._value is None else None
+        value = None if self._value is None else self._value.detach()
+        t_plan = native_plan(t_ptr)
+        graph = _lib.native().make_graph(self._rowptr, self._col, value, native_plan(self._rowptr), t_ptr, t_row, t_w,
+                                         t_plan, inv)
+        self._t_cache[key] = (version, graph)
+        return graph
+
+    def inverse_rowcount(self):
+        """1 / max(row length, 1), fp32."""
+        inv = getattr(self, "_inv_deg", None)
+        if inv is None:
+            inv = self._inv_deg = self.rowcount().to(torch.float32).clamp_(min=1).reciprocal_()
+        return inv
+
+
 class SparseTensor:
     def __init__(self, row=None, rowptr=None, col=None, value=None, sparse_sizes=None, is_sorted=False):
         assert col is not None and sparse_sizes is not None

@@ -125,13 +125,7 @@ def _inverse_degree(src):
             src._inv_deg = inv
         return inv
     st = src.storage
-    if st.value() is not None:
-        return None
-    inv = getattr(st, "_inv_deg", None)
-    if inv is None:
-        inv = st.rowcount().to(torch.float32).clamp_(min=1).reciprocal_()
-        st._inv_deg = inv
-    return inv
+    return None if st.value() is not None else st.inverse_rowcount()
 
 
 class qsage_layer(Function):
