@@ -111,6 +111,7 @@ bool rp_supported(int64_t D, int64_t k);
 Packed rp_quantize_pack(const Tensor& x, const Tensor& R, int64_t bits, uint64_t seed, uint64_t offset, int64_t row_offset,
                         Tensor* projection = nullptr);
 bool linear_supported(const Tensor& a);
+Tensor rows16(const Tensor& a);
 Tensor linear(const Tensor& a, const Tensor& w, const OptTensor& bias, const OptTensor& a2, const OptTensor& w2,
               const OptTensor& out, bool accumulate);
 Tensor grad_weight(const Tensor& g, int64_t bits, const Packed& q0, int64_t k0, const Packed* q1, int64_t k1);

@@ -70,6 +70,15 @@ Tensor weight_grad(const Tensor& g, const Compressed& c, int64_t bits, int64_t N
   return c.R.defined() ? at::mm(G, c.R.t()) : G.contiguous();
 }
 
+// A (x W^T) + b
+Tensor gcn_product(const Graph& g, const Tensor& x, const Tensor& w, const OptTensor& b) {
+  if (x.size(1) < w.size(0) && x.size(1) % 4 == 0)   // fewer columns in than out: (A x) W^T gathers the narrower operand
+    return linear(spmm(g.fw, g.fw.value, x, false), w, b, {}, {}, {}, false);
+  Tensor out = spmm(g.fw, g.fw.value, linear(x, w, {}, {}, {}, {}, false), false);
+  if (b) out.add_(*b);
+  return out;
+}
+
 }  // namespace
 
 // ---- activations --------------------------------------------------------------------------------------
@@ -120,13 +129,7 @@ struct GcnNode : Function<GcnNode> {
       if (b) out = out + *b;                 // half + float: float, as the promotion of the reference's add gives
     } else {
       s->x = compress(x, s->how, s->how.offset);
-      if (x.size(1) < w.size(0) && x.size(1) % 4 == 0) {
-        // fewer columns in than out: A (x W^T) = (A x) W^T gathers the narrower operand
-        out = linear(spmm(g.fw, g.fw.value, x, false), w, b, {}, {}, {}, false);
-      } else {
-        out = spmm(g.fw, g.fw.value, linear(x, w, {}, {}, {}, {}, false), false);
-        if (b) out.add_(*b);
-      }
+      out = gcn_product(g, x, w, b);
     }
     s->w = w;
     s->rows = x.size(0);
@@ -196,7 +199,8 @@ struct SageNode : Function<SageNode> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x_, const Tensor& w_l_, const OptTensor& b, const OptTensor& w_r_,
                         const c10::intrusive_ptr<SageState>& s) {
     const Graph& g = *s->graph;
-    const Tensor x = x_.contiguous(), w_l = w_l_.detach();
+    Tensor x = x_.contiguous();
+    const Tensor w_l = w_l_.detach();
     const int64_t out_f = w_l.size(0), in_f = w_l.size(1);
     OptTensor w_r;
     if (w_r_) w_r = w_r_->detach();
@@ -208,6 +212,7 @@ struct SageNode : Function<SageNode> {
     s->x = compress(x, s->how, offset);       // without lin_r nothing reads it; the noise stays that of the separate nodes
     if (!w_r) s->x = Compressed();
     offset += s->how.kept ? 2 : 1;
+    x = rows16(x);                            // several products below read it
     const int64_t k = s->how.kept, kp = (k + 3) / 4 * 4, op = (out_f + 3) / 4 * 4;
     Tensor out;
     if (s->projected_first && k && kp + op < in_f) {
@@ -298,6 +303,43 @@ Tensor sage_node(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const
   s->projected_first = projected_first;
   s->gradient_first = gradient_first;
   return SageNode::apply(x, w_l, b_l, w_r, s);
+}
+
+// ---- evaluation -----------------------------------------------------------------------------------------
+Tensor gcn_eval(const Tensor& x_, const Tensor& w, const OptTensor& b, const c10::intrusive_ptr<Graph>& graph, bool half) {
+  Plain plain;
+  const Graph& g = *graph;
+  if (!half) return gcn_product(g, x_.contiguous(), w, b);
+  const Tensor out = spmm(g.fw, g.fw.value, at::linear(x_.to(at::kHalf), w.to(at::kHalf)), false);
+  return b ? out + *b : out;
+}
+
+Tensor sage_eval(const Tensor& x_, const Tensor& w_l, const OptTensor& b, const OptTensor& w_r,
+                 const c10::intrusive_ptr<Graph>& graph, bool mean, bool half) {
+  Plain plain;
+  const Graph& g = *graph;
+  if (half) {
+    const Tensor x = x_.to(at::kHalf).contiguous();
+    OptTensor b16;
+    if (b) b16 = b->to(at::kHalf);
+    Tensor out = at::linear(spmm(g.fw, g.fw.value, x, mean), w_l.to(at::kHalf), b16);
+    return w_r ? out.add_(at::linear(x, w_r->to(at::kHalf))) : out;
+  }
+  const int64_t out_f = w_l.size(0), in_f = w_l.size(1), pad = (4 - out_f % 4) % 4;
+  const Tensor x = x_.contiguous();
+  if (out_f + pad >= in_f) {
+    const Tensor agg = spmm(g.fw, g.fw.value, x, mean);
+    OptTensor a2;
+    if (w_r) a2 = x;
+    return linear(agg, w_l, b, a2, w_r, {}, false);
+  }
+  // fewer outputs than inputs: reduce(A, x) W_l^T = reduce(A, x W_l^T) gathers the narrower operand
+  const Tensor rows = rows16(x);
+  const Tensor t = spmm(g.fw, g.fw.value, linear(rows, pad ? at::constant_pad_nd(w_l, {0, 0, 0, pad}) : w_l, {}, {}, {}, {}, false), mean);
+  Tensor out = pad ? t.narrow(1, 0, out_f) : t;
+  if (w_r) linear(rows, *w_r, b, {}, {}, out, true);
+  else if (b) out.add_(*b);
+  return out.contiguous();
 }
 
 }  // namespace exb

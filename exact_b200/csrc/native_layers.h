@@ -28,5 +28,9 @@ Tensor gcn_node(const Tensor& x, const Tensor& w, const OptTensor& b, const c10:
 Tensor sage_node(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const OptTensor& w_r,
                  const c10::intrusive_ptr<Graph>& graph, bool mean, const Saving& how, bool projected_first,
                  bool gradient_first);
+// The same layers without anything saved (evaluation).
+Tensor gcn_eval(const Tensor& x, const Tensor& w, const OptTensor& b, const c10::intrusive_ptr<Graph>& graph, bool half);
+Tensor sage_eval(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const OptTensor& w_r,
+                 const c10::intrusive_ptr<Graph>& graph, bool mean, bool half);
 
 }  // namespace exb

@@ -220,11 +220,12 @@ PyObject* make_plan(int64_t threshold, int64_t threshold_f16) {
   a->threshold_f16 = threshold_f16;
   return make_capsule(PlanPtr(std::move(a)));
 }
-PyObject* make_graph(const Tensor& rowptr, const Tensor& col, const OptTensor& value, const PlanPtr& plan, const Tensor& t_rowptr,
-                     const Tensor& t_col, const OptTensor& t_value, const PlanPtr& t_plan, const OptTensor& inv_degree) {
+// t_rowptr, t_col: the transpose, or None for a graph that is only evaluated
+PyObject* make_graph(const Tensor& rowptr, const Tensor& col, const OptTensor& value, const PlanPtr& plan, const OptTensor& t_rowptr,
+                     const OptTensor& t_col, const OptTensor& t_value, const PlanPtr& t_plan, const OptTensor& inv_degree) {
   auto g = c10::make_intrusive<Graph>();
   g->fw = Csr{rowptr, col, value, plan};
-  g->bw = Csr{t_rowptr, t_col, t_value, t_plan};
+  if (t_rowptr) g->bw = Csr{*t_rowptr, *t_col, t_value, t_plan};
   g->inv_degree = inv_degree;
   return make_capsule(std::move(g));
 }
@@ -295,7 +296,7 @@ PyMethodDef methods[] = {
     EXB_METHOD("quantize_pack", quantize_pack), EXB_METHOD("unpack", unpack), EXB_METHOD("rademacher", rademacher),
     EXB_METHOD("rp_quantize_pack", rp_quantize_pack_op), EXB_METHOD("bn_backward", bn_backward_op), EXB_METHOD("linear", linear), EXB_METHOD("grad_weight", grad_weight_op),
     EXB_METHOD("rows_scale_colsum", rows_scale_colsum), EXB_METHOD("spmm", spmm_op), EXB_METHOD("act", act_node),
-    EXB_METHOD("gcn", gcn_op), EXB_METHOD("sage", sage_op), {nullptr, nullptr, 0, nullptr}};
+    EXB_METHOD("gcn", gcn_op), EXB_METHOD("sage", sage_op), EXB_METHOD("gcn_eval", gcn_eval), EXB_METHOD("sage_eval", sage_eval), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

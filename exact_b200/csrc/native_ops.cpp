@@ -174,13 +174,13 @@ bool linear_supported(const Tensor& a) {
   return a.is_cuda() && a.scalar_type() == at::kFloat && a.dim() == 2 && a.size(0) >= 1024;
 }
 
-static Tensor rows16(const Tensor& a) {   // rows that start on 16-byte boundaries: `a` or a zero-padded copy
+// Rows that start on 16-byte boundaries, as tensor maps want them: `a`, or a copy with its rows zero-padded to whole
+// 16-byte pieces (one pass; a layer that multiplies the same rows twice makes the copy once and passes it on).
+Tensor rows16(const Tensor& a) {
   if (a.stride(1) == 1 && a.stride(0) % 4 == 0 && a.stride(0) >= a.size(1) && reinterpret_cast<uintptr_t>(a.data_ptr()) % 16 == 0)
     return a;
-  const int64_t K = a.size(1);
-  Tensor out = at::zeros({a.size(0), (K + 3) / 4 * 4}, a.options().requires_grad(false)).narrow(1, 0, K);
-  out.copy_(a);
-  return out;
+  const Tensor rows = a.stride(1) == 1 && a.stride(0) >= a.size(1) ? a : a.contiguous();
+  return std::get<0>(rows_scale_colsum(rows, {}, true, false)).narrow(1, 0, a.size(1));
 }
 
 Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const OptTensor& a2_, const OptTensor& w2_,

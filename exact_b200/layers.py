@@ -246,6 +246,9 @@ class QGCNConv(GCNConv):
             return _lib.native().gcn(x, self.weight, self.bias, st.native_graph("sum"), config.activation_compression_bits[0],
                                      kept, config.seed, config.take_offsets(2 if kept else 1), config.row_offset,
                                      config.fused_rp, torch.is_autocast_enabled("cuda"))
+        if not self.training and not torch.is_grad_enabled() and config.linear_tensor_core and self._native_takes(adj_t, x):
+            return _lib.native().gcn_eval(x, self.weight, self.bias, adj_t.storage.native_graph(None),
+                                          torch.is_autocast_enabled("cuda"))
         if self.training:
             # layers.py:252 passes lin_scheme in the `randmat` slot; the call is equivalent to this one.
             x = qlinear.apply(x, self.weight, None, None, None, self.lin_scheme, True)
@@ -261,8 +264,8 @@ class QGCNConv(GCNConv):
         if not isinstance(adj_t, SparseTensor) or self.msg_and_aggr_func.reduce != "sum":
             return False
         value = adj_t.storage._value
-        return (x.is_cuda and x.dim() == 2 and x.size(0) >= 1024 and (value is None or not value.requires_grad)
-                and (x.dtype == torch.float32 or torch.is_autocast_enabled("cuda")) and self.weight.dtype == torch.float32)
+        return (x.is_cuda and x.dim() == 2 and x.size(0) >= 1024
+                and (value is None or not value.requires_grad or not torch.is_grad_enabled()) and (x.dtype == torch.float32 or torch.is_autocast_enabled("cuda")) and self.weight.dtype == torch.float32)
 
     def message_and_aggregate(self, adj_t, x):
         return self.msg_and_aggr_func(adj_t, x)
@@ -303,6 +306,11 @@ class QSAGEConv(SAGEConv):
             return qsage_layer.apply(edge_index, x[0], self.lin_l.weight, self.lin_l.bias,
                                      self.lin_r.weight if self.root_weight else None,
                                      self.msg_and_aggr_func.reduce, self.scheme, self.lin_l.scheme)
+        if (l_eq_r and not self.training and not self.normalize and not torch.is_grad_enabled() and config.linear_tensor_core
+                and self._native_takes(edge_index, x[0])):
+            return _lib.native().sage_eval(x[0], self.lin_l.weight, self.lin_l.bias, self.lin_r.weight if self.root_weight else None,
+                                           edge_index.storage.native_graph(None), self.msg_and_aggr_func.reduce == "mean",
+                                           torch.is_autocast_enabled("cuda"))
         if l_eq_r and self.training:
             quantized, randmat, _ = project_and_quantize(x[0], self.scheme, True)
         else:
@@ -318,7 +326,8 @@ class QSAGEConv(SAGEConv):
 
     def _native_takes(self, adj_t, x):
         return (isinstance(adj_t, SparseTensor) and self.msg_and_aggr_func.reduce in ("sum", "mean") and x.is_cuda
-                and x.dim() == 2 and x.size(0) >= 1024 and x.dtype == torch.float32 and self.lin_l.weight.dtype == torch.float32)
+                and x.dim() == 2 and x.size(0) >= 1024 and self.lin_l.weight.dtype == torch.float32
+                and (x.dtype == torch.float32 or torch.is_autocast_enabled("cuda")))
 
     def message_and_aggregate(self, adj_t, x, quantized=None, randmat=None):
         return self.msg_and_aggr_func(adj_t, x[0], quantized=quantized, randmat=randmat)

@@ -86,7 +86,8 @@ class SparseStorage:
 
 
     def native_graph(self, reduce):
-        """The adjacency with its transpose and row plans for the layers' C++ nodes (_lib.native()), cached."""
+        """The adjacency with its transpose and row plans for the layers' C++ nodes (_lib.native()), cached.
+        reduce = None: without the transpose (evaluation)."""
         from . import _lib
         from .conf import config
         from .cpp_extension.spmm import native_plan
@@ -95,12 +96,14 @@ class SparseStorage:
         hit = self._t_cache.get(key)
         if hit is not None and hit[0] == version:
             return hit[1]
-        t_ptr, t_row, t_w = self.transposed("sum" if self._value is None else reduce)
-        inv = self.inverse_rowcount() if reduce == "mean" and self._value is None else None
         value = None if self._value is None else self._value.detach()
-        t_plan = native_plan(t_ptr)
-        graph = _lib.native().make_graph(self._rowptr, self._col, value, native_plan(self._rowptr), t_ptr, t_row, t_w,
-                                         t_plan, inv)
+        plan, transpose, inv = native_plan(self._rowptr), (None, None, None), None
+        t_plan = plan
+        if reduce is not None:
+            transpose = self.transposed("sum" if value is None else reduce)
+            t_plan = native_plan(transpose[0])
+            inv = self.inverse_rowcount() if reduce == "mean" and value is None else None
+        graph = _lib.native().make_graph(self._rowptr, self._col, value, plan, *transpose, t_plan, inv)
         self._t_cache[key] = (version, graph)
         return graph
 
