@@ -30,6 +30,7 @@ SIGNATURES = {
     "exact_version": (c_int, []),
     "exact_last_error": (ctypes.c_char_p, []),
     "exact_status": (c_int, [ctypes.POINTER(c_int), c_ptr]),
+    "exact_status_peek": (c_int, [ctypes.POINTER(c_int)]),
     "exact_status_async": (c_int, [c_ptr, c_ptr]),
     "exact_clear_status": (c_int, [c_ptr]),
     "exact_set_status": (c_int, [c_int, c_ptr]),
@@ -65,7 +66,9 @@ SIGNATURES = {
     "exact_act_quantized_backward_f16": (c_int, [c_int, c_ptr, c_ptr, c_i64, c_f32, c_ptr, c_ptr]),
     "exact_spmm_f16": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_int, c_ptr, c_ptr]),
     "exact_spmm_f16_planned": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_i64, c_int, c_ptr, c_i64, c_ptr,
-                                       c_i64, c_ptr, c_ptr]),
+                                       c_i64, c_ptr, c_ptr, c_ptr]),
+    "exact_spmm_planned": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_int, c_i64, c_ptr, c_ptr, c_ptr, c_ptr,
+                                   c_i64, c_ptr, c_ptr, c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr]),
     "exact_rows_scale_colsum_workspace_bytes": (c_i64, [c_i64]),
     "exact_rows_scale_colsum": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_ptr, c_i64, c_i64, c_ptr, c_ptr, c_i64, c_ptr]),
     "exact_bn_backward_workspace_bytes": (c_i64, [c_i64]),
@@ -96,6 +99,9 @@ SIGNATURES = {
     "exact_linear_workspace_bytes": (c_i64, [c_i64, c_i64, c_i64]),
     "exact_linear_forward": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_i64, c_ptr, c_i64, c_i64, c_ptr, c_i64,
                                      c_i64, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_ptr]),
+    "exact_linear_partial_bytes": (c_i64, [c_i64]),
+    "exact_linear_forward_strided": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_i64, c_i64, c_ptr, c_i64, c_i64, c_ptr,
+                                             c_i64, c_i64, c_i64, c_ptr, c_int, c_i64, c_ptr, c_ptr, c_ptr, c_i64, c_ptr]),
     "exact_spmm_minmax": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_i64, c_int, c_ptr, c_ptr, c_ptr]),
     "exact_spmm_value_bw": (c_int, [c_ptr, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_int, c_ptr, c_ptr]),
     "exact_spmm": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_int, c_ptr, c_ptr]),
@@ -230,15 +236,15 @@ def check_status(device=None, force=False):
 
 
 def poll_status(device=None):
-    """check_status without a synchronisation: looks at the copy of the status word enqueued by the previous
-    poll (if it has arrived) and enqueues the next one behind the work launched so far.  A training loop that
-    polls once per step learns of an abandoned kernel one step late and never waits for the GPU."""
+    """check_status without a synchronisation: looks at the status word as it is, so a training loop that polls once per
+    step learns of an abandoned kernel in the step after it (or while it still runs) and never waits for the GPU."""
     import torch
     dev = torch.cuda.current_device() if device is None else torch.device(device).index
-    word = native().poll_status(dev, bool(STATUS_PENDING.get(dev)))
-    if word >= 0:
-        STATUS_PENDING[dev] = False
-        raise_for_status(word)
+    word = native().peek_status(dev)
+    if word:
+        with torch.cuda.device(dev):
+            check(load().exact_clear_status(torch.cuda.current_stream(dev).cuda_stream), "exact_clear_status")
+    raise_for_status(word)
 
 
 # ---- launch accounting and optional per-kernel CUDA-event timing ----------------------------------

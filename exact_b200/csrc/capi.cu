@@ -25,9 +25,7 @@ int sm_count() {
   return cached;
 }
 
-// Library-wide status word: kernels with bounded on-chip waits OR a code into it when a wait expires.
-static __device__ int g_status_word;
-
+// Library-wide status words, one per device, in page-locked host memory that the devices see under the same address.
 int* status_word_ptr() {
   static std::mutex mu;
   static int* addr[64] = {nullptr};
@@ -36,7 +34,8 @@ int* status_word_ptr() {
   std::lock_guard<std::mutex> lock(mu);
   if (addr[dev] == nullptr) {
     void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess) return nullptr;
+    if (cudaHostAlloc(&p, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    *static_cast<volatile int*>(p) = 0;
     addr[dev] = static_cast<int*>(p);
   }
   return addr[dev];
@@ -52,8 +51,16 @@ int exact_status(int* status, void* stream) {
   EXB_REQUIRE(status != nullptr, "exact_status: null output");
   int* w = exb::status_word_ptr();
   EXB_REQUIRE(w != nullptr, "exact_status: no CUDA device");
-  EXB_CUDA_OK(cudaMemcpyAsync(status, w, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
   EXB_CUDA_OK(cudaStreamSynchronize((cudaStream_t)stream));
+  *status = *static_cast<volatile int*>(w);
+  return exb::EXB_OK;
+}
+
+int exact_status_peek(int* status) {
+  EXB_REQUIRE(status != nullptr, "exact_status_peek: null output");
+  int* w = exb::status_word_ptr();
+  EXB_REQUIRE(w != nullptr, "exact_status_peek: no CUDA device");
+  *status = *static_cast<volatile int*>(w);
   return exb::EXB_OK;
 }
 
@@ -61,22 +68,23 @@ int exact_status_async(int* pinned_host_status, void* stream) {
   EXB_REQUIRE(pinned_host_status != nullptr, "exact_status_async: null output");
   int* w = exb::status_word_ptr();
   EXB_REQUIRE(w != nullptr, "exact_status_async: no CUDA device");
-  EXB_CUDA_OK(cudaMemcpyAsync(pinned_host_status, w, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  EXB_CUDA_OK(cudaMemcpyAsync(pinned_host_status, w, sizeof(int), cudaMemcpyDefault, (cudaStream_t)stream));
   return exb::EXB_OK;
 }
 
 int exact_clear_status(void* stream) {
   int* w = exb::status_word_ptr();
   EXB_REQUIRE(w != nullptr, "exact_clear_status: no CUDA device");
-  EXB_CUDA_OK(cudaMemsetAsync(w, 0, sizeof(int), (cudaStream_t)stream));
+  EXB_CUDA_OK(cudaStreamSynchronize((cudaStream_t)stream));
+  *static_cast<volatile int*>(w) = 0;
   return exb::EXB_OK;
 }
 
 int exact_set_status(int code, void* stream) {
   int* w = exb::status_word_ptr();
   EXB_REQUIRE(w != nullptr, "exact_set_status: no CUDA device");
-  EXB_CUDA_OK(cudaMemcpyAsync(w, &code, sizeof(int), cudaMemcpyHostToDevice, (cudaStream_t)stream));
   EXB_CUDA_OK(cudaStreamSynchronize((cudaStream_t)stream));
+  *static_cast<volatile int*>(w) = code;
   return exb::EXB_OK;
 }
 

@@ -46,8 +46,9 @@ inline int fail(int code, const char* fmt, ...) {
 
 int sm_count();  // cached multiProcessorCount of the current device (capi.cu)
 
-// Device address of the library-wide status word on the current device (capi.cu), or null without a device.
+// Device address of the library-wide status word of the current device (capi.cu), or null without a device.
 // Kernels with bounded on-chip waits OR one of these codes into it when a wait expires; exact_status() reads it.
+// The word lives in page-locked host memory: the host looks at it without a copy or an event behind the launches.
 int* status_word_ptr();
 enum DeviceStatusBits : int { EXB_STATUS_RP_PACK = 1, EXB_STATUS_UNPACK_RP = 2, EXB_STATUS_LINEAR = 4, EXB_STATUS_GRAD_WEIGHT = 8 };
 
@@ -69,6 +70,14 @@ inline PhiloxKey make_philox_key(uint64_t seed) {
 }
 
 #ifdef __CUDACC__
+// Plain stores: the word is not in device memory.  Two kernels that give up at the same moment may leave one bit only.
+__device__ __forceinline__ void raise_status(int* word, int bit) {
+  if (word == nullptr) return;
+  volatile int* w = word;
+  *w = *w | bit;
+  __threadfence_system();
+}
+
 // ---- device helpers -----------------------------------------------------------------------------
 
 // Philox4x32-10 (Salmon et al., SC'11).  Counter (c0..c3), round keys from the constant bank.

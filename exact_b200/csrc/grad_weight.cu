@@ -66,7 +66,6 @@ struct GwParams {
   GwSegment seg[kGwMaxSeg];
   int nseg;
   float* partial;     // [grid, Opad, kpad]
-  int* status;
   int* lib_status;
   long long N;
   int O, Opad, kpad, bits;
@@ -402,10 +401,7 @@ grad_weight_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_consta
     tc_fence_after();
     tmem_dealloc(tmem_base, p.tmem_cols);
   }
-  if (threadIdx.x == 0 && s_abort) {
-    atomicExch(p.status, 1);
-    if (p.lib_status) atomicOr(p.lib_status, EXB_STATUS_GRAD_WEIGHT);
-  }
+  if (threadIdx.x == 0 && s_abort) raise_status(p.lib_status, EXB_STATUS_GRAD_WEIGHT);
 }
 
 // out[o, j] = sum over CTAs, in a fixed order, of partial[cta, o, j].
@@ -433,7 +429,7 @@ static int gw_pass(const float* g, int64_t N, int O, GwSegment a, const GwSegmen
     kpad += (b->k + 15) / 16 * 16;
     p.nseg = 2;
   }
-  p.partial = partial; p.status = reinterpret_cast<int*>(workspace); p.lib_status = status_word_ptr();
+  p.partial = partial; p.lib_status = status_word_ptr();
   p.N = N; p.O = O; p.Opad = (O + 127) / 128 * 128; p.kpad = kpad; p.bits = bits;
   p.mtiles = p.Opad / 128;
   p.kblocks = (N + kGwRows - 1) / kGwRows;
@@ -533,7 +529,6 @@ int exact_grad_weight_from_packed(const float* g, int64_t N, int64_t O, const ui
   EXB_REQUIRE(workspace_bytes >= 256 + grid * (int64_t)Opad * kpass * 4,
               "grad_weight_from_packed: workspace of %lld bytes is too small (%lld needed)", (long long)workspace_bytes,
               (long long)(256 + grid * (int64_t)Opad * kpass * 4));
-  EXB_CUDA_OK(cudaMemsetAsync(workspace, 0, 4, st));   // the call's status word
   const GwSegment s0{packed0, scale0, min0, (int)k0, (int)k0, 0, 0, 0}, s1{packed1, scale1, min1, (int)k1, (int)k1, 0, 0, 0};
   if (kpad <= 256) return gw_pass(g, N, (int)O, s0, k1 > 0 ? &s1 : nullptr, bits, (int)grid, workspace, out, ldo, st);
   // both activations do not fit one accumulator: each in passes of up to 256 of its columns

@@ -63,6 +63,8 @@ struct LinParams {
   int kblocks1, kblocks;   // K tiles of the first operand pair, and of both pairs together
   int num_tiles;
   int accumulate;          // C += ... instead of C = ...
+  int chunk;               // K tiles that are accumulated in TMEM before their sum is taken over in fp32
+  float* partial;          // [grid, Npad / 4, 128, 4]: running sums of the chunks before the last, per CTA
   int stages;              // K tiles the ring holds (2 at Npad = 256, up to 4 for narrow outputs)
   unsigned b_slot;         // bytes of a B_hi / B_lo slot = Npad * 128
   unsigned stage_bytes;    // A slot (32 KB) + two B slots
@@ -96,6 +98,9 @@ __device__ __forceinline__ LinPart lin_part(int it, const LinParams& p, uint32_t
   return r;
 }
 
+// CHUNKED: the contraction is drained from TMEM every p.chunk K tiles (a kernel of its own: its epilogue's registers and
+// code cost the unchunked product 5 %).
+template <bool CHUNKED>
 __global__ void __launch_bounds__(kLinThreads, 1)
 linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_a2,
                      const __grid_constant__ CUtensorMap tm_bh, const __grid_constant__ CUtensorMap tm_bl,
@@ -184,13 +189,19 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       const uint32_t idesc = umma_idesc_tf32(kLinTileM, p.Npad);
       int it = 0, t = 0;
       bool ok = true;
-      for (int tile = first; tile < p.num_tiles && ok; tile += step, t++) {
-        const int buf = t & 1;
-        const uint32_t tph = (uint32_t)(t >> 1) & 1u;
-        if (!mbar_wait(smem_u32(&s_tempty[buf]), tph ^ 1u, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * p.Npad);
+      for (int tile = first; tile < p.num_tiles && ok; tile += step) {
+        int buf = 0;
+        uint32_t d_tmem = 0;
         for (int kb = 0; kb < p.kblocks; kb++, it += 3) {
+          const bool opens = CHUNKED ? kb % p.chunk == 0 : kb == 0;
+          if (opens) {
+            buf = t & 1;
+            const uint32_t tph = (uint32_t)(t >> 1) & 1u;
+            if (!mbar_wait(smem_u32(&s_tempty[buf]), tph ^ 1u, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            d_tmem = tmem_base + (uint32_t)(buf * p.Npad);
+            t++;
+          }
           const LinPart qa = lin_part(it, p, ring), qh = lin_part(it + 1, p, ring), ql = lin_part(it + 2, p, ring);
           const int sa = qa.b, sh = qh.b, sl = ql.b;
           const uint32_t pl = ql.ph;
@@ -204,7 +215,7 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 #pragma unroll
           for (int k4 = 0; k4 < kLinTileK / 8; k4++) {
             const uint64_t o = (uint64_t)(k4 * 2);   // 8 tf32 = 32 bytes along K inside the swizzle atom
-            umma_tf32(d_tmem, alo + o, bhi + o, idesc, (kb | k4) != 0);
+            umma_tf32(d_tmem, alo + o, bhi + o, idesc, !opens || k4 != 0);
             umma_tf32(d_tmem, ahi + o, bhi + o, idesc, 1);
           }
           umma_commit(smem_u32(&s_empty[sh]));
@@ -217,8 +228,8 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
           }
           umma_commit(smem_u32(&s_empty[sa]));
           umma_commit(smem_u32(&s_empty[sl]));
+          if ((CHUNKED && (kb + 1) % p.chunk == 0) || kb + 1 == p.kblocks) umma_commit(smem_u32(&s_tfull[buf]));
         }
-        if (ok) umma_commit(smem_u32(&s_tfull[buf]));
       }
     }
   } else if (warp < 2 + kLinConvWarps) {
@@ -262,9 +273,55 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     const uint32_t stage_addr = stage_base + (uint32_t)quad * 4096u;
     int t = 0;
     bool ok = true;
-    for (int tile = first; tile < p.num_tiles && ok; tile += step, t++) {
+    const int chunks = CHUNKED ? (p.kblocks + p.chunk - 1) / p.chunk : 1;
+    // this thread's row of the running sums: 16 bytes per four columns, adjacent lanes adjacent
+    float4* __restrict__ part = !CHUNKED ? nullptr : reinterpret_cast<float4*>(p.partial) + (size_t)blockIdx.x * (p.Npad / 4) * kLinTileM + quad * 32 + lane;
+    for (int tile = first; tile < p.num_tiles && ok; tile += step) {
+      for (int ch = 0; CHUNKED && ch + 1 < chunks && ok; ch++, t++) {
+        const int buf = t & 1;
+        if (!mbar_wait<kLinSleepNs>(smem_u32(&s_tfull[buf]), (uint32_t)(t >> 1) & 1u, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.Npad);
+        for (int c0 = 0; c0 < p.Npad; c0 += 64) {
+          const int cols = p.Npad - c0 < 64 ? p.Npad - c0 : 64;
+          float4 old[16];
+          if (ch > 0) {
+#pragma unroll
+            for (int j = 0; j < 16; j++)
+              if (j * 4 < cols) old[j] = __ldcg(part + (size_t)(c0 / 4 + j) * kLinTileM);
+          }
+#pragma unroll
+          for (int h = 0; h < 4; h++) {
+            if (h * 16 < cols) {
+              float v[16];
+              tmem_ld16(taddr + (uint32_t)(c0 + h * 16), v);
+#pragma unroll
+              for (int j = 0; j < 4; j++) {
+                float4 o = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                if (ch > 0) {
+                  const float4 q = old[h * 4 + j];
+                  o.x += q.x; o.y += q.y; o.z += q.z; o.w += q.w;
+                }
+                __stcg(part + (size_t)(c0 / 4 + h * 4 + j) * kLinTileM, o);
+              }
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&s_tempty[buf]));
+      }
+      if (!ok) break;
       const int buf = t & 1;
       const uint32_t ph = (uint32_t)(t >> 1) & 1u;
+      t++;
+      float4 sum[8];         // the running sums of the next 32 columns
+      auto fetch = [&](int c0) {
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+          if (c0 + j * 4 < p.Npad) sum[j] = __ldcg(part + (size_t)(c0 / 4 + j) * kLinTileM);
+      };
+      if (CHUNKED) fetch(0);
       if (!mbar_wait<kLinSleepNs>(smem_u32(&s_tfull[buf]), ph, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.Npad);
@@ -274,6 +331,13 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         for (int h = 0; h * 16 < cols; h++) {
           float v[16];
           tmem_ld16(taddr + (uint32_t)(c0 + h * 16), v);
+          if (CHUNKED) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              const float4 q = h ? sum[4 + j] : sum[j];
+              v[4 * j] += q.x; v[4 * j + 1] += q.y; v[4 * j + 2] += q.z; v[4 * j + 3] += q.w;
+            }
+          }
 #pragma unroll
           for (int j = 0; j < 4; j++) {
             const uint32_t ci = (uint32_t)(h * 4 + j);
@@ -283,6 +347,7 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                          : "memory");
           }
         }
+        if (CHUNKED && c0 + 32 < p.Npad) fetch(c0 + 32);
         __syncwarp();
         const uint32_t ci = (uint32_t)lane & 7u;
         const int c = c0 + (int)ci * 4;
@@ -333,14 +398,15 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   }
   if (threadIdx.x == 0 && s_abort) {
     atomicExch(p.status, 1);
-    if (p.lib_status) atomicOr(p.lib_status, EXB_STATUS_LINEAR);
+    raise_status(p.lib_status, EXB_STATUS_LINEAR);
   }
 }
 
 // Heads and tails of [B | B2] (rows = output features), zero padded to [Npad, Kpad1 + Kpad2]; also
 // clears the status word.
-__global__ void linear_prepare_kernel(const float* __restrict__ B, int K, long long ldb, const float* __restrict__ B2,
-                                      int K2, long long ldb2, int N, int Npad, int Kpad1, int Kpad,
+__global__ void linear_prepare_kernel(const float* __restrict__ B, int K, long long ldb, long long incb,
+                                      const float* __restrict__ B2, int K2, long long ldb2, long long incb2, int N, int Npad,
+                                      int Kpad1, int Kpad,
                                       float* __restrict__ bh, float* __restrict__ bl, int* status) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *status = 0;
@@ -349,9 +415,9 @@ __global__ void linear_prepare_kernel(const float* __restrict__ B, int K, long l
   float v = 0.f;
   if (n < N) {
     if (kk < Kpad1) {
-      if (kk < K) v = B[(long long)n * ldb + kk];
+      if (kk < K) v = B[(long long)n * ldb + kk * incb];
     } else if (kk - Kpad1 < K2) {
-      v = B2[(long long)n * ldb2 + (kk - Kpad1)];
+      v = B2[(long long)n * ldb2 + (kk - Kpad1) * incb2];
     }
   }
   float hi, lo;
@@ -374,14 +440,29 @@ int64_t exact_linear_workspace_bytes(int64_t N, int64_t K, int64_t K2) {
   return 256 + 2 * Npad * (int64_t)(lin_kpad(K) + lin_kpad(K2)) * 4;
 }
 
+int64_t exact_linear_partial_bytes(int64_t N) {
+  const int64_t Npad = (N + 15) / 16 * 16;
+  return N > 0 ? (int64_t)sm_count() * Npad * kLinTileM * 4 : 0;
+}
+
 int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb,
                          const float* A2, int64_t K2, int64_t lda2, const float* B2, int64_t ldb2, int64_t N,
                          const float* bias, int accumulate, void* workspace, float* C, int64_t ldc, void* stream) {
+  return exact_linear_forward_strided(A, M, K, lda, B, ldb, 1, A2, K2, lda2, B2, ldb2, 1, N, bias, accumulate, 0, nullptr, workspace,
+                                      C, ldc, stream);
+}
+
+int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb, int64_t incb,
+                         const float* A2, int64_t K2, int64_t lda2, const float* B2, int64_t ldb2, int64_t incb2, int64_t N,
+                         const float* bias, int accumulate, int64_t k_chunk, float* partial, void* workspace, float* C,
+                         int64_t ldc, void* stream) {
+  EXB_REQUIRE(k_chunk >= 0 && k_chunk % kLinTileK == 0 && (k_chunk == 0 || (partial && (reinterpret_cast<uintptr_t>(partial) & 15) == 0)),
+              "linear_forward: k_chunk must be a multiple of 32 and needs a 16-byte aligned buffer of partial sums");
   EXB_REQUIRE(M >= 0 && K > 0 && N > 0 && K2 >= 0, "linear_forward: bad shape");
   if (M == 0) return EXB_OK;
   EXB_REQUIRE(A && B && C && workspace, "linear_forward: null pointer");
   EXB_REQUIRE((A2 != nullptr) == (K2 > 0) && (B2 != nullptr) == (K2 > 0), "linear_forward: the second operand pair needs A2, B2 and K2 > 0");
-  EXB_REQUIRE(lda >= K && ldb >= K && ldc >= N && (K2 == 0 || (lda2 >= K2 && ldb2 >= K2)), "linear_forward: leading dimension smaller than the row");
+  EXB_REQUIRE(lda >= K && (incb != 1 || ldb >= K) && ldc >= N && (K2 == 0 || (lda2 >= K2 && (incb2 != 1 || ldb2 >= K2))), "linear_forward: leading dimension smaller than the row");
   if (N > 256) return fail(EXB_ERR_UNSUPPORTED, "linear_forward: N = %lld exceeds one MMA tile (256); call per 256-column block", (long long)N);
   if (lda % 4 != 0 || (reinterpret_cast<uintptr_t>(A) & 15) != 0 ||
       (K2 > 0 && (lda2 % 4 != 0 || (reinterpret_cast<uintptr_t>(A2) & 15) != 0)))
@@ -395,7 +476,7 @@ int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t lda, cons
   float* bh = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + 256);
   float* bl = bh + (size_t)Npad * Kpad;
 
-  linear_prepare_kernel<<<(Npad * Kpad + 255) / 256, 256, 0, st>>>(B, (int)K, ldb, B2, (int)K2, ldb2, (int)N, Npad,
+  linear_prepare_kernel<<<(Npad * Kpad + 255) / 256, 256, 0, st>>>(B, (int)K, ldb, incb, B2, (int)K2, ldb2, incb2, (int)N, Npad,
                                                                    Kpad1, Kpad, bh, bl, status);
   EXB_CUDA_OK(cudaGetLastError());
 
@@ -418,6 +499,8 @@ int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t lda, cons
   p.kblocks1 = Kpad1 / kLinTileK; p.kblocks = Kpad / kLinTileK;
   p.num_tiles = (int)((M + kLinTileM - 1) / kLinTileM);
   p.accumulate = accumulate ? 1 : 0;
+  p.chunk = k_chunk > 0 ? (int)(k_chunk / kLinTileK) : p.kblocks;
+  p.partial = partial;
   p.b_slot = (unsigned)Npad * kLinTileK * 4;
   p.stage_bytes = kLinSlotBytes + 2 * p.b_slot;
   p.stages = (int)((kLinSlots * kLinSlotBytes) / p.stage_bytes);
@@ -428,8 +511,9 @@ int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t lda, cons
   const size_t dyn = (size_t)kLinSlots * kLinSlotBytes + 4 * 4096 + 1024;
   int grid = sm_count();
   if (grid > p.num_tiles) grid = p.num_tiles;
-  EXB_CUDA_OK(cudaFuncSetAttribute(linear_tf32x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-  linear_tf32x3_kernel<<<grid, kLinThreads, dyn, st>>>(tm_a, tm_a2, tm_bh, tm_bl, p);
+  auto* kern = p.chunk < p.kblocks ? linear_tf32x3_kernel<true> : linear_tf32x3_kernel<false>;
+  EXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+  kern<<<grid, kLinThreads, dyn, st>>>(tm_a, tm_a2, tm_bh, tm_bl, p);
   EXB_CUDA_OK(cudaGetLastError());
   return EXB_OK;
 }

@@ -37,12 +37,12 @@ struct LibraryError : std::runtime_error {   // becomes exact_b200.ExactB200Erro
   X(exact_act_quantized_relu_forward) X(exact_act_quantized_relu_backward) X(exact_act_quantized_leaky_relu_forward)  \
   X(exact_act_quantized_leaky_relu_backward) X(exact_act_quantized_dropout_forward)                                   \
   X(exact_act_quantized_dropout_backward) X(exact_act_quantized_relu_dropout_forward)                                 \
-  X(exact_act_quantized_forward_f16) X(exact_act_quantized_backward_f16) X(exact_spmm) X(exact_spmm_split)            \
-  X(exact_spmm_split_routed) X(exact_spmm_f16_planned) X(exact_rows_scale_colsum_workspace_bytes)                     \
+  X(exact_act_quantized_forward_f16) X(exact_act_quantized_backward_f16) X(exact_spmm_planned)                        \
+  X(exact_spmm_f16_planned) X(exact_rows_scale_colsum_workspace_bytes)                     \
   X(exact_rows_scale_colsum) X(exact_bn_backward_workspace_bytes) X(exact_bn_backward_from_packed)                    \
   X(exact_rp_workspace_bytes) X(exact_rp_quantize_pack) X(exact_rademacher) X(exact_grad_weight_workspace_bytes)      \
-  X(exact_grad_weight_from_packed) X(exact_linear_workspace_bytes) X(exact_linear_forward) X(exact_spmm_minmax)       \
-  X(exact_spmm_value_bw) X(exact_status_async) X(exact_clear_status)
+  X(exact_grad_weight_from_packed) X(exact_linear_workspace_bytes) X(exact_linear_partial_bytes) X(exact_linear_forward_strided) X(exact_spmm_minmax)       \
+  X(exact_spmm_value_bw) X(exact_status_peek)
 
 struct Library {
 #define EXB_POINTER(name) decltype(&::name) name = nullptr;
@@ -112,8 +112,9 @@ Packed rp_quantize_pack(const Tensor& x, const Tensor& R, int64_t bits, uint64_t
                         Tensor* projection = nullptr);
 bool linear_supported(const Tensor& a);
 Tensor rows16(const Tensor& a);
+// fp32 operands; w may be a transposed view (its rows are read through both strides)
 Tensor linear(const Tensor& a, const Tensor& w, const OptTensor& bias, const OptTensor& a2, const OptTensor& w2,
-              const OptTensor& out, bool accumulate);
+              const OptTensor& out, bool accumulate, int64_t k_chunk = 0);
 Tensor grad_weight(const Tensor& g, int64_t bits, const Packed& q0, int64_t k0, const Packed* q1, int64_t k1);
 std::tuple<Tensor, Tensor> rows_scale_colsum(const Tensor& g, const OptTensor& rowscale, bool want_scaled, bool want_colsum);
 std::tuple<Tensor, Tensor, Tensor> bn_backward(const Tensor& g, const Packed& q, int64_t bits, const OptTensor& weight,
@@ -147,15 +148,16 @@ struct RowPlan {
   mutable int64_t n_f16 = -1;
 };
 using PlanPtr = std::shared_ptr<const RowPlan>;
-Tensor spmm(const Tensor& rowptr, const Tensor& col, const RowPlan& plan, const OptTensor& value, const Tensor& mat, bool mean);
+Tensor spmm(const Tensor& rowptr, const Tensor& col, const RowPlan& plan, const OptTensor& value, const Tensor& mat, bool mean,
+            const OptTensor& bias = {});
 
 struct Csr {
   Tensor rowptr, col;
   OptTensor value;
   PlanPtr plan;
 };
-inline Tensor spmm(const Csr& a, const OptTensor& value, const Tensor& mat, bool mean) {
-  return spmm(a.rowptr, a.col, *a.plan, value, mat, mean);
+inline Tensor spmm(const Csr& a, const OptTensor& value, const Tensor& mat, bool mean, const OptTensor& bias = {}) {
+  return spmm(a.rowptr, a.col, *a.plan, value, mat, mean, bias);
 }
 
 }  // namespace exb

@@ -71,12 +71,10 @@ Tensor weight_grad(const Tensor& g, const Compressed& c, int64_t bits, int64_t N
 }
 
 // A (x W^T) + b
-Tensor gcn_product(const Graph& g, const Tensor& x, const Tensor& w, const OptTensor& b) {
+Tensor gcn_product(const Graph& g, const Tensor& x, const Tensor& w, const OptTensor& b, int64_t k_chunk = 0) {
   if (x.size(1) < w.size(0) && x.size(1) % 4 == 0)   // fewer columns in than out: (A x) W^T gathers the narrower operand
-    return linear(spmm(g.fw, g.fw.value, x, false), w, b, {}, {}, {}, false);
-  Tensor out = spmm(g.fw, g.fw.value, linear(x, w, {}, {}, {}, {}, false), false);
-  if (b) out.add_(*b);
-  return out;
+    return linear(spmm(g.fw, g.fw.value, x, false), w, b, {}, {}, {}, false, k_chunk);
+  return spmm(g.fw, g.fw.value, linear(x, w, {}, {}, {}, {}, false, k_chunk), false, b);
 }
 
 }  // namespace
@@ -125,8 +123,7 @@ struct GcnNode : Function<GcnNode> {
       x = x.to(at::kHalf);
       w = w.to(at::kHalf);
       s->x = compress(x, s->how, s->how.offset);
-      out = spmm(g.fw, g.fw.value, at::linear(x, w), false);
-      if (b) out = out + *b;                 // half + float: float, as the promotion of the reference's add gives
+      out = spmm(g.fw, g.fw.value, at::linear(x, w), false, b);   // with a bias: half + float is a float
     } else {
       s->x = compress(x, s->how, s->how.offset);
       out = gcn_product(g, x, w, b);
@@ -306,12 +303,15 @@ Tensor sage_node(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const
 }
 
 // ---- evaluation -----------------------------------------------------------------------------------------
+// Outputs that were products of the library's fp32 GEMM: contractions beyond 256 columns in chunks, so that the truncation
+// of the tensor core's accumulator stays below 2e-6 of a layer's output (4e-6 at 602 columns in one piece).
+constexpr int64_t kEvalChunk = 256;
+
 Tensor gcn_eval(const Tensor& x_, const Tensor& w, const OptTensor& b, const c10::intrusive_ptr<Graph>& graph, bool half) {
   Plain plain;
   const Graph& g = *graph;
-  if (!half) return gcn_product(g, x_.contiguous(), w, b);
-  const Tensor out = spmm(g.fw, g.fw.value, at::linear(x_.to(at::kHalf), w.to(at::kHalf)), false);
-  return b ? out + *b : out;
+  if (!half) return gcn_product(g, x_.contiguous(), w, b, kEvalChunk);
+  return spmm(g.fw, g.fw.value, at::linear(x_.to(at::kHalf), w.to(at::kHalf)), false, b);
 }
 
 Tensor sage_eval(const Tensor& x_, const Tensor& w_l, const OptTensor& b, const OptTensor& w_r,
@@ -331,13 +331,13 @@ Tensor sage_eval(const Tensor& x_, const Tensor& w_l, const OptTensor& b, const 
     const Tensor agg = spmm(g.fw, g.fw.value, x, mean);
     OptTensor a2;
     if (w_r) a2 = x;
-    return linear(agg, w_l, b, a2, w_r, {}, false);
+    return linear(agg, w_l, b, a2, w_r, {}, false, kEvalChunk);
   }
   // fewer outputs than inputs: reduce(A, x) W_l^T = reduce(A, x W_l^T) gathers the narrower operand
   const Tensor rows = rows16(x);
-  const Tensor t = spmm(g.fw, g.fw.value, linear(rows, pad ? at::constant_pad_nd(w_l, {0, 0, 0, pad}) : w_l, {}, {}, {}, {}, false), mean);
+  const Tensor t = spmm(g.fw, g.fw.value, linear(rows, pad ? at::constant_pad_nd(w_l, {0, 0, 0, pad}) : w_l, {}, {}, {}, {}, false, kEvalChunk), mean);
   Tensor out = pad ? t.narrow(1, 0, out_f) : t;
-  if (w_r) linear(rows, *w_r, b, {}, {}, out, true);
+  if (w_r) linear(rows, *w_r, b, {}, {}, out, true, kEvalChunk);
   else if (b) out.add_(*b);
   return out.contiguous();
 }

@@ -174,43 +174,11 @@ bool take_status_pending(int64_t device) {
   return (acct.status_pending.fetch_and(~bit) & bit) != 0;
 }
 
-// _lib.poll_status: a copy of the library's status word is enqueued behind the work launched so far, the next call looks at
-// it if it has arrived.  `also_pending`: launches outside this module are to be looked at.  Returns the word
-// (0: nothing to report, -1: the last copy is still in flight).
-int64_t poll_status(int64_t device, bool also_pending) {
-  struct Poll {
-    int* word = nullptr;      // pinned
-    cudaEvent_t event = nullptr;
-    bool in_flight = false;
-  };
-  static std::mutex mu;
-  static Poll polls[64];
-  if (device < 0 || device >= 64) throw std::runtime_error("poll_status: device out of range");
-  std::lock_guard<std::mutex> lock(mu);
-  Poll& p = polls[device];
-  int word = 0;
-  if (p.in_flight) {
-    if (cudaEventQuery(p.event) != cudaSuccess) {
-      cudaGetLastError();     // not ready: look again at the next poll
-      return -1;
-    }
-    word = *p.word;
-    p.in_flight = false;
-  }
-  const bool pending = take_status_pending(device) || also_pending;
-  if (word == 0 && !pending) return 0;
+int64_t peek_status(int64_t device) {
   c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
-  const cudaStream_t st = c10::cuda::getCurrentCUDAStream().stream();
-  if (p.word == nullptr) {
-    if (cudaHostAlloc(reinterpret_cast<void**>(&p.word), sizeof(int), cudaHostAllocPortable) != cudaSuccess ||
-        cudaEventCreateWithFlags(&p.event, cudaEventDisableTiming) != cudaSuccess)
-      throw LibraryError("poll_status: no pinned memory or event");
-  }
-  int rc = word != 0 ? lib.exact_clear_status(st) : 0;
-  if (rc == 0) rc = lib.exact_status_async(p.word, st);
-  if (rc != 0) library_failure("poll_status", rc);
-  cudaEventRecord(p.event, st);
-  p.in_flight = true;
+  int word = 0;
+  const int rc = lib.exact_status_peek(&word);
+  if (rc != 0) library_failure("exact_status_peek", rc);
   return word;
 }
 
@@ -228,6 +196,10 @@ PyObject* make_graph(const Tensor& rowptr, const Tensor& col, const OptTensor& v
   if (t_rowptr) g->bw = Csr{*t_rowptr, *t_col, t_value, t_plan};
   g->inv_degree = inv_degree;
   return make_capsule(std::move(g));
+}
+Tensor linear_op(const Tensor& a, const Tensor& w, const OptTensor& bias, const OptTensor& a2, const OptTensor& w2,
+                 const OptTensor& out, bool accumulate) {
+  return linear(a, w, bias, a2, w2, out, accumulate);
 }
 Tensor spmm_op(const Tensor& rowptr, const Tensor& col, const PlanPtr& plan, const OptTensor& value, const Tensor& mat, bool mean) {
   return spmm(rowptr, col, *plan, value, mat, mean);
@@ -292,9 +264,9 @@ PyMethodDef methods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&bind)), METH_FASTCALL, nullptr},
     EXB_METHOD("launches", launches), EXB_METHOD("set_timing", set_timing), EXB_METHOD("take_calls", take_calls),
     EXB_METHOD("set_clock", set_clock), EXB_METHOD("host_ns", host_ns), EXB_METHOD("host_calls", host_calls),
-    EXB_METHOD("take_status_pending", take_status_pending), EXB_METHOD("poll_status", poll_status), EXB_METHOD("make_plan", make_plan), EXB_METHOD("make_graph", make_graph),
+    EXB_METHOD("take_status_pending", take_status_pending), EXB_METHOD("peek_status", peek_status), EXB_METHOD("make_plan", make_plan), EXB_METHOD("make_graph", make_graph),
     EXB_METHOD("quantize_pack", quantize_pack), EXB_METHOD("unpack", unpack), EXB_METHOD("rademacher", rademacher),
-    EXB_METHOD("rp_quantize_pack", rp_quantize_pack_op), EXB_METHOD("bn_backward", bn_backward_op), EXB_METHOD("linear", linear), EXB_METHOD("grad_weight", grad_weight_op),
+    EXB_METHOD("rp_quantize_pack", rp_quantize_pack_op), EXB_METHOD("bn_backward", bn_backward_op), EXB_METHOD("linear", linear_op), EXB_METHOD("grad_weight", grad_weight_op),
     EXB_METHOD("rows_scale_colsum", rows_scale_colsum), EXB_METHOD("spmm", spmm_op), EXB_METHOD("act", act_node),
     EXB_METHOD("gcn", gcn_op), EXB_METHOD("sage", sage_op), EXB_METHOD("gcn_eval", gcn_eval), EXB_METHOD("sage_eval", sage_eval), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

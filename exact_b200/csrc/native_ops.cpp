@@ -184,21 +184,23 @@ Tensor rows16(const Tensor& a) {
 }
 
 Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const OptTensor& a2_, const OptTensor& w2_,
-              const OptTensor& out_, bool accumulate) {
+              const OptTensor& out_, bool accumulate, int64_t k_chunk) {
   c10::cuda::CUDAGuard guard(a_.device());
   const int64_t M = a_.size(0), K = a_.size(1), N = w_.size(0);
-  const Tensor a = rows16(a_), w = w_.stride(1) == 1 ? w_ : w_.contiguous();
+  const Tensor a = rows16(a_), w = w_;
   Tensor a2, w2, bias;
   int64_t K2 = 0;
   if (a2_) {
     K2 = a2_->size(1);
     a2 = rows16(*a2_);
-    w2 = w2_->stride(1) == 1 ? *w2_ : w2_->contiguous();
+    w2 = *w2_;
   }
   if (bias_) bias = bias_->contiguous();
   Tensor out = out_ ? *out_ : empty({M, N}, at::kFloat, a);
   if (!out_) accumulate = false;
   if (out.size(0) != M || out.size(1) != N || out.stride(1) != 1) throw std::runtime_error("linear: out does not fit");
+  Tensor partial;      // of a contraction in chunks (exact_linear_forward_chunked)
+  if (k_chunk > 0 && K + K2 > k_chunk) partial = empty({lib.exact_linear_partial_bytes(std::min<int64_t>(N, 256))}, at::kByte, a);
   for (int64_t n0 = 0; n0 < N; n0 += 256) {
     const int64_t n = std::min<int64_t>(N - n0, 256);
     Tensor ws = empty({lib.exact_linear_workspace_bytes(n, K, K2)}, at::kByte, a);
@@ -209,10 +211,11 @@ Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const 
     info.bytes = 4 * (M * (K + K2) + n * (K + K2) + M * n * (accumulate ? 2 : 1));
     info.flops = 6.0 * (double)M * (double)(K + K2) * (double)n;
     invoke("exact_linear_forward", info, [&](void* st) {
-      return lib.exact_linear_forward(ptr<float>(a), M, K, a.stride(0), wb, w.stride(0), K2 ? ptr<float>(a2) : nullptr, K2,
-                                      K2 ? a2.stride(0) : 0, w2b, K2 ? w2.stride(0) : 0, n,
-                                      bias.defined() ? ptr<float>(bias) + n0 : nullptr, accumulate ? 1 : 0, ptr(ws), cb,
-                                      out.stride(0), st);
+      return lib.exact_linear_forward_strided(ptr<float>(a), M, K, a.stride(0), wb, w.stride(0), w.stride(1), K2 ? ptr<float>(a2) : nullptr, K2,
+                                      K2 ? a2.stride(0) : 0, w2b, K2 ? w2.stride(0) : 0, K2 ? w2.stride(1) : 1, n,
+                                      bias.defined() ? ptr<float>(bias) + n0 : nullptr, accumulate ? 1 : 0,
+                                              partial.defined() ? k_chunk : 0, partial.defined() ? ptr<float>(partial) : nullptr, ptr(ws),
+                                              cb, out.stride(0), st);
     });
   }
   mark_status(a);
@@ -405,7 +408,8 @@ int64_t RowPlan::n_long_f16(const Tensor& rowptr) const {
   return n_f16;
 }
 
-Tensor spmm(const Tensor& rowptr, const Tensor& colt, const RowPlan& a, const OptTensor& value_, const Tensor& mat_, bool mean) {
+Tensor spmm(const Tensor& rowptr, const Tensor& colt, const RowPlan& a, const OptTensor& value_, const Tensor& mat_, bool mean,
+            const OptTensor& bias_) {
   const Tensor mat = mat_.contiguous();
   same_device(rowptr, mat);
   same_device(colt, mat);
@@ -414,11 +418,13 @@ Tensor spmm(const Tensor& rowptr, const Tensor& colt, const RowPlan& a, const Op
   const int ib = colt.scalar_type() == at::kInt ? 4 : 8;
   const int red = mean ? EXACT_REDUCE_MEAN : EXACT_REDUCE_SUM;
   const void *rp = ptr(rowptr), *col = ptr(colt);
+  OptTensor bias;
+  if (bias_) bias = bias_->detach().to(at::kFloat).contiguous();
   if (mat.scalar_type() == at::kHalf) {
     // the reference's half instantiation (spmm_cuda.cu:142): every step rounded to half, rows in CSR order
     OptTensor value;
     if (value_) value = value_->detach().to(at::kHalf).contiguous();
-    Tensor out = empty({M, K}, at::kHalf, mat), src = mat;
+    Tensor out = empty({M, K}, bias ? at::kFloat : at::kHalf, mat), src = mat;
     const int64_t ldm = (K + 7) / 8 * 8;
     if (ldm != K) {   // rows in whole 16-byte pieces: the copy is read and written once, the gathers nnz / N times
       src = empty({mat.size(0), ldm}, at::kHalf, mat);
@@ -428,7 +434,7 @@ Tensor spmm(const Tensor& rowptr, const Tensor& colt, const RowPlan& a, const Op
     const int64_t n_long = a.n_long_f16(rowptr);
     invoke("exact_spmm_f16", {nnz * (2 * K + ib) + 2 * M * K}, [&](void* st) {
       return lib.exact_spmm_f16_planned(rp, col, ib, ptr(value), ptr(src), ldm, M, K, red, order, a.threshold_f16,
-                                        n_long ? order : nullptr, n_long, ptr(out), st);
+                                        n_long ? order : nullptr, n_long, ptr<float>(bias), ptr(out), st);
     });
     return out;
   }
@@ -450,23 +456,12 @@ Tensor spmm(const Tensor& rowptr, const Tensor& colt, const RowPlan& a, const Op
     prow = ptr<int32_t>(pc.row); pslot = ptr<int32_t>(pc.slot); lrow = ptr<int32_t>(pc.long_row); lptr = ptr<int32_t>(pc.long_ptr);
     pb = ptr<int64_t>(pc.begin); pe = ptr<int64_t>(pc.end);
   }
-  if (K <= 64 && K % 4 == 0 && M > 0) {   // the kernel for narrow operands takes its rows in order of length
-    void* dst[1] = {ptr(out)};
-    const int32_t* order = ptr<int32_t>(a.row_order(rowptr));
-    invoke("exact_spmm_split_routed", info, [&](void* st) {
-      return lib.exact_spmm_split_routed(rp, col, ib, ptr<float>(value), ptr<float>(mat), M, K, red, pc.n ? a.threshold : 0, prow, pb,
-                                         pe, pslot, pc.n, lrow, lptr, pc.n_long, sc, order, M, 0, K, dst, 1, st);
-    });
-  } else if (pc.n == 0) {
-    invoke("exact_spmm", info, [&](void* st) {
-      return lib.exact_spmm(rp, col, ib, ptr<float>(value), ptr<float>(mat), M, K, red, ptr<float>(out), st);
-    });
-  } else {
-    invoke("exact_spmm_split", info, [&](void* st) {
-      return lib.exact_spmm_split(rp, col, ib, ptr<float>(value), ptr<float>(mat), M, K, red, a.threshold, prow, pb, pe, pslot, pc.n,
-                                  lrow, lptr, pc.n_long, sc, ptr<float>(out), st);
-    });
-  }
+  const bool narrow = K <= 64 && K % 4 == 0 && M > 0;   // the kernel for narrow operands takes its rows in order of length
+  const int32_t* order = narrow ? ptr<int32_t>(a.row_order(rowptr)) : nullptr;
+  invoke(narrow ? "exact_spmm_split_routed" : pc.n ? "exact_spmm_split" : "exact_spmm", info, [&](void* st) {
+    return lib.exact_spmm_planned(rp, col, ib, ptr<float>(value), ptr<float>(mat), M, K, red, pc.n ? a.threshold : 0, prow, pb, pe,
+                                  pslot, pc.n, lrow, lptr, pc.n_long, sc, order, ptr<float>(bias), ptr<float>(out), st);
+  });
   return out;
 }
 

@@ -260,7 +260,7 @@ rp_unpack_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
   }
   if (threadIdx.x == 0 && s_abort) {
     atomicExch(p.status, 1);
-    if (p.lib_status) atomicOr(p.lib_status, EXB_STATUS_UNPACK_RP);
+    raise_status(p.lib_status, EXB_STATUS_UNPACK_RP);
   }
 }
 
@@ -549,7 +549,7 @@ rp_unpack_stream_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_c
   }
   if (threadIdx.x == 0 && s_abort) {
     atomicExch(p.status, 1);
-    if (p.lib_status) atomicOr(p.lib_status, EXB_STATUS_UNPACK_RP);
+    raise_status(p.lib_status, EXB_STATUS_UNPACK_RP);
   }
 }
 

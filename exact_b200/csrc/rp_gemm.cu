@@ -382,7 +382,7 @@ rp_pack_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   }
   if (threadIdx.x == 0 && s_abort) {
     atomicExch(p.status, 1);
-    if (p.lib_status) atomicOr(p.lib_status, EXB_STATUS_RP_PACK);
+    raise_status(p.lib_status, EXB_STATUS_RP_PACK);
   }
 }
 

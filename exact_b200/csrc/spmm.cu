@@ -30,6 +30,7 @@ struct SpmmParams {
   const float* val;
   const float* mat;
   float* out;
+  const float* bias;   // [K] added to every row of the result, or null
   long long M, K;
   int mean;
   int regroup;   // the caller accepts a regrouped per-row sum (EXACT_SPMM_REGROUP)
@@ -214,6 +215,12 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_kernel(const __grid_
 #pragma unroll
       for (int x = 0; x < VEC; x++) acc[j][x] = __fdiv_rn(acc[j][x], dv);
   }
+  if (MODE == MODE_ROWS && p.bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < KVT; j++)
+#pragma unroll
+      for (int x = 0; x < VEC; x++) acc[j][x] = __fadd_rn(acc[j][x], __ldg(p.bias + cload[j] + x));
+  }
 #pragma unroll
   for (int j = 0; j < KVT; j++)
     if (FULL || cvalid[j]) st_vec<VEC>(dst + coff[j], acc[j]);
@@ -233,7 +240,8 @@ __global__ void __launch_bounds__(128) spmm_long_reduce_kernel(const __grid_cons
   for (long long c = threadIdx.x; c < p.K; c += blockDim.x) {
     float a = 0.f;
     for (int s = s0; s < s1; s++) a = __fadd_rn(a, p.scratch[(long long)s * p.K + c]);
-    dst[c] = p.mean ? __fdiv_rn(a, dv) : a;
+    if (p.mean) a = __fdiv_rn(a, dv);
+    dst[c] = p.bias != nullptr ? __fadd_rn(a, __ldg(p.bias + c)) : a;
   }
 }
 
@@ -343,6 +351,10 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_multi_kernel(const _
     const float dv = (float)(count > 0 ? count : 1);  // reducer.cuh:75-76
 #pragma unroll
     for (int x = 0; x < 4; x++) acc[x] = __fdiv_rn(acc[x], dv);
+  }
+  if (MODE == MODE_ROWS && p.bias != nullptr && cvalid) {
+#pragma unroll
+    for (int x = 0; x < 4; x++) acc[x] = __fadd_rn(acc[x], __ldg(p.bias + coff + x));
   }
   if (live && cvalid) *reinterpret_cast<float4*>(dst + coff) = make_float4(acc[0], acc[1], acc[2], acc[3]);
 }
@@ -581,6 +593,26 @@ int exact_spmm_split(const void* rowptr, const void* col, int idx_bytes, const f
   p.item_row = item_row; p.item_begin = reinterpret_cast<const long long*>(item_begin);
   p.item_end = reinterpret_cast<const long long*>(item_end); p.item_slot = item_slot; p.n_items = n_items;
   p.long_row = long_row; p.long_item_ptr = long_item_ptr; p.n_long = n_long; p.scratch = scratch;
+  return spmm_common(p, idx_bytes, reduce, (cudaStream_t)stream);
+}
+
+int exact_spmm_planned(const void* rowptr, const void* col, int idx_bytes, const float* value, const float* mat, int64_t M,
+                       int64_t K, int reduce, int64_t long_threshold, const int32_t* item_row, const int64_t* item_begin,
+                       const int64_t* item_end, const int32_t* item_slot, int64_t n_items, const int32_t* long_row,
+                       const int32_t* long_item_ptr, int64_t n_long, float* scratch, const int32_t* row_order,
+                       const float* bias, float* out, void* stream) {
+  EXB_REQUIRE(long_threshold >= 0 && n_items >= 0 && n_long >= 0, "spmm_planned: negative plan size");
+  EXB_REQUIRE(n_items <= 2147483647LL && n_long <= 2147483647LL, "spmm_planned: plan too large");
+  if (n_items > 0)
+    EXB_REQUIRE(long_threshold > 0 && item_row && item_begin && item_end && long_row && long_item_ptr && scratch && n_long > 0,
+                "spmm_planned: null plan array or scratch");
+  SpmmParams p{};
+  p.rowptr = rowptr; p.col = col; p.val = value; p.mat = mat; p.out = out; p.bias = bias; p.M = M; p.K = K;
+  p.long_threshold = n_items > 0 ? long_threshold : 0;
+  p.item_row = item_row; p.item_begin = reinterpret_cast<const long long*>(item_begin);
+  p.item_end = reinterpret_cast<const long long*>(item_end); p.item_slot = item_slot; p.n_items = n_items;
+  p.long_row = long_row; p.long_item_ptr = long_item_ptr; p.n_long = n_long; p.scratch = scratch;
+  p.row_order = row_order;
   return spmm_common(p, idx_bytes, reduce, (cudaStream_t)stream);
 }
 

@@ -33,7 +33,8 @@ struct SpmmF16Params {
   const void* col;
   const __half* val;
   const __half* mat;
-  __half* out;
+  void* out;                  // halves, or fp32 with a bias
+  const float* bias;          // [K] added to every row in fp32, or null
   long long M, K, ldm;
   int mean;
   long long long_threshold;   // rows with more edges are left to the hub warps (0: none)
@@ -164,8 +165,24 @@ __global__ void __launch_bounds__(kF16Warps * 32, 4) spmm_f16_rows_kernel(const 
 #pragma unroll
       for (int x = 0; x < NH; x++) acc[x] = h2_mean(acc[x], dv);
     }
-    __half* dst = p.out + row * p.K + c;
-    if (VEC == 8) {
+    if (p.bias != nullptr) {
+      float* dst = static_cast<float*>(p.out) + row * p.K + c;
+      float v[2 * NH];
+#pragma unroll
+      for (int x = 0; x < 2 * NH; x++) {
+        v[x] = __half2float(__ushort_as_half((unsigned short)(acc[x / 2] >> (x & 1) * 16)));
+        if (c + x < p.K) v[x] = __fadd_rn(v[x], __ldg(p.bias + c + x));
+      }
+      if (VEC == 8 && p.K % 8 == 0) {
+        reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2 % (2 * NH)], v[3 % (2 * NH)]);
+        reinterpret_cast<float4*>(dst)[1] = make_float4(v[4 % (2 * NH)], v[5 % (2 * NH)], v[6 % (2 * NH)], v[7 % (2 * NH)]);
+      } else {
+#pragma unroll
+        for (int x = 0; x < (VEC == 8 ? 8 : 1); x++)
+          if (c + x < p.K) dst[x] = v[x % (2 * NH)];
+      }
+    } else if (VEC == 8) {
+      __half* dst = static_cast<__half*>(p.out) + row * p.K + c;
       if (p.K % 8 == 0) {
         *reinterpret_cast<uint4*>(dst) = make_uint4(acc[0], acc[NH > 1 ? 1 : 0], acc[NH > 2 ? 2 : 0], acc[NH > 3 ? 3 : 0]);
       } else {
@@ -174,7 +191,7 @@ __global__ void __launch_bounds__(kF16Warps * 32, 4) spmm_f16_rows_kernel(const 
           if (c + x < p.K) dst[x] = __ushort_as_half((unsigned short)(acc[x / 2 < NH ? x / 2 : 0] >> (x & 1) * 16));
       }
     } else {
-      dst[0] = __ushort_as_half((unsigned short)acc[0]);
+      static_cast<__half*>(p.out)[row * p.K + c] = __ushort_as_half((unsigned short)acc[0]);
     }
   }
   // The rows may start before the long rows' kernel in front of them has finished (they touch nothing of it); the
@@ -295,7 +312,13 @@ __device__ void f16_hub_add(const SpmmF16Params& p, long long row, long long c0,
   }
   if (p.mean) acc = h2_mean(acc, rh((float)(end - begin > 0 ? end - begin : 1)));
   const long long c = c0 + lane * 2;
-  __half* dst = p.out + row * p.K + c;
+  if (p.bias != nullptr) {
+    float* dst = static_cast<float*>(p.out) + row * p.K + c;
+    if (c < p.K) dst[0] = __fadd_rn(__half2float(__ushort_as_half((unsigned short)acc)), __ldg(p.bias + c));
+    if (c + 1 < p.K) dst[1] = __fadd_rn(__half2float(__ushort_as_half((unsigned short)(acc >> 16))), __ldg(p.bias + c + 1));
+    return;
+  }
+  __half* dst = static_cast<__half*>(p.out) + row * p.K + c;
   if (c < p.K) dst[0] = __ushort_as_half((unsigned short)acc);
   if (c + 1 < p.K) dst[1] = __ushort_as_half((unsigned short)(acc >> 16));
 }
@@ -384,16 +407,17 @@ extern "C" {
 
 int exact_spmm_f16(const void* rowptr, const void* col, int idx_bytes, const void* value, const void* mat, int64_t M,
                    int64_t K, int reduce, void* out, void* stream) {
-  return exact_spmm_f16_planned(rowptr, col, idx_bytes, value, mat, K, M, K, reduce, nullptr, 0, nullptr, 0, out, stream);
+  return exact_spmm_f16_planned(rowptr, col, idx_bytes, value, mat, K, M, K, reduce, nullptr, 0, nullptr, 0, nullptr, out, stream);
 }
 
 int exact_spmm_f16_planned(const void* rowptr, const void* col, int idx_bytes, const void* value, const void* mat,
                            int64_t ldm, int64_t M, int64_t K, int reduce, const int32_t* row_order,
-                           int64_t long_threshold, const int32_t* long_row, int64_t n_long, void* out, void* stream) {
+                           int64_t long_threshold, const int32_t* long_row, int64_t n_long, const float* bias, void* out,
+                           void* stream) {
   EXB_REQUIRE(n_long >= 0 && (n_long == 0 || (long_row && long_threshold > 0)), "spmm_f16: null plan array");
   SpmmF16Params p{};
   p.rowptr = rowptr; p.col = col; p.val = static_cast<const __half*>(value); p.mat = static_cast<const __half*>(mat);
-  p.out = static_cast<__half*>(out); p.M = M; p.K = K; p.ldm = ldm;
+  p.out = out; p.bias = bias; p.M = M; p.K = K; p.ldm = ldm;
   p.row_order = row_order; p.long_row = long_row; p.n_long = n_long;
   p.long_threshold = n_long > 0 ? long_threshold : 0;
   return spmm_f16_common(p, idx_bytes, reduce, (cudaStream_t)stream);

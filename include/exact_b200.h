@@ -50,6 +50,8 @@ EXACT_API const char* exact_last_error(void);
  * incomplete.  exact_set_status writes the word, so that a host can exercise its error path without making
  * a wait expire.  No counterpart in the reference (its kernels never wait). */
 EXACT_API int exact_status(int* status, void* stream);
+/* The word as it is now, without waiting for anything (it lives in page-locked host memory). */
+EXACT_API int exact_status_peek(int* status);
 /* The same copy without the synchronisation: *pinned_host_status (page-locked host memory) is valid once the
  * work enqueued on `stream` so far has completed. */
 EXACT_API int exact_status_async(int* pinned_host_status, void* stream);
@@ -300,11 +302,12 @@ EXACT_API int exact_spmm_f16(const void* rowptr, const void* col, int idx_bytes,
 /* exact_spmm_f16 with a plan of the adjacency's rows: operand rows of pitch `ldm` elements (when ldm is a multiple of 8
  * and mat 16-byte aligned, the columns K .. ldm - 1 are read and ignored), `row_order` (or NULL) the order in which the
  * rows are taken, `long_row` the n_long rows with more than `long_threshold` edges, longest first (their sums run on
- * warps of their own, still one chain in CSR order).  Same bits as exact_spmm_f16. */
+ * warps of their own, still one chain in CSR order).  Same bits as exact_spmm_f16.  With `bias` [K] fp32 (or NULL) `out` is
+ * fp32 and receives float(half result) + bias, what adding an fp32 bias to the half result gives (layers.py:261-263). */
 EXACT_API int exact_spmm_f16_planned(const void* rowptr, const void* col, int idx_bytes, const void* value, const void* mat,
                                      int64_t ldm, int64_t M, int64_t K, int reduce, const int32_t* row_order,
-                                     int64_t long_threshold, const int32_t* long_row, int64_t n_long, void* out,
-                                     void* stream);
+                                     int64_t long_threshold, const int32_t* long_row, int64_t n_long, const float* bias,
+                                     void* out, void* stream);
 
 /* exact_spmm_split with the second exchange folded into it (no counterpart in the reference): instead of a local
  * [M, K] result followed by exact_rows_scatter, every output row r is stored, by the warp that summed it,
@@ -323,6 +326,15 @@ EXACT_API int exact_spmm_split_routed(const void* rowptr, const void* col, int i
                                       const int32_t* long_item_ptr, int64_t n_long, float* scratch,
                                       const int32_t* row_order, int64_t shard, int64_t col0, int64_t ldd,
                                       void* const* dst, int n_dst, void* stream);
+
+/* exact_spmm_split (or exact_spmm, with n_items = 0) into a local result, with a row order for narrow operands (or NULL) and
+ * `bias` [K] (or NULL) added to every row of the result: out = reduce(A, mat) + bias, the sum and the addition rounded
+ * separately as `out + bias` after the aggregation rounds them (layers.py:261-263). */
+EXACT_API int exact_spmm_planned(const void* rowptr, const void* col, int idx_bytes, const float* value, const float* mat,
+                                 int64_t M, int64_t K, int reduce, int64_t long_threshold, const int32_t* item_row,
+                                 const int64_t* item_begin, const int64_t* item_end, const int32_t* item_slot,
+                                 int64_t n_items, const int32_t* long_row, const int32_t* long_item_ptr, int64_t n_long,
+                                 float* scratch, const int32_t* row_order, const float* bias, float* out, void* stream);
 
 /* Buffers that the ranks of a row-sharded run write into each other (one process per GPU, one node).  No
  * counterpart in the reference.  These are the only entry points that allocate or free device memory:
@@ -411,6 +423,17 @@ EXACT_API int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t
                                    const float* A2, int64_t K2, int64_t lda2, const float* B2, int64_t ldb2,
                                    int64_t N, const float* bias, int accumulate, void* workspace, float* C,
                                    int64_t ldc, void* stream);
+/* exact_linear_forward with two more choices.  incb, incb2: distance between the elements of a row of B, B2 (ldb = 1 and incb =
+ * the pitch: the transposed weight, without a copy).  k_chunk: the contraction is cut into chunks of k_chunk columns (a
+ * multiple of 32; 0: one chunk).  The tensor core truncates its fp32 accumulator at every MMA, a bias of about 7e-9 of the
+ * result per contracted column; each chunk's sum is added to the previous ones by an fp32 addition instead (at 256 columns
+ * the bias stays below 2e-6 whatever K is).  partial: exact_linear_partial_bytes(N) bytes, 16-byte aligned. */
+EXACT_API int64_t exact_linear_partial_bytes(int64_t N);
+EXACT_API int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb,
+                                           int64_t incb, const float* A2, int64_t K2, int64_t lda2, const float* B2,
+                                           int64_t ldb2, int64_t incb2, int64_t N, const float* bias, int accumulate,
+                                           int64_t k_chunk, float* partial, void* workspace, float* C, int64_t ldc,
+                                           void* stream);
 
 /* Weight gradient of a quantised linear layer from the packed activation(s), on the tensor cores:
  *     out[O, kpad] = g^T [O x N] . dequantise(packed) [N x k]
@@ -423,7 +446,7 @@ EXACT_API int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t
  *   g [N, O] fp32, 16-byte aligned, O % 4 == 0, O <= 256; other shapes return code 3 (the caller unpacks and
  *   uses a library GEMM).  tf32 inputs, fp32 accumulation: about 5e-4 relative.
  *   workspace: exact_grad_weight_workspace_bytes(O, pad16(k0) + pad16(k1), SM count) bytes, 256-byte aligned:
- *   its first int32 is the status word (see exact_rp_quantize_pack), the rest holds one partial result per CTA (of at
+ *   it holds one partial result per CTA (of at
  *   most 256 columns: more are multiplied in passes), added in a fixed order by a second kernel (the result does not
  *   depend on timing). */
 EXACT_API int64_t exact_grad_weight_workspace_bytes(int64_t O, int64_t k_total_padded, int max_ctas);
