@@ -152,14 +152,7 @@ def spmm_value_bw(row, rowptr, col, mat, grad, reduce):
         raise RuntimeError("mat and grad must be float32 matrices")
     if not (row.dtype == col.dtype == rowptr.dtype) or col.dtype not in (torch.int32, torch.int64):
         raise RuntimeError("row, rowptr and col must all be int32 or all int64")
-    mat, grad = mat.contiguous(), grad.contiguous()
-    row, col, rowptr = row.contiguous(), col.contiguous(), rowptr.contiguous()
-    E, K = col.numel(), mat.size(1)
-    out = torch.empty(E, dtype=torch.float32, device=mat.device)
-    ib = 4 if col.dtype == torch.int32 else 8
-    _lib.invoke("exact_spmm_value_bw", E * (8 * K + 2 * ib + 4), _lib.ptr(row), _lib.ptr(rowptr), _lib.ptr(col), ib,
-                _lib.ptr(mat), _lib.ptr(grad), E, K, _lib.REDUCE[reduce], _lib.ptr(out), _lib.stream_ptr())
-    return out
+    return _lib.native().spmm_value_backward(row.contiguous(), rowptr.contiguous(), col.contiguous(), mat, grad, reduce == "mean")
 
 
 def spmm_sum_bw(row, rowptr, col, value, colptr, csr2csc, mat, grad_out, has_value, value_requires_grad,
@@ -201,17 +194,8 @@ def _spmm_minmax(rowptr, col, value, mat, is_max):
         raise RuntimeError("mat must be a float32 matrix")
     if rowptr.dtype != col.dtype or col.dtype not in (torch.int32, torch.int64):
         raise RuntimeError("rowptr and col must both be int32 or both int64")
-    mat, rowptr, col = mat.contiguous(), rowptr.contiguous(), col.contiguous()
-    if value is not None:
-        value = value.detach().to(torch.float32).contiguous()
-    M, K, nnz = rowptr.numel() - 1, mat.size(1), col.numel()
-    out = torch.empty((M, K), dtype=torch.float32, device=mat.device)
-    arg_out = torch.empty((M, K), dtype=col.dtype, device=mat.device)
-    ib = 4 if col.dtype == torch.int32 else 8
-    _lib.invoke("exact_spmm_minmax", nnz * (K * 4 + ib) + M * K * (4 + ib), _lib.ptr(rowptr), _lib.ptr(col), ib,
-                _lib.ptr(value), _lib.ptr(mat), M, K, nnz, 1 if is_max else 0, _lib.ptr(out), _lib.ptr(arg_out),
-                _lib.stream_ptr())
-    return out, arg_out
+    rowptr, col = rowptr.contiguous(), col.contiguous()
+    return _lib.native().spmm_minmax(rowptr, col, native_plan(rowptr), value, mat, is_max)
 
 
 def spmm_max_fw(rowptr, col, value, mat):
@@ -226,28 +210,9 @@ def spmm_min_fw(rowptr, col, value, mat):
 
 def spmm_max_bw(col, value, mat, arg_out, grad_out, has_value, value_requires_grad, mat_requires_grad):
     """spmm.cc:159-193 (and 210-241 for min, the same arithmetic): gradients routed to the winning edges."""
-    arg_out = arg_out.to(torch.int64)
-    invalid = arg_out == col.size(0)
-    arg_out = arg_out.masked_fill(invalid, 0)
-    ind = col.to(torch.int64).index_select(0, arg_out.flatten()).view_as(arg_out)
-    grad_value = None
-    if has_value and value_requires_grad:
-        out = mat.gather(-2, ind)
-        out.mul_(grad_out)
-        out.masked_fill_(invalid, 0)
-        grad_value = torch.zeros_like(value)
-        grad_value.scatter_add_(0, arg_out.flatten(), out.flatten())
-    grad_mat = None
-    if mat_requires_grad:
-        if has_value:
-            v = value.detach().index_select(0, arg_out.flatten()).view_as(arg_out)
-            v = v * grad_out
-        else:
-            v = grad_out.clone()
-        v.masked_fill_(invalid, 0)
-        grad_mat = torch.zeros_like(mat)
-        grad_mat.scatter_add_(-2, ind, v)
-    return grad_value, grad_mat
+    need_value = has_value and value_requires_grad
+    return _lib.native().spmm_minmax_backward(col.contiguous(), value if has_value else None, mat if need_value else None,
+                                              arg_out, grad_out, need_value, mat_requires_grad, mat.size(0))
 
 
 spmm_min_bw = spmm_max_bw

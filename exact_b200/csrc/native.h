@@ -41,7 +41,8 @@ struct LibraryError : std::runtime_error {   // becomes exact_b200.ExactB200Erro
   X(exact_spmm_f16_planned) X(exact_rows_scale_colsum_workspace_bytes)                     \
   X(exact_rows_scale_colsum) X(exact_bn_backward_workspace_bytes) X(exact_bn_backward_from_packed)                    \
   X(exact_rp_workspace_bytes) X(exact_rp_quantize_pack) X(exact_rademacher) X(exact_grad_weight_workspace_bytes)      \
-  X(exact_grad_weight_from_packed) X(exact_linear_workspace_bytes) X(exact_linear_partial_bytes) X(exact_linear_forward_strided) X(exact_spmm_minmax)       \
+  X(exact_grad_weight_from_packed) X(exact_linear_workspace_bytes) X(exact_linear_partial_bytes) X(exact_linear_forward_strided)                            \
+  X(exact_spmm_minmax_scratch_bytes) X(exact_spmm_minmax_planned) X(exact_spmm_minmax_backward)                       \
   X(exact_spmm_value_bw) X(exact_status_peek)
 
 struct Library {
@@ -150,6 +151,15 @@ struct RowPlan {
 using PlanPtr = std::shared_ptr<const RowPlan>;
 Tensor spmm(const Tensor& rowptr, const Tensor& col, const RowPlan& plan, const OptTensor& value, const Tensor& mat, bool mean,
             const OptTensor& bias = {});
+
+// (best value, winning edge) of the max / min aggregation, and its gradients (grad_value, grad_mat)
+std::tuple<Tensor, Tensor> spmm_minmax(const Tensor& rowptr, const Tensor& col, const RowPlan& plan, const OptTensor& value,
+                                       const Tensor& mat, bool is_max);
+std::tuple<Tensor, Tensor> spmm_minmax_backward(const Tensor& col, const OptTensor& value, const OptTensor& mat, const Tensor& arg,
+                                                const Tensor& grad, bool need_value, bool need_mat, int64_t mat_rows);
+// gradient with respect to the edge values of a sum or mean
+Tensor spmm_value_backward(const Tensor& row, const Tensor& rowptr, const Tensor& col, const Tensor& mat, const Tensor& grad,
+                           bool mean);
 
 struct Csr {
   Tensor rowptr, col;

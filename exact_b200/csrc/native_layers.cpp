@@ -302,6 +302,71 @@ Tensor sage_node(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const
   return SageNode::apply(x, w_l, b_l, w_r, s);
 }
 
+// ---- aggregation: qspmm_sum / mean / max / min (ops.py:257-436) --------------------------------------------
+struct AggregateState : torch::CustomClassHolder {
+  c10::intrusive_ptr<Graph> graph;
+  Saving how;
+  OptTensor value, row;
+  Compressed x;        // only when the edge values get a gradient: nothing else reads it
+  Tensor arg;
+  int64_t reduce, rows;
+  bool keep_x;
+};
+
+struct AggregateNode : Function<AggregateNode> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x_, const OptTensor& value, const c10::intrusive_ptr<AggregateState>& s) {
+    const Graph& g = *s->graph;
+    const Tensor x = x_.contiguous();
+    Tensor out;
+    if (s->reduce <= 1) {
+      out = spmm(g.fw, value, x, s->reduce == 1);
+    } else {
+      auto [best, arg] = spmm_minmax(g.fw.rowptr, g.fw.col, *g.fw.plan, value, x, s->reduce == 2);
+      out = best;
+      s->arg = arg;
+    }
+    if (s->keep_x) s->x = compress(x, s->how, s->how.offset);
+    if (value) s->value = value->detach();
+    s->rows = x.size(0);
+    ctx->saved_data["s"] = c10::IValue::make_capsule(s);
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    Plain plain;
+    auto s = state_of<AggregateState>(ctx);
+    const Graph& gr = *s->graph;
+    const bool need_x = ctx->needs_input_grad(0), need_v = s->value && ctx->needs_input_grad(1);
+    const Tensor g = grads[0].contiguous();
+    Tensor gx, gv, x;
+    if (need_v) {
+      x = unpack(s->x.q.codes, s->how.bits, s->x.q.scale, s->x.q.mn, s->rows, s->x.width);
+      if (s->x.R.defined()) x = linear_supported(x) ? linear(x, s->x.R, {}, {}, {}, {}, false) : at::matmul(x, s->x.R.t());
+    }
+    if (s->reduce <= 1) {
+      if (need_v) gv = spmm_value_backward(*s->row, gr.fw.rowptr, gr.fw.col, x, g, s->reduce == 1);
+      if (need_x) gx = spmm(gr.bw, gr.bw.value, g, false);
+    } else {
+      OptTensor mat;
+      if (need_v) mat = x;
+      auto [v, m] = spmm_minmax_backward(gr.fw.col, s->value, mat, s->arg, g, need_v, need_x, s->rows);
+      gv = v;
+      gx = m;
+    }
+    return {gx, gv, {}};
+  }
+};
+
+Tensor aggregate_node(const Tensor& x, const OptTensor& value, const OptTensor& row, const c10::intrusive_ptr<Graph>& graph,
+                      int64_t reduce, bool keep_x, const Saving& how) {
+  auto s = c10::make_intrusive<AggregateState>();
+  s->keep_x = keep_x;
+  s->graph = graph;
+  s->how = how;
+  s->row = row;
+  s->reduce = reduce;
+  return AggregateNode::apply(x, value, s);
+}
+
 // ---- evaluation -----------------------------------------------------------------------------------------
 // Outputs that were products of the library's fp32 GEMM: contractions beyond 256 columns in chunks, so that the truncation
 // of the tensor core's accumulator stays below 2e-6 of a layer's output (4e-6 at 602 columns in one piece).

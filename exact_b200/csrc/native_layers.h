@@ -28,6 +28,12 @@ Tensor gcn_node(const Tensor& x, const Tensor& w, const OptTensor& b, const c10:
 Tensor sage_node(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const OptTensor& w_r,
                  const c10::intrusive_ptr<Graph>& graph, bool mean, const Saving& how, bool projected_first,
                  bool gradient_first);
+// reduce(A, x) with gradients to x and, when they ask for one, the edge values (qspmm_sum / mean / max / min).
+// reduce: 0 sum, 1 mean, 2 max, 3 min; the graph's transpose carries the weights of the reduction.  row: the row of every edge
+// (needed for the values' gradient of a sum or mean).  keep_x: the values' gradient will be asked for, x is saved compressed.
+Tensor aggregate_node(const Tensor& x, const OptTensor& value, const OptTensor& row, const c10::intrusive_ptr<Graph>& graph,
+                      int64_t reduce, bool keep_x, const Saving& how);
+
 // The same layers without anything saved (evaluation).
 Tensor gcn_eval(const Tensor& x, const Tensor& w, const OptTensor& b, const c10::intrusive_ptr<Graph>& graph, bool half);
 Tensor sage_eval(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const OptTensor& w_r,

@@ -233,6 +233,16 @@ Tensor sage_op(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const O
                    gradient_first);
 }
 
+Tensor aggregate_op(const Tensor& x, const OptTensor& value, const OptTensor& row, const c10::intrusive_ptr<Graph>& graph,
+                    int64_t reduce, bool keep_x, int64_t bits, int64_t kept, uint64_t seed, uint64_t offset, int64_t row_offset,
+                    bool fused) {
+  return aggregate_node(x, value, row, graph, reduce, keep_x, Saving{bits, kept, seed, offset, row_offset, fused});
+}
+std::tuple<Tensor, Tensor> spmm_minmax_op(const Tensor& rowptr, const Tensor& col, const PlanPtr& plan, const OptTensor& value,
+                                          const Tensor& mat, bool is_max) {
+  return spmm_minmax(rowptr, col, *plan, value, mat, is_max);
+}
+
 // bind(path of libexact_b200.so, ExactB200Error)
 PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 2) {
@@ -268,6 +278,8 @@ PyMethodDef methods[] = {
     EXB_METHOD("quantize_pack", quantize_pack), EXB_METHOD("unpack", unpack), EXB_METHOD("rademacher", rademacher),
     EXB_METHOD("rp_quantize_pack", rp_quantize_pack_op), EXB_METHOD("bn_backward", bn_backward_op), EXB_METHOD("linear", linear_op), EXB_METHOD("grad_weight", grad_weight_op),
     EXB_METHOD("rows_scale_colsum", rows_scale_colsum), EXB_METHOD("spmm", spmm_op), EXB_METHOD("act", act_node),
+    EXB_METHOD("aggregate", aggregate_op), EXB_METHOD("spmm_minmax", spmm_minmax_op),
+    EXB_METHOD("spmm_minmax_backward", spmm_minmax_backward), EXB_METHOD("spmm_value_backward", spmm_value_backward),
     EXB_METHOD("gcn", gcn_op), EXB_METHOD("sage", sage_op), EXB_METHOD("gcn_eval", gcn_eval), EXB_METHOD("sage_eval", sage_eval), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -456,11 +456,72 @@ Tensor spmm(const Tensor& rowptr, const Tensor& colt, const RowPlan& a, const Op
     prow = ptr<int32_t>(pc.row); pslot = ptr<int32_t>(pc.slot); lrow = ptr<int32_t>(pc.long_row); lptr = ptr<int32_t>(pc.long_ptr);
     pb = ptr<int64_t>(pc.begin); pe = ptr<int64_t>(pc.end);
   }
-  const bool narrow = K <= 64 && K % 4 == 0 && M > 0;   // the kernel for narrow operands takes its rows in order of length
-  const int32_t* order = narrow ? ptr<int32_t>(a.row_order(rowptr)) : nullptr;
+  const bool narrow = K <= 64 && K % 4 == 0 && M > 0;
+  const int32_t* order = M > 0 ? ptr<int32_t>(a.row_order(rowptr)) : nullptr;
   invoke(narrow ? "exact_spmm_split_routed" : pc.n ? "exact_spmm_split" : "exact_spmm", info, [&](void* st) {
     return lib.exact_spmm_planned(rp, col, ib, ptr<float>(value), ptr<float>(mat), M, K, red, pc.n ? a.threshold : 0, prow, pb, pe,
                                   pslot, pc.n, lrow, lptr, pc.n_long, sc, order, ptr<float>(bias), ptr<float>(out), st);
+  });
+  return out;
+}
+
+std::tuple<Tensor, Tensor> spmm_minmax(const Tensor& rowptr, const Tensor& col, const RowPlan& plan, const OptTensor& value_,
+                                       const Tensor& mat_, bool is_max) {
+  const Tensor mat = mat_.contiguous();
+  check_type(mat.scalar_type() == at::kFloat, "mat");
+  same_device(rowptr, mat);
+  same_device(col, mat);
+  c10::cuda::CUDAGuard guard(mat.device());
+  OptTensor value;
+  if (value_) value = value_->detach().to(at::kFloat).contiguous();
+  const int64_t M = rowptr.size(0) - 1, K = mat.size(1), nnz = col.size(0);
+  const int ib = col.scalar_type() == at::kInt ? 4 : 8;
+  Tensor out = empty({M, K}, at::kFloat, mat), arg = empty({M, K}, col.scalar_type(), mat), scratch;
+  const RowPlan::Pieces& pc = plan.pieces(rowptr, col);
+  if (pc.n) scratch = empty({lib.exact_spmm_minmax_scratch_bytes(pc.n, K)}, at::kByte, mat);
+  invoke("exact_spmm_minmax", {nnz * (K * 4 + ib) + M * K * (4 + ib)}, [&](void* st) {
+    return lib.exact_spmm_minmax_planned(ptr(rowptr), ptr(col), ib, ptr<float>(value), ptr<float>(mat), M, K, nnz, is_max ? 1 : 0,
+                                         pc.n ? plan.threshold : 0, pc.n ? ptr<int64_t>(pc.begin) : nullptr,
+                                         pc.n ? ptr<int64_t>(pc.end) : nullptr, pc.n ? ptr<int32_t>(pc.slot) : nullptr, pc.n,
+                                         pc.n ? ptr<int32_t>(pc.long_row) : nullptr, pc.n ? ptr<int32_t>(pc.long_ptr) : nullptr,
+                                         pc.n_long, pc.n ? ptr(scratch) : nullptr, ptr<float>(out), ptr(arg), st);
+  });
+  return {out, arg};
+}
+
+std::tuple<Tensor, Tensor> spmm_minmax_backward(const Tensor& col, const OptTensor& value_, const OptTensor& mat, const Tensor& arg,
+                                                const Tensor& grad_, bool need_value, bool need_mat, int64_t mat_rows) {
+  const Tensor grad = grad_.contiguous();
+  c10::cuda::CUDAGuard guard(grad.device());
+  OptTensor value;
+  if (value_) value = value_->detach().to(at::kFloat).contiguous();
+  const int64_t M = grad.size(0), K = grad.size(1), nnz = col.size(0);
+  const int ib = col.scalar_type() == at::kInt ? 4 : 8;
+  Tensor gv, gm;
+  const auto opts = grad.options().requires_grad(false);
+  if (need_value) gv = at::zeros({nnz}, opts);
+  if (need_mat) gm = at::zeros({mat_rows, K}, opts);
+  invoke("exact_spmm_minmax_backward", {M * K * (8 + ib) + (need_mat ? mat_rows * K * 4 : 0)}, [&](void* st) {
+    return lib.exact_spmm_minmax_backward(ptr(col), ib, ptr<float>(value), ptr<float>(mat), ptr(arg), ptr<float>(grad), M, K, nnz,
+                                          need_mat ? ptr<float>(gm) : nullptr, need_value ? ptr<float>(gv) : nullptr, st);
+  });
+  return {gv, gm};
+}
+
+Tensor spmm_value_backward(const Tensor& row, const Tensor& rowptr, const Tensor& col, const Tensor& mat_, const Tensor& grad_,
+                           bool mean) {
+  const Tensor mat = mat_.contiguous(), grad = grad_.contiguous();
+  check_type(mat.scalar_type() == at::kFloat && grad.scalar_type() == at::kFloat, "mat or grad");
+  check_type(row.scalar_type() == col.scalar_type() && rowptr.scalar_type() == col.scalar_type(), "row, rowptr or col");
+  same_device(row, mat);
+  same_device(col, grad);
+  c10::cuda::CUDAGuard guard(mat.device());
+  const int64_t E = col.size(0), K = mat.size(1);
+  const int ib = col.scalar_type() == at::kInt ? 4 : 8;
+  Tensor out = empty({E}, at::kFloat, mat);
+  invoke("exact_spmm_value_bw", {E * (8 * K + 2 * ib + 4)}, [&](void* st) {
+    return lib.exact_spmm_value_bw(ptr(row), ptr(rowptr), ptr(col), ib, ptr<float>(mat), ptr<float>(grad), E, K,
+                                   mean ? EXACT_REDUCE_MEAN : EXACT_REDUCE_SUM, ptr<float>(out), st);
   });
   return out;
 }

@@ -61,6 +61,7 @@ __device__ __forceinline__ float* output_row(const SpmmParams& p, long long row)
 }
 
 constexpr int kSpmmWarps = 4;
+constexpr int kRowWarps = 8, kRowBlocks = 4, kRowBatch = 8;   // persistent row kernel: warps per block, blocks per SM, gathers in flight
 constexpr int kEdgeUnroll = 16;   // gathers in flight per lane (16 against 8: 3 % faster at 128 M edges x 256 columns)
 
 template <int VEC>
@@ -226,6 +227,128 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_kernel(const __grid_
     if (FULL || cvalid[j]) st_vec<VEC>(dst + coff[j], acc[j]);
 }
 
+template <int U, int VEC, bool HAS_VAL>
+__device__ __forceinline__ void row_group(const char* __restrict__ mat0, unsigned long long row_bytes, const uint32_t* idx,
+                                          const float* val, float (&acc)[VEC]) {
+  float m[U][VEC];
+#pragma unroll
+  for (int u = 0; u < U; u++) ldg_vec<VEC>(reinterpret_cast<const float*>(mat0 + (unsigned long long)idx[u] * row_bytes), m[u]);
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const float w = HAS_VAL ? val[u] : 1.f;
+#pragma unroll
+    for (int x = 0; x < VEC; x++) {
+      if (HAS_VAL) acc[x] = __fmaf_rn(w, m[u][x], acc[x]);
+      else acc[x] = __fadd_rn(acc[x], m[u][x]);
+    }
+  }
+}
+
+// Wide operands, rows in length-sorted order, by persistent warps.  With a warp per row and blocks of four rows, a graph of
+// short rows was a chain of memory latencies per row (extent, indices, gathers) at 40 % occupancy, a block's slot being held
+// by its longest row.  Here a warp takes every W-th row of a tile, keeps the next row's indices, the extent of the one after
+// and the id of the third on their way, and gathers eight edges at a time; 64 registers, 32 warps per SM (24 with 16
+// gathers: 4 - 13 % slower, 40 with 48 registers: 10 - 20 % slower).  256 columns, with the pieces of long rows: 169,343
+// nodes / 2.54 M edges 335 -> 258 us, 500,000 / 6.4 M 877 -> 634, 232,965 / 23 M 1,240 -> 1,176, 2.45 M / 126 M 9,590 -> 8,800.
+// Without the order the strided rows are unbalanced (426 us at 2.54 M edges): calls without one take the kernel above.
+// The pieces stay with that kernel too: 256 edges each, they want its 48 warps per SM and run 20 % slower in this one.
+// Tiles of 128 columns stay separate passes over the graph (all of a tile's rows before the next tile).
+template <typename IdxT, int VEC, bool HAS_VAL>
+__global__ void __launch_bounds__(kRowWarps * 32, kRowBlocks) spmm_rows_kernel(const __grid_constant__ SpmmParams p) {
+  __shared__ uint32_t s_idx[kRowWarps][32];
+  __shared__ float s_val[kRowWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const IdxT* __restrict__ rowptr = reinterpret_cast<const IdxT*>(p.rowptr);
+  const IdxT* __restrict__ col = reinterpret_cast<const IdxT*>(p.col);
+  const long long K = p.K;
+  const unsigned long long row_bytes = (unsigned long long)K * 4ull;
+  const long long stride = (long long)gridDim.x * kRowWarps;
+  uint32_t* const my_idx = s_idx[warp];
+  float* const my_val = s_val[warp];
+
+  for (long long c0 = 0; c0 < K; c0 += 32 * VEC) {
+    const long long coff = c0 + lane * VEC;
+    const bool cvalid = coff < K;
+    const long long cload = cvalid ? coff : c0;     // lanes past K gather what the first lane gathers and drop it
+    const char* __restrict__ mat0 = reinterpret_cast<const char*>(p.mat + cload);
+    long long u = (long long)blockIdx.x * kRowWarps + warp;
+    auto row_at = [&](long long q) -> int { return q < p.M ? p.row_order[q] : -1; };
+    auto extent = [&](int r, IdxT& b, IdxT& e) {
+      b = e = 0;
+      if (r >= 0) {
+        b = rowptr[r];
+        e = rowptr[r + 1];
+      }
+    };
+    auto first_edges = [&](IdxT b, IdxT e, uint32_t& i, float& v) {
+      i = 0;
+      v = 0.f;
+      if (b + lane < e) {
+        i = (uint32_t)col[b + lane];
+        if (HAS_VAL) v = __ldg(p.val + b + lane);
+      }
+    };
+    IdxT b, e, b1, e1;
+    int row = row_at(u), row1 = row_at(u + stride), row2 = row_at(u + 2 * stride);
+    extent(row, b, e);
+    extent(row1, b1, e1);
+    uint32_t idx;
+    float val;
+    first_edges(b, e, idx, val);
+    for (; u < p.M; u += stride) {
+      __syncwarp();
+      my_idx[lane] = idx;
+      if (HAS_VAL) my_val[lane] = val;
+      __syncwarp();
+      IdxT b2, e2;
+      const int row3 = row_at(u + 3 * stride);
+      extent(row2, b2, e2);
+      first_edges(b1, e1, idx, val);
+      const long long len = (long long)(e - b);
+      if (!(p.long_threshold > 0 && len > p.long_threshold)) {
+        float acc[VEC];
+#pragma unroll
+        for (int x = 0; x < VEC; x++) acc[x] = 0.f;
+        for (long long base = 0; base < len; base += 32) {
+          if (base > 0) {
+            const long long at = (long long)b + base + lane;
+            uint32_t i = 0;
+            float v = 0.f;
+            if (at < (long long)e) {
+              i = (uint32_t)col[at];
+              if (HAS_VAL) v = __ldg(p.val + at);
+            }
+            __syncwarp();
+            my_idx[lane] = i;
+            if (HAS_VAL) my_val[lane] = v;
+            __syncwarp();
+          }
+          const int cnt = len - base < 32 ? (int)(len - base) : 32;
+          int t = 0;
+#pragma unroll 1
+          for (; t + kRowBatch <= cnt; t += kRowBatch) row_group<kRowBatch, VEC, HAS_VAL>(mat0, row_bytes, my_idx + t, my_val + t, acc);
+          if (kRowBatch > 8 && (cnt & 8)) { row_group<8, VEC, HAS_VAL>(mat0, row_bytes, my_idx + t, my_val + t, acc); t += 8; }
+          if (cnt & 4) { row_group<4, VEC, HAS_VAL>(mat0, row_bytes, my_idx + t, my_val + t, acc); t += 4; }
+          if (cnt & 2) { row_group<2, VEC, HAS_VAL>(mat0, row_bytes, my_idx + t, my_val + t, acc); t += 2; }
+          if (cnt & 1) row_group<1, VEC, HAS_VAL>(mat0, row_bytes, my_idx + t, my_val + t, acc);
+        }
+        if (p.mean) {
+          const float dv = (float)(len > 0 ? len : 1);  // reducer.cuh:75-76
+#pragma unroll
+          for (int x = 0; x < VEC; x++) acc[x] = __fdiv_rn(acc[x], dv);
+        }
+        if (p.bias != nullptr) {
+#pragma unroll
+          for (int x = 0; x < VEC; x++) acc[x] = __fadd_rn(acc[x], __ldg(p.bias + cload + x));
+        }
+        if (cvalid) st_vec<VEC>(output_row(p, row) + coff, acc);
+      }
+      b = b1; e = e1; b1 = b2; e1 = e2;
+      row = row1; row1 = row2; row2 = row3;
+    }
+  }
+}
+
 // Adds the partial sums of each long row in item order and writes the row of the output.
 template <typename IdxT>
 __global__ void __launch_bounds__(128) spmm_long_reduce_kernel(const __grid_constant__ SpmmParams p) {
@@ -255,7 +378,7 @@ __global__ void __launch_bounds__(128) spmm_long_reduce_kernel(const __grid_cons
 // strict CSR-order sum (the pieces of long rows are still added separately).  The groups of a warp run until
 // the longest of their rows is done; callers that pass `row_order` (rows sorted by length) give every warp rows
 // of equal length.
-template <typename IdxT, bool HAS_VAL, int MODE, int LPE>
+template <typename IdxT, bool HAS_VAL, int LPE>
 __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_multi_kernel(const __grid_constant__ SpmmParams p) {
   constexpr int kRows = 32 / LPE;              // rows (or long-row pieces) per warp
   constexpr int kBatch = 8;                    // edges per step and group
@@ -272,21 +395,18 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_multi_kernel(const _
   long long begin = 0, len = 0;
   float* dst = nullptr;
   bool live = false;
-  if (MODE == MODE_ROWS) {
-    if (unit < p.M) {
-      const long long row = p.row_order ? (long long)p.row_order[unit] : unit;
-      begin = (long long)rowptr[row];
-      len = (long long)rowptr[row + 1] - begin;
-      live = !(p.long_threshold > 0 && len > p.long_threshold);
-      dst = output_row(p, row);
-    }
-  } else {
-    if (unit < p.n_items) {
-      begin = p.item_begin[unit];
-      len = p.item_end[unit] - begin;
-      live = true;
-      dst = p.scratch + (long long)(p.item_slot ? p.item_slot[unit] : (int)unit) * K;
-    }
+  const bool is_row = unit >= p.n_items;     // the pieces of long rows come first
+  if (!is_row) {
+    begin = p.item_begin[unit];
+    len = p.item_end[unit] - begin;
+    live = true;
+    dst = p.scratch + (long long)(p.item_slot ? p.item_slot[unit] : (int)unit) * K;
+  } else if (unit - p.n_items < p.M) {
+    const long long row = p.row_order ? (long long)p.row_order[unit - p.n_items] : unit - p.n_items;
+    begin = (long long)rowptr[row];
+    len = (long long)rowptr[row + 1] - begin;
+    live = !(p.long_threshold > 0 && len > p.long_threshold);
+    dst = output_row(p, row);
   }
   const long long count = len;
   if (!live) len = 0;
@@ -347,35 +467,34 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_multi_kernel(const _
       val[q] = nval[q];
     }
   }
-  if (MODE == MODE_ROWS && p.mean) {
+  if (is_row && p.mean) {
     const float dv = (float)(count > 0 ? count : 1);  // reducer.cuh:75-76
 #pragma unroll
     for (int x = 0; x < 4; x++) acc[x] = __fdiv_rn(acc[x], dv);
   }
-  if (MODE == MODE_ROWS && p.bias != nullptr && cvalid) {
+  if (is_row && p.bias != nullptr && cvalid) {
 #pragma unroll
     for (int x = 0; x < 4; x++) acc[x] = __fadd_rn(acc[x], __ldg(p.bias + coff + x));
   }
   if (live && cvalid) *reinterpret_cast<float4*>(dst + coff) = make_float4(acc[0], acc[1], acc[2], acc[3]);
 }
 
+template <typename IdxT>
+static int launch_long_reduce(const SpmmParams& p, cudaStream_t st) {
+  if (p.n_items == 0) return EXB_OK;
+  spmm_long_reduce_kernel<IdxT><<<(unsigned)p.n_long, 128, 0, st>>>(p);
+  EXB_CUDA_OK(cudaGetLastError());
+  return EXB_OK;
+}
+
 template <typename IdxT, bool HAS_VAL, int LPE>
 static int launch_spmm_multi(const SpmmParams& p, cudaStream_t st) {
   const unsigned gy = (unsigned)((p.K + 4 * LPE - 1) / (4 * LPE));
   constexpr long long per_cta = (long long)kSpmmWarps * (32 / LPE);
-  {
-    dim3 grid((unsigned)((p.M + per_cta - 1) / per_cta), gy);
-    spmm_csr_multi_kernel<IdxT, HAS_VAL, MODE_ROWS, LPE><<<grid, kSpmmWarps * 32, 0, st>>>(p);
-    EXB_CUDA_OK(cudaGetLastError());
-  }
-  if (p.n_items > 0) {
-    dim3 grid((unsigned)((p.n_items + per_cta - 1) / per_cta), gy);
-    spmm_csr_multi_kernel<IdxT, HAS_VAL, MODE_ITEMS, LPE><<<grid, kSpmmWarps * 32, 0, st>>>(p);
-    EXB_CUDA_OK(cudaGetLastError());
-    spmm_long_reduce_kernel<IdxT><<<(unsigned)p.n_long, 128, 0, st>>>(p);
-    EXB_CUDA_OK(cudaGetLastError());
-  }
-  return EXB_OK;
+  dim3 grid((unsigned)((p.n_items + p.M + per_cta - 1) / per_cta), gy);
+  spmm_csr_multi_kernel<IdxT, HAS_VAL, LPE><<<grid, kSpmmWarps * 32, 0, st>>>(p);
+  EXB_CUDA_OK(cudaGetLastError());
+  return launch_long_reduce<IdxT>(p, st);
 }
 
 template <typename IdxT, bool HAS_VAL>
@@ -389,7 +508,12 @@ template <typename IdxT, int VEC, int KVT, bool HAS_VAL, bool FULL>
 static int launch_spmm_mode(const SpmmParams& p, cudaStream_t st) {
   const long long C = p.K / VEC;
   const unsigned gy = (unsigned)((C + 32 * KVT - 1) / (32 * KVT));
-  {
+  if (p.row_order != nullptr && p.M < 2147483647LL) {
+    long long blocks = (p.M + kRowWarps - 1) / kRowWarps;
+    if (blocks > sm_count() * kRowBlocks) blocks = sm_count() * kRowBlocks;
+    spmm_rows_kernel<IdxT, VEC, HAS_VAL><<<(unsigned)blocks, kRowWarps * 32, 0, st>>>(p);
+    EXB_CUDA_OK(cudaGetLastError());
+  } else {
     dim3 grid((unsigned)((p.M + kSpmmWarps - 1) / kSpmmWarps), gy);
     spmm_csr_kernel<IdxT, VEC, KVT, HAS_VAL, FULL, MODE_ROWS><<<grid, kSpmmWarps * 32, 0, st>>>(p);
     EXB_CUDA_OK(cudaGetLastError());
@@ -398,10 +522,8 @@ static int launch_spmm_mode(const SpmmParams& p, cudaStream_t st) {
     dim3 grid((unsigned)((p.n_items + kSpmmWarps - 1) / kSpmmWarps), gy);
     spmm_csr_kernel<IdxT, VEC, KVT, HAS_VAL, FULL, MODE_ITEMS><<<grid, kSpmmWarps * 32, 0, st>>>(p);
     EXB_CUDA_OK(cudaGetLastError());
-    spmm_long_reduce_kernel<IdxT><<<(unsigned)p.n_long, 128, 0, st>>>(p);
-    EXB_CUDA_OK(cudaGetLastError());
   }
-  return EXB_OK;
+  return launch_long_reduce<IdxT>(p, st);
 }
 
 template <typename IdxT, int VEC, bool HAS_VAL>
@@ -456,64 +578,248 @@ static int spmm_common(SpmmParams& p, int idx_bytes, int reduce, cudaStream_t st
   return p.val ? launch_spmm_vec<int64_t, true>(p, st) : launch_spmm_vec<int64_t, false>(p, st);
 }
 
-// Gradient with respect to the edge values (spmm_cuda.cu:172-209): one warp per edge,
-// out[e] = dot(mat[col[e], :], grad[row[e], :]) (/ max(row length, 1) for mean).  Lane l accumulates columns
-// l, l + 32, ... with one FMA each, then the lanes are added by the reference's shuffle-down tree, so the
-// value equals the reference's bit for bit.
+// Gradient with respect to the edge values (spmm_cuda.cu:172-209): out[e] = dot(mat[col[e], :], grad[row[e], :])
+// (/ max(row length, 1) for mean).  Lane l accumulates columns l, l + 32, ... with one FMA each, then the lanes are added by
+// the reference's shuffle-down tree (l + 16, + 8, ...), so the value equals the reference's bit for bit.
+// A warp takes 32 consecutive edges.  Their rows of mat are gathered eight edges at a time, the row of grad stays in
+// registers while the edges belong to one row, and the 32 trees are folded into one another: at each level a lane keeps the
+// half of the edges its bit names and adds the other lane's value, 31 shuffles for 32 edges instead of 160 (an addition's
+// operands change places, which does not change its result).  One warp per edge was bound by issue slots and latency:
+// 2.5 M edges x 128 columns 402 us, 186 us this way.
 template <typename IdxT>
-__global__ void __launch_bounds__(256) spmm_value_bw_kernel(const IdxT* __restrict__ row, const IdxT* __restrict__ rowptr,
+__global__ void __launch_bounds__(128) spmm_value_bw_kernel(const IdxT* __restrict__ row, const IdxT* __restrict__ rowptr,
                                                             const IdxT* __restrict__ col, const float* __restrict__ mat,
                                                             const float* __restrict__ grad, long long E, long long K,
                                                             int mean, float* __restrict__ out) {
+  constexpr int kCols = 4;    // column groups of 32 held at a time
   const int lane = threadIdx.x & 31;
-  const long long e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (e >= E) return;
-  const long long r = (long long)row[e], c = (long long)col[e];
-  const float* m = mat + c * K;
-  const float* g = grad + r * K;
-  float val = 0.f;
-  for (long long k = lane; k < K; k += 32) val = __fmaf_rn(__ldg(m + k), __ldg(g + k), val);
+  const long long e0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) << 5;
+  if (e0 >= E) return;
+  const long long last = E - 1 - e0;
+  const long long mine = e0 + (lane < last ? lane : last);      // edges past the end repeat the last one
+  const long long my_row = (long long)row[mine], my_col = (long long)col[mine];
+  float acc[32];
 #pragma unroll
-  for (int i = 16; i > 0; i >>= 1) val = __fadd_rn(val, __shfl_down_sync(0xffffffffu, val, i));
-  if (lane == 0) {
+  for (int u = 0; u < 32; u++) acc[u] = 0.f;
+  for (long long k0 = 0; k0 < K; k0 += 32 * kCols) {
+    const long long k = k0 + lane;
+    long long held = -1;
+    float g[kCols];
+#pragma unroll
+    for (int u0 = 0; u0 < 32; u0 += 8) {
+      float m[8][kCols];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const float* __restrict__ src = mat + __shfl_sync(0xffffffffu, my_col, u0 + u) * K;
+#pragma unroll
+        for (int j = 0; j < kCols; j++) m[u][j] = k + 32 * j < K ? __ldg(src + k + 32 * j) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const long long r = __shfl_sync(0xffffffffu, my_row, u0 + u);
+        if (r != held) {
+          held = r;
+          const float* __restrict__ src = grad + r * K;
+#pragma unroll
+          for (int j = 0; j < kCols; j++) g[j] = k + 32 * j < K ? __ldg(src + k + 32 * j) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < kCols; j++) acc[u0 + u] = __fmaf_rn(m[u][j], g[j], acc[u0 + u]);   // (0 * 0 past the last column)
+      }
+    }
+  }
+#pragma unroll
+  for (int half = 16; half > 0; half >>= 1) {
+    const bool upper = (lane & half) != 0;
+#pragma unroll
+    for (int u = 0; u < half; u++) {
+      const float keep = upper ? acc[u + half] : acc[u], give = upper ? acc[u] : acc[u + half];
+      acc[u] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, half));
+    }
+  }
+  if (lane <= last) {
+    float val = acc[0];
     if (mean) {
-      const long long deg = (long long)rowptr[r + 1] - (long long)rowptr[r];
+      const long long deg = (long long)rowptr[my_row + 1] - (long long)rowptr[my_row];
       val = __fdiv_rn(val, (float)(deg > 1 ? deg : 1));
     }
-    out[e] = val;
+    out[e0 + lane] = val;
   }
 }
 
 // max / min aggregation with the position of the winning edge (spmm_cuda.cu:27-104 with REDUCE = MAX / MIN;
 // reducer.cuh:43-85): out[r, c] = max_e value[e] * mat[col[e], c], arg[r, c] = the first edge that attains it
 // (a later edge replaces the current one only when strictly greater / smaller), rows without edges give 0 and
-// arg = nnz.  One warp per row and 32 columns; lane = column, edges in CSR order.
-template <typename IdxT, bool HAS_VAL, bool IS_MAX>
-__global__ void __launch_bounds__(256) spmm_minmax_kernel(const IdxT* __restrict__ rowptr, const IdxT* __restrict__ col,
-                                                          const float* __restrict__ val, const float* __restrict__ mat,
-                                                          long long M, long long K, long long nnz, float* __restrict__ out,
-                                                          IdxT* __restrict__ arg_out) {
+// arg = nnz.  One warp per row and 32 * VEC columns, edges in CSR order, eight gathers in flight; rows above the plan's
+// threshold are cut into pieces (warps of their own, best value and position to scratch) that a last kernel compares in
+// order, which picks the same edge.  With one gather at a time and no pieces 2.5 M edges x 128 columns took 2,270 us, now
+// 259 (the gradient 500 us as a chain of tensor ops, 125 us below).
+struct MinMaxParams {
+  const void* rowptr;
+  const void* col;
+  const float* val;
+  const float* mat;
+  float* out;
+  void* arg;
+  long long M, K, nnz, long_threshold, n_items, n_long;
+  const long long* item_begin;
+  const long long* item_end;
+  const int* item_slot;
+  const int* long_row;
+  const int* long_item_ptr;
+  float* best;          // [n_items, K]
+  long long* best_arg;  // [n_items, K]
+};
+
+template <typename IdxT, int VEC, bool HAS_VAL, bool IS_MAX>
+__global__ void __launch_bounds__(128) spmm_minmax_kernel(const __grid_constant__ MinMaxParams p) {
+  constexpr int kBatch = 8;
   const int lane = threadIdx.x & 31;
-  const long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long c = (long long)blockIdx.y * 32 + lane;
-  if (r >= M) return;
-  const long long begin = (long long)rowptr[r], end = (long long)rowptr[r + 1];
-  float best = IS_MAX ? -3.402823466e+38f : 3.402823466e+38f;   // numeric_limits lowest() / max()
-  long long arg = nnz;
-  for (long long e = begin; e < end; e++) {
+  const long long unit = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;   // pieces of long rows first
+  const IdxT* __restrict__ rowptr = static_cast<const IdxT*>(p.rowptr);
+  const IdxT* __restrict__ col = static_cast<const IdxT*>(p.col);
+  const long long coff = ((long long)blockIdx.y * 32 + lane) * VEC;
+  const bool cvalid = coff < p.K;
+  const bool piece = unit < p.n_items;
+  long long begin, end, row = 0;
+  if (piece) {
+    begin = p.item_begin[unit];
+    end = p.item_end[unit];
+  } else {
+    row = unit - p.n_items;
+    if (row >= p.M) return;
+    begin = (long long)rowptr[row];
+    end = (long long)rowptr[row + 1];
+    if (p.long_threshold > 0 && end - begin > p.long_threshold) return;
+  }
+  const float* __restrict__ mat0 = p.mat + (cvalid ? coff : 0);
+  float best[VEC];
+  long long arg[VEC];
+#pragma unroll
+  for (int x = 0; x < VEC; x++) {
+    best[x] = IS_MAX ? -3.402823466e+38f : 3.402823466e+38f;   // numeric_limits lowest() / max()
+    arg[x] = p.nnz;
+  }
+  for (long long base = begin; base < end; base += 32) {
+    const long long e = base + lane < end ? base + lane : end - 1;   // past the end the last edge again: never strictly better
     const long long src = (long long)col[e];
-    if (c < K) {
-      float v = __ldg(mat + src * K + c);
-      if (HAS_VAL) v = __fmul_rn(__ldg(val + e), v);
-      if (IS_MAX ? (v > best) : (v < best)) {
-        best = v;
-        arg = e;
+    const float w = HAS_VAL ? __ldg(p.val + e) : 1.f;
+    const int cnt = end - base < 32 ? (int)(end - base) : 32;
+#pragma unroll 1
+    for (int t = 0; t < cnt; t += kBatch) {
+      float m[kBatch][VEC];
+#pragma unroll
+      for (int u = 0; u < kBatch; u++) ldg_vec<VEC>(mat0 + __shfl_sync(0xffffffffu, src, t + u) * p.K, m[u]);
+#pragma unroll
+      for (int u = 0; u < kBatch; u++) {
+        const float wu = HAS_VAL ? __shfl_sync(0xffffffffu, w, t + u) : 1.f;
+#pragma unroll
+        for (int x = 0; x < VEC; x++) {
+          const float v = HAS_VAL ? __fmul_rn(wu, m[u][x]) : m[u][x];
+          if (IS_MAX ? (v > best[x]) : (v < best[x])) {
+            best[x] = v;
+            arg[x] = base + t + u;
+          }
+        }
       }
     }
   }
-  if (c < K) {
-    out[r * K + c] = end > begin ? best : 0.f;           // reducer.cuh:78-84
-    arg_out[r * K + c] = end > begin ? (IdxT)arg : (IdxT)nnz;
+  if (!cvalid) return;
+  if (piece) {
+    const long long at = (long long)p.item_slot[unit] * p.K + coff;
+#pragma unroll
+    for (int x = 0; x < VEC; x++) {
+      p.best[at + x] = best[x];
+      p.best_arg[at + x] = arg[x];
+    }
+    return;
+  }
+  const bool any = end > begin;                                  // reducer.cuh:78-84
+  float o[VEC];
+#pragma unroll
+  for (int x = 0; x < VEC; x++) o[x] = any ? best[x] : 0.f;
+  st_vec<VEC>(p.out + row * p.K + coff, o);
+  IdxT* arg_out = static_cast<IdxT*>(p.arg) + row * p.K + coff;
+#pragma unroll
+  for (int x = 0; x < VEC; x++) arg_out[x] = (IdxT)arg[x];
+}
+
+template <typename IdxT, bool IS_MAX>
+__global__ void __launch_bounds__(128) spmm_minmax_long_kernel(const __grid_constant__ MinMaxParams p) {
+  const long long i = blockIdx.x;
+  const long long row = p.long_row[i];
+  const int s0 = p.long_item_ptr[i], s1 = p.long_item_ptr[i + 1];
+  for (long long c = threadIdx.x; c < p.K; c += blockDim.x) {
+    float best = IS_MAX ? -3.402823466e+38f : 3.402823466e+38f;
+    long long arg = p.nnz;
+    for (int s = s0; s < s1; s++) {
+      const float v = p.best[(long long)s * p.K + c];
+      if (IS_MAX ? (v > best) : (v < best)) {
+        best = v;
+        arg = p.best_arg[(long long)s * p.K + c];
+      }
+    }
+    p.out[row * p.K + c] = best;
+    static_cast<IdxT*>(p.arg)[row * p.K + c] = (IdxT)arg;
+  }
+}
+
+template <typename IdxT, int VEC, bool HAS_VAL, bool IS_MAX>
+static int launch_minmax(const MinMaxParams& p, cudaStream_t st) {
+  dim3 grid((unsigned)((p.n_items + p.M + 3) / 4), (unsigned)((p.K + 32 * VEC - 1) / (32 * VEC)));
+  spmm_minmax_kernel<IdxT, VEC, HAS_VAL, IS_MAX><<<grid, 128, 0, st>>>(p);
+  EXB_CUDA_OK(cudaGetLastError());
+  if (p.n_items > 0) {
+    spmm_minmax_long_kernel<IdxT, IS_MAX><<<(unsigned)p.n_long, 128, 0, st>>>(p);
+    EXB_CUDA_OK(cudaGetLastError());
+  }
+  return EXB_OK;
+}
+template <typename IdxT, bool HAS_VAL, bool IS_MAX>
+static int launch_minmax_vec(const MinMaxParams& p, cudaStream_t st) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p.mat) | reinterpret_cast<uintptr_t>(p.out);
+  if (p.K % 4 == 0 && a % 16 == 0) return launch_minmax<IdxT, 4, HAS_VAL, IS_MAX>(p, st);
+  if (p.K % 2 == 0 && a % 8 == 0) return launch_minmax<IdxT, 2, HAS_VAL, IS_MAX>(p, st);
+  return launch_minmax<IdxT, 1, HAS_VAL, IS_MAX>(p, st);
+}
+template <typename IdxT>
+static int launch_minmax_idx(const MinMaxParams& p, bool is_max, cudaStream_t st) {
+  if (p.val) return is_max ? launch_minmax_vec<IdxT, true, true>(p, st) : launch_minmax_vec<IdxT, true, false>(p, st);
+  return is_max ? launch_minmax_vec<IdxT, false, true>(p, st) : launch_minmax_vec<IdxT, false, false>(p, st);
+}
+
+// Gradients of the max / min aggregation, routed to the winning edges (spmm.cc:159-193, 210-241): with e = arg[r, c],
+//   grad_mat[col[e], c] += value[e] * grad[r, c],   grad_value[e] += mat[col[e], c] * grad[r, c];
+// rows without edges (e = nnz) contribute nothing.  One pass over arg and grad with reductions into zeroed outputs, where the
+// reference's chain of tensor ops reads and writes a dozen [M, K] tensors (four of them int64).  One warp per row.
+template <typename IdxT>
+__global__ void __launch_bounds__(256) spmm_minmax_bw_kernel(const IdxT* __restrict__ col, const float* __restrict__ val,
+                                                             const float* __restrict__ mat, const IdxT* __restrict__ arg,
+                                                             const float* __restrict__ grad, long long M, long long K,
+                                                             long long nnz, float* __restrict__ grad_mat,
+                                                             float* __restrict__ grad_value) {
+  constexpr int kBatch = 4;
+  const int lane = threadIdx.x & 31;
+  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < M; r += warps) {
+    for (long long c0 = lane; c0 < K; c0 += 32 * kBatch) {
+      long long e[kBatch], dst[kBatch];
+      float g[kBatch];
+#pragma unroll
+      for (int u = 0; u < kBatch; u++) {
+        const long long c = c0 + 32 * u;
+        e[u] = c < K ? (long long)arg[r * K + c] : nnz;
+        g[u] = c < K ? __ldg(grad + r * K + c) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < kBatch; u++) dst[u] = e[u] < nnz ? (long long)col[e[u]] * K + c0 + 32 * u : -1;
+#pragma unroll
+      for (int u = 0; u < kBatch; u++) {
+        if (dst[u] < 0) continue;
+        if (grad_mat) atomicAdd(grad_mat + dst[u], val ? __fmul_rn(__ldg(val + e[u]), g[u]) : g[u]);
+        if (grad_value) atomicAdd(grad_value + e[u], __fmul_rn(__ldg(mat + dst[u]), g[u]));
+      }
+    }
   }
 }
 
@@ -527,22 +833,53 @@ int exact_spmm_minmax(const void* rowptr, const void* col, int idx_bytes, const 
                       int64_t M, int64_t K, int64_t nnz, int is_max, float* out, void* arg_out, void* stream) {
   EXB_REQUIRE(idx_bytes == 4 || idx_bytes == 8, "spmm_minmax: idx_bytes must be 4 or 8 (got %d)", idx_bytes);
   EXB_REQUIRE(M >= 0 && K >= 0 && nnz >= 0, "spmm_minmax: negative shape");
+  return exact_spmm_minmax_planned(rowptr, col, idx_bytes, value, mat, M, K, nnz, is_max, 0, nullptr, nullptr, nullptr, 0, nullptr,
+                                   nullptr, 0, nullptr, out, arg_out, stream);
+}
+
+int64_t exact_spmm_minmax_scratch_bytes(int64_t n_items, int64_t K) { return n_items > 0 && K > 0 ? n_items * K * 12 : 0; }
+
+int exact_spmm_minmax_planned(const void* rowptr, const void* col, int idx_bytes, const float* value, const float* mat, int64_t M,
+                              int64_t K, int64_t nnz, int is_max, int64_t long_threshold, const int64_t* item_begin,
+                              const int64_t* item_end, const int32_t* item_slot, int64_t n_items, const int32_t* long_row,
+                              const int32_t* long_item_ptr, int64_t n_long, void* scratch, float* out, void* arg_out,
+                              void* stream) {
+  EXB_REQUIRE(idx_bytes == 4 || idx_bytes == 8, "spmm_minmax: idx_bytes must be 4 or 8 (got %d)", idx_bytes);
+  EXB_REQUIRE(M >= 0 && K >= 0 && nnz >= 0, "spmm_minmax: negative shape");
   if (M == 0 || K == 0) return EXB_OK;
   EXB_REQUIRE(rowptr && mat && out && arg_out && (nnz == 0 || col), "spmm_minmax: null pointer");
-  EXB_REQUIRE((M + 7) / 8 <= 2147483647LL && (K + 31) / 32 <= 65535, "spmm_minmax: shape too large");
-  dim3 grid((unsigned)((M + 7) / 8), (unsigned)((K + 31) / 32));
-  cudaStream_t st = (cudaStream_t)stream;
-#define EXB_MM(IDX_, HV_, MX_)                                                                                   \
-  spmm_minmax_kernel<IDX_, HV_, MX_><<<grid, 256, 0, st>>>(static_cast<const IDX_*>(rowptr), static_cast<const IDX_*>(col), \
-                                                           value, mat, M, K, nnz, out, static_cast<IDX_*>(arg_out))
-  if (idx_bytes == 4) {
-    if (value) { if (is_max) EXB_MM(int32_t, true, true); else EXB_MM(int32_t, true, false); }
-    else { if (is_max) EXB_MM(int32_t, false, true); else EXB_MM(int32_t, false, false); }
-  } else {
-    if (value) { if (is_max) EXB_MM(int64_t, true, true); else EXB_MM(int64_t, true, false); }
-    else { if (is_max) EXB_MM(int64_t, false, true); else EXB_MM(int64_t, false, false); }
-  }
-#undef EXB_MM
+  EXB_REQUIRE(n_items >= 0 && n_long >= 0 && n_items + M <= 4LL * 2147483647LL && (K + 31) / 32 <= 65535, "spmm_minmax: shape too large");
+  if (n_items > 0)
+    EXB_REQUIRE(long_threshold > 0 && item_begin && item_end && item_slot && long_row && long_item_ptr && scratch && n_long > 0 &&
+                    (reinterpret_cast<uintptr_t>(scratch) & 7) == 0,
+                "spmm_minmax: null plan array or misaligned scratch");
+  MinMaxParams p{};
+  p.rowptr = rowptr; p.col = col; p.val = value; p.mat = mat; p.out = out; p.arg = arg_out; p.M = M; p.K = K; p.nnz = nnz;
+  p.long_threshold = n_items > 0 ? long_threshold : 0;
+  p.n_items = n_items; p.n_long = n_long; p.item_begin = reinterpret_cast<const long long*>(item_begin);
+  p.item_end = reinterpret_cast<const long long*>(item_end); p.item_slot = item_slot; p.long_row = long_row;
+  p.long_item_ptr = long_item_ptr;
+  p.best_arg = static_cast<long long*>(scratch);
+  p.best = reinterpret_cast<float*>(p.best_arg + n_items * K);
+  return idx_bytes == 4 ? launch_minmax_idx<int32_t>(p, is_max != 0, (cudaStream_t)stream)
+                        : launch_minmax_idx<int64_t>(p, is_max != 0, (cudaStream_t)stream);
+}
+
+int exact_spmm_minmax_backward(const void* col, int idx_bytes, const float* value, const float* mat, const void* arg,
+                               const float* grad_out, int64_t M, int64_t K, int64_t nnz, float* grad_mat, float* grad_value,
+                               void* stream) {
+  EXB_REQUIRE(idx_bytes == 4 || idx_bytes == 8, "spmm_minmax_backward: idx_bytes must be 4 or 8 (got %d)", idx_bytes);
+  EXB_REQUIRE(M >= 0 && K >= 0 && nnz >= 0, "spmm_minmax_backward: negative shape");
+  if (M == 0 || K == 0 || (!grad_mat && !grad_value)) return EXB_OK;
+  EXB_REQUIRE(col && arg && grad_out && (!grad_value || mat), "spmm_minmax_backward: null pointer");
+  long long blocks = (M + 7) / 8;
+  if (blocks > (long long)sm_count() * 8) blocks = (long long)sm_count() * 8;
+  if (idx_bytes == 4)
+    spmm_minmax_bw_kernel<int32_t><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
+        static_cast<const int32_t*>(col), value, mat, static_cast<const int32_t*>(arg), grad_out, M, K, nnz, grad_mat, grad_value);
+  else
+    spmm_minmax_bw_kernel<int64_t><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
+        static_cast<const int64_t*>(col), value, mat, static_cast<const int64_t*>(arg), grad_out, M, K, nnz, grad_mat, grad_value);
   EXB_CUDA_OK(cudaGetLastError());
   return EXB_OK;
 }
@@ -555,14 +892,14 @@ int exact_spmm_value_bw(const void* row, const void* rowptr, const void* col, in
   if (E == 0) return EXB_OK;
   EXB_REQUIRE(row && col && mat && grad && out && (reduce == EXACT_REDUCE_SUM || rowptr), "spmm_value_bw: null pointer");
   EXB_REQUIRE((E + 7) / 8 <= 2147483647LL, "spmm_value_bw: too many edges");
-  const unsigned blocks = (unsigned)((E + 7) / 8);
+  const unsigned blocks = (unsigned)((E + 127) / 128);   // four warps of 32 edges
   const int mean = reduce == EXACT_REDUCE_MEAN;
   if (idx_bytes == 4)
-    spmm_value_bw_kernel<int32_t><<<blocks, 256, 0, (cudaStream_t)stream>>>(
+    spmm_value_bw_kernel<int32_t><<<blocks, 128, 0, (cudaStream_t)stream>>>(
         static_cast<const int32_t*>(row), static_cast<const int32_t*>(rowptr), static_cast<const int32_t*>(col), mat, grad, E,
         K, mean, out);
   else
-    spmm_value_bw_kernel<int64_t><<<blocks, 256, 0, (cudaStream_t)stream>>>(
+    spmm_value_bw_kernel<int64_t><<<blocks, 128, 0, (cudaStream_t)stream>>>(
         static_cast<const int64_t*>(row), static_cast<const int64_t*>(rowptr), static_cast<const int64_t*>(col), mat, grad, E,
         K, mean, out);
   EXB_CUDA_OK(cudaGetLastError());

@@ -85,13 +85,14 @@ class SparseStorage:
         return out
 
 
-    def native_graph(self, reduce):
+    def native_graph(self, reduce, weighted=False):
         """The adjacency with its transpose and row plans for the layers' C++ nodes (_lib.native()), cached.
-        reduce = None: without the transpose (evaluation)."""
+        reduce = None: without the transpose (evaluation, max / min).  weighted: the transpose of a mean carries its weights
+        per edge instead of leaving them to a scaling of the rows."""
         from . import _lib
         from .conf import config
         from .cpp_extension.spmm import native_plan
-        key = ("native", reduce, config.spmm_long_row)
+        key = ("native", reduce, weighted, config.spmm_long_row)
         version = None if self._value is None else self._value._version
         hit = self._t_cache.get(key)
         if hit is not None and hit[0] == version:
@@ -100,9 +101,9 @@ class SparseStorage:
         plan, transpose, inv = native_plan(self._rowptr), (None, None, None), None
         t_plan = plan
         if reduce is not None:
-            transpose = self.transposed("sum" if value is None else reduce)
+            transpose = self.transposed("sum" if value is None and not weighted else reduce)
             t_plan = native_plan(transpose[0])
-            inv = self.inverse_rowcount() if reduce == "mean" and value is None else None
+            inv = self.inverse_rowcount() if reduce == "mean" and value is None and not weighted else None
         graph = _lib.native().make_graph(self._rowptr, self._col, value, plan, *transpose, t_plan, inv)
         self._t_cache[key] = (version, graph)
         return graph

@@ -5,6 +5,7 @@ from torch.amp import custom_bwd, custom_fwd
 import torch.nn.functional as F
 from torch.autograd.function import Function
 
+from . import _lib
 from .conf import config
 from .cpp_extension import backward_func as ext_backward_func
 from .cpp_extension import quantization as ext_quantization
@@ -13,6 +14,9 @@ from .ops import (_rademacher, linear_backward_from_compressed, project_and_quan
                   qspmm_sum)
 from .qscheme import QScheme
 from .utils import empty_cache
+
+
+_NATIVE_REDUCE = {"sum": 0, "add": 0, "mean": 1, "max": 2, "min": 3}
 
 
 def qmatmul(src, other, reduce="sum", quantized=None, randmat=None, scheme=None):
@@ -27,6 +31,19 @@ def qmatmul(src, other, reduce="sum", quantized=None, randmat=None, scheme=None)
     rowptr, col, value = src.csr()
     has_value = value is not None
     st = src.storage
+    code = _NATIVE_REDUCE.get(reduce)
+    if (code is not None and quantized is None and other.is_cuda and other.dim() == 2 and other.dtype == torch.float32
+            and config.native_layers() and not torch.is_autocast_enabled("cuda")
+            and (not has_value or value.dtype == torch.float32)):
+        # one C++ node: the same saved tensors and noise offsets as the nodes below
+        value_rg = has_value and value.requires_grad and torch.is_grad_enabled()
+        need_t = code < 2 and other.requires_grad and torch.is_grad_enabled()
+        kept = config.kept_columns(other.size(1)) if code < 2 else 0
+        draws = (2 if kept else 1) if value_rg or code >= 2 else 0
+        return _lib.native().aggregate(other, value, st.row() if value_rg and code < 2 else None,
+                                       st.native_graph(("sum", "mean")[code] if need_t else None, weighted=need_t and code == 1),
+                                       code, value_rg, config.activation_compression_bits[0], kept, config.seed, config.take_offsets(draws),
+                                       config.row_offset, config.fused_rp)
     value_rg = has_value and value.requires_grad
     if reduce in ["sum", "add"]:
         row, csr2csc, colptr = st._row, st._csr2csc, st._colptr

@@ -185,6 +185,19 @@ EXACT_API int exact_spmm(const void* rowptr, const void* col, int idx_bytes, con
 EXACT_API int exact_spmm_minmax(const void* rowptr, const void* col, int idx_bytes, const float* value,
                                 const float* mat, int64_t M, int64_t K, int64_t nnz, int is_max, float* out,
                                 void* arg_out, void* stream);
+/* The same with a plan of the long rows (item_*, long_*: see exact_spmm_split; n_items = 0: none), whose pieces are compared in
+ * order.  scratch: exact_spmm_minmax_scratch_bytes(n_items, K) bytes, 8-byte aligned. */
+EXACT_API int64_t exact_spmm_minmax_scratch_bytes(int64_t n_items, int64_t K);
+EXACT_API int exact_spmm_minmax_planned(const void* rowptr, const void* col, int idx_bytes, const float* value, const float* mat,
+                                        int64_t M, int64_t K, int64_t nnz, int is_max, int64_t long_threshold,
+                                        const int64_t* item_begin, const int64_t* item_end, const int32_t* item_slot,
+                                        int64_t n_items, const int32_t* long_row, const int32_t* long_item_ptr,
+                                        int64_t n_long, void* scratch, float* out, void* arg_out, void* stream);
+/* Gradients of the max / min aggregation (spmm.cc:159-193, 210-241), added into grad_mat [rows of mat, K] and grad_value
+ * [nnz], which the caller has zeroed (either may be NULL; mat is read for grad_value only). */
+EXACT_API int exact_spmm_minmax_backward(const void* col, int idx_bytes, const float* value, const float* mat, const void* arg,
+                                         const float* grad_out, int64_t M, int64_t K, int64_t nnz, float* grad_mat,
+                                         float* grad_value, void* stream);
 
 /* Gradient with respect to the edge values, spmm_value_bw of spmm.cc:66-68, 125-126 (kernel
  * spmm_cuda.cu:172-209): out[e] = dot(mat[col[e], :], grad[row[e], :]), divided by max(length of row[e], 1)
