@@ -11,11 +11,15 @@
 // in one byte at (n / (8/bits)) * D + d.  An 8-row tile therefore covers whole bytes for every bit
 // width.  `tpt` threads own one tile; each thread keeps 8 rows x V chunks x VEC columns in registers,
 // so bytes are assembled thread-locally and stored VEC at a time, and the activation is read from
-// HBM exactly once.  Row min/max go through redux.sync (sub-warp groups when tpt < 32) and, when a
+// HBM exactly once.  Row min/max go through redux.sync (folded shuffles when tpt < 32) and, when a
 // tile spans several warps, a double-buffered shared-memory exchange with named barriers.  While a
 // tile is processed, the next one (a contiguous run of 8*D elements) is pulled into L2 with one
 // cp.async.bulk.prefetch.  The arithmetic uses the paired fp32 instructions of sm_100 (two elements per issue slot,
 // each rounded exactly like the scalar instruction).
+#include <cuda_fp16.h>
+
+#include <type_traits>
+
 #include "common.cuh"
 #include "exact_b200.h"
 
@@ -51,29 +55,103 @@ __device__ __forceinline__ void group_barrier(int grp, int nthreads) {
 struct TileCtx {
   long long N, D, G;
   int tpt, grp, tl, lane, lane_base;
-  unsigned gmask;
   bool multi;
+};
+
+struct HalfBits { uint16_t bits; };   // fp16 activations: the half arithmetic of the reference's half kernels (pack_f16.cu)
+
+// VEC adjacent elements of a row as loaded.  16-bit types stay packed in pairs: half the registers of the widened tile, and
+// their minimum and maximum are taken two at a time.
+template <typename InT, int VEC>
+struct Raw {
+  static constexpr int kWords = (VEC + 1) / 2;
+  uint32_t w[kWords];
+  __device__ __forceinline__ void load(const InT* p) {
+    if (VEC == 4) {
+      const uint2 t = __ldcs(reinterpret_cast<const uint2*>(p));
+      w[0] = t.x;
+      w[kWords - 1] = t.y;
+    } else if (VEC == 2) {
+      w[0] = __ldcs(reinterpret_cast<const uint32_t*>(p));
+    } else {
+      w[0] = __ldcs(reinterpret_cast<const uint16_t*>(p));
+    }
+  }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < kWords; i++) w[i] = 0u;
+  }
+  static __device__ __forceinline__ float low(uint32_t v) {
+    if (std::is_same<InT, HalfBits>::value) return __half2float(__ushort_as_half((unsigned short)v));
+    return __uint_as_float(v << 16);
+  }
+  static __device__ __forceinline__ float high(uint32_t v) {
+    if (std::is_same<InT, HalfBits>::value) return __half2float(__ushort_as_half((unsigned short)(v >> 16)));
+    return __uint_as_float(v & 0xffff0000u);
+  }
+  __device__ __forceinline__ float at(int e) const { return (e & 1) ? high(w[e >> 1]) : low(w[e >> 1]); }
+  static __device__ __forceinline__ uint32_t pair_min(uint32_t a, uint32_t b) {
+    uint32_t r;
+    if (std::is_same<InT, HalfBits>::value) asm("min.NaN.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    else asm("min.NaN.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+  }
+  static __device__ __forceinline__ uint32_t pair_max(uint32_t a, uint32_t b) {
+    uint32_t r;
+    if (std::is_same<InT, HalfBits>::value) asm("max.NaN.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    else asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+  }
+  __device__ __forceinline__ void range(float& lo, float& hi) const {
+    if (VEC == 1) {
+      const float v = low(w[0]);
+      lo = min_nan(lo, v);
+      hi = max_nan(hi, v);
+      return;
+    }
+    const uint32_t a = VEC == 4 ? pair_min(w[0], w[kWords - 1]) : w[0], b = VEC == 4 ? pair_max(w[0], w[kWords - 1]) : w[0];
+    lo = min_nan3(lo, low(a), high(a));
+    hi = max_nan3(hi, low(b), high(b));
+  }
+};
+template <int VEC>
+struct Raw<float, VEC> {
+  float v[VEC];
+  __device__ __forceinline__ void load(const float* p) { Ld<float, VEC>::load(p, v); }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int e = 0; e < VEC; e++) v[e] = 0.f;
+  }
+  __device__ __forceinline__ float at(int e) const { return v[e]; }
+  __device__ __forceinline__ void range(float& lo, float& hi) const {
+    if (VEC == 1) {
+      lo = min_nan(lo, v[0]);
+      hi = max_nan(hi, v[0]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < VEC; e += 2) {
+        lo = min_nan3(lo, v[e], v[(e + 1) % VEC]);
+        hi = max_nan3(hi, v[e], v[(e + 1) % VEC]);
+      }
+    }
+  }
 };
 
 // FULL: all 8 rows of the tile exist; one 64-bit base per chunk, rows addressed by 32-bit offsets.
 template <typename InT, int VEC, int V, bool FULL>
 __device__ __forceinline__ void load_tile(const InT* __restrict__ x, const TileCtx& c, long long tile,
                                           const long long (&col)[V], const bool (&cvalid)[V],
-                                          float (&xv)[8][V][VEC]) {
+                                          Raw<InT, VEC> (&xv)[8][V]) {
   const long long row0 = tile << 3;
-  const int rows_valid = FULL ? 8 : ((c.N - row0 >= 8) ? 8 : (int)(c.N - row0));
+  const int rows_valid = FULL ? 8 : c.N - row0 >= 8 ? 8 : c.N > row0 ? (int)(c.N - row0) : 0;
   const unsigned Du = (unsigned)c.D;
 #pragma unroll
   for (int v = 0; v < V; v++) {
     const InT* __restrict__ base = x + row0 * c.D + col[v];
 #pragma unroll
     for (int r = 0; r < 8; r++) {
-      if ((FULL || r < rows_valid) && cvalid[v]) {
-        Ld<InT, VEC>::load(base + r * Du, xv[r][v]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < VEC; e++) xv[r][v][e] = 0.f;
-      }
+      if ((FULL || r < rows_valid) && cvalid[v]) xv[r][v].load(base + r * Du);
+      else xv[r][v].clear();
     }
   }
 }
@@ -103,13 +181,45 @@ __device__ __forceinline__ uint32_t load_bytes(const uint8_t* p) {
   return __ldcs(p);
 }
 
+__device__ __forceinline__ float round_to_half(float f) { return __half2float(__float2half_rn(f)); }
+// half(half(x - min) * scale) of elements e and e + 1, widened: the paired half instructions round each result once, which is
+// what rounding the fp32 difference and product of halves to half gives (24 >= 2 * 11 + 2 digits).
+template <typename InT, int VEC>
+__device__ __forceinline__ f32x2 half_scaled(const Raw<InT, VEC>& x, int e, float mn, float sc) {
+  if constexpr (std::is_same<InT, HalfBits>::value) {
+    const uint32_t m = (uint32_t)__half_as_ushort(__float2half_rn(mn)) * 0x10001u;
+    const uint32_t s = (uint32_t)__half_as_ushort(__float2half_rn(sc)) * 0x10001u;
+    uint32_t d;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(x.w[e >> 1]), "r"(m));
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(d), "r"(s));
+    return f2_pack(__half2float(__ushort_as_half((unsigned short)d)), __half2float(__ushort_as_half((unsigned short)(d >> 16))));
+  } else {
+    return f2_pack(0.f, 0.f);
+  }
+}
+
+// (2^b - 1) / (max - min) as ops.py:39 evaluates it, reciprocal(mx - mn) * (2^b - 1), in the activation's arithmetic.
+template <typename InT>
+__device__ __forceinline__ float scale_of(float lo, float hi, float B) {
+  if (std::is_same<InT, HalfBits>::value)
+    return round_to_half(__fmul_rn(round_to_half(__fdiv_rn(1.0f, round_to_half(__fsub_rn(hi, lo)))), B));
+  return __fmul_rn(__frcp_rn(__fsub_rn(hi, lo)), B);
+}
+// How the statistics are stored: bf16 for fp32 and bf16 activations, fp16 for fp16 ones (ops.py:80-83).
+template <typename InT>
+__device__ __forceinline__ uint16_t stat_bits(float f) {
+  if (std::is_same<InT, HalfBits>::value) return __half_as_ushort(__float2half_rn(f));
+  return f32_to_bf16_bits(f);
+}
+
 // Quantise the 8 x (V*VEC) register tile with stochastic rounding and assemble the packed bytes.
 // MAGIC (only with FAST, and only when every scale of the tile is a finite non-zero number): the
 // rounding is done by adding 1.5 * 2^23, the code being the low byte of the sum.
 template <typename InT, int BITS, int VEC, int V, bool FAST, bool MAGIC>
 __device__ __forceinline__ void quantize_rows(const PackParams& p, const TileCtx& c, long long tile, int rows_valid,
                                               const long long (&col)[V], const bool (&cvalid)[V],
-                                              float (&xv)[8][V][VEC], const float (&mn)[8], const float (&sc)[8]) {
+                                              const Raw<InT, VEC> (&xv)[8][V], const float (&mn)[8], const float (&sc)[8]) {
+  constexpr bool HALF = std::is_same<InT, HalfBits>::value;
   constexpr int WPT = 8 / BITS;
   constexpr int GPT = BITS;
   const long long row0 = tile << 3;
@@ -127,6 +237,11 @@ __device__ __forceinline__ void quantize_rows(const PackParams& p, const TileCtx
     uint32_t acc[GPT];
 #pragma unroll
     for (int g = 0; g < GPT; g++) acc[g] = 0u;
+    // MAGIC and fp32 arithmetic: with Philox noise (at most 1 - 2^-9) no code exceeds 2^bits - 1, so the rows of a byte may be
+    // added instead of masked and OR-ed, on the floats' bit patterns (the exponent's share of the sum lies above the low
+    // byte): one multiply-add per element instead of 1.25 permutes, shifts and masks.
+    constexpr bool SUM = MAGIC && !HALF && VEC >= 2;
+    uint32_t sum[VEC];
 
     // One Philox block per 8-row tile and PAIR of columns: its 16 bytes are the noise of rows 0..7 of the
     // even and the odd column (byte 2 r + (column & 1)), 8 bits per element: u = (h + 0.5) / 256.
@@ -163,8 +278,14 @@ __device__ __forceinline__ void quantize_rows(const PackParams& p, const TileCtx
               const float f1 = u8_to_1p(w[e >> 1][r >> 1], (r & 1) * 2 + 1);
               u2 = noise8_to_unit(f2_pack(f0, f1));
             }
-            const f32x2 a2 = f2_sub(f2_pack(xv[r][v][e], xv[r][v][(e + 1) % VEC]), mn2);
-            f32x2 t2 = f2_add(f2_fma(a2, sc2, u2), neg_half);
+            f32x2 t2;
+            if (HALF) {
+              // Half (op) Half rounded to half each time, then fp32 (quantization_cuda_kernel.cu:89 on c10::Half)
+              t2 = f2_add(f2_add(half_scaled(xv[r][v], e, mn[r], sc[r]), u2), neg_half);
+            } else {
+              const f32x2 a2 = f2_sub(f2_pack(xv[r][v].at(e), xv[r][v].at((e + 1) % VEC)), mn2);
+              t2 = f2_add(f2_fma(a2, sc2, u2), neg_half);
+            }
             float t0, t1;
             if (MAGIC) {
               t2 = f2_add(t2, magic);
@@ -180,8 +301,17 @@ __device__ __forceinline__ void quantize_rows(const PackParams& p, const TileCtx
         } else {
           const float u = (!FAST && nbase != nullptr) ? un[0]
                           : noise8_to_unit(u8_to_1p(w[0][r >> 1], (r & 1) * 2 + odd));
-          const float t = __fsub_rn(__fmaf_rn(__fsub_rn(xv[r][v][0], mn[r]), sc[r], u), 0.5f);
+          const float x0 = xv[r][v].at(0);
+          const float t = HALF ? __fsub_rn(__fadd_rn(round_to_half(__fmul_rn(round_to_half(__fsub_rn(x0, mn[r])), sc[r])), u), 0.5f)
+                               : __fsub_rn(__fmaf_rn(__fsub_rn(x0, mn[r]), sc[r], u), 0.5f);
           code[0] = __float2uint_rn(t) & 0xffu;
+        }
+        if (SUM) {
+#pragma unroll
+          for (int e = 0; e < VEC; e++)
+            sum[e] = r % WPT == 0 ? code[e] : sum[e] + code[e] * (1u << ((r % WPT) * BITS));
+          if (r % WPT == WPT - 1) acc[r / WPT] = bytes_of<VEC>(sum);
+          continue;
         }
         const uint32_t word = bytes_of<VEC>(code);
         constexpr uint32_t kOnes = 0x01010101u;
@@ -199,16 +329,48 @@ __device__ __forceinline__ void quantize_rows(const PackParams& p, const TileCtx
   }
 }
 
+// Minimum over the lanes of a tile of 8 or 16 lanes of the eight lo[] and the eight hi[] (maxima negated: a negation is exact,
+// and -min(-a, -b) treats NaN and signed zeros as max does), folded: at each level a lane keeps the half of the values that
+// one bit of its index names and hands the other half over, so 16 reductions take 14 or 15 shuffles.  redux.sync takes one
+// value per instruction, once per tile of the warp: 64 columns (two tiles a warp) 179 us against 113 us for 128 columns and
+// the same 128 M elements; 125 us with the folded shuffles (which at one tile a warp lose to redux, 125 against 113 us).
+// tpt = 16: lane l of the tile ends with row l & 7 (maximum for l >= 8) in v0; 8: rows 2 (l & 3) in v0 and 2 (l & 3) + 1 in
+// v1 (l >= 4).  All lanes of the warp take part.
+__device__ __forceinline__ void reduce_rows(const float (&lo)[8], const float (&hi)[8], int tpt, int lane, float& v0, float& v1) {
+  float v[8];
+  int h = tpt >> 1;
+  bool upper = (lane & h) != 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) v[i] = min_nan(upper ? -hi[i] : lo[i], __shfl_xor_sync(0xffffffffu, upper ? lo[i] : -hi[i], h));
+  h >>= 1;
+  upper = (lane & h) != 0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) v[i] = min_nan(upper ? v[i + 4] : v[i], __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + 4], h));
+  h >>= 1;
+  upper = (lane & h) != 0;
+#pragma unroll
+  for (int i = 0; i < 2; i++) v[i] = min_nan(upper ? v[i + 2] : v[i], __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + 2], h));
+  v0 = v[0];
+  v1 = v[1];
+  if (tpt > 8) {
+    h >>= 1;
+    upper = (lane & h) != 0;
+    v0 = min_nan(upper ? v[1] : v[0], __shfl_xor_sync(0xffffffffu, upper ? v[0] : v[1], h));
+  }
+}
+
+enum TileKind { TILE_SUB = 0, TILE_WARP = 1, TILE_MULTI = 2 };   // threads per tile: 8 or 16, 32, several warps
+
 // FAST: the tile has all 8 rows and the noise is drawn from Philox.  Then there is no per-row
 // validity test, and -- when all 8 scales are finite and non-zero, i.e. no row is constant or holds
 // an infinity or a NaN -- round-to-nearest-even is done by adding 1.5 * 2^23 (the code is then the
 // low byte of the float) instead of a float->int conversion.
-template <typename InT, int BITS, int VEC, int V, bool FAST>
+template <typename InT, int BITS, int VEC, int V, int KIND, bool FAST>
 __device__ __forceinline__ bool process_tile(const PackParams& p, const TileCtx& c, long long tile, int it,
                                              const long long (&col)[V], const bool (&cvalid)[V],
-                                             float (&xv)[8][V][VEC], float* s_part, float* s_fin) {
+                                             const Raw<InT, VEC> (&xv)[8][V], float* s_part, float* s_fin) {
   const long long row0 = tile << 3;
-  const int rows_valid = FAST ? 8 : ((c.N - row0 >= 8) ? 8 : (int)(c.N - row0));
+  const int rows_valid = FAST ? 8 : c.N - row0 >= 8 ? 8 : c.N > row0 ? (int)(c.N - row0) : 0;   // 0: past the end, with its warp
   const float B = (float)((1 << BITS) - 1);
 
   // ---- row statistics ----------------------------------------------------------------------------
@@ -218,41 +380,64 @@ __device__ __forceinline__ bool process_tile(const PackParams& p, const TileCtx&
     lo[r] = __int_as_float(0x7f800000);
     hi[r] = __int_as_float(0xff800000);
 #pragma unroll
-    for (int v = 0; v < V; v++) {
-      if (cvalid[v]) {
-#pragma unroll
-        for (int e = 0; e < VEC; e++) {
-          lo[r] = min_nan(lo[r], xv[r][v][e]);
-          hi[r] = max_nan(hi[r], xv[r][v][e]);
-        }
-      }
+    for (int v = 0; v < V; v++)
+      if (cvalid[v]) xv[r][v].range(lo[r], hi[r]);
+    if (KIND != TILE_SUB) {
+      lo[r] = redux_min_nan(lo[r], 0xffffffffu);
+      hi[r] = redux_max_nan(hi[r], 0xffffffffu);
     }
-    lo[r] = redux_min_nan(lo[r], c.gmask);
-    hi[r] = redux_max_nan(hi[r], c.gmask);
   }
   bool finite = true;  // all 8 scales are finite numbers (warp-uniform)
-  if (!c.multi) {
-    // lane (tl & 7) turns row (tl & 7)'s range into a scale, then the group shares the 8 scales.
-    const int my = c.tl & 7;
-    float lo_my = lo[0], hi_my = hi[0];
-#pragma unroll
-    for (int r = 1; r < 8; r++) {
-      lo_my = (my == r) ? lo[r] : lo_my;
-      hi_my = (my == r) ? hi[r] : hi_my;
-    }
-    // ops.py:39 evaluates (2^b - 1) / (mx - mn) as reciprocal(mx - mn) * (2^b - 1).
-    const float s_my = __fmul_rn(__frcp_rn(__fsub_rn(hi_my, lo_my)), B);
+  if (KIND != TILE_MULTI) {
+    const float inf = __int_as_float(0x7f800000);
     // 0 < s < inf  <=>  the row's range is a finite non-zero number, hence every x in it is finite
-    if (FAST) finite = __all_sync(c.gmask, s_my > 0.f && s_my < __int_as_float(0x7f800000));
+    if (KIND == TILE_WARP) {
+      // lane (tl & 7) turns row (tl & 7)'s range into a scale, then the group shares the 8 scales.
+      const int my = c.tl & 7;
+      float lo_my = lo[0], hi_my = hi[0];
 #pragma unroll
-    for (int r = 0; r < 8; r++) {
-      sc[r] = __shfl_sync(c.gmask, s_my, c.lane_base + r);
-      mn[r] = lo[r];
+      for (int r = 1; r < 8; r++) {
+        lo_my = (my == r) ? lo[r] : lo_my;
+        hi_my = (my == r) ? hi[r] : hi_my;
+      }
+      const float s_my = scale_of<InT>(lo_my, hi_my, B);
+      if (FAST) finite = __all_sync(0xffffffffu, s_my > 0.f && s_my < inf);
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        sc[r] = __shfl_sync(0xffffffffu, s_my, r);
+        mn[r] = lo[r];
+      }
+    } else {
+      float v0, v1;
+      reduce_rows(lo, hi, c.tpt, c.lane, v0, v1);
+      const int half = c.tpt >> 1;                             // the lane's partner across `half` holds the other extreme
+      const float o0 = __shfl_xor_sync(0xffffffffu, v0, half), o1 = c.tpt == 8 ? __shfl_xor_sync(0xffffffffu, v1, half) : 0.f;
+      const bool holds_max = (c.tl & half) != 0;
+      const float lo0 = holds_max ? o0 : v0, s0 = scale_of<InT>(lo0, -(holds_max ? v0 : o0), B);
+      float lo1 = 0.f, s1 = 1.f;
+      if (c.tpt == 8) {
+        lo1 = holds_max ? o1 : v1;
+        s1 = scale_of<InT>(lo1, -(holds_max ? v1 : o1), B);
+      }
+      if (FAST) finite = __all_sync(0xffffffffu, s0 > 0.f && s0 < inf && s1 > 0.f && s1 < inf);
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        const int from = c.lane_base + (c.tpt == 8 ? r >> 1 : r);
+        mn[r] = __shfl_sync(0xffffffffu, c.tpt == 8 && (r & 1) ? lo1 : lo0, from);
+        sc[r] = __shfl_sync(0xffffffffu, c.tpt == 8 && (r & 1) ? s1 : s0, from);
+      }
     }
-    if (c.tl < rows_valid) {  // tl < 8 here because rows_valid <= 8
+    // lane tl < 8 of the tile writes row tl's statistics
+    if (c.tl < rows_valid) {
+      float s_my = sc[0], lo_my = mn[0];
+#pragma unroll
+      for (int r = 1; r < 8; r++) {
+        s_my = (c.tl == r) ? sc[r] : s_my;
+        lo_my = (c.tl == r) ? mn[r] : lo_my;
+      }
       const long long row = row0 + c.tl;
-      if (p.scale_bf16) p.scale_bf16[row] = f32_to_bf16_bits(s_my);
-      if (p.min_bf16) p.min_bf16[row] = f32_to_bf16_bits(lo_my);
+      if (p.scale_bf16) p.scale_bf16[row] = stat_bits<InT>(s_my);
+      if (p.min_bf16) p.min_bf16[row] = stat_bits<InT>(lo_my);
       if (p.scale_f32) p.scale_f32[row] = s_my;
       if (p.min_f32) p.min_f32[row] = lo_my;
     }
@@ -275,13 +460,13 @@ __device__ __forceinline__ bool process_tile(const PackParams& p, const TileCtx&
         lo_f = min_nan(lo_f, part[w * 16 + c.tl]);
         hi_f = max_nan(hi_f, part[w * 16 + 8 + c.tl]);
       }
-      const float s_f = __fmul_rn(__frcp_rn(__fsub_rn(hi_f, lo_f)), B);
+      const float s_f = scale_of<InT>(lo_f, hi_f, B);
       fin[c.tl] = lo_f;
       fin[8 + c.tl] = s_f;
       if (c.tl < rows_valid) {
         const long long row = row0 + c.tl;
-        if (p.scale_bf16) p.scale_bf16[row] = f32_to_bf16_bits(s_f);
-        if (p.min_bf16) p.min_bf16[row] = f32_to_bf16_bits(lo_f);
+        if (p.scale_bf16) p.scale_bf16[row] = stat_bits<InT>(s_f);
+        if (p.min_bf16) p.min_bf16[row] = stat_bits<InT>(lo_f);
         if (p.scale_f32) p.scale_f32[row] = s_f;
         if (p.min_f32) p.min_f32[row] = lo_f;
       }
@@ -318,8 +503,8 @@ __device__ __forceinline__ bool process_tile(const PackParams& p, const TileCtx&
   return true;
 }
 
-template <typename InT, int BITS, int VEC, int V>
-__global__ void __launch_bounds__(256)
+template <typename InT, int BITS, int VEC, int V, int KIND>
+__global__ void __launch_bounds__(256, KIND == TILE_MULTI && V == 2 && VEC <= 2 ? 3 : 1)
 quantize_pack_kernel(const __grid_constant__ PackParams p) {
   constexpr int WPT = 8 / BITS;
   __shared__ float s_part[2 * kMaxGroupsPerCta * kMaxWarpsPerTile * 16];
@@ -333,7 +518,6 @@ quantize_pack_kernel(const __grid_constant__ PackParams p) {
   c.tl = threadIdx.x - c.grp * c.tpt;
   c.lane = threadIdx.x & 31;
   c.lane_base = (c.tpt < 32) ? (c.lane / c.tpt) * c.tpt : 0;
-  c.gmask = (c.tpt < 32) ? (((1u << c.tpt) - 1u) << c.lane_base) : 0xffffffffu;
   c.multi = c.tpt > 32;
   const int tiles_per_cta = blockDim.x / c.tpt;
   const long long num_tiles = (p.N + 7) >> 3;
@@ -355,23 +539,26 @@ quantize_pack_kernel(const __grid_constant__ PackParams p) {
   const long long tile_bytes = 8 * p.D * (long long)sizeof(InT);
   const bool can_prefetch = (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 && (tile_bytes & 15) == 0;
   const bool philox = p.noise == nullptr;
-  float xv[8][V][VEC];
+  Raw<InT, VEC> xv[8][V];
   int it = 0;
-  for (long long tile = (long long)blockIdx.x * tiles_per_cta + c.grp; tile < num_tiles; tile += stride, ++it) {
+  // The tiles of a warp (several when tpt < 32) go through the loop together, past the end and on the general path too: the
+  // shuffles below always have all lanes.
+  const int in_warp = KIND == TILE_SUB ? c.lane / c.tpt : 0, last_in_warp = KIND == TILE_SUB ? 32 / c.tpt - 1 : 0;
+  for (long long tile = (long long)blockIdx.x * tiles_per_cta + c.grp; tile - in_warp < num_tiles; tile += stride, ++it) {
     const long long next = tile + stride;
     if (c.tl == 0 && can_prefetch && next < full_tiles) {  // never the ragged last tile
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(x + (next << 3) * p.D), "r"((uint32_t)tile_bytes)
                    : "memory");
     }
     bool done = false;
-    if (philox && tile < full_tiles) {
+    if (philox && tile - in_warp + last_in_warp < full_tiles) {
       load_tile<InT, VEC, V, true>(x, c, tile, col, cvalid, xv);
-      done = process_tile<InT, BITS, VEC, V, true>(p, c, tile, it, col, cvalid, xv, s_part, s_fin);
+      done = process_tile<InT, BITS, VEC, V, KIND, true>(p, c, tile, it, col, cvalid, xv, s_part, s_fin);
       if (!done) ++it;  // the redo below exchanges its statistics through the other shared-memory buffer
     }
     if (!done) {
       load_tile<InT, VEC, V, false>(x, c, tile, col, cvalid, xv);
-      process_tile<InT, BITS, VEC, V, false>(p, c, tile, it, col, cvalid, xv, s_part, s_fin);
+      process_tile<InT, BITS, VEC, V, KIND, false>(p, c, tile, it, col, cvalid, xv, s_part, s_fin);
     }
   }
 }
@@ -427,11 +614,24 @@ struct UnpackParams {
   const uint8_t* packed;
   const void* scale;  // [N] fp32 or bf16 bits
   const void* mn;     // [N]
-  float* out;         // [N, D]
+  void* out;          // [N, D], fp32 (fp16 with fp16 statistics)
   long long N, D;
   int tpt;
   int vec_stats;  // 1: scale/min are 16-byte aligned, whole-tile vector loads are legal
 };
+
+template <int VEC>
+__device__ __forceinline__ void store_halves(__half* p, const float (&o)[VEC]) {
+  if (VEC == 4) {
+    const __half2 a = __floats2half2_rn(o[0], o[1 % VEC]), b = __floats2half2_rn(o[2 % VEC], o[3 % VEC]);
+    __stcs(reinterpret_cast<uint2*>(p), make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b)));
+  } else if (VEC == 2) {
+    const __half2 a = __floats2half2_rn(o[0], o[1 % VEC]);
+    __stcs(reinterpret_cast<uint32_t*>(p), *reinterpret_cast<const uint32_t*>(&a));
+  } else {
+    *p = __float2half_rn(o[0]);
+  }
+}
 
 // code / s by the Markstein sequence q0 = c*r, rem = fma(-q0, s, c), q = fma(rem, r, q0) with r the
 // correctly rounded reciprocal of s: equal to the IEEE quotient for every code 0..255 and every normal
@@ -442,9 +642,12 @@ __device__ __forceinline__ bool scale_is_tame(float s) {
   return e >= 27u && e <= 227u;
 }
 
-template <int BITS, int VEC, int V, bool STATS_BF16>
+// STATS: 0 fp32, 1 bf16 (fp32 result), 2 fp16 (fp16 result, every step rounded to half: quantization_cuda_kernel.cu:182 on
+// c10::Half).
+template <int BITS, int VEC, int V, int STATS>
 __global__ void __launch_bounds__(256)
 unpack_dequant_kernel(const __grid_constant__ UnpackParams p) {
+  constexpr bool STATS_BF16 = STATS == 1, HALF = STATS == 2;
   constexpr int WPT = 8 / BITS;
   constexpr int GPT = BITS;
   constexpr uint32_t MASKREP = 0x01010101u * ((1u << BITS) - 1u);
@@ -483,17 +686,18 @@ unpack_dequant_kernel(const __grid_constant__ UnpackParams p) {
 
     float s[8], m[8];
     if (rows_valid == 8 && p.vec_stats) {
-      if (STATS_BF16) {
+      if (STATS_BF16 || HALF) {
         const uint4 sv = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.scale) + row0));
         const uint4 mv = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.mn) + row0));
         const uint32_t sw[4] = {sv.x, sv.y, sv.z, sv.w};
         const uint32_t mw[4] = {mv.x, mv.y, mv.z, mv.w};
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-          s[2 * i] = __uint_as_float(sw[i] << 16);
-          s[2 * i + 1] = __uint_as_float(sw[i] & 0xffff0000u);
-          m[2 * i] = __uint_as_float(mw[i] << 16);
-          m[2 * i + 1] = __uint_as_float(mw[i] & 0xffff0000u);
+          using Stat = Raw<typename std::conditional<HALF, HalfBits, uint16_t>::type, 2>;
+          s[2 * i] = Stat::low(sw[i]);
+          s[2 * i + 1] = Stat::high(sw[i]);
+          m[2 * i] = Stat::low(mw[i]);
+          m[2 * i + 1] = Stat::high(mw[i]);
         }
       } else {
         const float4* sp = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.scale) + row0);
@@ -506,9 +710,10 @@ unpack_dequant_kernel(const __grid_constant__ UnpackParams p) {
 #pragma unroll
       for (int r = 0; r < 8; r++) {
         if (r < rows_valid) {
-          if (STATS_BF16) {
-            s[r] = bf16_bits_to_f32(__ldg(reinterpret_cast<const uint16_t*>(p.scale) + row0 + r));
-            m[r] = bf16_bits_to_f32(__ldg(reinterpret_cast<const uint16_t*>(p.mn) + row0 + r));
+          if (STATS_BF16 || HALF) {
+            using Stat = Raw<typename std::conditional<HALF, HalfBits, uint16_t>::type, 1>;
+            s[r] = Stat::low(__ldg(reinterpret_cast<const uint16_t*>(p.scale) + row0 + r));
+            m[r] = Stat::low(__ldg(reinterpret_cast<const uint16_t*>(p.mn) + row0 + r));
           } else {
             s[r] = __ldg(reinterpret_cast<const float*>(p.scale) + row0 + r);
             m[r] = __ldg(reinterpret_cast<const float*>(p.mn) + row0 + r);
@@ -553,16 +758,91 @@ unpack_dequant_kernel(const __grid_constant__ UnpackParams p) {
                 const f32x2 q0 = f2_mul(c2, r2);
                 const f32x2 rem = f2_fma(q0, ns2, c2);
                 const f32x2 q = f2_fma(rem, r2, q0);
-                f2_unpack(f2_add(q, m2), o[e], o[(e + 1) % VEC]);
+                if (HALF) {
+                  float q0r, q1r;
+                  f2_unpack(q, q0r, q1r);
+                  f2_unpack(f2_add(f2_pack(round_to_half(q0r), round_to_half(q1r)), m2), o[e], o[(e + 1) % VEC]);
+                } else {
+                  f2_unpack(f2_add(q, m2), o[e], o[(e + 1) % VEC]);
+                }
               }
             } else {
 #pragma unroll
               for (int e = 0; e < VEC; e++)  // quantization_cuda_kernel.cu:182: IEEE division, then addition
-                o[e] = __fadd_rn(__fdiv_rn(__fsub_rn(cf[e], 8388608.f), s[r]), m[r]);
+              {
+                const float q = __fdiv_rn(__fsub_rn(cf[e], 8388608.f), s[r]);
+                o[e] = __fadd_rn(HALF ? round_to_half(q) : q, m[r]);
+              }
             }
-            StF32<VEC>::store(p.out + (row0 + r) * D + col[v], o);
+            if (HALF) store_halves<VEC>(static_cast<__half*>(p.out) + (row0 + r) * D + col[v], o);
+            else StF32<VEC>::store(static_cast<float*>(p.out) + (row0 + r) * D + col[v], o);
           }
         }
+      }
+    }
+  }
+}
+
+// Unpack + dequantise of an odd number of columns.  Rows then start on odd elements and the tiled kernel stores one element per
+// lane; here the output is one run of elements and a thread makes four adjacent ones, whatever rows they fall into, and stores
+// them together.  300,001 x 47 at INT2: 62 us in the tiled kernel (fp16 64, 42 in the plain one), 37 here.
+template <int BITS, int STATS>
+__global__ void __launch_bounds__(256) unpack_flat_kernel(const __grid_constant__ UnpackParams p) {
+  constexpr bool HALF = STATS == 2;
+  constexpr int WPT = 8 / BITS;
+  constexpr uint32_t MASK = (1u << BITS) - 1u;
+  const long long total = p.N * p.D;
+  const uint32_t D = (uint32_t)p.D;
+  for (long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i0 < total; i0 += (long long)gridDim.x * blockDim.x * 4) {
+    long long n = total < (1LL << 32) ? (long long)((uint32_t)i0 / D) : i0 / p.D;
+    uint32_t d = (uint32_t)(i0 - n * p.D);
+    float s = 1.f, m = 0.f, rcp = 1.f;
+    bool tame = true;
+    const uint8_t* src = nullptr;
+    int sh = 0;
+    auto row = [&]() {
+      if (STATS == 0) {
+        s = __ldg(reinterpret_cast<const float*>(p.scale) + n);
+        m = __ldg(reinterpret_cast<const float*>(p.mn) + n);
+      } else {
+        using Stat = Raw<typename std::conditional<HALF, HalfBits, uint16_t>::type, 1>;
+        s = Stat::low(__ldg(reinterpret_cast<const uint16_t*>(p.scale) + n));
+        m = Stat::low(__ldg(reinterpret_cast<const uint16_t*>(p.mn) + n));
+      }
+      rcp = __frcp_rn(s);
+      tame = scale_is_tame(s);
+      src = p.packed + (n / WPT) * p.D;
+      sh = (int)(n % WPT) * BITS;
+    };
+    row();
+    float o[4];
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      o[x] = 0.f;
+      if (i0 + x < total) {
+        const float c = (float)((__ldg(src + d) >> sh) & MASK);
+        float q;
+        if (tame) {
+          const float q0 = __fmul_rn(c, rcp);
+          q = __fmaf_rn(__fmaf_rn(-q0, s, c), rcp, q0);
+        } else {
+          q = __fdiv_rn(c, s);
+        }
+        o[x] = __fadd_rn(HALF ? round_to_half(q) : q, m);
+        if (++d == D && x < 3 && i0 + x + 1 < total) {
+          d = 0;
+          n++;
+          row();
+        }
+      }
+    }
+    if (i0 + 4 <= total) {
+      if (HALF) store_halves<4>(static_cast<__half*>(p.out) + i0, o);
+      else StF32<4>::store(static_cast<float*>(p.out) + i0, o);
+    } else {
+      for (int x = 0; i0 + x < total; x++) {
+        if (HALF) static_cast<__half*>(p.out)[i0 + x] = __float2half_rn(o[x]);
+        else static_cast<float*>(p.out)[i0 + x] = o[x];
       }
     }
   }
@@ -595,7 +875,7 @@ static bool choose_shape(long long D, int max_vec, TileShape* s) {
   } else if (C <= 512) {
     v = 2;
     tpt = (int)(((C + 1) / 2 + 31) / 32) * 32;
-  } else if (C <= 1024 && vec == 4) {
+  } else if (C <= 1024) {
     v = 4;
     tpt = (int)(((C + 3) / 4 + 31) / 32) * 32;
   } else {
@@ -624,18 +904,20 @@ static int launch_pack(const PackParams& p, const TileShape& s, cudaStream_t st)
   const int tiles_per_cta = s.block / s.tpt;
   const long long ctas = (tiles + tiles_per_cta - 1) / tiles_per_cta;
   int grid = 1;
-#define EXB_PACK_CASE(VEC_, V_)                                                        \
-  if (s.vec == VEC_ && s.v == V_) {                                                    \
-    auto k = quantize_pack_kernel<InT, BITS, VEC_, V_>;                                \
+  const int kind = s.tpt < 32 ? TILE_SUB : s.tpt == 32 ? TILE_WARP : TILE_MULTI;
+#define EXB_PACK_CASE(VEC_, V_, KIND_)                                                 \
+  if (s.vec == VEC_ && s.v == V_ && kind == KIND_) {                                   \
+    auto k = quantize_pack_kernel<InT, BITS, VEC_, V_, KIND_>;                         \
     int rc = persistent_grid(k, s.block, ctas, &grid);                                 \
     if (rc) return rc;                                                                 \
     k<<<grid, s.block, 0, st>>>(p);                                                    \
     EXB_CUDA_OK(cudaGetLastError());                                                   \
     return EXB_OK;                                                                     \
   }
-  EXB_PACK_CASE(4, 1) EXB_PACK_CASE(4, 2) EXB_PACK_CASE(4, 4)
-  EXB_PACK_CASE(2, 1) EXB_PACK_CASE(2, 2)
-  EXB_PACK_CASE(1, 1) EXB_PACK_CASE(1, 2)
+  EXB_PACK_CASE(4, 1, TILE_SUB) EXB_PACK_CASE(4, 1, TILE_WARP) EXB_PACK_CASE(4, 2, TILE_WARP) EXB_PACK_CASE(4, 2, TILE_MULTI)
+  EXB_PACK_CASE(4, 4, TILE_MULTI) EXB_PACK_CASE(2, 4, TILE_MULTI) EXB_PACK_CASE(1, 4, TILE_MULTI)
+  EXB_PACK_CASE(2, 1, TILE_SUB) EXB_PACK_CASE(2, 1, TILE_WARP) EXB_PACK_CASE(2, 2, TILE_WARP) EXB_PACK_CASE(2, 2, TILE_MULTI)
+  EXB_PACK_CASE(1, 1, TILE_SUB) EXB_PACK_CASE(1, 1, TILE_WARP) EXB_PACK_CASE(1, 2, TILE_WARP) EXB_PACK_CASE(1, 2, TILE_MULTI)
 #undef EXB_PACK_CASE
   return fail(EXB_ERR_UNSUPPORTED, "no pack kernel for vec=%d v=%d", s.vec, s.v);
 }
@@ -674,13 +956,15 @@ static int align_vec(const void* ptr, int elem_bytes) {
   return 1;
 }
 
+constexpr int kDtypeHalf = 2;   // inside the library: exact_quantize_pack_f16
+
 static int pack_common(const void* x, int dtype, long long N, long long D, int bits,
                        const float* noise, const float* mn_in, const float* scale_in,
                        unsigned long long seed, unsigned long long offset, long long row_offset,
                        uint8_t* packed, uint16_t* scale_bf16, uint16_t* min_bf16, float* scale_f32,
                        float* min_f32, cudaStream_t st) {
   EXB_REQUIRE(bits == 1 || bits == 2 || bits == 4 || bits == 8, "bits must be 1, 2, 4 or 8 (got %d)", bits);
-  EXB_REQUIRE(dtype == EXACT_DTYPE_F32 || dtype == EXACT_DTYPE_BF16,
+  EXB_REQUIRE(dtype == EXACT_DTYPE_F32 || dtype == EXACT_DTYPE_BF16 || dtype == kDtypeHalf,
               "pack: dtype must be EXACT_DTYPE_F32 or EXACT_DTYPE_BF16 (got %d)", dtype);
   EXB_REQUIRE(N >= 0 && D >= 0, "pack: negative shape %lld x %lld", N, D);
   EXB_REQUIRE(row_offset >= 0 && row_offset % 8 == 0, "pack: row_offset must be a non-negative multiple of 8");
@@ -704,13 +988,21 @@ static int pack_common(const void* x, int dtype, long long N, long long D, int b
   if (pa != 0) max_vec = (pa == 2 && max_vec >= 2) ? 2 : 1;
   TileShape s;
   if (!choose_shape(D, max_vec, &s))
-    return fail(EXB_ERR_UNSUPPORTED, "pack: D=%lld is beyond the register-tiled kernels (max 4096 when D%%4==0, 1024 when D%%2==0, 512 otherwise)", D);
+    return fail(EXB_ERR_UNSUPPORTED, "pack: D=%lld is beyond the register-tiled kernels (max 4096 when D%%4==0, 2048 when D%%2==0, 1024 otherwise)", D);
   p.tpt = s.tpt;
+  if (dtype == kDtypeHalf) return launch_pack_bits<HalfBits>(p, bits, s, st);
   if (dtype == EXACT_DTYPE_F32) return launch_pack_bits<float>(p, bits, s, st);
   return launch_pack_bits<uint16_t>(p, bits, s, st);
 }
 
-template <int BITS, bool BF>
+int quantize_pack_half(const void* x, long long N, long long D, int bits, const float* noise, unsigned long long seed,
+                       unsigned long long offset, long long row_offset, uint8_t* packed, uint16_t* scale, uint16_t* mn,
+                       cudaStream_t st) {
+  return pack_common(x, kDtypeHalf, N, D, bits, noise, nullptr, nullptr, seed, offset, row_offset, packed, scale, mn, nullptr,
+                     nullptr, st);
+}
+
+template <int BITS, int STATS>
 static int launch_unpack(const UnpackParams& p, const TileShape& s, cudaStream_t st) {
   const long long tiles = (p.N + 7) / 8;
   const int tiles_per_cta = s.block / s.tpt;
@@ -718,7 +1010,7 @@ static int launch_unpack(const UnpackParams& p, const TileShape& s, cudaStream_t
   int grid = 1;
 #define EXB_UNPACK_CASE(VEC_, V_)                                                      \
   if (s.vec == VEC_ && s.v == V_) {                                                    \
-    auto k = unpack_dequant_kernel<BITS, VEC_, V_, BF>;                                \
+    auto k = unpack_dequant_kernel<BITS, VEC_, V_, STATS>;                                \
     int rc = persistent_grid(k, s.block, ctas, &grid);                                 \
     if (rc) return rc;                                                                 \
     k<<<grid, s.block, 0, st>>>(p);                                                    \
@@ -726,10 +1018,63 @@ static int launch_unpack(const UnpackParams& p, const TileShape& s, cudaStream_t
     return EXB_OK;                                                                     \
   }
   EXB_UNPACK_CASE(4, 1) EXB_UNPACK_CASE(4, 2) EXB_UNPACK_CASE(4, 4)
-  EXB_UNPACK_CASE(2, 1) EXB_UNPACK_CASE(2, 2)
-  EXB_UNPACK_CASE(1, 1) EXB_UNPACK_CASE(1, 2)
+  EXB_UNPACK_CASE(2, 1) EXB_UNPACK_CASE(2, 2) EXB_UNPACK_CASE(2, 4)
+  EXB_UNPACK_CASE(1, 1) EXB_UNPACK_CASE(1, 2) EXB_UNPACK_CASE(1, 4)
 #undef EXB_UNPACK_CASE
   return fail(EXB_ERR_UNSUPPORTED, "no unpack kernel for vec=%d v=%d", s.vec, s.v);
+}
+
+// stats: the STATS of the kernel
+static int unpack_common(const uint8_t* packed, int bits, const void* scale, const void* min, int stats, long long N, long long D,
+                         void* out, cudaStream_t st) {
+  EXB_REQUIRE(bits == 1 || bits == 2 || bits == 4 || bits == 8, "bits must be 1, 2, 4 or 8 (got %d)", bits);
+  EXB_REQUIRE(N >= 0 && D >= 0, "unpack: negative shape");
+  if (N == 0 || D == 0) return EXB_OK;
+  EXB_REQUIRE(packed && scale && min && out, "unpack: null pointer");
+  int max_vec = align_vec(out, stats == 2 ? 2 : 4);
+  if (D % 2 != 0 && max_vec == 4 && D < (1LL << 31)) {
+    UnpackParams p{};
+    p.packed = packed; p.scale = scale; p.mn = min; p.out = out; p.N = N; p.D = D;
+    long long blocks = (N * D + 1023) / 1024;
+    if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
+#define EXB_FLAT(BITS_)                                                                                        \
+  if (stats == 2) unpack_flat_kernel<BITS_, 2><<<(int)blocks, 256, 0, st>>>(p);                                \
+  else if (stats == 1) unpack_flat_kernel<BITS_, 1><<<(int)blocks, 256, 0, st>>>(p);                           \
+  else unpack_flat_kernel<BITS_, 0><<<(int)blocks, 256, 0, st>>>(p);                                           \
+  break
+    switch (bits) {
+      case 1: EXB_FLAT(1);
+      case 2: EXB_FLAT(2);
+      case 4: EXB_FLAT(4);
+      default: EXB_FLAT(8);
+    }
+#undef EXB_FLAT
+    EXB_CUDA_OK(cudaGetLastError());
+    return EXB_OK;
+  }
+  const int pa = (int)(reinterpret_cast<uintptr_t>(packed) & 3);
+  if (pa != 0) max_vec = (pa == 2 && max_vec >= 2) ? 2 : 1;
+  TileShape s;
+  if (!choose_shape(D, max_vec, &s))
+    return fail(EXB_ERR_UNSUPPORTED, "unpack: D=%lld is beyond the register-tiled kernels", D);
+  UnpackParams p;
+  p.packed = packed; p.scale = scale; p.mn = min; p.out = out; p.N = N; p.D = D; p.tpt = s.tpt;
+  p.vec_stats = (reinterpret_cast<uintptr_t>(scale) % 16 == 0 && reinterpret_cast<uintptr_t>(min) % 16 == 0) ? 1 : 0;
+#define EXB_UNPACK_STATS(BITS_)                                                                             \
+  return stats == 2 ? launch_unpack<BITS_, 2>(p, s, st) : stats == 1 ? launch_unpack<BITS_, 1>(p, s, st)    \
+                                                                     : launch_unpack<BITS_, 0>(p, s, st)
+  switch (bits) {
+    case 1: EXB_UNPACK_STATS(1);
+    case 2: EXB_UNPACK_STATS(2);
+    case 4: EXB_UNPACK_STATS(4);
+    default: EXB_UNPACK_STATS(8);
+  }
+#undef EXB_UNPACK_STATS
+}
+
+int unpack_half(const uint8_t* packed, int bits, const void* scale, const void* min, long long N, long long D, void* out,
+                cudaStream_t st) {
+  return unpack_common(packed, bits, scale, min, 2, N, D, out, st);
 }
 
 }  // namespace exb
@@ -756,29 +1101,9 @@ int exact_pack_single_precision(const void* data, int dtype, const float* min, c
 
 int exact_unpack_single_precision(const uint8_t* packed, int bits, const void* scale, const void* min,
                                   int stats_dtype, int64_t N, int64_t D, float* out, void* stream) {
-  EXB_REQUIRE(bits == 1 || bits == 2 || bits == 4 || bits == 8, "bits must be 1, 2, 4 or 8 (got %d)", bits);
   EXB_REQUIRE(stats_dtype == EXACT_DTYPE_F32 || stats_dtype == EXACT_DTYPE_BF16,
               "unpack: scale/min dtype must be EXACT_DTYPE_F32 or EXACT_DTYPE_BF16 (got %d)", stats_dtype);
-  EXB_REQUIRE(N >= 0 && D >= 0, "unpack: negative shape");
-  if (N == 0 || D == 0) return EXB_OK;
-  EXB_REQUIRE(packed && scale && min && out, "unpack: null pointer");
-  int max_vec = align_vec(out, 4);
-  const int pa = (int)(reinterpret_cast<uintptr_t>(packed) & 3);
-  if (pa != 0) max_vec = (pa == 2 && max_vec >= 2) ? 2 : 1;
-  TileShape s;
-  if (!choose_shape(D, max_vec, &s))
-    return fail(EXB_ERR_UNSUPPORTED, "unpack: D=%lld is beyond the register-tiled kernels", (long long)D);
-  UnpackParams p;
-  p.packed = packed; p.scale = scale; p.mn = min; p.out = out; p.N = N; p.D = D; p.tpt = s.tpt;
-  p.vec_stats = (reinterpret_cast<uintptr_t>(scale) % 16 == 0 && reinterpret_cast<uintptr_t>(min) % 16 == 0) ? 1 : 0;
-  cudaStream_t st = (cudaStream_t)stream;
-  const bool bf = stats_dtype == EXACT_DTYPE_BF16;
-  switch (bits) {
-    case 1: return bf ? launch_unpack<1, true>(p, s, st) : launch_unpack<1, false>(p, s, st);
-    case 2: return bf ? launch_unpack<2, true>(p, s, st) : launch_unpack<2, false>(p, s, st);
-    case 4: return bf ? launch_unpack<4, true>(p, s, st) : launch_unpack<4, false>(p, s, st);
-    default: return bf ? launch_unpack<8, true>(p, s, st) : launch_unpack<8, false>(p, s, st);
-  }
+  return unpack_common(packed, bits, scale, min, stats_dtype == EXACT_DTYPE_BF16 ? 1 : 0, N, D, out, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -9,14 +9,23 @@
 // and the row statistics of an fp16 activation stay fp16 (exact/exact/ops.py:82-83): min = min_d x,
 // scale = half(float(half(1 / float(half(max - min)))) * (2^bits - 1)), the half ops of torch behind
 // `(2 ** bits - 1) / (mx - mn)` (ops.py:39: reciprocal, then multiplication by the scalar).
-// The packed layout is that of the fp32 path.  These are plain streaming kernels (one thread per 8-row tile and
-// column, one warp per row for the statistics); the fp32 / bf16 path is the tuned one.
+// The packed layout is that of the fp32 path, and quantise + pack and unpack run on its register-tiled kernels (pack.cu) with
+// the half arithmetic above.  The plain kernels here (one thread per 8-row tile and column, one warp per row for the
+// statistics) take caller-computed statistics and the widths beyond a register tile (169,343 x 256 at INT2: statistics + pack
+// 137 us and unpack 103 us in these, 37 and 27 there).
 #include <cuda_fp16.h>
 
 #include "exact_b200.h"
 #include "common.cuh"
 
 namespace exb {
+
+// pack.cu; EXB_ERR_UNSUPPORTED for a width beyond its register tiles
+int quantize_pack_half(const void* x, long long N, long long D, int bits, const float* noise, unsigned long long seed,
+                       unsigned long long offset, long long row_offset, uint8_t* packed, uint16_t* scale, uint16_t* mn,
+                       cudaStream_t st);
+int unpack_half(const uint8_t* packed, int bits, const void* scale, const void* min, long long N, long long D, void* out,
+                cudaStream_t st);
 
 __device__ __forceinline__ float h_bits_to_f32(uint16_t b) { return __half2float(__ushort_as_half(b)); }
 __device__ __forceinline__ uint16_t f32_to_h_bits(float f) { return __half_as_ushort(__float2half_rn(f)); }
@@ -188,6 +197,8 @@ int exact_quantize_pack_f16(const void* x, int64_t N, int64_t D, int bits, const
   if (N == 0 || D == 0) return EXB_OK;
   EXB_REQUIRE(x && packed && scale_f16 && min_f16, "quantize_pack_f16: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
+  const int rc = quantize_pack_half(x, N, D, bits, noise, seed, offset, row_offset, packed, scale_f16, min_f16, st);
+  if (rc != EXB_ERR_UNSUPPORTED) return rc;
   long long blocks = (N + 7) / 8;
   const long long cap = (long long)sm_count() * 16;
   if (blocks > cap) blocks = cap;
@@ -205,6 +216,8 @@ int exact_unpack_single_precision_f16(const uint8_t* packed, int bits, const voi
   if (N == 0 || D == 0) return EXB_OK;
   EXB_REQUIRE(packed && scale && min && out, "unpack_f16: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
+  const int rc = unpack_half(packed, bits, scale, min, N, D, out, st);
+  if (rc != EXB_ERR_UNSUPPORTED) return rc;
   const int grid = f16_grid(((N + 7) / 8) * D);
   const uint16_t* s = static_cast<const uint16_t*>(scale);
   const uint16_t* m = static_cast<const uint16_t*>(min);
