@@ -71,6 +71,10 @@ SIGNATURES = {
                                    c_i64, c_ptr, c_ptr, c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr]),
     "exact_rows_scale_colsum_workspace_bytes": (c_i64, [c_i64]),
     "exact_rows_scale_colsum": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_ptr, c_i64, c_i64, c_ptr, c_ptr, c_i64, c_ptr]),
+    "exact_bn_forward_workspace_bytes": (c_i64, [c_i64]),
+    "exact_bn_forward": (c_int, [c_ptr, c_i64, c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_f32, c_f32, c_ptr, c_i64, c_ptr, c_ptr, c_ptr,
+                                 c_ptr]),
+    "exact_rows_half_colsum": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_i64, c_i64, c_ptr, c_ptr, c_i64, c_ptr]),
     "exact_bn_backward_workspace_bytes": (c_i64, [c_i64]),
     "exact_bn_backward_from_packed": (c_int, [c_ptr, c_i64, c_i64, c_ptr, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_int,
                                               c_ptr, c_i64, c_ptr, c_ptr, c_ptr, c_ptr]),

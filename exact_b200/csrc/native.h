@@ -39,7 +39,7 @@ struct LibraryError : std::runtime_error {   // becomes exact_b200.ExactB200Erro
   X(exact_act_quantized_dropout_backward) X(exact_act_quantized_relu_dropout_forward)                                 \
   X(exact_act_quantized_forward_f16) X(exact_act_quantized_backward_f16) X(exact_spmm_planned)                        \
   X(exact_spmm_f16_planned) X(exact_rows_scale_colsum_workspace_bytes)                     \
-  X(exact_rows_scale_colsum) X(exact_bn_backward_workspace_bytes) X(exact_bn_backward_from_packed)                    \
+  X(exact_rows_scale_colsum) X(exact_bn_forward_workspace_bytes) X(exact_bn_forward) X(exact_rows_half_colsum) X(exact_bn_backward_workspace_bytes) X(exact_bn_backward_from_packed)                    \
   X(exact_rp_workspace_bytes) X(exact_rp_quantize_pack) X(exact_rademacher) X(exact_grad_weight_workspace_bytes)      \
   X(exact_grad_weight_from_packed) X(exact_linear_workspace_bytes) X(exact_linear_partial_bytes) X(exact_linear_forward_strided)                            \
   X(exact_spmm_minmax_scratch_bytes) X(exact_spmm_minmax_planned) X(exact_spmm_minmax_backward)                       \
@@ -118,6 +118,12 @@ Tensor linear(const Tensor& a, const Tensor& w, const OptTensor& bias, const Opt
               const OptTensor& out, bool accumulate, int64_t k_chunk = 0);
 Tensor grad_weight(const Tensor& g, int64_t bits, const Packed& q0, int64_t k0, const Packed* q1, int64_t k1);
 std::tuple<Tensor, Tensor> rows_scale_colsum(const Tensor& g, const OptTensor& rowscale, bool want_scaled, bool want_colsum);
+// (fp16 copy of g zero-padded to whole 16-byte pieces, g.sum(0))
+std::tuple<Tensor, Tensor> rows_half_colsum(const Tensor& g, bool want_colsum);
+// (y, mean, invstd); the running statistics are moved in place
+std::tuple<Tensor, Tensor, Tensor> bn_forward(const Tensor& x, const OptTensor& weight, const OptTensor& bias,
+                                              const OptTensor& running_mean, const OptTensor& running_var, double momentum,
+                                              double eps);
 std::tuple<Tensor, Tensor, Tensor> bn_backward(const Tensor& g, const Packed& q, int64_t bits, const OptTensor& weight,
                                                const Tensor& mean, const Tensor& invstd, bool train, bool want_input,
                                                bool want_weight, bool want_bias);

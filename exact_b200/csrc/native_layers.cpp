@@ -108,7 +108,7 @@ struct GcnState : torch::CustomClassHolder {
   Saving how;
   Compressed x;
   Tensor w;            // as used by the products (half under autocast)
-  bool has_bias, half;
+  bool has_bias, half, x_half = false;
   int64_t rows;
 };
 
@@ -120,6 +120,7 @@ struct GcnNode : Function<GcnNode> {
     Tensor out;
     if (s->half) {
       // autocast: the quantised ops cast to half (ops.py:130, 260), the products are the library's half GEMMs
+      s->x_half = x.scalar_type() == at::kHalf;
       x = x.to(at::kHalf);
       w = w.to(at::kHalf);
       s->x = compress(x, s->how, s->how.offset);
@@ -142,11 +143,16 @@ struct GcnNode : Function<GcnNode> {
     Tensor g = grads[0].contiguous(), gb, gw, gx;
     const int64_t O = g.size(1);
     if (s->half) {
-      if (s->has_bias) gb = std::get<1>(rows_scale_colsum(g.to(at::kFloat), {}, false, true));
+      Tensor g16 = g;      // without a bias the output, and so its gradient, is half
+      if (g.scalar_type() == at::kFloat) {
+        auto [h, sum] = rows_half_colsum(g, s->has_bias);
+        g16 = h;           // padded with zero columns to whole 16-byte pieces
+        gb = sum;
+      }
       if (need_x || need_w) {
-        const Tensor gh = spmm(gr.bw, gr.bw.value, g.to(at::kHalf), false);
+        const Tensor gh = spmm(gr.bw, gr.bw.value, g16, false).narrow(1, 0, O);
         if (need_w) gw = weight_grad(gh, s->x, s->how.bits, s->rows).to(at::kFloat);
-        if (need_x) gx = at::mm(gh, s->w).to(at::kFloat);
+        if (need_x) gx = s->x_half ? at::mm(gh, s->w) : at::mm(gh, s->w, at::kFloat);
       }
       return {gx, gw, gb, {}};
     }
@@ -300,6 +306,42 @@ Tensor sage_node(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const
   s->projected_first = projected_first;
   s->gradient_first = gradient_first;
   return SageNode::apply(x, w_l, b_l, w_r, s);
+}
+
+// ---- batch norm: qbatch_norm (ops.py:206-254) ---------------------------------------------------------------
+struct BnState : torch::CustomClassHolder {
+  Packed x;
+  Tensor mean, invstd;
+  OptTensor weight;
+  int64_t bits;
+};
+
+struct BnNode : Function<BnNode> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x_, const OptTensor& weight, const OptTensor& bias,
+                        const OptTensor& running_mean, const OptTensor& running_var, double momentum, double eps,
+                        const c10::intrusive_ptr<BnState>& s, const Saving& how) {
+    const Tensor x = x_.contiguous();
+    s->x = quantize_pack(x, how.bits, {}, how.seed, how.offset, how.row_offset);
+    auto [y, mean, invstd] = bn_forward(x, weight, bias, running_mean, running_var, momentum, eps);
+    s->mean = mean;
+    s->invstd = invstd;
+    if (weight) s->weight = weight->detach();
+    s->bits = how.bits;
+    ctx->saved_data["s"] = c10::IValue::make_capsule(s);
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    Plain plain;
+    auto s = state_of<BnState>(ctx);
+    auto [gx, gw, gb] = bn_backward(grads[0], s->x, s->bits, s->weight, s->mean, s->invstd, true, ctx->needs_input_grad(0),
+                                    s->weight && ctx->needs_input_grad(1), s->weight && ctx->needs_input_grad(2));
+    return {gx, gw, gb, {}, {}, {}, {}, {}, {}};
+  }
+};
+
+Tensor bn_node(const Tensor& x, const OptTensor& weight, const OptTensor& bias, const OptTensor& running_mean,
+               const OptTensor& running_var, double momentum, double eps, const Saving& how) {
+  return BnNode::apply(x, weight, bias, running_mean, running_var, momentum, eps, c10::make_intrusive<BnState>(), how);
 }
 
 // ---- aggregation: qspmm_sum / mean / max / min (ops.py:257-436) --------------------------------------------

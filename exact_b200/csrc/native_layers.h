@@ -28,6 +28,10 @@ Tensor gcn_node(const Tensor& x, const Tensor& w, const OptTensor& b, const c10:
 Tensor sage_node(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const OptTensor& w_r,
                  const c10::intrusive_ptr<Graph>& graph, bool mean, const Saving& how, bool projected_first,
                  bool gradient_first);
+// Training batch norm with its input saved compressed (qbatch_norm, ops.py:206-254).
+Tensor bn_node(const Tensor& x, const OptTensor& weight, const OptTensor& bias, const OptTensor& running_mean,
+               const OptTensor& running_var, double momentum, double eps, const Saving& how);
+
 // reduce(A, x) with gradients to x and, when they ask for one, the edge values (qspmm_sum / mean / max / min).
 // reduce: 0 sum, 1 mean, 2 max, 3 min; the graph's transpose carries the weights of the reduction.  row: the row of every edge
 // (needed for the values' gradient of a sum or mean).  keep_x: the values' gradient will be asked for, x is saved compressed.

@@ -263,6 +263,41 @@ std::tuple<Tensor, Tensor> rows_scale_colsum(const Tensor& g, const OptTensor& r
   return {out, colsum};
 }
 
+std::tuple<Tensor, Tensor> rows_half_colsum(const Tensor& g, bool want_colsum) {
+  c10::cuda::CUDAGuard guard(g.device());
+  const int64_t N = g.size(0), K = g.size(1), Kout = (K + 7) / 8 * 8;
+  Tensor out = empty({N, Kout}, at::kHalf, g), colsum, ws;
+  int64_t ws_bytes = 0;
+  if (want_colsum) {
+    colsum = empty({K}, at::kFloat, g);
+    ws_bytes = lib.exact_rows_scale_colsum_workspace_bytes(Kout);
+    ws = empty({ws_bytes}, at::kByte, g);
+  }
+  invoke("exact_rows_half_colsum", {4 * N * K + 2 * N * Kout}, [&](void* st) {
+    return lib.exact_rows_half_colsum(ptr<float>(g), N, K, g.stride(0), ptr(out), Kout, Kout, want_colsum ? ptr<float>(colsum) : nullptr,
+                                      want_colsum ? ptr(ws) : nullptr, ws_bytes, st);
+  });
+  return {out, colsum};
+}
+
+std::tuple<Tensor, Tensor, Tensor> bn_forward(const Tensor& x, const OptTensor& weight_, const OptTensor& bias_,
+                                              const OptTensor& running_mean, const OptTensor& running_var, double momentum,
+                                              double eps) {
+  c10::cuda::CUDAGuard guard(x.device());
+  OptTensor weight, bias;
+  if (weight_) weight = weight_->detach().contiguous();
+  if (bias_) bias = bias_->detach().contiguous();
+  const int64_t N = x.size(0), D = x.size(1), ws_bytes = lib.exact_bn_forward_workspace_bytes(D);
+  Tensor ws = empty({ws_bytes}, at::kByte, x), y = empty({N, D}, at::kFloat, x), mean = empty({D}, at::kFloat, x),
+         invstd = empty({D}, at::kFloat, x);
+  invoke("exact_bn_forward", {12 * N * D}, [&](void* st) {
+    return lib.exact_bn_forward(ptr<float>(x), N, D, ptr<float>(weight), ptr<float>(bias), ptr<float>(running_mean),
+                                ptr<float>(running_var), (float)momentum, (float)eps, ptr(ws), ws_bytes, ptr<float>(y),
+                                ptr<float>(mean), ptr<float>(invstd), st);
+  });
+  return {y, mean, invstd};
+}
+
 std::tuple<Tensor, Tensor, Tensor> bn_backward(const Tensor& g_, const Packed& q, int64_t bits, const OptTensor& weight_,
                                                const Tensor& mean_, const Tensor& invstd_, bool train, bool want_input,
                                                bool want_weight, bool want_bias) {

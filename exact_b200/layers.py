@@ -220,6 +220,15 @@ class QBatchNorm1d(torch.nn.BatchNorm1d):
             else:
                 exponential_average_factor = self.momentum
         bn_training = True
+        if (config.native_layers() and config.bn_backward_from_packed and input.is_cuda and input.dim() == 2
+                and input.dtype == torch.float32 and input.size(1) % 4 == 0 and input.size(0) >= 1024
+                and (self.weight is None or self.weight.dtype == torch.float32)):
+            # fewer rows: the framework's one-launch kernels are as fast
+            track = self.track_running_stats
+            return _lib.native().batch_norm(input, self.weight, self.bias, self.running_mean if track else None,
+                                            self.running_var if track else None, exponential_average_factor, self.eps,
+                                            config.activation_compression_bits[0], config.seed, config.take_offsets(1),
+                                            config.row_offset)
         return qbatch_norm.apply(
             input,
             self.running_mean if not self.training or self.track_running_stats else None,
@@ -264,8 +273,9 @@ class QGCNConv(GCNConv):
         if not isinstance(adj_t, SparseTensor) or self.msg_and_aggr_func.reduce != "sum":
             return False
         value = adj_t.storage._value
-        return (x.is_cuda and x.dim() == 2 and x.size(0) >= 1024
-                and (value is None or not value.requires_grad or not torch.is_grad_enabled()) and (x.dtype == torch.float32 or torch.is_autocast_enabled("cuda")) and self.weight.dtype == torch.float32)
+        return (x.is_cuda and x.dim() == 2 and x.size(0) >= 1024 and self.weight.dtype == torch.float32
+                and (value is None or not value.requires_grad or not torch.is_grad_enabled())
+                and (x.dtype == torch.float32 or torch.is_autocast_enabled("cuda")))
 
     def message_and_aggregate(self, adj_t, x):
         return self.msg_and_aggr_func(adj_t, x)

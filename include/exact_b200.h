@@ -283,6 +283,9 @@ EXACT_API int64_t exact_rows_scale_colsum_workspace_bytes(int64_t Kout);
 EXACT_API int exact_rows_scale_colsum(const float* g, int64_t n, int64_t K, int64_t ldg, const float* rowscale, float* out,
                                       int64_t Kout, int64_t ldo, float* colsum, void* workspace,
                                       int64_t workspace_bytes, void* stream);
+/* The same pass with an fp16 copy of g in place of the scaled one: out_f16 [n, ldo] halves, zero-padded to Kout columns. */
+EXACT_API int exact_rows_half_colsum(const float* g, int64_t n, int64_t K, int64_t ldg, void* out_f16, int64_t Kout, int64_t ldo,
+                                     float* colsum, void* workspace, int64_t workspace_bytes, void* stream);
 
 /* Batch-norm backward straight from the packed input: native_batch_norm_backward as called by the reference's
  * qbatch_norm.backward (exact/exact/ops.py:248-251) with the dequantize_activation of ops.py:238 folded into
@@ -302,6 +305,14 @@ EXACT_API int exact_bn_backward_from_packed(const float* grad_out, int64_t N, in
                                             const float* mean, const float* invstd, int training, void* workspace,
                                             int64_t workspace_bytes, float* grad_input, float* grad_weight,
                                             float* grad_bias, void* stream);
+
+/* Batch norm of a training step, forward (native_batch_norm of ops.py:222-229): batch statistics of x [N, D] (fp32, D % 4 == 0,
+ * 16-byte aligned; other widths return code 3), y, the saved mean and 1 / sqrt(var + eps), and the running statistics (both or
+ * neither may be NULL) moved by `momentum`.  workspace: exact_bn_forward_workspace_bytes(D) bytes. */
+EXACT_API int64_t exact_bn_forward_workspace_bytes(int64_t D);
+EXACT_API int exact_bn_forward(const float* x, int64_t N, int64_t D, const float* weight, const float* bias, float* running_mean,
+                               float* running_var, float momentum, float eps, void* workspace, int64_t workspace_bytes,
+                               float* y, float* save_mean, float* save_invstd, void* stream);
 
 /* CSR SpMM on fp16 operands with the arithmetic of the reference's half instantiation (spmm_cuda.cu:142; AMP runs
  * cast the operands to fp16, exact/exact/ops.py:260, 313): term = half(value[e] * mat[col[e], c]) (the bare operand
