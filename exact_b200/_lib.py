@@ -37,6 +37,7 @@ SIGNATURES = {
     "exact_packed_bytes": (c_i64, [c_i64, c_i64, c_int]),
     "exact_quantize_pack": (c_int, [c_ptr, c_int, c_i64, c_i64, c_int, c_ptr, c_u64, c_u64, c_i64,
                                     c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr]),
+    "exact_quantize_pack_rows": (c_int, [c_ptr, c_int, c_i64, c_i64, c_i64, c_int, c_u64, c_u64, c_i64, c_ptr, c_ptr, c_ptr, c_ptr]),
     "exact_pack_single_precision": (c_int, [c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_int, c_ptr,
                                             c_u64, c_u64, c_i64, c_ptr, c_ptr]),
     "exact_unpack_single_precision": (c_int, [c_ptr, c_int, c_ptr, c_ptr, c_int, c_i64, c_i64, c_ptr, c_ptr]),
@@ -74,6 +75,8 @@ SIGNATURES = {
     "exact_bn_forward_workspace_bytes": (c_i64, [c_i64]),
     "exact_bn_forward": (c_int, [c_ptr, c_i64, c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_f32, c_f32, c_ptr, c_i64, c_ptr, c_ptr, c_ptr,
                                  c_ptr]),
+    "exact_rows_scale_copy_colsum": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_ptr, c_ptr, c_i64, c_i64, c_ptr, c_ptr, c_i64,
+                                             c_ptr]),
     "exact_rows_half_colsum": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_i64, c_i64, c_ptr, c_ptr, c_i64, c_ptr]),
     "exact_bn_backward_workspace_bytes": (c_i64, [c_i64]),
     "exact_bn_backward_from_packed": (c_int, [c_ptr, c_i64, c_i64, c_ptr, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_int,
@@ -91,6 +94,8 @@ SIGNATURES = {
     "exact_rp_workspace_bytes": (c_i64, [c_i64, c_i64]),
     "exact_rp_quantize_pack": (c_int, [c_ptr, c_i64, c_i64, c_ptr, c_i64, c_int, c_u64, c_u64, c_i64, c_ptr, c_ptr,
                                        c_ptr, c_ptr, c_ptr, c_ptr]),
+    "exact_rp_quantize_pack_rows": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_i64, c_int, c_u64, c_u64, c_i64, c_ptr, c_ptr,
+                                            c_ptr, c_ptr, c_ptr, c_ptr]),
     "exact_unpack_rp_workspace_bytes": (c_i64, [c_i64, c_i64]),
     "exact_unpack_dequant_rp": (c_int, [c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_ptr, c_i64, c_ptr, c_ptr, c_ptr]),
     "exact_rademacher": (c_int, [c_u64, c_u64, c_i64, c_i64, c_ptr, c_ptr]),
@@ -105,7 +110,7 @@ SIGNATURES = {
                                      c_i64, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_ptr]),
     "exact_linear_partial_bytes": (c_i64, [c_i64]),
     "exact_linear_forward_strided": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_i64, c_i64, c_ptr, c_i64, c_i64, c_ptr,
-                                             c_i64, c_i64, c_i64, c_ptr, c_int, c_i64, c_ptr, c_ptr, c_ptr, c_i64, c_ptr]),
+                                             c_i64, c_i64, c_i64, c_ptr, c_ptr, c_i64, c_i64, c_ptr, c_ptr, c_ptr, c_i64, c_ptr]),
     "exact_spmm_minmax": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_i64, c_int, c_ptr, c_ptr, c_ptr]),
     "exact_spmm_minmax_scratch_bytes": (c_i64, [c_i64, c_i64]),
     "exact_spmm_minmax_planned": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_i64, c_int, c_i64, c_ptr, c_ptr,

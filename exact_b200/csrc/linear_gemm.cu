@@ -62,7 +62,8 @@ struct LinParams {
   int N, Npad;
   int kblocks1, kblocks;   // K tiles of the first operand pair, and of both pairs together
   int num_tiles;
-  int accumulate;          // C += ... instead of C = ...
+  const float* addend;     // [M, ldadd] added to the product (C itself: C += ...), or null
+  long long ldadd;
   int chunk;               // K tiles that are accumulated in TMEM before their sum is taken over in fp32
   float* partial;          // [grid, Npad / 4, 128, 4]: running sums of the chunks before the last, per CTA
   int stages;              // K tiles the ring holds (2 at Npad = 256, up to 4 for narrow outputs)
@@ -269,7 +270,8 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   } else {
     // ---------------- epilogue: the last four warps ----------------
     const int quad = warp & 3;   // TMEM lanes 32*quad .. 32*quad+31
-    const bool vec = (p.N & 3) == 0 && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
+    const bool vec = (p.N & 3) == 0 && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 &&
+                     (p.addend == nullptr || ((p.ldadd & 3) == 0 && (reinterpret_cast<uintptr_t>(p.addend) & 15) == 0));
     const uint32_t stage_addr = stage_base + (uint32_t)quad * 4096u;
     int t = 0;
     bool ok = true;
@@ -365,11 +367,12 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
           const uint32_t addr = stage_addr + (uint32_t)rr * 128u + ((ci ^ ((uint32_t)rr & 7u)) << 4);
           asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(addr));
           if (nn < p.M && (int)ci * 4 < cols && c < p.N) {
-            float* __restrict__ d = p.C + nn * p.ldc + c;
+            float* d = p.C + nn * p.ldc + c;
+            const float* add = p.addend ? p.addend + nn * p.ldadd + c : nullptr;
             o.x += bv[0]; o.y += bv[1]; o.z += bv[2]; o.w += bv[3];
             if (vec) {   // N % 4 == 0, so c + 4 <= N
-              if (p.accumulate) {
-                const float4 old = *reinterpret_cast<const float4*>(d);
+              if (add) {
+                const float4 old = *reinterpret_cast<const float4*>(add);
                 o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
               }
               __stcs(reinterpret_cast<float4*>(d), o);
@@ -377,7 +380,7 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
               const float ov[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
               for (int bb = 0; bb < 4; bb++)
-                if (c + bb < p.N) d[bb] = p.accumulate ? d[bb] + ov[bb] : ov[bb];
+                if (c + bb < p.N) d[bb] = add ? add[bb] + ov[bb] : ov[bb];
             }
           }
         }
@@ -448,14 +451,14 @@ int64_t exact_linear_partial_bytes(int64_t N) {
 int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb,
                          const float* A2, int64_t K2, int64_t lda2, const float* B2, int64_t ldb2, int64_t N,
                          const float* bias, int accumulate, void* workspace, float* C, int64_t ldc, void* stream) {
-  return exact_linear_forward_strided(A, M, K, lda, B, ldb, 1, A2, K2, lda2, B2, ldb2, 1, N, bias, accumulate, 0, nullptr, workspace,
-                                      C, ldc, stream);
+  return exact_linear_forward_strided(A, M, K, lda, B, ldb, 1, A2, K2, lda2, B2, ldb2, 1, N, bias, accumulate ? C : nullptr,
+                                      accumulate ? ldc : 0, 0, nullptr, workspace, C, ldc, stream);
 }
 
 int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb, int64_t incb,
                          const float* A2, int64_t K2, int64_t lda2, const float* B2, int64_t ldb2, int64_t incb2, int64_t N,
-                         const float* bias, int accumulate, int64_t k_chunk, float* partial, void* workspace, float* C,
-                         int64_t ldc, void* stream) {
+                         const float* bias, const float* addend, int64_t ldadd, int64_t k_chunk, float* partial, void* workspace,
+                         float* C, int64_t ldc, void* stream) {
   EXB_REQUIRE(k_chunk >= 0 && k_chunk % kLinTileK == 0 && (k_chunk == 0 || (partial && (reinterpret_cast<uintptr_t>(partial) & 15) == 0)),
               "linear_forward: k_chunk must be a multiple of 32 and needs a 16-byte aligned buffer of partial sums");
   EXB_REQUIRE(M >= 0 && K > 0 && N > 0 && K2 >= 0, "linear_forward: bad shape");
@@ -463,6 +466,7 @@ int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t l
   EXB_REQUIRE(A && B && C && workspace, "linear_forward: null pointer");
   EXB_REQUIRE((A2 != nullptr) == (K2 > 0) && (B2 != nullptr) == (K2 > 0), "linear_forward: the second operand pair needs A2, B2 and K2 > 0");
   EXB_REQUIRE(lda >= K && (incb != 1 || ldb >= K) && ldc >= N && (K2 == 0 || (lda2 >= K2 && (incb2 != 1 || ldb2 >= K2))), "linear_forward: leading dimension smaller than the row");
+  EXB_REQUIRE(addend == nullptr || ldadd >= N, "linear_forward: leading dimension of the addend smaller than the row");
   if (N > 256) return fail(EXB_ERR_UNSUPPORTED, "linear_forward: N = %lld exceeds one MMA tile (256); call per 256-column block", (long long)N);
   if (lda % 4 != 0 || (reinterpret_cast<uintptr_t>(A) & 15) != 0 ||
       (K2 > 0 && (lda2 % 4 != 0 || (reinterpret_cast<uintptr_t>(A2) & 15) != 0)))
@@ -498,7 +502,7 @@ int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t l
   p.C = C; p.bias = bias; p.status = status; p.lib_status = status_word_ptr(); p.M = M; p.ldc = ldc; p.N = (int)N; p.Npad = Npad;
   p.kblocks1 = Kpad1 / kLinTileK; p.kblocks = Kpad / kLinTileK;
   p.num_tiles = (int)((M + kLinTileM - 1) / kLinTileM);
-  p.accumulate = accumulate ? 1 : 0;
+  p.addend = addend; p.ldadd = ldadd;
   p.chunk = k_chunk > 0 ? (int)(k_chunk / kLinTileK) : p.kblocks;
   p.partial = partial;
   p.b_slot = (unsigned)Npad * kLinTileK * 4;

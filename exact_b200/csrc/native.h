@@ -39,8 +39,10 @@ struct LibraryError : std::runtime_error {   // becomes exact_b200.ExactB200Erro
   X(exact_act_quantized_dropout_backward) X(exact_act_quantized_relu_dropout_forward)                                 \
   X(exact_act_quantized_forward_f16) X(exact_act_quantized_backward_f16) X(exact_spmm_planned)                        \
   X(exact_spmm_f16_planned) X(exact_rows_scale_colsum_workspace_bytes)                     \
-  X(exact_rows_scale_colsum) X(exact_bn_forward_workspace_bytes) X(exact_bn_forward) X(exact_rows_half_colsum) X(exact_bn_backward_workspace_bytes) X(exact_bn_backward_from_packed)                    \
-  X(exact_rp_workspace_bytes) X(exact_rp_quantize_pack) X(exact_rademacher) X(exact_grad_weight_workspace_bytes)      \
+  X(exact_rows_scale_colsum) X(exact_bn_forward_workspace_bytes) X(exact_bn_forward) X(exact_rows_half_colsum) \
+  X(exact_rows_scale_copy_colsum) X(exact_quantize_pack_rows) X(exact_rp_quantize_pack_rows)                          \
+  X(exact_bn_backward_workspace_bytes) X(exact_bn_backward_from_packed)                                               \
+  X(exact_rp_workspace_bytes) X(exact_rademacher) X(exact_grad_weight_workspace_bytes)      \
   X(exact_grad_weight_from_packed) X(exact_linear_workspace_bytes) X(exact_linear_partial_bytes) X(exact_linear_forward_strided)                            \
   X(exact_spmm_minmax_scratch_bytes) X(exact_spmm_minmax_planned) X(exact_spmm_minmax_backward)                       \
   X(exact_spmm_value_bw) X(exact_status_peek)
@@ -106,18 +108,23 @@ struct Packed {           // a compressed activation: quantize_activation's resu
 };
 
 Packed quantize_pack(const Tensor& x, int64_t bits, const OptTensor& noise, uint64_t seed, uint64_t offset, int64_t row_offset);
+// the same with Philox noise on fp32 rows of any pitch
+Packed quantize_pack_rows(const Tensor& x, int64_t bits, uint64_t seed, uint64_t offset, int64_t row_offset);
 Tensor unpack(const Tensor& codes, int64_t bits, const Tensor& scale, const Tensor& mn, int64_t N, int64_t D);
 Tensor rademacher(int64_t rows, int64_t cols, uint64_t seed, uint64_t offset, const Tensor& like);
 bool rp_supported(int64_t D, int64_t k);
+// x: rows of any pitch
 Packed rp_quantize_pack(const Tensor& x, const Tensor& R, int64_t bits, uint64_t seed, uint64_t offset, int64_t row_offset,
                         Tensor* projection = nullptr);
 bool linear_supported(const Tensor& a);
 Tensor rows16(const Tensor& a);
-// fp32 operands; w may be a transposed view (its rows are read through both strides)
+// fp32 operands; w may be a transposed view (its rows are read through both strides); addend: rows of any pitch
 Tensor linear(const Tensor& a, const Tensor& w, const OptTensor& bias, const OptTensor& a2, const OptTensor& w2,
-              const OptTensor& out, bool accumulate, int64_t k_chunk = 0);
+              const OptTensor& out, bool accumulate, int64_t k_chunk = 0, const OptTensor& addend = {});
 Tensor grad_weight(const Tensor& g, int64_t bits, const Packed& q0, int64_t k0, const Packed* q1, int64_t k1);
 std::tuple<Tensor, Tensor> rows_scale_colsum(const Tensor& g, const OptTensor& rowscale, bool want_scaled, bool want_colsum);
+// (D^-1 g, g itself, both zero-padded to whole 16-byte pieces, g.sum(0))
+std::tuple<Tensor, Tensor, Tensor> rows_scale_copy_colsum(const Tensor& g, const OptTensor& rowscale, bool want_colsum);
 // (fp16 copy of g zero-padded to whole 16-byte pieces, g.sum(0))
 std::tuple<Tensor, Tensor> rows_half_colsum(const Tensor& g, bool want_colsum);
 // (y, mean, invstd); the running statistics are moved in place

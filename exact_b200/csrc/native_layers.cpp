@@ -212,10 +212,10 @@ struct SageNode : Function<SageNode> {
     s->rows = x.size(0);
     s->has_bias = b.has_value();
     uint64_t offset = s->how.offset;
-    s->x = compress(x, s->how, offset);       // without lin_r nothing reads it; the noise stays that of the separate nodes
-    if (!w_r) s->x = Compressed();
-    offset += s->how.kept ? 2 : 1;
-    x = rows16(x);                            // several products below read it
+    const Tensor rows = rows16(x);            // several products read them, the projection among them
+    if (w_r) s->x = compress(s->how.kept ? rows : x, s->how, offset);
+    offset += s->how.kept ? 2 : 1;            // without lin_r nothing reads it; the noise stays that of the separate nodes
+    x = rows;
     const int64_t k = s->how.kept, kp = (k + 3) / 4 * 4, op = (out_f + 3) / 4 * 4;
     Tensor out;
     if (s->projected_first && k && kp + op < in_f) {
@@ -227,10 +227,10 @@ struct SageNode : Function<SageNode> {
       wcat.narrow(0, 0, k).copy_(s->agg.R.t());
       wcat.narrow(0, kp, out_f).copy_(w_l);
       const Tensor t = spmm(g.fw, g.fw.value, linear(x, wcat, {}, {}, {}, {}, false), s->mean);
-      s->agg.q = quantize_pack(t.narrow(1, 0, k).contiguous(), s->how.bits, {}, s->how.seed, offset + 1, s->how.row_offset);
-      out = t.narrow(1, kp, out_f).contiguous();
-      if (b) out.add_(*b);
-      if (w_r) linear(x, *w_r, {}, {}, {}, out, true);
+      s->agg.q = quantize_pack_rows(t.narrow(1, 0, k), s->how.bits, s->how.seed, offset + 1, s->how.row_offset);
+      const Tensor part = t.narrow(1, kp, out_f);
+      if (w_r) out = linear(x, *w_r, b, {}, {}, {}, false, 0, part);
+      else out = b ? part.add(*b) : part.contiguous();
     } else {
       const Tensor agg = spmm(g.fw, g.fw.value, x, s->mean);
       s->agg = compress(agg, s->how, offset);
@@ -251,17 +251,21 @@ struct SageNode : Function<SageNode> {
     const int64_t O = g.size(1), in_f = s->w_l.size(1), k = s->agg.width;
     const bool aggregate_g = need_x && s->gradient_first && O <= in_f;
     const bool by_degree = s->mean && gr.inv_degree.has_value();
-    // One pass over g: D^-1 g (zero-padded to whole column groups), the operand of the transposed mean, and the bias
-    // gradient g.sum(0) (backward_func.cc:88-90).
+    // One pass over g: D^-1 g, the operand of the transposed mean, g with its rows padded to whole 16-byte pieces for the
+    // products below, and the bias gradient g.sum(0) (backward_func.cc:88-90).
     Tensor scaled;
-    if (aggregate_g && (by_degree || O % 4)) {
-      auto [sc, sum] = rows_scale_colsum(g, by_degree ? gr.inv_degree : OptTensor(), true, s->has_bias);
+    if (aggregate_g && by_degree && O % 4) {
+      auto [sc, padded, sum] = rows_scale_copy_colsum(g, gr.inv_degree, s->has_bias);
       scaled = sc;
+      g = padded;
+      gb = sum;
+    } else if (O % 4 || (aggregate_g && by_degree)) {
+      auto [sc, sum] = rows_scale_colsum(g, O % 4 ? OptTensor() : gr.inv_degree, true, s->has_bias);
+      (O % 4 ? g : scaled) = sc;
       gb = sum;
     } else if (s->has_bias) {
       gb = std::get<1>(rows_scale_colsum(g, {}, false, true));
     }
-    if (O % 4) g = at::constant_pad_nd(g, {0, 4 - O % 4});   // rows in 16-byte pieces for the products below
     // both weight gradients in one pass over g: g^T [Xq_agg | Xq_x], then the two small transposed projections
     if (O <= 256) {
       const int64_t k0pad = (k + 15) / 16 * 16;
@@ -443,10 +447,9 @@ Tensor sage_eval(const Tensor& x_, const Tensor& w_l, const OptTensor& b, const 
   // fewer outputs than inputs: reduce(A, x) W_l^T = reduce(A, x W_l^T) gathers the narrower operand
   const Tensor rows = rows16(x);
   const Tensor t = spmm(g.fw, g.fw.value, linear(rows, pad ? at::constant_pad_nd(w_l, {0, 0, 0, pad}) : w_l, {}, {}, {}, {}, false, kEvalChunk), mean);
-  Tensor out = pad ? t.narrow(1, 0, out_f) : t;
-  if (w_r) linear(rows, *w_r, b, {}, {}, out, true, kEvalChunk);
-  else if (b) out.add_(*b);
-  return out.contiguous();
+  const Tensor part = t.narrow(1, 0, out_f);
+  if (w_r) return linear(rows, *w_r, b, {}, {}, {}, false, kEvalChunk, part);
+  return b ? part.add(*b) : part.contiguous();
 }
 
 }  // namespace exb

@@ -99,6 +99,19 @@ Packed quantize_pack(const Tensor& x, int64_t bits, const OptTensor& noise, uint
   return q;
 }
 
+Packed quantize_pack_rows(const Tensor& x, int64_t bits, uint64_t seed, uint64_t offset, int64_t row_offset) {
+  check_type(x.is_cuda() && x.dim() == 2 && x.stride(1) == 1 && x.scalar_type() == at::kFloat, "data");
+  check_bits(bits);
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t N = x.size(0), D = x.size(1), bytes = lib.exact_packed_bytes(N, D, (int)bits);
+  Packed q{empty({bytes + 1}, at::kChar, x), empty({N}, at::kBFloat16, x), empty({N}, at::kBFloat16, x)};
+  invoke("exact_quantize_pack", {N * D * 4 + bytes + 4 * N}, [&](void* st) {
+    return lib.exact_quantize_pack_rows(ptr(x), EXACT_DTYPE_F32, N, D, x.stride(0), (int)bits, seed, offset, row_offset,
+                                        ptr<uint8_t>(q.codes), ptr<uint16_t>(q.scale), ptr<uint16_t>(q.mn), st);
+  });
+  return q;
+}
+
 Tensor unpack(const Tensor& codes, int64_t bits, const Tensor& scale, const Tensor& mn, int64_t N, int64_t D) {
   if (!codes.is_cuda() || !codes.is_contiguous() || codes.dim() != 1 || codes.scalar_type() != at::kChar)
     throw std::runtime_error("The type of data is not correct!");
@@ -147,7 +160,7 @@ bool rp_supported(int64_t D, int64_t k) {
 
 Packed rp_quantize_pack(const Tensor& x, const Tensor& R, int64_t bits, uint64_t seed, uint64_t offset, int64_t row_offset,
                         Tensor* projection) {
-  check_tensor(x, "data", 2);
+  if (!x.is_cuda() || x.dim() != 2 || x.stride(1) != 1 || x.stride(0) < x.size(1)) check_tensor(x, "data", 2);   // any pitch
   check_type(x.scalar_type() == at::kFloat, "data");
   check_tensor(R, "R", 2);
   check_type(R.scalar_type() == at::kFloat, "R");
@@ -162,7 +175,7 @@ Packed rp_quantize_pack(const Tensor& x, const Tensor& R, int64_t bits, uint64_t
   const int64_t bytes = lib.exact_packed_bytes(N, k, (int)bits);
   Packed q{empty({bytes + 1}, at::kChar, x), empty({N}, at::kBFloat16, x), empty({N}, at::kBFloat16, x)};
   invoke("exact_rp_quantize_pack", {N * D * 4 + D * k * 4 + bytes + 4 * N}, [&](void* st) {
-    return lib.exact_rp_quantize_pack(ptr<float>(x), N, D, ptr<float>(R), k, (int)bits, seed, offset, row_offset, ptr(ws),
+    return lib.exact_rp_quantize_pack_rows(ptr<float>(x), N, D, N > 1 ? x.stride(0) : D, ptr<float>(R), k, (int)bits, seed, offset, row_offset, ptr(ws),
                                       ptr<uint8_t>(q.codes), ptr<uint16_t>(q.scale), ptr<uint16_t>(q.mn),
                                       projection ? ptr<float>(*projection) : nullptr, st);
   });
@@ -184,7 +197,7 @@ Tensor rows16(const Tensor& a) {
 }
 
 Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const OptTensor& a2_, const OptTensor& w2_,
-              const OptTensor& out_, bool accumulate, int64_t k_chunk) {
+              const OptTensor& out_, bool accumulate, int64_t k_chunk, const OptTensor& addend_) {
   c10::cuda::CUDAGuard guard(a_.device());
   const int64_t M = a_.size(0), K = a_.size(1), N = w_.size(0);
   const Tensor a = rows16(a_), w = w_;
@@ -197,7 +210,7 @@ Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const 
   }
   if (bias_) bias = bias_->contiguous();
   Tensor out = out_ ? *out_ : empty({M, N}, at::kFloat, a);
-  if (!out_) accumulate = false;
+  const OptTensor addend = addend_ ? addend_ : out_ && accumulate ? OptTensor(out) : OptTensor();
   if (out.size(0) != M || out.size(1) != N || out.stride(1) != 1) throw std::runtime_error("linear: out does not fit");
   Tensor partial;      // of a contraction in chunks (exact_linear_forward_chunked)
   if (k_chunk > 0 && K + K2 > k_chunk) partial = empty({lib.exact_linear_partial_bytes(std::min<int64_t>(N, 256))}, at::kByte, a);
@@ -208,12 +221,13 @@ Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const 
     const float* w2b = K2 ? ptr<float>(w2) + n0 * w2.stride(0) : nullptr;
     float* cb = ptr<float>(out) + n0;
     CallInfo info;
-    info.bytes = 4 * (M * (K + K2) + n * (K + K2) + M * n * (accumulate ? 2 : 1));
+    info.bytes = 4 * (M * (K + K2) + n * (K + K2) + M * n * (addend ? 2 : 1));
     info.flops = 6.0 * (double)M * (double)(K + K2) * (double)n;
     invoke("exact_linear_forward", info, [&](void* st) {
       return lib.exact_linear_forward_strided(ptr<float>(a), M, K, a.stride(0), wb, w.stride(0), w.stride(1), K2 ? ptr<float>(a2) : nullptr, K2,
                                       K2 ? a2.stride(0) : 0, w2b, K2 ? w2.stride(0) : 0, K2 ? w2.stride(1) : 1, n,
-                                      bias.defined() ? ptr<float>(bias) + n0 : nullptr, accumulate ? 1 : 0,
+                                      bias.defined() ? ptr<float>(bias) + n0 : nullptr,
+                                              addend ? ptr<float>(addend) + n0 : nullptr, addend ? addend->stride(0) : 0,
                                               partial.defined() ? k_chunk : 0, partial.defined() ? ptr<float>(partial) : nullptr, ptr(ws),
                                               cb, out.stride(0), st);
     });
@@ -261,6 +275,24 @@ std::tuple<Tensor, Tensor> rows_scale_colsum(const Tensor& g, const OptTensor& r
                                        want_colsum ? ptr<float>(colsum) : nullptr, want_colsum ? ptr(ws) : nullptr, ws_bytes, st);
   });
   return {out, colsum};
+}
+
+std::tuple<Tensor, Tensor, Tensor> rows_scale_copy_colsum(const Tensor& g, const OptTensor& rowscale, bool want_colsum) {
+  c10::cuda::CUDAGuard guard(g.device());
+  const int64_t N = g.size(0), K = g.size(1), Kout = (K + 3) / 4 * 4;
+  Tensor out = empty({N, Kout}, at::kFloat, g), copy = empty({N, Kout}, at::kFloat, g), colsum, ws;
+  int64_t ws_bytes = 0;
+  if (want_colsum) {
+    colsum = empty({K}, at::kFloat, g);
+    ws_bytes = lib.exact_rows_scale_colsum_workspace_bytes(Kout);
+    ws = empty({ws_bytes}, at::kByte, g);
+  }
+  invoke("exact_rows_scale_colsum", {4 * N * K + 8 * N * Kout}, [&](void* st) {
+    return lib.exact_rows_scale_copy_colsum(ptr<float>(g), N, K, g.stride(0), ptr<float>(rowscale), ptr<float>(out), ptr<float>(copy),
+                                            Kout, Kout, want_colsum ? ptr<float>(colsum) : nullptr, want_colsum ? ptr(ws) : nullptr,
+                                            ws_bytes, st);
+  });
+  return {out, copy, colsum};
 }
 
 std::tuple<Tensor, Tensor> rows_half_colsum(const Tensor& g, bool want_colsum) {

@@ -35,7 +35,7 @@ struct PackParams {
   uint16_t* min_bf16;     // [N] or null
   float* scale_f32;       // [N] or null
   float* min_f32;         // [N] or null
-  long long N, D;
+  long long N, D, ldx;    // ldx: pitch of x in elements
   long long row_offset;   // global index of row 0 (multiple of 8): keys the noise for row-sharded runs
   int tpt;                // threads per 8-row tile
   uint32_t off_lo, off_hi;
@@ -53,7 +53,7 @@ __device__ __forceinline__ void group_barrier(int grp, int nthreads) {
 
 // Per-thread view of the tiling, fixed for the whole kernel.
 struct TileCtx {
-  long long N, D, G;
+  long long N, D, G, ldx;
   int tpt, grp, tl, lane, lane_base;
   bool multi;
 };
@@ -144,10 +144,10 @@ __device__ __forceinline__ void load_tile(const InT* __restrict__ x, const TileC
                                           Raw<InT, VEC> (&xv)[8][V]) {
   const long long row0 = tile << 3;
   const int rows_valid = FULL ? 8 : c.N - row0 >= 8 ? 8 : c.N > row0 ? (int)(c.N - row0) : 0;
-  const unsigned Du = (unsigned)c.D;
+  const unsigned Du = (unsigned)c.ldx;
 #pragma unroll
   for (int v = 0; v < V; v++) {
-    const InT* __restrict__ base = x + row0 * c.D + col[v];
+    const InT* __restrict__ base = x + row0 * c.ldx + col[v];
 #pragma unroll
     for (int r = 0; r < 8; r++) {
       if ((FULL || r < rows_valid) && cvalid[v]) xv[r][v].load(base + r * Du);
@@ -511,7 +511,7 @@ quantize_pack_kernel(const __grid_constant__ PackParams p) {
   __shared__ __align__(16) float s_fin[2 * kMaxGroupsPerCta * 16];
 
   TileCtx c;
-  c.N = p.N; c.D = p.D;
+  c.N = p.N; c.D = p.D; c.ldx = p.ldx;
   c.G = (p.N + WPT - 1) / WPT;
   c.tpt = p.tpt;
   c.grp = threadIdx.x / c.tpt;
@@ -537,7 +537,7 @@ quantize_pack_kernel(const __grid_constant__ PackParams p) {
   // instruction while the current one is processed, so the register loads of the next iteration
   // find their lines on chip.
   const long long tile_bytes = 8 * p.D * (long long)sizeof(InT);
-  const bool can_prefetch = (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 && (tile_bytes & 15) == 0;
+  const bool can_prefetch = p.ldx == p.D && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 && (tile_bytes & 15) == 0;
   const bool philox = p.noise == nullptr;
   Raw<InT, VEC> xv[8][V];
   int it = 0;
@@ -958,7 +958,7 @@ static int align_vec(const void* ptr, int elem_bytes) {
 
 constexpr int kDtypeHalf = 2;   // inside the library: exact_quantize_pack_f16
 
-static int pack_common(const void* x, int dtype, long long N, long long D, int bits,
+static int pack_common(const void* x, int dtype, long long N, long long D, long long ldx, int bits,
                        const float* noise, const float* mn_in, const float* scale_in,
                        unsigned long long seed, unsigned long long offset, long long row_offset,
                        uint8_t* packed, uint16_t* scale_bf16, uint16_t* min_bf16, float* scale_f32,
@@ -974,7 +974,7 @@ static int pack_common(const void* x, int dtype, long long N, long long D, int b
   p.x = x; p.noise = noise; p.mn_in = mn_in; p.scale_in = scale_in;
   p.packed = packed; p.scale_bf16 = scale_bf16; p.min_bf16 = min_bf16;
   p.scale_f32 = scale_f32; p.min_f32 = min_f32;
-  p.N = N; p.D = D; p.row_offset = row_offset; p.tpt = 0;
+  p.N = N; p.D = D; p.ldx = ldx; p.row_offset = row_offset; p.tpt = 0;
   p.off_lo = (uint32_t)offset; p.off_hi = (uint32_t)(offset >> 32);
   p.key = make_philox_key(seed);
   if (mn_in != nullptr) {
@@ -983,6 +983,7 @@ static int pack_common(const void* x, int dtype, long long N, long long D, int b
   }
   const int eb = dtype == EXACT_DTYPE_F32 ? 4 : 2;
   int max_vec = align_vec(x, eb);
+  if (ldx % 4 != 0) max_vec = ldx % 2 != 0 ? 1 : max_vec < 2 ? max_vec : 2;
   if (noise) max_vec = max_vec < align_vec(noise, 4) ? max_vec : align_vec(noise, 4);
   const int pa = (int)(reinterpret_cast<uintptr_t>(packed) & 3);
   if (pa != 0) max_vec = (pa == 2 && max_vec >= 2) ? 2 : 1;
@@ -998,7 +999,7 @@ static int pack_common(const void* x, int dtype, long long N, long long D, int b
 int quantize_pack_half(const void* x, long long N, long long D, int bits, const float* noise, unsigned long long seed,
                        unsigned long long offset, long long row_offset, uint8_t* packed, uint16_t* scale, uint16_t* mn,
                        cudaStream_t st) {
-  return pack_common(x, kDtypeHalf, N, D, bits, noise, nullptr, nullptr, seed, offset, row_offset, packed, scale, mn, nullptr,
+  return pack_common(x, kDtypeHalf, N, D, D, bits, noise, nullptr, nullptr, seed, offset, row_offset, packed, scale, mn, nullptr,
                      nullptr, st);
 }
 
@@ -1087,15 +1088,22 @@ int exact_quantize_pack(const void* x, int dtype, int64_t N, int64_t D, int bits
                         uint64_t seed, uint64_t offset, int64_t row_offset, uint8_t* packed,
                         uint16_t* scale_bf16, uint16_t* min_bf16, float* scale_f32, float* min_f32,
                         void* stream) {
-  return pack_common(x, dtype, N, D, bits, noise, nullptr, nullptr, seed, offset, row_offset, packed,
+  return pack_common(x, dtype, N, D, D, bits, noise, nullptr, nullptr, seed, offset, row_offset, packed,
                      scale_bf16, min_bf16, scale_f32, min_f32, (cudaStream_t)stream);
+}
+
+int exact_quantize_pack_rows(const void* x, int dtype, int64_t N, int64_t D, int64_t ldx, int bits, uint64_t seed, uint64_t offset,
+                             int64_t row_offset, uint8_t* packed, uint16_t* scale_bf16, uint16_t* min_bf16, void* stream) {
+  EXB_REQUIRE(ldx >= D && ldx < (1LL << 28), "quantize_pack_rows: the pitch must be at least the row and below 2^28");
+  return pack_common(x, dtype, N, D, ldx, bits, nullptr, nullptr, nullptr, seed, offset, row_offset, packed, scale_bf16, min_bf16,
+                     nullptr, nullptr, (cudaStream_t)stream);
 }
 
 int exact_pack_single_precision(const void* data, int dtype, const float* min, const float* scale,
                                 int64_t N, int64_t D, int bits, const float* noise, uint64_t seed,
                                 uint64_t offset, int64_t row_offset, uint8_t* packed, void* stream) {
   if (N > 0 && D > 0) EXB_REQUIRE(min != nullptr && scale != nullptr, "pack_single_precision: null min/scale");
-  return pack_common(data, dtype, N, D, bits, noise, min, scale, seed, offset, row_offset, packed,
+  return pack_common(data, dtype, N, D, D, bits, noise, min, scale, seed, offset, row_offset, packed,
                      nullptr, nullptr, nullptr, nullptr, (cudaStream_t)stream);
 }
 

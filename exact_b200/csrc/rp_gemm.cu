@@ -65,6 +65,7 @@ struct RpParams {
   int* lib_status;    // library-wide status word of this device (capi.cu), or null
   long long N;
   long long row_offset;
+  long long ldx;
   int D, k, kpad, bits;
   int num_tiles, kblocks, stages;
   unsigned stage_bytes;
@@ -218,8 +219,8 @@ rp_pack_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         // A producer warp has an SM sub-partition to itself, so the per-piece address arithmetic is kept to a
         // few independent instructions: source and destination advance by constants from row to row.
         const long long n0 = (long long)tile * kRpTileM + rg;
-        const float* src = p.x + n0 * p.D + col;
-        const long long src_step = (long long)rpp * p.D;
+        const float* src = p.x + n0 * p.ldx + col;
+        const long long src_step = (long long)rpp * p.ldx;
         uint32_t dst_row = tiles_base + (uint32_t)s * p.stage_bytes + (uint32_t)(rg * 128 + within);
         const long long rows_left = p.N - n0;     // rows n0, n0 + rpp, ... below N are real
         const int passes = kRpTileM / rpp;        // 16 (8-byte pieces) or 32 (4-byte pieces)
@@ -451,6 +452,15 @@ int exact_rp_quantize_pack(const float* x, int64_t N, int64_t D, const float* R,
                            uint64_t seed, uint64_t offset, int64_t row_offset, void* workspace,
                            uint8_t* packed, uint16_t* scale_bf16, uint16_t* min_bf16, float* y_out,
                            void* stream) {
+  return exact_rp_quantize_pack_rows(x, N, D, D, R, k, bits, seed, offset, row_offset, workspace, packed, scale_bf16, min_bf16,
+                                     y_out, stream);
+}
+
+int exact_rp_quantize_pack_rows(const float* x, int64_t N, int64_t D, int64_t ldx, const float* R, int64_t k, int bits,
+                                uint64_t seed, uint64_t offset, int64_t row_offset, void* workspace,
+                                uint8_t* packed, uint16_t* scale_bf16, uint16_t* min_bf16, float* y_out,
+                                void* stream) {
+  EXB_REQUIRE(ldx >= D, "rp_quantize_pack: the pitch must be at least the row");
   EXB_REQUIRE(bits == 1 || bits == 2 || bits == 4 || bits == 8, "bits must be 1, 2, 4 or 8 (got %d)", bits);
   EXB_REQUIRE(N >= 0 && D > 0 && k > 0, "rp_quantize_pack: bad shape");
   EXB_REQUIRE(row_offset >= 0 && row_offset % 8 == 0, "rp_quantize_pack: row_offset must be a non-negative multiple of 8");
@@ -461,7 +471,7 @@ int exact_rp_quantize_pack(const float* x, int64_t N, int64_t D, const float* R,
   if (kpad > 512) return fail(EXB_ERR_UNSUPPORTED, "rp_quantize_pack: k = %lld exceeds the 512 accumulator columns of TMEM", (long long)k);
   EXB_REQUIRE((reinterpret_cast<uintptr_t>(x) & 3) == 0, "rp_quantize_pack: x must be 4-byte aligned");
   // rows that a tensor map cannot describe (pitch or base not a multiple of 16 bytes) are copied by cp.async
-  const bool async_a = D % 4 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0;
+  const bool async_a = ldx % 4 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0;
   EXB_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "rp_quantize_pack: workspace must be 256-byte aligned");
   // the epilogue stores 32-bit words of packed bytes when k % 4 == 0
   EXB_REQUIRE(k % 4 != 0 || (reinterpret_cast<uintptr_t>(packed) & 3) == 0, "rp_quantize_pack: packed must be 4-byte aligned when k %% 4 == 0");
@@ -476,7 +486,7 @@ int exact_rp_quantize_pack(const float* x, int64_t N, int64_t D, const float* R,
   CUtensorMap tm_x, tm_rt;
   int rc;
   if (!async_a) {
-    rc = make_tensor_map_2d_f32(&tm_x, x, (unsigned long long)D, (unsigned long long)N, (unsigned long long)D * 4, kRpTileK, kRpTileM);
+    rc = make_tensor_map_2d_f32(&tm_x, x, (unsigned long long)D, (unsigned long long)N, (unsigned long long)ldx * 4, kRpTileK, kRpTileM);
     if (rc) return rc;
   } else {
     memset(&tm_x, 0, sizeof(tm_x));   // not read: the cp.async producers take x itself
@@ -488,7 +498,8 @@ int exact_rp_quantize_pack(const float* x, int64_t N, int64_t D, const float* R,
   RpParams p{};
   p.packed = packed; p.scale_bf16 = scale_bf16; p.min_bf16 = min_bf16; p.y_out = y_out; p.status = status; p.lib_status = status_word_ptr();
   p.x = x;
-  p.piece = (D % 2 == 0 && (reinterpret_cast<uintptr_t>(x) & 7) == 0) ? 8 : 4;
+  p.ldx = ldx;
+  p.piece = (D % 2 == 0 && ldx % 2 == 0 && (reinterpret_cast<uintptr_t>(x) & 7) == 0) ? 8 : 4;
   p.N = N; p.row_offset = row_offset; p.D = (int)D; p.k = (int)k; p.kpad = kpad; p.bits = bits;
   p.num_tiles = (int)((N + kRpTileM - 1) / kRpTileM);
   p.kblocks = Dpad / kRpTileK;

@@ -78,6 +78,10 @@ EXACT_API int exact_quantize_pack(const void* x, int dtype, int64_t N, int64_t D
                                   const float* noise, uint64_t seed, uint64_t offset,
                                   int64_t row_offset, uint8_t* packed, uint16_t* scale_bf16,
                                   uint16_t* min_bf16, float* scale_f32, float* min_f32, void* stream);
+/* The same with Philox noise on rows of pitch ldx >= D elements (a column block of a wider matrix). */
+EXACT_API int exact_quantize_pack_rows(const void* x, int dtype, int64_t N, int64_t D, int64_t ldx, int bits, uint64_t seed,
+                                       uint64_t offset, int64_t row_offset, uint8_t* packed, uint16_t* scale_bf16,
+                                       uint16_t* min_bf16, void* stream);
 
 /* quantization.pack_single_precision(data, min, max, scale, bits, stochastic)
  * (quantization.cc:37-48; kernel quantization_cuda_kernel.cu:63-94) with caller-computed fp32 row
@@ -283,6 +287,10 @@ EXACT_API int64_t exact_rows_scale_colsum_workspace_bytes(int64_t Kout);
 EXACT_API int exact_rows_scale_colsum(const float* g, int64_t n, int64_t K, int64_t ldg, const float* rowscale, float* out,
                                       int64_t Kout, int64_t ldo, float* colsum, void* workspace,
                                       int64_t workspace_bytes, void* stream);
+/* The same pass with an unscaled zero-padded copy of g beside the scaled one (same Kout and ldo). */
+EXACT_API int exact_rows_scale_copy_colsum(const float* g, int64_t n, int64_t K, int64_t ldg, const float* rowscale, float* out,
+                                           float* copy, int64_t Kout, int64_t ldo, float* colsum, void* workspace,
+                                           int64_t workspace_bytes, void* stream);
 /* The same pass with an fp16 copy of g in place of the scaled one: out_f16 [n, ldo] halves, zero-padded to Kout columns. */
 EXACT_API int exact_rows_half_colsum(const float* g, int64_t n, int64_t K, int64_t ldg, void* out_f16, int64_t Kout, int64_t ldo,
                                      float* colsum, void* workspace, int64_t workspace_bytes, void* stream);
@@ -414,6 +422,11 @@ EXACT_API int exact_rp_quantize_pack(const float* x, int64_t N, int64_t D, const
                                      uint64_t seed, uint64_t offset, int64_t row_offset, void* workspace,
                                      uint8_t* packed, uint16_t* scale_bf16, uint16_t* min_bf16, float* y_out,
                                      void* stream);
+/* The same on rows of pitch ldx >= D elements: rows padded to 16-byte pieces take the tensor-map path whatever D is. */
+EXACT_API int exact_rp_quantize_pack_rows(const float* x, int64_t N, int64_t D, int64_t ldx, const float* R, int64_t k, int bits,
+                                          uint64_t seed, uint64_t offset, int64_t row_offset, void* workspace,
+                                          uint8_t* packed, uint16_t* scale_bf16, uint16_t* min_bf16, float* y_out,
+                                          void* stream);
 
 /* Fused unpack + dequantise + transpose projection: the backward chain dequantize_activation ->
  * rp2input of exact/exact/ops.py:164-166 (unpack_single_precision, quantization.cc:50-62, then
@@ -447,7 +460,8 @@ EXACT_API int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t
                                    const float* A2, int64_t K2, int64_t lda2, const float* B2, int64_t ldb2,
                                    int64_t N, const float* bias, int accumulate, void* workspace, float* C,
                                    int64_t ldc, void* stream);
-/* exact_linear_forward with two more choices.  incb, incb2: distance between the elements of a row of B, B2 (ldb = 1 and incb =
+/* exact_linear_forward with three more choices.  addend: [M, N] with pitch ldadd, added to the product in place of what C held
+ * (NULL: nothing; it may be C).  incb, incb2: distance between the elements of a row of B, B2 (ldb = 1 and incb =
  * the pitch: the transposed weight, without a copy).  k_chunk: the contraction is cut into chunks of k_chunk columns (a
  * multiple of 32; 0: one chunk).  The tensor core truncates its fp32 accumulator at every MMA, a bias of about 7e-9 of the
  * result per contracted column; each chunk's sum is added to the previous ones by an fp32 addition instead (at 256 columns
@@ -455,9 +469,9 @@ EXACT_API int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t
 EXACT_API int64_t exact_linear_partial_bytes(int64_t N);
 EXACT_API int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb,
                                            int64_t incb, const float* A2, int64_t K2, int64_t lda2, const float* B2,
-                                           int64_t ldb2, int64_t incb2, int64_t N, const float* bias, int accumulate,
-                                           int64_t k_chunk, float* partial, void* workspace, float* C, int64_t ldc,
-                                           void* stream);
+                                           int64_t ldb2, int64_t incb2, int64_t N, const float* bias, const float* addend,
+                                           int64_t ldadd, int64_t k_chunk, float* partial, void* workspace, float* C,
+                                           int64_t ldc, void* stream);
 
 /* Weight gradient of a quantised linear layer from the packed activation(s), on the tensor cores:
  *     out[O, kpad] = g^T [O x N] . dequantise(packed) [N x k]
