@@ -16,21 +16,30 @@
 // rows, but an infinite element turns its output row into NaN where an fp32 GEMM gives +-inf (its tail is
 // inf - inf).
 //
-// Structure (one CTA per SM, persistent over 128-row tiles of A, 14 warps):
-//   warp 0     TMA producer.  Shared memory is a 192 KB ring of K-tile stages; a 32-column K tile uses three
-//              parts: A (raw fp32 [128 x 32], 16 KB, the tail tile goes into the part's other half),
-//              B_hi [Npad x 32] and B_lo [Npad x 32]: two stages at Npad = 256, up to four for narrow
+// Structure (one CTA per SM, persistent over 128-row tiles of A, 18 warps).  Two CTAs of a cluster work as a pair on two
+// neighbouring tiles (tcgen05.mma.cta_group::2, M = 256): each holds its rows of A and half of the rows of B, so a CTA fetches and
+// its tensor core reads half as much of B, which is what the product is bound by once the roles keep up (at 256 x 256 the
+// shared-memory traffic of a K tile takes as long as its MMAs), and the ring holds three K tiles instead of two.
+//   warp 0     producer.  Shared memory is a 192 KB ring of K-tile stages; a 32-column K tile uses three
+//              parts: A (raw fp32 [128 x 32] by TMA, 16 KB, the tail tile goes into the part's other half),
+//              B_hi and B_lo (the CTA's rows x 32, one contiguous run): three stages at Npad = 256, four for narrow
 //              outputs.  128-byte swizzle, no multicast.
 //              The A tile of four K tiles ahead is requested into L2 (tensor prefetch): A is read from
-//              HBM exactly once and the ring is only two K tiles deep.
-//   warps 2-9  converter: rewrite the raw A tile in place as a_hi and write a_lo beside it (same swizzled
-//              offsets), fence.proxy.async, signal.
-//   warp 1     MMA issuer: tcgen05.mma.cta_group::1.kind::tf32, M = 128, N = Npad, K = 8; per K tile
-//              8 MMAs (hi*hi, lo*hi) then release B_hi, 4 MMAs (hi*lo) then release A and B_lo.
-//              Accumulators are double-buffered in TMEM.
-//   warps 10-13 epilogue: tcgen05.ld -> per-warp staging tile in shared memory -> (+ bias, + old C)
-//              -> coalesced global stores.
-// B_hi / B_lo are produced once per call from the (small) weight matrix by a preparation kernel.
+//              HBM exactly once and the ring is only a few K tiles deep.
+//   warps 2-9  converters: rewrite the raw A tile in place as a_hi and write a_lo beside it (same swizzled
+//              offsets), fence.proxy.async, signal.  Two groups of four take alternate K tiles: a K tile is a chain of wait,
+//              reads, conversions, stores, fence and arrival, 1,250 cycles whatever the width of the output.  The first
+//              warp of a group also waits for B, so that the issuing thread has one wait per K tile.
+//   warp 1     MMA issuer (of the pair's first CTA): kind::tf32, N = Npad, K = 8; per K tile 12 MMAs (hi*hi, lo*hi, hi*lo),
+//              then one commit that frees the stage (in both CTAs).  Its chain of waits and index arithmetic was what the
+//              kernel was bound by (2,500 cycles per K tile at any width; the MMAs take 1,536 at 256 columns): stage and
+//              parity are counted instead of divided out.  Accumulators are double-buffered in TMEM.
+//   warps 10-17 epilogue: tcgen05.ld -> per-warp staging tile in shared memory -> (+ bias, + addend)
+//              -> coalesced global stores; two groups of four take alternate blocks of 32 columns.
+// Measured (us, before -> now): 2,449,029 x 256 -> 256: 1,673 -> 1,400, with a second operand pair of 256 3,365 -> 2,460; 48 -> 256:
+// 1,046 -> 630; 256 -> 47: 1,305 -> 880; 232,965 x 604 -> 256: 368 -> 299; 169,343 x 128 -> 256: 100 -> 66.  With the pair alone and
+// the chains as they were it lost (1,710 -> 2,008).
+// The weight is split, padded and laid out as the tiles once per call by a preparation kernel.
 //
 // Every mbarrier wait is bounded; on expiry the CTA raises an abort flag, all roles leave their loops,
 // bulk copies in flight are waited for (bounded), TMEM is freed and the status word is set.
@@ -43,17 +52,19 @@ namespace exb {
 
 constexpr int kLinTileM = 128;
 constexpr int kLinTileK = 32;
-constexpr int kLinConvWarps = 8;
-constexpr int kLinThreads = (2 + kLinConvWarps + 4) * 32;   // TMA, MMA, converters, epilogue
+constexpr int kLinConvWarps = 8;                // in two groups that take alternate K tiles
+constexpr int kLinConvGroup = kLinConvWarps / 2;
+constexpr int kLinEpiGroups = 2;                // four warps each (one per 32 lanes of TMEM), alternate column blocks
+constexpr int kLinThreads = (2 + kLinConvWarps + 4 * kLinEpiGroups) * 32;   // TMA, MMA, converters, epilogue
 constexpr int kLinSlots = 6;                    // ring capacity in 32 KB units
 constexpr int kLinMaxStages = 4;
-constexpr int kLinBars = kLinMaxStages * 3;
 constexpr uint32_t kLinSlotBytes = 32 * 1024;
 constexpr uint32_t kLinHalf = 16 * 1024;        // raw / tail halves of an A slot
-constexpr int kLinSleepNs = 200;                // back-off between polls of the roles that wait long (producer, epilogue)
+constexpr int kLinSleepNs = 200;                // back-off between polls of the epilogue, which waits long
 constexpr int kLinPrefetch = 4;                 // K tiles of A requested into L2 ahead of their TMA load
 
 struct LinParams {
+  const float* b;         // heads and tails of the weight, as linear_prepare_kernel lays them out
   float* C;
   const float* bias;
   int* status;
@@ -66,8 +77,8 @@ struct LinParams {
   long long ldadd;
   int chunk;               // K tiles that are accumulated in TMEM before their sum is taken over in fp32
   float* partial;          // [grid, Npad / 4, 128, 4]: running sums of the chunks before the last, per CTA
-  int stages;              // K tiles the ring holds (2 at Npad = 256, up to 4 for narrow outputs)
-  unsigned b_slot;         // bytes of a B_hi / B_lo slot = Npad * 128
+  int stages;              // K tiles the ring holds
+  unsigned b_slot;         // bytes of a B_hi / B_lo slot: 128 per row of B in this CTA
   unsigned stage_bytes;    // A slot (32 KB) + two B slots
   unsigned tmem_cols;
 };
@@ -86,114 +97,132 @@ __device__ __forceinline__ void fence_proxy_async_smem_lin() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// Part `it` of the stream of ring parts (three per K tile: A, B_hi, B_lo): barrier index, phase, address.
-struct LinPart { int b; uint32_t ph; uint32_t addr; };
-__device__ __forceinline__ LinPart lin_part(int it, const LinParams& p, uint32_t ring) {
-  const int kt = it / 3, part = it - kt * 3;
-  const int stage = kt % p.stages;
-  LinPart r;
-  r.b = stage * 3 + part;
-  r.ph = (uint32_t)(kt / p.stages) & 1u;
-  r.addr = ring + (uint32_t)stage * p.stage_bytes +
-           (part == 0 ? 0u : (part == 1 ? kLinSlotBytes : kLinSlotBytes + p.b_slot));
-  return r;
-}
+// The ring's next stage and the parity of its round.
+struct LinStage {
+  int s = 0;
+  uint32_t ph = 0;
+  __device__ __forceinline__ void next(int stages) {
+    if (++s == stages) {
+      s = 0;
+      ph ^= 1u;
+    }
+  }
+};
 
 // CHUNKED: the contraction is drained from TMEM every p.chunk K tiles (a kernel of its own: its epilogue's registers and
 // code cost the unchunked product 5 %).
-template <bool CHUNKED>
+template <bool CHUNKED, bool PAIR>
 __global__ void __launch_bounds__(kLinThreads, 1)
 linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_a2,
-                     const __grid_constant__ CUtensorMap tm_bh, const __grid_constant__ CUtensorMap tm_bl,
                      const __grid_constant__ LinParams p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) unsigned long long s_full[kLinBars];
-  __shared__ __align__(8) unsigned long long s_empty[kLinBars];
-  __shared__ __align__(8) unsigned long long s_conv[kLinBars];
+  __shared__ __align__(8) unsigned long long s_full[kLinMaxStages];    // A has landed
+  __shared__ __align__(8) unsigned long long s_bfull[kLinMaxStages];   // B has landed
+  __shared__ __align__(8) unsigned long long s_ready[kLinMaxStages];   // A is split (in both CTAs of a pair) and B is there
+  __shared__ __align__(8) unsigned long long s_empty[kLinMaxStages];
   __shared__ __align__(8) unsigned long long s_tfull[2];
   __shared__ __align__(8) unsigned long long s_tempty[2];
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = PAIR ? (int)cluster_rank() : 0;
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t stage_base = ring + kLinSlots * kLinSlotBytes;   // 4 x 4 KB epilogue staging tiles
+  const uint32_t stage_base = ring + kLinSlots * kLinSlotBytes;   // 4 KB of staging per epilogue warp
   volatile int* abort_flag = &s_abort;
 
   if (threadIdx.x == 0) {
     s_abort = 0;
-    for (int s = 0; s < kLinBars; s++) {
+    for (int s = 0; s < kLinMaxStages; s++) {
       mbar_init(smem_u32(&s_full[s]), 1);
+      mbar_init(smem_u32(&s_bfull[s]), 1);
+      mbar_init(smem_u32(&s_ready[s]), PAIR ? 2 * kLinConvGroup : kLinConvGroup);   // one arrival per converter warp
       mbar_init(smem_u32(&s_empty[s]), 1);
-      mbar_init(smem_u32(&s_conv[s]), kLinConvWarps);   // one arrival per converter warp
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(smem_u32(&s_tfull[b]), 1);
-      mbar_init(smem_u32(&s_tempty[b]), 4);
+      mbar_init(smem_u32(&s_tempty[b]), (PAIR ? 8 : 4) * kLinEpiGroups);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(smem_u32(&s_tmem_base), p.tmem_cols);
+  if (warp == 1) {
+    if (PAIR) tmem_alloc_pair(smem_u32(&s_tmem_base), p.tmem_cols);
+    else tmem_alloc(smem_u32(&s_tmem_base), p.tmem_cols);
+  }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();     // the other CTA arrives on these barriers
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
 
-  const int first = blockIdx.x, step = gridDim.x;
-  const uint32_t b_bytes = (uint32_t)p.Npad * kLinTileK * 4;
+  // the tiles of a pair are neighbours; one past the last (an odd number of tiles) reads zeros and stores nothing
+  const int first = blockIdx.x, step = gridDim.x, tiles = PAIR ? (p.num_tiles + 1) / 2 * 2 : p.num_tiles;
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      int it = 0;   // slot uses so far (three per K tile)
+      LinStage st;
+      int uses = 0;   // K tiles requested so far, at most p.stages
       bool ok = true;
-      for (int tile = first; tile < p.num_tiles && ok; tile += step) {
-        for (int kb = 0; kb < p.kblocks && ok; kb++) {
-          for (int u = 0; u < 3; u++, it++) {
-            const LinPart pt_ = lin_part(it, p, ring);
-            if (!mbar_wait<kLinSleepNs>(smem_u32(&s_empty[pt_.b]), pt_.ph ^ 1u, abort_flag)) { ok = false; break; }
-            const uint32_t full = smem_u32(&s_full[pt_.b]);
-            const uint32_t dst = pt_.addr;
-            if (u == 0) {
-              mbar_arrive_expect_tx(full, kLinHalf);
-              if (kb < p.kblocks1) tma_load_2d(dst, &tm_a, kb * kLinTileK, tile * kLinTileM, full);
-              else tma_load_2d(dst, &tm_a2, (kb - p.kblocks1) * kLinTileK, tile * kLinTileM, full);
-              // A comes from HBM exactly once: pull the tile that will be loaded kLinPrefetch K tiles from
-              // now into L2, so that its TMA load later pays L2 latency only (the ring holds two K tiles)
-              int pk = kb + kLinPrefetch, pt = tile;
-              if (pk >= p.kblocks) { pk -= p.kblocks; pt += step; }
-              if (pt < p.num_tiles && pk < p.kblocks) {
-                if (pk < p.kblocks1) tma_prefetch_2d(&tm_a, pk * kLinTileK, pt * kLinTileM);
-                else tma_prefetch_2d(&tm_a2, (pk - p.kblocks1) * kLinTileK, pt * kLinTileM);
-              }
-            } else {
-              mbar_arrive_expect_tx(full, b_bytes);
-              tma_load_2d(dst, u == 1 ? &tm_bh : &tm_bl, kb * kLinTileK, 0, full);
-            }
+      for (int tile = first; tile < tiles && ok; tile += step) {
+        for (int kb = 0; kb < p.kblocks; kb++, st.next(p.stages)) {
+          if (!mbar_wait(smem_u32(&s_empty[st.s]), st.ph ^ 1u, abort_flag)) { ok = false; break; }
+          const uint32_t full = smem_u32(&s_full[st.s]), bfull = smem_u32(&s_bfull[st.s]);
+          const uint32_t dst = ring + (uint32_t)st.s * p.stage_bytes;
+          mbar_arrive_expect_tx(full, kLinHalf);
+          if (kb < p.kblocks1) tma_load_2d(dst, &tm_a, kb * kLinTileK, tile * kLinTileM, full);
+          else tma_load_2d(dst, &tm_a2, (kb - p.kblocks1) * kLinTileK, tile * kLinTileM, full);
+          mbar_arrive_expect_tx(bfull, 2 * p.b_slot);
+          bulk_load(dst + kLinSlotBytes, reinterpret_cast<const char*>(p.b) + (size_t)(PAIR ? 2 * kb + rank : kb) * (2 * p.b_slot),
+                    2 * p.b_slot, bfull);
+          if (uses < p.stages) uses++;
+          // A comes from HBM exactly once: pull the tile that will be loaded kLinPrefetch K tiles from
+          // now into L2, so that its TMA load later pays L2 latency only (the ring holds two or three K tiles)
+          int pk = kb + kLinPrefetch, pt = tile;
+          if (pk >= p.kblocks) { pk -= p.kblocks; pt += step; }
+          if (pt < p.num_tiles && pk < p.kblocks) {
+            if (pk < p.kblocks1) tma_prefetch_2d(&tm_a, pk * kLinTileK, pt * kLinTileM);
+            else tma_prefetch_2d(&tm_a2, (pk - p.kblocks1) * kLinTileK, pt * kLinTileM);
           }
         }
       }
-      if (!ok) {
-        // leave no bulk copy in flight: wait (bounded) for every slot that was armed last
-        const long long t0 = clock64();
-        for (int j = 0; j < p.stages * 3 && j < it; j++) {
-          const LinPart q = lin_part(it - 1 - j, p, ring);
-          const uint32_t bar = smem_u32(&s_full[q.b]);
-          const uint32_t ph = q.ph;
-          while (!mbar_try_wait(bar, ph) && clock64() - t0 < kWaitLimitCycles) {}
+      // the latest round of every stage that was used: the stage before `st` and those before it
+      const long long t0 = clock64();
+      for (int j = 0; j < uses; j++) {
+        if (--st.s < 0) {
+          st.s = p.stages - 1;
+          st.ph ^= 1u;
+        }
+        if (PAIR && ok) {
+          // the pair's commits arrive in both CTAs: none may be under way when one of them exits
+          ok = mbar_wait(smem_u32(&s_empty[st.s]), st.ph, abort_flag);
+        }
+        if (!ok) {
+          // leave no bulk copy in flight (bounded)
+          while (!(mbar_try_wait(smem_u32(&s_full[st.s]), st.ph) && mbar_try_wait(smem_u32(&s_bfull[st.s]), st.ph)) &&
+                 clock64() - t0 < kWaitLimitCycles) {}
         }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_tf32(kLinTileM, p.Npad);
-      int it = 0, t = 0;
+    if (lane == 0 && rank == 0) {   // the first CTA of a pair issues for both
+      const uint32_t idesc = umma_idesc_tf32(PAIR ? 2 * kLinTileM : kLinTileM, p.Npad);
+      auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+        if (PAIR) umma_tf32_pair(d, a, b, idesc, acc);
+        else umma_tf32(d, a, b, idesc, acc);
+      };
+      auto commit = [&](uint32_t bar) {
+        if (PAIR) umma_commit_pair(bar);
+        else umma_commit(bar);
+      };
+      LinStage st;
+      int t = 0;
       bool ok = true;
-      for (int tile = first; tile < p.num_tiles && ok; tile += step) {
+      for (int tile = first; tile < tiles && ok; tile += step) {
         int buf = 0;
         uint32_t d_tmem = 0;
-        for (int kb = 0; kb < p.kblocks; kb++, it += 3) {
+        for (int kb = 0; kb < p.kblocks; kb++, st.next(p.stages)) {
           const bool opens = CHUNKED ? kb % p.chunk == 0 : kb == 0;
           if (opens) {
             buf = t & 1;
@@ -203,97 +232,103 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
             d_tmem = tmem_base + (uint32_t)(buf * p.Npad);
             t++;
           }
-          const LinPart qa = lin_part(it, p, ring), qh = lin_part(it + 1, p, ring), ql = lin_part(it + 2, p, ring);
-          const int sa = qa.b, sh = qh.b, sl = ql.b;
-          const uint32_t pl = ql.ph;
-          if (!mbar_wait(smem_u32(&s_conv[sa]), qa.ph, abort_flag)) { ok = false; break; }
-          if (!mbar_wait(smem_u32(&s_full[sh]), qh.ph, abort_flag)) { ok = false; break; }
+          if (!mbar_wait(smem_u32(&s_ready[st.s]), st.ph, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const uint64_t ahi = umma_desc_sw128(qa.addr);
-          const uint64_t alo = umma_desc_sw128(qa.addr + kLinHalf);
-          const uint64_t bhi = umma_desc_sw128(qh.addr);
-          const uint64_t blo = umma_desc_sw128(ql.addr);
+          const uint32_t base = ring + (uint32_t)st.s * p.stage_bytes;
+          const uint64_t ahi = umma_desc_sw128(base);
+          const uint64_t alo = umma_desc_sw128(base + kLinHalf);
+          const uint64_t bhi = umma_desc_sw128(base + kLinSlotBytes);
+          const uint64_t blo = umma_desc_sw128(base + kLinSlotBytes + p.b_slot);
 #pragma unroll
           for (int k4 = 0; k4 < kLinTileK / 8; k4++) {
             const uint64_t o = (uint64_t)(k4 * 2);   // 8 tf32 = 32 bytes along K inside the swizzle atom
-            umma_tf32(d_tmem, alo + o, bhi + o, idesc, !opens || k4 != 0);
-            umma_tf32(d_tmem, ahi + o, bhi + o, idesc, 1);
+            mma(d_tmem, alo + o, bhi + o, !opens || k4 != 0);
+            mma(d_tmem, ahi + o, bhi + o, 1);
           }
-          umma_commit(smem_u32(&s_empty[sh]));
-          if (!mbar_wait(smem_u32(&s_full[sl]), pl, abort_flag)) { ok = false; break; }
-          tc_fence_after();
 #pragma unroll
           for (int k4 = 0; k4 < kLinTileK / 8; k4++) {
             const uint64_t o = (uint64_t)(k4 * 2);
-            umma_tf32(d_tmem, ahi + o, blo + o, idesc, 1);
+            mma(d_tmem, ahi + o, blo + o, 1);
           }
-          umma_commit(smem_u32(&s_empty[sa]));
-          umma_commit(smem_u32(&s_empty[sl]));
-          if ((CHUNKED && (kb + 1) % p.chunk == 0) || kb + 1 == p.kblocks) umma_commit(smem_u32(&s_tfull[buf]));
+          commit(smem_u32(&s_empty[st.s]));
+          if ((CHUNKED && (kb + 1) % p.chunk == 0) || kb + 1 == p.kblocks) commit(smem_u32(&s_tfull[buf]));
         }
       }
     }
   } else if (warp < 2 + kLinConvWarps) {
     // ---------------- converter: warps 2 .. 2 + kLinConvWarps - 1 ----------------
-    const int ct = threadIdx.x - 64;   // 0 .. 32 * kLinConvWarps - 1
-    constexpr int kPer = (int)(kLinHalf / 16) / (32 * kLinConvWarps);   // 16-byte chunks per thread
-    int it = 0;
+    const int group = (warp - 2) / kLinConvGroup, ct = threadIdx.x - 64 - group * 32 * kLinConvGroup;
+    constexpr int kPer = (int)(kLinHalf / 16) / (32 * kLinConvGroup);   // 16-byte chunks per thread
+    constexpr int kBatch = 4;
+    LinStage st;
+    int turn = group;
     bool ok = true;
-    for (int tile = first; tile < p.num_tiles && ok; tile += step) {
-      for (int kb = 0; kb < p.kblocks; kb++, it += 3) {
-        const LinPart qa = lin_part(it, p, ring);
-        const int s = qa.b;
-        if (!mbar_wait(smem_u32(&s_full[s]), qa.ph, abort_flag)) { ok = false; break; }
-        const uint32_t base = qa.addr + (uint32_t)ct * 16u;
+    for (int tile = first; tile < tiles && ok; tile += step) {
+      for (int kb = 0; kb < p.kblocks; kb++, st.next(p.stages), turn ^= 1) {
+        if (turn) continue;
+        if (!mbar_wait(smem_u32(&s_full[st.s]), st.ph, abort_flag)) { ok = false; break; }
+        const uint32_t base = ring + (uint32_t)st.s * p.stage_bytes + (uint32_t)ct * 16u;
 #pragma unroll
-        for (int i = 0; i < kPer; i++) {
-          const uint32_t addr = base + (uint32_t)i * (32u * kLinConvWarps * 16u);
-          float a[4], h[4], l[4];
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]) : "r"(addr));
+        for (int i0 = 0; i0 < kPer; i0 += kBatch) {
+          float a[kBatch][4];
 #pragma unroll
-          for (int e = 0; e < 4; e++) h[e] = __uint_as_float(rna_tf32(a[e]));
+          for (int i = 0; i < kBatch; i++)
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a[i][0]), "=f"(a[i][1]), "=f"(a[i][2]), "=f"(a[i][3])
+                         : "r"(base + (uint32_t)(i0 + i) * (32u * kLinConvGroup * 16u)));
 #pragma unroll
-          for (int e = 0; e < 4; e += 2) {   // tails: paired subtract, then round to tf32
-            float d0, d1;
-            f2_unpack(f2_sub(f2_pack(a[e], a[e + 1]), f2_pack(h[e], h[e + 1])), d0, d1);
-            l[e] = __uint_as_float(rna_tf32(d0));
-            l[e + 1] = __uint_as_float(rna_tf32(d1));
+          for (int i = 0; i < kBatch; i++) {
+            const uint32_t addr = base + (uint32_t)(i0 + i) * (32u * kLinConvGroup * 16u);
+            float h[4], l[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) h[e] = __uint_as_float(rna_tf32(a[i][e]));
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {   // tails: paired subtract, then round to tf32
+              float d0, d1;
+              f2_unpack(f2_sub(f2_pack(a[i][e], a[i][e + 1]), f2_pack(h[e], h[e + 1])), d0, d1);
+              l[e] = __uint_as_float(rna_tf32(d0));
+              l[e + 1] = __uint_as_float(rna_tf32(d1));
+            }
+            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(h[0]), "f"(h[1]), "f"(h[2]), "f"(h[3]) : "memory");
+            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr + kLinHalf), "f"(l[0]), "f"(l[1]), "f"(l[2]), "f"(l[3]) : "memory");
           }
-          asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(h[0]), "f"(h[1]), "f"(h[2]), "f"(h[3]) : "memory");
-          asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr + kLinHalf), "f"(l[0]), "f"(l[1]), "f"(l[2]), "f"(l[3]) : "memory");
         }
         fence_proxy_async_smem_lin();  // generic-proxy stores -> visible to the tensor core's reads
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&s_conv[s]));
+        if (ct < 32 && !mbar_wait(smem_u32(&s_bfull[st.s]), st.ph, abort_flag)) { ok = false; break; }   // for the MMA's one wait
+        if (lane == 0) {
+          if (PAIR) mbar_arrive_leader(smem_u32(&s_ready[st.s]));
+          else mbar_arrive(smem_u32(&s_ready[st.s]));
+        }
       }
     }
   } else {
-    // ---------------- epilogue: the last four warps ----------------
+    // ---------------- epilogue: the last warps ----------------
     const int quad = warp & 3;   // TMEM lanes 32*quad .. 32*quad+31
+    const int share = (warp - 2 - kLinConvWarps) / 4;   // every kLinEpiGroups-th block of columns
     const bool vec = (p.N & 3) == 0 && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 &&
                      (p.addend == nullptr || ((p.ldadd & 3) == 0 && (reinterpret_cast<uintptr_t>(p.addend) & 15) == 0));
-    const uint32_t stage_addr = stage_base + (uint32_t)quad * 4096u;
+    const uint32_t stage_addr = stage_base + (uint32_t)(share * 4 + quad) * 4096u;
     int t = 0;
     bool ok = true;
     const int chunks = CHUNKED ? (p.kblocks + p.chunk - 1) / p.chunk : 1;
     // this thread's row of the running sums: 16 bytes per four columns, adjacent lanes adjacent
     float4* __restrict__ part = !CHUNKED ? nullptr : reinterpret_cast<float4*>(p.partial) + (size_t)blockIdx.x * (p.Npad / 4) * kLinTileM + quad * 32 + lane;
-    for (int tile = first; tile < p.num_tiles && ok; tile += step) {
+    for (int tile = first; tile < tiles && ok; tile += step) {
       for (int ch = 0; CHUNKED && ch + 1 < chunks && ok; ch++, t++) {
         const int buf = t & 1;
         if (!mbar_wait<kLinSleepNs>(smem_u32(&s_tfull[buf]), (uint32_t)(t >> 1) & 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.Npad);
-        for (int c0 = 0; c0 < p.Npad; c0 += 64) {
-          const int cols = p.Npad - c0 < 64 ? p.Npad - c0 : 64;
-          float4 old[16];
+        for (int c0 = share * 32; c0 < p.Npad; c0 += 32 * kLinEpiGroups) {
+          const int cols = p.Npad - c0 < 32 ? p.Npad - c0 : 32;
+          float4 old[8];
           if (ch > 0) {
 #pragma unroll
-            for (int j = 0; j < 16; j++)
+            for (int j = 0; j < 8; j++)
               if (j * 4 < cols) old[j] = __ldcg(part + (size_t)(c0 / 4 + j) * kLinTileM);
           }
 #pragma unroll
-          for (int h = 0; h < 4; h++) {
+          for (int h = 0; h < 2; h++) {
             if (h * 16 < cols) {
               float v[16];
               tmem_ld16(taddr + (uint32_t)(c0 + h * 16), v);
@@ -311,7 +346,10 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&s_tempty[buf]));
+        if (lane == 0) {
+        if (PAIR) mbar_arrive_leader(smem_u32(&s_tempty[buf]));
+        else mbar_arrive(smem_u32(&s_tempty[buf]));
+      }
       }
       if (!ok) break;
       const int buf = t & 1;
@@ -323,12 +361,12 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         for (int j = 0; j < 8; j++)
           if (c0 + j * 4 < p.Npad) sum[j] = __ldcg(part + (size_t)(c0 / 4 + j) * kLinTileM);
       };
-      if (CHUNKED) fetch(0);
+      if (CHUNKED) fetch(share * 32);
       if (!mbar_wait<kLinSleepNs>(smem_u32(&s_tfull[buf]), ph, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.Npad);
       const long long row_base = (long long)tile * kLinTileM + quad * 32;
-      for (int c0 = 0; c0 < p.Npad; c0 += 32) {
+      for (int c0 = share * 32; c0 < p.Npad; c0 += 32 * kLinEpiGroups) {
         const int cols = (p.Npad - c0) < 32 ? (p.Npad - c0) : 32;   // 16 or 32
         for (int h = 0; h * 16 < cols; h++) {
           float v[16];
@@ -349,7 +387,7 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                          : "memory");
           }
         }
-        if (CHUNKED && c0 + 32 < p.Npad) fetch(c0 + 32);
+        if (CHUNKED && c0 + 32 * kLinEpiGroups < p.Npad) fetch(c0 + 32 * kLinEpiGroups);
         __syncwarp();
         const uint32_t ci = (uint32_t)lane & 7u;
         const int c = c0 + (int)ci * 4;
@@ -388,29 +426,36 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&s_tempty[buf]));
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_leader(smem_u32(&s_tempty[buf]));
+        else mbar_arrive(smem_u32(&s_tempty[buf]));
+      }
     }
   }
 
   // ---------------- teardown ----------------
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, p.tmem_cols);
+    if (PAIR) tmem_dealloc_pair(tmem_base, p.tmem_cols);
+    else tmem_dealloc(tmem_base, p.tmem_cols);
   }
+  if (PAIR) cluster_sync();
   if (threadIdx.x == 0 && s_abort) {
     atomicExch(p.status, 1);
     raise_status(p.lib_status, EXB_STATUS_LINEAR);
   }
 }
 
-// Heads and tails of [B | B2] (rows = output features), zero padded to [Npad, Kpad1 + Kpad2]; also
-// clears the status word.
+// Heads and tails of [B | B2] (rows = output features), zero padded to [Npad, Kpad1 + Kpad2], in the order and with the swizzle
+// of the shared-memory tiles: K tile by K tile, in it the share of each CTA of a pair (b_rows rows), in that the heads and then
+// the tails, so that a CTA's part of a K tile is one contiguous run.  Also clears the status word.
 __global__ void linear_prepare_kernel(const float* __restrict__ B, int K, long long ldb, long long incb,
                                       const float* __restrict__ B2, int K2, long long ldb2, long long incb2, int N, int Npad,
                                       int Kpad1, int Kpad,
-                                      float* __restrict__ bh, float* __restrict__ bl, int* status) {
+                                      int b_rows, float* __restrict__ out, int* status) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *status = 0;
   if (i >= Npad * Kpad) return;
@@ -425,8 +470,10 @@ __global__ void linear_prepare_kernel(const float* __restrict__ B, int K, long l
   }
   float hi, lo;
   split_tf32(v, hi, lo);
-  bh[i] = hi;
-  bl[i] = lo;
+  const int share = n / b_rows, r = n - share * b_rows, kb = kk / kLinTileK, e = kk - kb * kLinTileK;
+  const size_t at = (size_t)(kb * (Npad / b_rows) + share) * 2 * b_rows * kLinTileK + r * kLinTileK + (((e >> 2) ^ (r & 7)) << 2) + (e & 3);
+  out[at] = hi;
+  out[at + (size_t)b_rows * kLinTileK] = lo;
 }
 
 static inline int lin_kpad(long long K) { return (int)((K + kLinTileK - 1) / kLinTileK * kLinTileK); }
@@ -477,14 +524,17 @@ int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t l
   const int Npad = (int)((N + 15) / 16 * 16);
   const int Kpad1 = lin_kpad(K), Kpad2 = lin_kpad(K2), Kpad = Kpad1 + Kpad2;
   int* status = reinterpret_cast<int*>(workspace);
-  float* bh = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + 256);
-  float* bl = bh + (size_t)Npad * Kpad;
+  float* b = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + 256);
+  const int num_tiles = (int)((M + kLinTileM - 1) / kLinTileM);
+  // Pairs need whole 16-row groups of B in each half; a single tile has no partner.
+  const bool pair = num_tiles >= 2 && Npad % 32 == 0;
+  const int b_rows = pair ? Npad / 2 : Npad;   // of B in one CTA
 
   linear_prepare_kernel<<<(Npad * Kpad + 255) / 256, 256, 0, st>>>(B, (int)K, ldb, incb, B2, (int)K2, ldb2, incb2, (int)N, Npad,
-                                                                   Kpad1, Kpad, bh, bl, status);
+                                                                   Kpad1, Kpad, b_rows, b, status);
   EXB_CUDA_OK(cudaGetLastError());
 
-  CUtensorMap tm_a, tm_a2, tm_bh, tm_bl;
+  CUtensorMap tm_a, tm_a2;
   int rc = make_tensor_map_2d_f32(&tm_a, A, (unsigned long long)K, (unsigned long long)M, (unsigned long long)lda * 4, kLinTileK, kLinTileM);
   if (rc) return rc;
   if (K2 > 0) {
@@ -493,31 +543,41 @@ int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t l
   } else {
     tm_a2 = tm_a;
   }
-  rc = make_tensor_map_2d_f32(&tm_bh, bh, (unsigned long long)Kpad, (unsigned long long)Npad, (unsigned long long)Kpad * 4, kLinTileK, (unsigned)Npad);
-  if (rc) return rc;
-  rc = make_tensor_map_2d_f32(&tm_bl, bl, (unsigned long long)Kpad, (unsigned long long)Npad, (unsigned long long)Kpad * 4, kLinTileK, (unsigned)Npad);
-  if (rc) return rc;
 
   LinParams p{};
-  p.C = C; p.bias = bias; p.status = status; p.lib_status = status_word_ptr(); p.M = M; p.ldc = ldc; p.N = (int)N; p.Npad = Npad;
+  p.b = b; p.C = C; p.bias = bias; p.status = status; p.lib_status = status_word_ptr(); p.M = M; p.ldc = ldc; p.N = (int)N; p.Npad = Npad;
   p.kblocks1 = Kpad1 / kLinTileK; p.kblocks = Kpad / kLinTileK;
-  p.num_tiles = (int)((M + kLinTileM - 1) / kLinTileM);
+  p.num_tiles = num_tiles;
   p.addend = addend; p.ldadd = ldadd;
   p.chunk = k_chunk > 0 ? (int)(k_chunk / kLinTileK) : p.kblocks;
   p.partial = partial;
-  p.b_slot = (unsigned)Npad * kLinTileK * 4;
+  p.b_slot = (unsigned)b_rows * kLinTileK * 4;
   p.stage_bytes = kLinSlotBytes + 2 * p.b_slot;
   p.stages = (int)((kLinSlots * kLinSlotBytes) / p.stage_bytes);
   if (p.stages > kLinMaxStages) p.stages = kLinMaxStages;
   unsigned cols = 32;
   while (cols < (unsigned)(2 * Npad)) cols <<= 1;
   p.tmem_cols = cols;
-  const size_t dyn = (size_t)kLinSlots * kLinSlotBytes + 4 * 4096 + 1024;
+  const size_t dyn = (size_t)kLinSlots * kLinSlotBytes + 4 * kLinEpiGroups * 4096 + 1024;
+  const bool chunked = p.chunk < p.kblocks;
+  auto* kern = pair ? (chunked ? linear_tf32x3_kernel<true, true> : linear_tf32x3_kernel<false, true>)
+                    : (chunked ? linear_tf32x3_kernel<true, false> : linear_tf32x3_kernel<false, false>);
+  EXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
   int grid = sm_count();
   if (grid > p.num_tiles) grid = p.num_tiles;
-  auto* kern = p.chunk < p.kblocks ? linear_tf32x3_kernel<true> : linear_tf32x3_kernel<false>;
-  EXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-  kern<<<grid, kLinThreads, dyn, st>>>(tm_a, tm_a2, tm_bh, tm_bl, p);
+  if (pair) grid = grid == sm_count() ? grid / 2 * 2 : (grid + 1) / 2 * 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kLinThreads);
+  cfg.dynamicSmemBytes = dyn;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pair ? 1 : 0;
+  EXB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tm_a, tm_a2, p));
   EXB_CUDA_OK(cudaGetLastError());
   return EXB_OK;
 }
