@@ -143,6 +143,18 @@ __device__ __forceinline__ void gw_column(uint32_t from, uint32_t pitch, int sli
   }
 }
 
+// Places of one block of 32 rows in both rings.
+struct GwStages {
+  RingStage raw, mma;
+  __device__ __forceinline__ GwStages(const GwParams& p, int n) { skip(p, n); }
+  __device__ __forceinline__ void skip(const GwParams& p, int n) {
+    for (int i = 0; i < n; i++) {
+      raw.next(p.raw_stages);
+      mma.next(p.stages);
+    }
+  }
+};
+
 template <int BITS>
 __global__ void __launch_bounds__(kGwThreads, 1)
 grad_weight_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ GwParams p) {
@@ -204,9 +216,10 @@ grad_weight_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_consta
     if (lane == 0) {
       bool ok = true;
       long long it = 0;
-      for (; it < nblk && ok; it++) {
-        const int s = (int)(it % p.raw_stages);
-        const uint32_t ph = (uint32_t)(it / p.raw_stages) & 1u;
+      RingStage st;
+      for (; it < nblk && ok; it++, st.next(p.raw_stages)) {
+        const int s = st.s;
+        const uint32_t ph = st.ph;
         if (!mbar_wait(smem_u32(&s_rempty[s]), ph ^ 1u, abort_flag)) { ok = false; break; }
         const uint32_t full = smem_u32(&s_rfull[s]);
         const uint32_t dst = tiles_base + (uint32_t)s * p.raw_bytes;
@@ -239,9 +252,10 @@ grad_weight_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_consta
     if (lane == 0) {
       const uint32_t idesc = umma_idesc_tf32(128, p.kpad);
       bool ok = true;
-      for (long long it = 0; it < nblk && ok; it++) {
-        const int s = (int)(it % p.stages);
-        const uint32_t ph = (uint32_t)(it / p.stages) & 1u;
+      RingStage st;
+      for (long long it = 0; it < nblk && ok; it++, st.next(p.stages)) {
+        const int s = st.s;
+        const uint32_t ph = st.ph;
         if (!mbar_wait(smem_u32(&s_full[s]), ph, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t a_addr = tiles_base + mma_off + (uint32_t)s * p.stage_bytes;
@@ -260,9 +274,10 @@ grad_weight_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_consta
   } else if (warp >= 6) {
     // ---------------- converters (warps 6..9): raw box [32 rows x O] -> A^T tiles [128 outputs x 32 rows] ----------------
     const int pair = (warp - 6) >> 1, t = threadIdx.x - 192 - pair * 64;   // output modulo 64
-    for (long long it = pair; it < nblk; it += 2) {
-      const int rs = (int)(it % p.raw_stages), s = (int)(it % p.stages);
-      const uint32_t rph = (uint32_t)(it / p.raw_stages) & 1u, ph = (uint32_t)(it / p.stages) & 1u;
+    GwStages st(p, pair);
+    for (long long it = pair; it < nblk; it += 2, st.skip(p, 2)) {
+      const int rs = st.raw.s, s = st.mma.s;
+      const uint32_t rph = st.raw.ph, ph = st.mma.ph;
       // the same outcome in every lane, so that a warp leaves the loop as a whole
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_rfull[rs]), rph, abort_flag))) break;
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[s]), ph ^ 1u, abort_flag))) break;
@@ -315,10 +330,10 @@ grad_weight_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_consta
       }
     };
     if (grp_id < nblk) load_stats(grp_id);
-    for (long long it = grp_id; it < nblk && ok; it += 2) {
-      const int rs = (int)(it % p.raw_stages), s = (int)(it % p.stages);
-      const uint32_t rph = (uint32_t)(it / p.raw_stages) & 1u, ph = (uint32_t)(it / p.stages) & 1u;
-      
+    GwStages st(p, grp_id);
+    for (long long it = grp_id; it < nblk && ok; it += 2, st.skip(p, 2)) {
+      const int rs = st.raw.s, s = st.mma.s;
+      const uint32_t rph = st.raw.ph, ph = st.mma.ph;
       const int sb = (int)((it >> 1) & 1);
 #pragma unroll
       for (int sg = 0; sg < kGwMaxSeg; sg++) {

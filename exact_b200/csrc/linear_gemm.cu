@@ -97,18 +97,6 @@ __device__ __forceinline__ void fence_proxy_async_smem_lin() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// The ring's next stage and the parity of its round.
-struct LinStage {
-  int s = 0;
-  uint32_t ph = 0;
-  __device__ __forceinline__ void next(int stages) {
-    if (++s == stages) {
-      s = 0;
-      ph ^= 1u;
-    }
-  }
-};
-
 // CHUNKED: the contraction is drained from TMEM every p.chunk K tiles (a kernel of its own: its epilogue's registers and
 // code cost the unchunked product 5 %).
 template <bool CHUNKED, bool PAIR>
@@ -161,7 +149,7 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      LinStage st;
+      RingStage st;
       int uses = 0;   // K tiles requested so far, at most p.stages
       bool ok = true;
       for (int tile = first; tile < tiles && ok; tile += step) {
@@ -216,7 +204,7 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         if (PAIR) umma_commit_pair(bar);
         else umma_commit(bar);
       };
-      LinStage st;
+      RingStage st;
       int t = 0;
       bool ok = true;
       for (int tile = first; tile < tiles && ok; tile += step) {
@@ -260,7 +248,7 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     const int group = (warp - 2) / kLinConvGroup, ct = threadIdx.x - 64 - group * 32 * kLinConvGroup;
     constexpr int kPer = (int)(kLinHalf / 16) / (32 * kLinConvGroup);   // 16-byte chunks per thread
     constexpr int kBatch = 4;
-    LinStage st;
+    RingStage st;
     int turn = group;
     bool ok = true;
     for (int tile = first; tile < tiles && ok; tile += step) {

@@ -134,11 +134,12 @@ rp_pack_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     // ---------------- TMA producer ----------------
     if (lane == 0) {
       int it = 0;
+      RingStage st;
       bool ok = true;
       for (int tile = first; tile < p.num_tiles && ok; tile += step) {
-        for (int kb = 0; kb < p.kblocks; kb++, it++) {
-          const int s = it % p.stages;
-          const uint32_t ph = (uint32_t)(it / p.stages) & 1u;
+        for (int kb = 0; kb < p.kblocks; kb++, it++, st.next(p.stages)) {
+          const int s = st.s;
+          const uint32_t ph = st.ph;
           if (!mbar_wait(smem_u32(&s_empty[s]), ph ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t full = smem_u32(&s_full[s]);
           const uint32_t dst = tiles_base + (uint32_t)s * p.stage_bytes;
@@ -169,7 +170,8 @@ rp_pack_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       const int n_lo = p.kpad <= 256 ? p.kpad : 256, n_hi = p.kpad - n_lo;
       const uint32_t idesc = umma_idesc_tf32(kRpTileM, n_lo);
       const uint32_t idesc_hi = umma_idesc_tf32(kRpTileM, n_hi > 0 ? n_hi : 16);
-      int it = 0, t = 0;
+      RingStage st;
+      int t = 0;
       bool ok = true;
       for (int tile = first; tile < p.num_tiles && ok; tile += step, t++) {
         const int buf = p.nbuf == 2 ? (t & 1) : 0;
@@ -177,9 +179,9 @@ rp_pack_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         if (!mbar_wait(smem_u32(&s_tempty[buf]), tph ^ 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * p.kpad);
-        for (int kb = 0; kb < p.kblocks; kb++, it++) {
-          const int s = it % p.stages;
-          const uint32_t ph = (uint32_t)(it / p.stages) & 1u;
+        for (int kb = 0; kb < p.kblocks; kb++, st.next(p.stages)) {
+          const int s = st.s;
+          const uint32_t ph = st.ph;
           if (!mbar_wait(smem_u32(&s_full[s]), ph, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_addr = tiles_base + (uint32_t)s * p.stage_bytes;
@@ -207,11 +209,12 @@ rp_pack_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     const int cbytes = pi * p.piece;                        // byte offset of the piece inside a tile row
     const int chunk = cbytes >> 4, within = cbytes & 15;
     int it = 0;
+    RingStage st, landed;                                   // the stage being filled, the one p.lag iterations before it
     bool ok = true;
     for (int tile = first; tile < p.num_tiles && ok; tile += step) {
-      for (int kb = 0; kb < p.kblocks; kb++, it++) {
-        const int s = it % p.stages;
-        const uint32_t ph = (uint32_t)(it / p.stages) & 1u;
+      for (int kb = 0; kb < p.kblocks; kb++, it++, st.next(p.stages)) {
+        const int s = st.s;
+        const uint32_t ph = st.ph;
         if (!mbar_wait(smem_u32(&s_empty[s]), ph ^ 1u, abort_flag)) { ok = false; break; }
         const int col = kb * kRpTileK + (cbytes >> 2);
         // a piece is inside the row or outside as a whole: 8-byte pieces are only used for even D
@@ -247,14 +250,15 @@ rp_pack_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         if (it >= p.lag) {
           cp_async_wait_pending(p.lag);          // the copies of iteration it - lag have landed
           fence_proxy_async_smem();
-          mbar_arrive(smem_u32(&s_full[(it - p.lag) % p.stages]));
+          mbar_arrive(smem_u32(&s_full[landed.s]));
+          landed.next(p.stages);
         }
       }
     }
     cp_async_wait_pending(0);
     if (ok) {
       fence_proxy_async_smem();
-      for (int j = it > p.lag ? it - p.lag : 0; j < it; j++) mbar_arrive(smem_u32(&s_full[j % p.stages]));
+      for (int j = it > p.lag ? it - p.lag : 0; j < it; j++, landed.next(p.stages)) mbar_arrive(smem_u32(&s_full[landed.s]));
     }
   } else {
     // ---------------- epilogue: warps 2..5, thread = row ----------------
