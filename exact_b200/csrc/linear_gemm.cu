@@ -113,7 +113,7 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // known to be uniform
   const int rank = PAIR ? (int)cluster_rank() : 0;
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t stage_base = ring + kLinSlots * kLinSlotBytes;   // 4 KB of staging per epilogue warp
@@ -194,7 +194,11 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0 && rank == 0) {   // the first CTA of a pair issues for both
+    // The first CTA of a pair issues for both.  The whole warp walks the loop and one elected lane issues: descriptors and
+    // addresses then live in uniform registers, which the instructions take; from a branch of one lane each of the twelve
+    // MMAs first moved its operands there.
+    if (rank == 0) {
+      const bool elected = elect_one();
       const uint32_t idesc = umma_idesc_tf32(PAIR ? 2 * kLinTileM : kLinTileM, p.Npad);
       auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
         if (PAIR) umma_tf32_pair(d, a, b, idesc, acc);
@@ -215,31 +219,34 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
           if (opens) {
             buf = t & 1;
             const uint32_t tph = (uint32_t)(t >> 1) & 1u;
-            if (!mbar_wait(smem_u32(&s_tempty[buf]), tph ^ 1u, abort_flag)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_tempty[buf]), tph ^ 1u, abort_flag))) { ok = false; break; }
             tc_fence_after();
             d_tmem = tmem_base + (uint32_t)(buf * p.Npad);
             t++;
           }
-          if (!mbar_wait(smem_u32(&s_ready[st.s]), st.ph, abort_flag)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_ready[st.s]), st.ph, abort_flag))) { ok = false; break; }
           tc_fence_after();
           const uint32_t base = ring + (uint32_t)st.s * p.stage_bytes;
           const uint64_t ahi = umma_desc_sw128(base);
           const uint64_t alo = umma_desc_sw128(base + kLinHalf);
           const uint64_t bhi = umma_desc_sw128(base + kLinSlotBytes);
           const uint64_t blo = umma_desc_sw128(base + kLinSlotBytes + p.b_slot);
+          if (elected) {
 #pragma unroll
-          for (int k4 = 0; k4 < kLinTileK / 8; k4++) {
-            const uint64_t o = (uint64_t)(k4 * 2);   // 8 tf32 = 32 bytes along K inside the swizzle atom
-            mma(d_tmem, alo + o, bhi + o, !opens || k4 != 0);
-            mma(d_tmem, ahi + o, bhi + o, 1);
-          }
+            for (int k4 = 0; k4 < kLinTileK / 8; k4++) {
+              const uint64_t o = (uint64_t)(k4 * 2);   // 8 tf32 = 32 bytes along K inside the swizzle atom
+              mma(d_tmem, alo + o, bhi + o, !opens || k4 != 0);
+              mma(d_tmem, ahi + o, bhi + o, 1);
+            }
 #pragma unroll
-          for (int k4 = 0; k4 < kLinTileK / 8; k4++) {
-            const uint64_t o = (uint64_t)(k4 * 2);
-            mma(d_tmem, ahi + o, blo + o, 1);
+            for (int k4 = 0; k4 < kLinTileK / 8; k4++) {
+              const uint64_t o = (uint64_t)(k4 * 2);
+              mma(d_tmem, ahi + o, blo + o, 1);
+            }
+            commit(smem_u32(&s_empty[st.s]));
+            if ((CHUNKED && (kb + 1) % p.chunk == 0) || kb + 1 == p.kblocks) commit(smem_u32(&s_tfull[buf]));
           }
-          commit(smem_u32(&s_empty[st.s]));
-          if ((CHUNKED && (kb + 1) % p.chunk == 0) || kb + 1 == p.kblocks) commit(smem_u32(&s_tfull[buf]));
+          __syncwarp();
         }
       }
     }
