@@ -279,8 +279,10 @@ grad_weight_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_consta
       const int rs = st.raw.s, s = st.mma.s;
       const uint32_t rph = st.raw.ph, ph = st.mma.ph;
       // the same outcome in every lane, so that a warp leaves the loop as a whole
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_rfull[rs]), rph, abort_flag))) break;
+      // The stage first: a pair meets a place of an odd ring in every second round, which a parity alone does not tell apart; the
+      // block that used the stage before has been consumed, so the one that used the raw place before (no later) has landed.
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[s]), ph ^ 1u, abort_flag))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_rfull[rs]), rph, abort_flag))) break;
       const float* raw = reinterpret_cast<const float*>(tiles_ptr + (size_t)rs * p.raw_bytes);
       uint8_t* at = tiles_ptr + mma_off + (size_t)s * p.stage_bytes;
       for (int o = t; o < p.Opad; o += 64) {
@@ -345,8 +347,9 @@ grad_weight_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_consta
       __syncwarp();                           // this warp's copy of the stage's statistics is in shared memory
       if (it + 2 < nblk) load_stats(it + 2);
       // the same outcome in every lane, so that a warp leaves the loop as a whole
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_rfull[rs]), rph, abort_flag))) { ok = false; break; }
+      // the stage first: see the converters
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[s]), ph ^ 1u, abort_flag))) { ok = false; break; }
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_rfull[rs]), rph, abort_flag))) { ok = false; break; }
       uint8_t* btile = tiles_ptr + mma_off + (size_t)s * p.stage_bytes + p.a_bytes;
       const long long grp0 = (kb0 + it) * GROUPS;
       const long long groups_left = (p.N + WPT - 1) / WPT - grp0;

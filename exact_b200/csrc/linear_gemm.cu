@@ -256,11 +256,16 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     constexpr int kPer = (int)(kLinHalf / 16) / (32 * kLinConvGroup);   // 16-byte chunks per thread
     constexpr int kBatch = 4;
     RingStage st;
-    int turn = group;
+    int turn = group, seen = 0;   // seen: K tiles so far, up to a full ring
     bool ok = true;
     for (int tile = first; tile < tiles && ok; tile += step) {
       for (int kb = 0; kb < p.kblocks; kb++, st.next(p.stages), turn ^= 1) {
+        const bool again = seen >= p.stages;
+        if (!again) seen++;
         if (turn) continue;
+        // A parity tells a round from its neighbours only, and with an odd number of stages this group meets a stage in every
+        // second round.  So first see that the other group's round has been consumed; then `full` can only be one behind.
+        if (again && !mbar_wait(smem_u32(&s_empty[st.s]), st.ph ^ 1u, abort_flag)) { ok = false; break; }
         if (!mbar_wait(smem_u32(&s_full[st.s]), st.ph, abort_flag)) { ok = false; break; }
         const uint32_t base = ring + (uint32_t)st.s * p.stage_bytes + (uint32_t)ct * 16u;
 #pragma unroll

@@ -30,3 +30,16 @@ def test_tiles_and_widths(M, K, K2, N, chunk):
     assert (out.double() - want).norm() <= 5e-6 * want.norm()
     assert (out.double() - want).abs().max() <= 1e-5 * want.abs().max()
     _lib.check_status(force=True)
+
+
+@pytest.mark.parametrize("N", [256, 128, 47])
+def test_same_result_whatever_the_timing_of_the_loads(N):
+    """Cold and warm operands: the groups of warps that take alternate K tiles must not meet a stage a round early."""
+    from exact_b200.cpp_extension import backward_func as B
+    a, w = torch.randn(128 * 700, 256, device="cuda"), torch.randn(N, 256, device="cuda")
+    flush = torch.empty(64 << 20, device="cuda")
+    want = B.linear_forward(a, w)
+    for i in range(20):
+        if i % 2:
+            flush.fill_(float(i))
+        assert torch.equal(B.linear_forward(a, w), want)
