@@ -68,7 +68,7 @@ SIGNATURES = {
     "exact_spmm_f16": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_int, c_ptr, c_ptr]),
     "exact_spmm_f16_planned": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_i64, c_int, c_ptr, c_i64, c_ptr,
                                        c_i64, c_ptr, c_ptr, c_ptr]),
-    "exact_spmm_planned": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_int, c_i64, c_ptr, c_ptr, c_ptr, c_ptr,
+    "exact_spmm_planned": (c_int, [c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_i64, c_int, c_i64, c_ptr, c_ptr, c_ptr, c_ptr,
                                    c_i64, c_ptr, c_ptr, c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr]),
     "exact_rows_scale_colsum_workspace_bytes": (c_i64, [c_i64]),
     "exact_rows_scale_colsum": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_ptr, c_i64, c_i64, c_ptr, c_ptr, c_i64, c_ptr]),

@@ -513,9 +513,19 @@ Tensor spmm(const Tensor& rowptr, const Tensor& colt, const RowPlan& a, const Op
   info.bytes = mat.size(0) * K * 4 + index_bytes + M * K * 4;   // what must cross HBM at least once
   info.l2_bytes = nnz * K * 4 + index_bytes + M * K * 4;        // what the gathers request when no source row is reused
   info.edge_columns = nnz * K;
+  // Rows of whole 16-byte pieces: an odd width is gathered element by element in 32-column passes over the graph, an even one in
+  // pairs.  The padded copy is one pass over the operand, which a call of a few microseconds does not repay; a wide odd
+  // operand of a small graph is bound by latency, and its many narrow passes hide that better (18.7 M edges x 47 columns
+  // 598 -> 390 us, x 90 922 -> 649, x 145 1,452 -> 1,229; 0.46 M x 47 56 -> 39, x 90 81 -> 70, x 145 88 -> 103).
+  int64_t ldm = K;
+  Tensor src = mat;
+  if (K % 4 && nnz >= 2 * mat.size(0) && nnz * K >= (K <= 64 || K % 2 == 0 ? 1LL << 22 : 1LL << 27)) {
+    ldm = (K + 3) / 4 * 4;
+    src = std::get<0>(rows_scale_colsum(mat, {}, true, false));
+  }
   const RowPlan::Pieces& pc = a.pieces(rowptr, colt);
   Tensor scratch;
-  if (pc.n) scratch = empty({pc.n, K}, at::kFloat, mat);
+  if (pc.n) scratch = empty({pc.n, ldm}, at::kFloat, mat);
   float* sc = pc.n ? ptr<float>(scratch) : nullptr;
   const int32_t *prow = nullptr, *pslot = nullptr, *lrow = nullptr, *lptr = nullptr;
   const int64_t *pb = nullptr, *pe = nullptr;
@@ -523,10 +533,10 @@ Tensor spmm(const Tensor& rowptr, const Tensor& colt, const RowPlan& a, const Op
     prow = ptr<int32_t>(pc.row); pslot = ptr<int32_t>(pc.slot); lrow = ptr<int32_t>(pc.long_row); lptr = ptr<int32_t>(pc.long_ptr);
     pb = ptr<int64_t>(pc.begin); pe = ptr<int64_t>(pc.end);
   }
-  const bool narrow = K <= 64 && K % 4 == 0 && M > 0;
+  const bool narrow = ldm <= 64 && ldm % 4 == 0 && M > 0;
   const int32_t* order = M > 0 ? ptr<int32_t>(a.row_order(rowptr)) : nullptr;
   invoke(narrow ? "exact_spmm_split_routed" : pc.n ? "exact_spmm_split" : "exact_spmm", info, [&](void* st) {
-    return lib.exact_spmm_planned(rp, col, ib, ptr<float>(value), ptr<float>(mat), M, K, red, pc.n ? a.threshold : 0, prow, pb, pe,
+    return lib.exact_spmm_planned(rp, col, ib, ptr<float>(value), ptr<float>(src), ldm, M, K, red, pc.n ? a.threshold : 0, prow, pb, pe,
                                   pslot, pc.n, lrow, lptr, pc.n_long, sc, order, ptr<float>(bias), ptr<float>(out), st);
   });
   return out;

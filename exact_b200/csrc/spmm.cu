@@ -32,6 +32,7 @@ struct SpmmParams {
   float* out;
   const float* bias;   // [K] added to every row of the result, or null
   long long M, K;
+  long long Kout;      // columns of the result: K, or up to three fewer when the operand's rows are padded to 16-byte pieces
   int mean;
   int regroup;   // the caller accepts a regrouped per-row sum (EXACT_SPMM_REGROUP)
   long long long_threshold;  // rows with more edges are skipped by the row kernel (0: none)
@@ -44,7 +45,7 @@ struct SpmmParams {
   const int* long_row;
   const int* long_item_ptr;
   long long n_long;
-  float* scratch;  // [n_items, K]
+  float* scratch;      // [n_items, K]
   // Routed output (feature-parallel aggregation): row r is written to columns route_col0 .. + K - 1 of row
   // r % route_shard of the [route_shard, route_ld] matrix at route_dst[r / route_shard], which may be another
   // GPU's memory (plain stores).  route_n == 0: the rows go to `out`.
@@ -55,7 +56,7 @@ struct SpmmParams {
 };
 
 __device__ __forceinline__ float* output_row(const SpmmParams& p, long long row) {
-  if (p.route_n == 0) return p.out + row * p.K;
+  if (p.route_n == 0) return p.out + row * p.Kout;
   const long long owner = row / p.route_shard;
   return p.route_dst[owner] + (row - owner * p.route_shard) * p.route_ld + p.route_col0;
 }
@@ -84,6 +85,22 @@ __device__ __forceinline__ void st_vec(float* p, const float (&a)[VEC]) {
   if (VEC == 4) *reinterpret_cast<float4*>(p) = make_float4(a[0], a[1 % VEC], a[2 % VEC], a[3 % VEC]);
   else if (VEC == 2) *reinterpret_cast<float2*>(p) = make_float2(a[0], a[1 % VEC]);
   else p[0] = a[0];
+}
+
+// Columns c .. c + VEC - 1 of a row of the result, bias added.
+template <int VEC>
+__device__ __forceinline__ void store_row(const SpmmParams& p, long long row, long long c, const float (&acc)[VEC]) {
+  float* d = output_row(p, row) + c;
+  if (p.Kout == p.K) {
+    float o[VEC];
+#pragma unroll
+    for (int x = 0; x < VEC; x++) o[x] = p.bias != nullptr ? __fadd_rn(acc[x], __ldg(p.bias + c + x)) : acc[x];
+    st_vec<VEC>(d, o);
+  } else {
+#pragma unroll
+    for (int x = 0; x < VEC; x++)
+      if (c + x < p.Kout) d[x] = p.bias != nullptr ? __fadd_rn(acc[x], __ldg(p.bias + c + x)) : acc[x];
+  }
 }
 
 // acc += sum over edges [begin, end) of val[e] * mat[col[e], column tile], in edge order.
@@ -185,7 +202,7 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_kernel(const __grid_
     for (int e = 0; e < VEC; e++) acc[j][e] = 0.f;
 
   long long begin, end;
-  float* dst;
+  float* dst = nullptr;
   long long count = 0;
   if (MODE == MODE_ROWS) {
     if (unit >= p.M) return;
@@ -193,7 +210,6 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_kernel(const __grid_
     end = (long long)rowptr[unit + 1];
     count = end - begin;
     if (p.long_threshold > 0 && count > p.long_threshold) return;
-    dst = output_row(p, unit);
   } else {
     if (unit >= p.n_items) return;
     begin = p.item_begin[unit];
@@ -216,15 +232,12 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_kernel(const __grid_
 #pragma unroll
       for (int x = 0; x < VEC; x++) acc[j][x] = __fdiv_rn(acc[j][x], dv);
   }
-  if (MODE == MODE_ROWS && p.bias != nullptr) {
 #pragma unroll
-    for (int j = 0; j < KVT; j++)
-#pragma unroll
-      for (int x = 0; x < VEC; x++) acc[j][x] = __fadd_rn(acc[j][x], __ldg(p.bias + cload[j] + x));
+  for (int j = 0; j < KVT; j++) {
+    if (!FULL && !cvalid[j]) continue;
+    if (MODE == MODE_ROWS) store_row<VEC>(p, unit, coff[j], acc[j]);
+    else st_vec<VEC>(dst + coff[j], acc[j]);
   }
-#pragma unroll
-  for (int j = 0; j < KVT; j++)
-    if (FULL || cvalid[j]) st_vec<VEC>(dst + coff[j], acc[j]);
 }
 
 template <int U, int VEC, bool HAS_VAL>
@@ -337,11 +350,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, kRowBlocks) spmm_rows_kernel(c
 #pragma unroll
           for (int x = 0; x < VEC; x++) acc[x] = __fdiv_rn(acc[x], dv);
         }
-        if (p.bias != nullptr) {
-#pragma unroll
-          for (int x = 0; x < VEC; x++) acc[x] = __fadd_rn(acc[x], __ldg(p.bias + cload + x));
-        }
-        if (cvalid) st_vec<VEC>(output_row(p, row) + coff, acc);
+        if (cvalid) store_row<VEC>(p, row, coff, acc);
       }
       b = b1; e = e1; b1 = b2; e1 = e2;
       row = row1; row1 = row2; row2 = row3;
@@ -360,7 +369,7 @@ __global__ void __launch_bounds__(128) spmm_long_reduce_kernel(const __grid_cons
   const long long cnt = (long long)rowptr[row + 1] - (long long)rowptr[row];
   const float dv = (float)(cnt > 0 ? cnt : 1);
   float* __restrict__ dst = output_row(p, row);
-  for (long long c = threadIdx.x; c < p.K; c += blockDim.x) {
+  for (long long c = threadIdx.x; c < p.Kout; c += blockDim.x) {
     float a = 0.f;
     for (int s = s0; s < s1; s++) a = __fadd_rn(a, p.scratch[(long long)s * p.K + c]);
     if (p.mean) a = __fdiv_rn(a, dv);
@@ -392,7 +401,7 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_multi_kernel(const _
   const long long coff = ((long long)blockIdx.y * LPE + hl) * 4;
   const bool cvalid = coff < K;
 
-  long long begin = 0, len = 0;
+  long long begin = 0, len = 0, row = 0;
   float* dst = nullptr;
   bool live = false;
   const bool is_row = unit >= p.n_items;     // the pieces of long rows come first
@@ -402,11 +411,10 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_multi_kernel(const _
     live = true;
     dst = p.scratch + (long long)(p.item_slot ? p.item_slot[unit] : (int)unit) * K;
   } else if (unit - p.n_items < p.M) {
-    const long long row = p.row_order ? (long long)p.row_order[unit - p.n_items] : unit - p.n_items;
+    row = p.row_order ? (long long)p.row_order[unit - p.n_items] : unit - p.n_items;
     begin = (long long)rowptr[row];
     len = (long long)rowptr[row + 1] - begin;
     live = !(p.long_threshold > 0 && len > p.long_threshold);
-    dst = output_row(p, row);
   }
   const long long count = len;
   if (!live) len = 0;
@@ -472,11 +480,10 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_multi_kernel(const _
 #pragma unroll
     for (int x = 0; x < 4; x++) acc[x] = __fdiv_rn(acc[x], dv);
   }
-  if (is_row && p.bias != nullptr && cvalid) {
-#pragma unroll
-    for (int x = 0; x < 4; x++) acc[x] = __fadd_rn(acc[x], __ldg(p.bias + coff + x));
+  if (live && cvalid) {
+    if (is_row) store_row<4>(p, row, coff, acc);
+    else st_vec<4>(dst + coff, acc);
   }
-  if (live && cvalid) *reinterpret_cast<float4*>(dst + coff) = make_float4(acc[0], acc[1], acc[2], acc[3]);
 }
 
 template <typename IdxT>
@@ -508,7 +515,9 @@ template <typename IdxT, int VEC, int KVT, bool HAS_VAL, bool FULL>
 static int launch_spmm_mode(const SpmmParams& p, cudaStream_t st) {
   const long long C = p.K / VEC;
   const unsigned gy = (unsigned)((C + 32 * KVT - 1) / (32 * KVT));
-  if (p.row_order != nullptr && p.M < 2147483647LL) {
+  // From 16 rows a warp on: with fewer the rows' own latency counts, and the other kernel keeps twice the gathers in flight
+  // (12,093 rows x 256 columns 66 us here, 58 there; 38,146 rows 93 and 89; 169,343 rows 241 and 276).
+  if (p.row_order != nullptr && p.M < 2147483647LL && p.M >= 16LL * sm_count() * kRowBlocks * kRowWarps) {
     long long blocks = (p.M + kRowWarps - 1) / kRowWarps;
     if (blocks > sm_count() * kRowBlocks) blocks = sm_count() * kRowBlocks;
     spmm_rows_kernel<IdxT, VEC, HAS_VAL><<<(unsigned)blocks, kRowWarps * 32, 0, st>>>(p);
@@ -547,7 +556,7 @@ static int launch_spmm_kvt(const SpmmParams& p, cudaStream_t st) {
 
 template <typename IdxT, bool HAS_VAL>
 static int launch_spmm_vec(const SpmmParams& p, cudaStream_t st) {
-  uintptr_t a = reinterpret_cast<uintptr_t>(p.mat) | reinterpret_cast<uintptr_t>(p.out);
+  uintptr_t a = reinterpret_cast<uintptr_t>(p.mat) | (p.Kout == p.K ? reinterpret_cast<uintptr_t>(p.out) : 0);
   if (p.scratch) a |= reinterpret_cast<uintptr_t>(p.scratch);
   for (int i = 0; i < p.route_n; i++) a |= reinterpret_cast<uintptr_t>(p.route_dst[i]);
   if (p.route_n) a |= (uintptr_t)(p.route_ld * 4) | (uintptr_t)(p.route_col0 * 4);
@@ -563,6 +572,7 @@ static int spmm_common(SpmmParams& p, int idx_bytes, int reduce, cudaStream_t st
   reduce &= ~EXACT_SPMM_REGROUP;
   EXB_REQUIRE(reduce == EXACT_REDUCE_SUM || reduce == EXACT_REDUCE_MEAN, "spmm: reduce must be sum or mean");
   EXB_REQUIRE(p.M >= 0 && p.K >= 0, "spmm: negative shape");
+  if (p.Kout == 0) p.Kout = p.K;
   if (p.M == 0 || p.K == 0) return EXB_OK;
   EXB_REQUIRE(p.rowptr && p.mat && (p.out || p.route_n > 0), "spmm: null pointer");
   EXB_REQUIRE((p.M + kSpmmWarps - 1) / kSpmmWarps <= 2147483647LL, "spmm: too many rows");
@@ -933,18 +943,19 @@ int exact_spmm_split(const void* rowptr, const void* col, int idx_bytes, const f
   return spmm_common(p, idx_bytes, reduce, (cudaStream_t)stream);
 }
 
-int exact_spmm_planned(const void* rowptr, const void* col, int idx_bytes, const float* value, const float* mat, int64_t M,
-                       int64_t K, int reduce, int64_t long_threshold, const int32_t* item_row, const int64_t* item_begin,
+int exact_spmm_planned(const void* rowptr, const void* col, int idx_bytes, const float* value, const float* mat, int64_t ldm,
+                       int64_t M, int64_t K, int reduce, int64_t long_threshold, const int32_t* item_row, const int64_t* item_begin,
                        const int64_t* item_end, const int32_t* item_slot, int64_t n_items, const int32_t* long_row,
                        const int32_t* long_item_ptr, int64_t n_long, float* scratch, const int32_t* row_order,
                        const float* bias, float* out, void* stream) {
+  EXB_REQUIRE(K >= 0 && (ldm == K || (ldm > K && ldm < K + 4 && ldm % 4 == 0)), "spmm_planned: ldm must be K, or K rounded up to a multiple of 4");
   EXB_REQUIRE(long_threshold >= 0 && n_items >= 0 && n_long >= 0, "spmm_planned: negative plan size");
   EXB_REQUIRE(n_items <= 2147483647LL && n_long <= 2147483647LL, "spmm_planned: plan too large");
   if (n_items > 0)
     EXB_REQUIRE(long_threshold > 0 && item_row && item_begin && item_end && long_row && long_item_ptr && scratch && n_long > 0,
                 "spmm_planned: null plan array or scratch");
   SpmmParams p{};
-  p.rowptr = rowptr; p.col = col; p.val = value; p.mat = mat; p.out = out; p.bias = bias; p.M = M; p.K = K;
+  p.rowptr = rowptr; p.col = col; p.val = value; p.mat = mat; p.out = out; p.bias = bias; p.M = M; p.K = ldm; p.Kout = K;
   p.long_threshold = n_items > 0 ? long_threshold : 0;
   p.item_row = item_row; p.item_begin = reinterpret_cast<const long long*>(item_begin);
   p.item_end = reinterpret_cast<const long long*>(item_end); p.item_slot = item_slot; p.n_items = n_items;

@@ -361,9 +361,10 @@ EXACT_API int exact_spmm_split_routed(const void* rowptr, const void* col, int i
 
 /* exact_spmm_split (or exact_spmm, with n_items = 0) into a local result, with a row order for narrow operands (or NULL) and
  * `bias` [K] (or NULL) added to every row of the result: out = reduce(A, mat) + bias, the sum and the addition rounded
- * separately as `out + bias` after the aggregation rounds them (layers.py:261-263). */
+ * separately as `out + bias` after the aggregation rounds them (layers.py:261-263).  ldm: pitch of mat, K or K rounded up to a
+ * multiple of 4 (rows padded to 16-byte pieces are gathered a piece at a time; out stays [M, K], scratch is [n_items, ldm]). */
 EXACT_API int exact_spmm_planned(const void* rowptr, const void* col, int idx_bytes, const float* value, const float* mat,
-                                 int64_t M, int64_t K, int reduce, int64_t long_threshold, const int32_t* item_row,
+                                 int64_t ldm, int64_t M, int64_t K, int reduce, int64_t long_threshold, const int32_t* item_row,
                                  const int64_t* item_begin, const int64_t* item_end, const int32_t* item_slot,
                                  int64_t n_items, const int32_t* long_row, const int32_t* long_item_ptr, int64_t n_long,
                                  float* scratch, const int32_t* row_order, const float* bias, float* out, void* stream);
