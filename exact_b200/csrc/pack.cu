@@ -359,7 +359,22 @@ __device__ __forceinline__ void reduce_rows(const float (&lo)[8], const float (&
   }
 }
 
-enum TileKind { TILE_SUB = 0, TILE_WARP = 1, TILE_MULTI = 2 };   // threads per tile: 8 or 16, 32, several warps
+enum TileKind { TILE_SUB = 0, TILE_WARP = 1, TILE_MULTI = 2, TILE_PAIR = 3 };   // threads per tile: 8 or 16, 32, several warps, two
+
+// Resident CTAs of 256 threads the compiler is told to leave registers for (the second launch bound).  One lets it spend up to 168
+// registers on a tile's rows, which is the faster way for most classes; the exceptions (us for 80 M elements, 1 | the bound taken):
+//   two warps a tile, two loads of four columns (260 - 512 columns): 128 registers keep a fourth CTA of 128 threads resident.
+//     320 columns, INT2: fp32 102 | 94, bf16 111 | 98, fp16 105 | 95.  With three or four warps a tile one stays the better
+//     bound (640 columns, INT8: fp32 85 | 84, fp16 82 | 93), which is why two warps are a class of their own;
+//   one warp a tile, two loads of four columns, bf16 (132 - 256 columns): 200 columns, INT2 90 | 86 (fp32 78 | 80, left at one);
+//   several warps, two loads of one or two columns: three.  602 columns, INT2: fp32 109 | 96 (a 16-byte spill included), fp16 100 | 105,
+//     bf16 91 | 98; INT4: 102 | 97, 115 | 107, 93 | 99.
+template <typename InT>
+constexpr int resident_ctas(int vec, int v, int kind) {
+  if (v != 2) return 1;
+  if (vec == 4) return kind == TILE_PAIR || (kind == TILE_WARP && std::is_same<InT, uint16_t>::value) ? 2 : 1;
+  return kind >= TILE_MULTI ? 3 : 1;
+}
 
 // FAST: the tile has all 8 rows and the noise is drawn from Philox.  Then there is no per-row
 // validity test, and -- when all 8 scales are finite and non-zero, i.e. no row is constant or holds
@@ -388,7 +403,7 @@ __device__ __forceinline__ bool process_tile(const PackParams& p, const TileCtx&
     }
   }
   bool finite = true;  // all 8 scales are finite numbers (warp-uniform)
-  if (KIND != TILE_MULTI) {
+  if (KIND < TILE_MULTI) {
     const float inf = __int_as_float(0x7f800000);
     // 0 < s < inf  <=>  the row's range is a finite non-zero number, hence every x in it is finite
     if (KIND == TILE_WARP) {
@@ -504,7 +519,7 @@ __device__ __forceinline__ bool process_tile(const PackParams& p, const TileCtx&
 }
 
 template <typename InT, int BITS, int VEC, int V, int KIND>
-__global__ void __launch_bounds__(256, KIND == TILE_MULTI && V == 2 && VEC <= 2 ? 3 : 1)
+__global__ void __launch_bounds__(256, resident_ctas<InT>(VEC, V, KIND))
 quantize_pack_kernel(const __grid_constant__ PackParams p) {
   constexpr int WPT = 8 / BITS;
   __shared__ float s_part[2 * kMaxGroupsPerCta * kMaxWarpsPerTile * 16];
@@ -904,7 +919,7 @@ static int launch_pack(const PackParams& p, const TileShape& s, cudaStream_t st)
   const int tiles_per_cta = s.block / s.tpt;
   const long long ctas = (tiles + tiles_per_cta - 1) / tiles_per_cta;
   int grid = 1;
-  const int kind = s.tpt < 32 ? TILE_SUB : s.tpt == 32 ? TILE_WARP : TILE_MULTI;
+  const int kind = s.tpt < 32 ? TILE_SUB : s.tpt == 32 ? TILE_WARP : s.tpt == 64 && s.vec == 4 ? TILE_PAIR : TILE_MULTI;
 #define EXB_PACK_CASE(VEC_, V_, KIND_)                                                 \
   if (s.vec == VEC_ && s.v == V_ && kind == KIND_) {                                   \
     auto k = quantize_pack_kernel<InT, BITS, VEC_, V_, KIND_>;                         \
@@ -914,7 +929,7 @@ static int launch_pack(const PackParams& p, const TileShape& s, cudaStream_t st)
     EXB_CUDA_OK(cudaGetLastError());                                                   \
     return EXB_OK;                                                                     \
   }
-  EXB_PACK_CASE(4, 1, TILE_SUB) EXB_PACK_CASE(4, 1, TILE_WARP) EXB_PACK_CASE(4, 2, TILE_WARP) EXB_PACK_CASE(4, 2, TILE_MULTI)
+  EXB_PACK_CASE(4, 1, TILE_SUB) EXB_PACK_CASE(4, 1, TILE_WARP) EXB_PACK_CASE(4, 2, TILE_WARP) EXB_PACK_CASE(4, 2, TILE_PAIR) EXB_PACK_CASE(4, 2, TILE_MULTI)
   EXB_PACK_CASE(4, 4, TILE_MULTI) EXB_PACK_CASE(2, 4, TILE_MULTI) EXB_PACK_CASE(1, 4, TILE_MULTI)
   EXB_PACK_CASE(2, 1, TILE_SUB) EXB_PACK_CASE(2, 1, TILE_WARP) EXB_PACK_CASE(2, 2, TILE_WARP) EXB_PACK_CASE(2, 2, TILE_MULTI)
   EXB_PACK_CASE(1, 1, TILE_SUB) EXB_PACK_CASE(1, 1, TILE_WARP) EXB_PACK_CASE(1, 2, TILE_WARP) EXB_PACK_CASE(1, 2, TILE_MULTI)

@@ -32,3 +32,10 @@ def test_pack_and_unpack(N, D, dtype, bits):
     assert np.array_equal(scale.view(torch.int16).cpu().numpy().view(np.uint16), osc.view(np.uint16))
     assert np.array_equal(mn.view(torch.int16).cpu().numpy().view(np.uint16), omn.view(np.uint16))
     assert np.array_equal(out.numpy(), ref, equal_nan=True)
+
+
+@pytest.mark.parametrize("bits", [1, 4, 8])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,D", [(17, 256), (41, 260), (1027, 320), (8, 384), (63, 512), (25, 516)])
+def test_pack_at_the_edges_of_two_warps_a_tile(N, D, dtype, bits):
+    test_pack_and_unpack(N, D, dtype, bits)
