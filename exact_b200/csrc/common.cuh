@@ -70,11 +70,11 @@ inline PhiloxKey make_philox_key(uint64_t seed) {
 }
 
 #ifdef __CUDACC__
-// Plain stores: the word is not in device memory.  Two kernels that give up at the same moment may leave one bit only.
+// CTAs and kernels that give up at the same moment all leave their bit: an atomic on mapped host memory is one for all threads of
+// the device that maps it, and the host writes the word only to clear or set it, after the stream it was asked for.
 __device__ __forceinline__ void raise_status(int* word, int bit) {
   if (word == nullptr) return;
-  volatile int* w = word;
-  *w = *w | bit;
+  atomicOr(word, bit);
   __threadfence_system();
 }
 
