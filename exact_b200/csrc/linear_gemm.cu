@@ -204,6 +204,10 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         if (PAIR) umma_tf32_pair(d, a, b, idesc, acc);
         else umma_tf32(d, a, b, idesc, acc);
       };
+      auto wait = [&](uint32_t bar, uint32_t parity) {
+        const bool there = PAIR ? mbar_wait_pair(bar, parity, abort_flag) : mbar_wait(bar, parity, abort_flag);
+        return __all_sync(0xffffffffu, there) != 0;
+      };
       auto commit = [&](uint32_t bar) {
         if (PAIR) umma_commit_pair(bar);
         else umma_commit(bar);
@@ -219,12 +223,12 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
           if (opens) {
             buf = t & 1;
             const uint32_t tph = (uint32_t)(t >> 1) & 1u;
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_tempty[buf]), tph ^ 1u, abort_flag))) { ok = false; break; }
+            if (!wait(smem_u32(&s_tempty[buf]), tph ^ 1u)) { ok = false; break; }
             tc_fence_after();
             d_tmem = tmem_base + (uint32_t)(buf * p.Npad);
             t++;
           }
-          if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_ready[st.s]), st.ph, abort_flag))) { ok = false; break; }
+          if (!wait(smem_u32(&s_ready[st.s]), st.ph)) { ok = false; break; }
           tc_fence_after();
           const uint32_t base = ring + (uint32_t)st.s * p.stage_bytes;
           const uint64_t ahi = umma_desc_sw128(base);

@@ -120,15 +120,43 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// One arrival on the barrier at this CTA's address `bar` in the pair's first CTA.  What it announces is shared memory written
-// before a proxy fence and TMEM read before a tcgen05 fence; with cluster scope the arrival also drained everything else that
-// the thread had written and took 1,400 cycles.
+// One arrival on the barrier at this CTA's address `bar` in the pair's first CTA.  It announces this CTA's shared memory, written
+// before a proxy fence by this warp, to the thread that issues the pair's MMAs (mbar_wait_pair), and tensor memory that has been
+// read (tcgen05 fences).  The release has cluster scope, as the waiting thread is in another CTA, and covers shared memory only:
+// an arrive.release.cluster also drained the thread's global stores and took 1,400 cycles.
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
   asm volatile(
       "{\n\t.reg .b32 ra;\n\t"
       "mapa.shared::cluster.u32 ra, %0, 0;\n\t"
-      "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar)
+      "fence.release.sync_restrict::shared::cta.cluster;\n\t"
+      "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar)
       : "memory");
+}
+// The wait that goes with it: of the first CTA's issuing thread, bounded as mbar_wait.
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_pair(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (!mbar_try_wait_cluster(bar, parity)) {
+    const long long t0 = clock64();
+    while (!mbar_try_wait_cluster(bar, parity)) {
+      if (*abort_flag) return false;
+      if (clock64() - t0 > kWaitLimitCycles) {
+        *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+  asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+  return true;
 }
 // Both CTAs of the pair call these; the columns are the same in both.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {
