@@ -50,8 +50,8 @@ class QuantizationConfig:
         # (fp32-equivalent accuracy); False: the library's fp32 GEMM.
         self.linear_tensor_core = True
         # Weight gradients of the quantised linear layers straight from the packed activation on the tensor
-        # cores (tf32 inputs, fp32 accumulation: about 5e-4 relative, far below the quantisation noise of the
-        # activation); False: unpack, then the library's fp32 GEMM.
+        # cores (operands split into fp16 heads and tails: as accurate as an fp32 product); False: unpack, then the
+        # library's fp32 GEMM.
         self.grad_weight_tensor_core = True
         # qbatch_norm.backward reads the saved input in its packed form (two passes over the packed bytes) instead
         # of dequantising it into an [N, D] tensor for ATen's backward.

@@ -1,7 +1,7 @@
 """Stand-in for the reference's `exact.cpp_extension.backward_func` module
 (exact/exact/cpp_extension/backward_func.cc:83-107): the dense-layer GEMMs and ATen batch-norm
 pass-throughs.  The tall GEMMs (rows = nodes) go to the tensor-core kernel with fp32-equivalent accuracy
-(exact_linear_forward); the weight-gradient reductions and unsupported shapes stay library GEMMs."""
+(exact_linear_forward), the weight gradients to exact_grad_weight_from_packed; unsupported shapes stay library GEMMs."""
 import torch
 
 from .. import _lib
@@ -57,9 +57,9 @@ def rows_reduce_mm(g, x, batches=512):
 
 
 def grad_weight_supported(g, k0, k1, bits):
-    """Shapes exact_grad_weight_from_packed takes: fp32 g [N, O] with O <= 256 (padded to a multiple of 4), at least 4,096 rows
-    (below that the library GEMM on the unpacked activation is as fast), and few enough activation columns for
-    four producer warps (k0 + k1 <= 1024 * bits / 256)."""
+    """The shapes at which the product needs the fewest reads of g: fp32 g [N, O] with O <= 256 (padded to a multiple of 4), at
+    least 4,096 rows, few activation columns.  Kept for callers that choose by it; the layers take the kernel for every
+    shape of grad_weight_takes."""
     if not (config.grad_weight_tensor_core and g.is_cuda and g.dtype == torch.float32 and g.dim() == 2):
         return False
     N, O = g.shape
@@ -67,6 +67,12 @@ def grad_weight_supported(g, k0, k1, bits):
     # a width that is not a multiple of 4 (47 classes) goes in as a zero-padded copy of g
     return (N >= 4096 and (O + 3) // 4 * 4 <= 256 and kpad <= 256 and (k0 + k1) * (32 // (8 // bits)) <= 1024
             and g.is_contiguous() and (g.data_ptr() % 16 == 0 or O % 4 != 0))
+
+
+def grad_weight_takes(g):
+    """Whether the layers' weight gradients come from exact_grad_weight_from_packed: fp32 g [N, O], O <= 256, on the GPU.  The rule
+    is the C++ nodes' own, so a switch that sends a layer through the Python nodes does not change the route."""
+    return config.grad_weight_tensor_core and g.is_cuda and _lib.native().grad_weight_takes(g)
 
 
 def grad_weight_from_packed(g, q0, k0, q1=None, k1=0):

@@ -62,10 +62,11 @@ Compressed compress(const Tensor& x, const Saving& how, uint64_t offset) {
 // g^T x_hat for a saved activation: [O, in_features].
 Tensor weight_grad(const Tensor& g, const Compressed& c, int64_t bits, int64_t N) {
   Tensor G;
-  if (g.scalar_type() == at::kFloat && g.size(1) <= 256) {
-    G = grad_weight(g.contiguous(), bits, c.q, c.width, nullptr, 0).narrow(1, 0, c.width);
+  if (grad_weight_takes(g)) {
+    G = grad_weight(g, bits, c.q, c.width, nullptr, 0).narrow(1, 0, c.width);
   } else {
-    G = at::mm(g.t(), unpack(c.q.codes, bits, c.q.scale, c.q.mn, N, c.width));
+    const Tensor x = unpack(c.q.codes, bits, c.q.scale, c.q.mn, N, c.width);
+    G = g.scalar_type() == at::kFloat ? rows_reduce_mm(g.contiguous(), x) : at::mm(g.t(), x);
   }
   return c.R.defined() ? at::mm(G, c.R.t()) : G.contiguous();
 }
@@ -267,7 +268,7 @@ struct SageNode : Function<SageNode> {
       gb = std::get<1>(rows_scale_colsum(g, {}, false, true));
     }
     // both weight gradients in one pass over g: g^T [Xq_agg | Xq_x], then the two small transposed projections
-    if (O <= 256) {
+    if (grad_weight_takes(g)) {
       const int64_t k0pad = (k + 15) / 16 * 16;
       const Tensor G = grad_weight(g, s->how.bits, s->agg.q, k, has_r ? &s->x.q : nullptr, has_r ? s->x.width : 0).narrow(0, 0, O);
       gl = G.narrow(1, 0, k);

@@ -281,7 +281,7 @@ PyMethodDef methods[] = {
     EXB_METHOD("set_clock", set_clock), EXB_METHOD("host_ns", host_ns), EXB_METHOD("host_calls", host_calls),
     EXB_METHOD("take_status_pending", take_status_pending), EXB_METHOD("peek_status", peek_status), EXB_METHOD("make_plan", make_plan), EXB_METHOD("make_graph", make_graph),
     EXB_METHOD("quantize_pack", quantize_pack), EXB_METHOD("unpack", unpack), EXB_METHOD("rademacher", rademacher),
-    EXB_METHOD("rp_quantize_pack", rp_quantize_pack_op), EXB_METHOD("bn_backward", bn_backward_op), EXB_METHOD("linear", linear_op), EXB_METHOD("grad_weight", grad_weight_op),
+    EXB_METHOD("rp_quantize_pack", rp_quantize_pack_op), EXB_METHOD("bn_backward", bn_backward_op), EXB_METHOD("linear", linear_op), EXB_METHOD("grad_weight", grad_weight_op), EXB_METHOD("grad_weight_takes", grad_weight_takes),
     EXB_METHOD("rows_scale_colsum", rows_scale_colsum), EXB_METHOD("spmm", spmm_op), EXB_METHOD("act", act_node),
     EXB_METHOD("batch_norm", bn_op), EXB_METHOD("aggregate", aggregate_op), EXB_METHOD("spmm_minmax", spmm_minmax_op),
     EXB_METHOD("spmm_minmax_backward", spmm_minmax_backward), EXB_METHOD("spmm_value_backward", spmm_value_backward),

@@ -236,14 +236,31 @@ Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const 
   return out;
 }
 
+// The one rule of which weight gradients the kernel forms; the others are unpacked and go to rows_reduce_mm.
+bool grad_weight_takes(const Tensor& g) {
+  return g.is_cuda() && g.scalar_type() == at::kFloat && g.dim() == 2 && g.size(0) > 0 && g.size(1) <= 256;
+}
+
+// g^T x with the reduction over rows cut into products that one batched library GEMM computes in parallel: a single one leaves
+// most SMs idle on this shape, and its sums are longer.
+Tensor rows_reduce_mm(const Tensor& g, const Tensor& x, int64_t batches) {
+  const int64_t M = g.size(0);
+  if (!g.is_cuda() || M < 64 * batches || !g.is_contiguous() || !x.is_contiguous()) return at::mm(g.t(), x);
+  const int64_t rows = M / batches * batches;
+  Tensor out = at::bmm(g.narrow(0, 0, rows).view({batches, -1, g.size(1)}).transpose(1, 2), x.narrow(0, 0, rows).view({batches, -1, x.size(1)})).sum(0);
+  if (rows < M) out.addmm_(g.narrow(0, rows, M - rows).t(), x.narrow(0, rows, M - rows));
+  return out;
+}
+
 // g^T . dequantise(q0 | q1): [O, pad16(k0) + pad16(k1)] with the second block from column pad16(k0) on.
 Tensor grad_weight(const Tensor& g_, int64_t bits, const Packed& q0, int64_t k0, const Packed* q1, int64_t k1) {
   c10::cuda::CUDAGuard guard(g_.device());
-  const Tensor g = g_.size(1) % 4 ? at::constant_pad_nd(g_, {0, 4 - g_.size(1) % 4}) : g_;
+  Tensor g = g_.size(1) % 4 ? at::constant_pad_nd(g_, {0, 4 - g_.size(1) % 4}) : g_.contiguous();
+  if (reinterpret_cast<uintptr_t>(g.data_ptr()) % 16) g = g.clone();      // a view off the 16 bytes that a tensor map wants
   const int64_t N = g.size(0), O = g.size(1);
   const int64_t kpad = (k0 + 15) / 16 * 16 + (q1 ? (k1 + 15) / 16 * 16 : 0);
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  const int64_t ws_bytes = lib.exact_grad_weight_workspace_bytes(O, std::min<int64_t>(kpad, 256), sms);
+  const int64_t ws_bytes = lib.exact_grad_weight_workspace_bytes(O, kpad, sms);
   Tensor ws = empty({ws_bytes}, at::kByte, g), out = empty({O, kpad}, at::kFloat, g);
   CallInfo info;
   info.bytes = 4 * N * O + (N * (k0 + (q1 ? k1 : 0)) * bits) / 8 + 4 * N * (q1 ? 2 : 1);

@@ -11,11 +11,11 @@ namespace exb {
 
 constexpr int kSumSlices = 16;
 
-// Every thread of a (32, kSumSlices) block calls it; the sum is returned to the threads of slice 0.
-__device__ __forceinline__ float sum_partials(const float* __restrict__ column, long long stride, int n, bool valid,
-                                              float (*s_part)[33]) {
+// Every thread of a (32, kSumSlices) block calls it; the sum (in the precision of s_part) is returned to the threads of slice 0.
+template <typename Sum>
+__device__ __forceinline__ Sum sum_partials(const float* __restrict__ column, long long stride, int n, bool valid, Sum (*s_part)[33]) {
   const int sl = threadIdx.y;
-  float a = 0.f;
+  Sum a = 0;
   if (valid) {
     int i = sl;
     for (; i + 7 * kSumSlices < n; i += 8 * kSumSlices) {
@@ -23,17 +23,17 @@ __device__ __forceinline__ float sum_partials(const float* __restrict__ column, 
 #pragma unroll
       for (int u = 0; u < 8; u++) v[u] = column[(long long)(i + u * kSumSlices) * stride];
 #pragma unroll
-      for (int u = 0; u < 8; u++) a = __fadd_rn(a, v[u]);
+      for (int u = 0; u < 8; u++) a += v[u];
     }
-    for (; i < n; i += kSumSlices) a = __fadd_rn(a, column[(long long)i * stride]);
+    for (; i < n; i += kSumSlices) a += column[(long long)i * stride];
   }
   __syncthreads();          // s_part may still be read for the previous sum
   s_part[sl][threadIdx.x] = a;
   __syncthreads();
-  float t = 0.f;
+  Sum t = 0;
   if (sl == 0) {
 #pragma unroll
-    for (int y = 0; y < kSumSlices; y++) t = __fadd_rn(t, s_part[y][threadIdx.x]);
+    for (int y = 0; y < kSumSlices; y++) t += s_part[y][threadIdx.x];
   }
   return t;
 }

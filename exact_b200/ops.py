@@ -214,7 +214,7 @@ def linear_backward_from_compressed(quantized, weight, bias, randmat, ori_input_
     input = None
     if (config.compress_activation and not config.simulate and not config.swap and quantized[1] is not None
             and len(q_input_shape) == 2 and (not projected or config.grad_weight_in_projected_space)
-            and ext_backward_func.grad_weight_supported(grad_output, q_input_shape[1], 0, quantized[1])):
+            and ext_backward_func.grad_weight_takes(grad_output)):
         # g^T Xq on the tensor cores with the dequantisation in the operand path: the [N, k] fp32 activation is
         # never written; with a projection, (g^T Xq) R^T instead of g^T (Xq R^T)
         grad_weight, _ = ext_backward_func.grad_weight_from_packed(grad_output, quantized, q_input_shape[1])

@@ -260,7 +260,7 @@ class qsage_layer(Function):
             grad_w_r = None
             if (config.compress_activation and not config.simulate and not config.swap and q_agg[1] is not None
                     and config.grad_weight_in_projected_space and both_projected
-                    and ext_backward_func.grad_weight_supported(g, k_agg, k_x if w_r is not None else 0, q_agg[1])):
+                    and ext_backward_func.grad_weight_takes(g)):
                 # both weight gradients in one pass over g: g^T [Xq_agg | Xq_x] on the tensor cores, dequantised
                 # on the way in, then the two small transposed projections
                 ga, gx = ext_backward_func.grad_weight_from_packed(g, q_agg, k_agg, q_x if w_r is not None else None,

@@ -483,11 +483,11 @@ EXACT_API int exact_linear_forward_strided(const float* A, int64_t M, int64_t K,
  * inputs of a GraphSAGE layer, layers.py:163-170) go in one pass: columns [0, k0) of `out` belong to the first,
  * columns [pad16(k0), pad16(k0) + k1) to the second (k1 = 0: one activation); ldo >= pad16(k0) + pad16(k1).
  *   g [N, O] fp32, 16-byte aligned, O % 4 == 0, O <= 256; other shapes return code 3 (the caller unpacks and
- *   uses a library GEMM).  tf32 inputs, fp32 accumulation: about 5e-4 relative.
+ *   uses a library GEMM).  Both operands split into fp16 heads and tails under a power of two per 64 rows, fp32
+ *   accumulation: 0.4e-7 .. 4e-7 relative (Frobenius) against fp64, as an fp32 GEMM.
  *   workspace: exact_grad_weight_workspace_bytes(O, pad16(k0) + pad16(k1), SM count) bytes, 256-byte aligned:
- *   it holds one partial result per CTA (of at
- *   most 256 columns: more are multiplied in passes), added in a fixed order by a second kernel (the result does not
- *   depend on timing). */
+ *   it holds one partial result per CTA (of 128 outputs and at most 128 columns), added in a fixed order by a second
+ *   kernel (the result does not depend on timing). */
 EXACT_API int64_t exact_grad_weight_workspace_bytes(int64_t O, int64_t k_total_padded, int max_ctas);
 EXACT_API int exact_grad_weight_from_packed(const float* g, int64_t N, int64_t O, const uint8_t* packed0,
                                             const uint16_t* scale0, const uint16_t* min0, int64_t k0,
