@@ -61,6 +61,7 @@ constexpr int kLinMaxStages = 4;
 constexpr uint32_t kLinSlotBytes = 32 * 1024;
 constexpr uint32_t kLinHalf = 16 * 1024;        // raw / tail halves of an A slot
 constexpr int kLinSleepNs = 200;                // back-off between polls of the epilogue, which waits long
+constexpr float kLinLoss = 1.1920929e-7f;       // 2^-23: what a chunk of two K tiles loses to the truncating accumulator on average
 constexpr int kLinPrefetch = 4;                 // K tiles of A requested into L2 ahead of their TMA load
 
 struct LinParams {
@@ -97,8 +98,11 @@ __device__ __forceinline__ void fence_proxy_async_smem_lin() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// CHUNKED: the contraction is drained from TMEM every p.chunk K tiles (a kernel of its own: its epilogue's registers and
-// code cost the unchunked product 5 %).
+// CHUNKED: the contraction is drained from TMEM every p.chunk K tiles, in fp32 and with a chunk's average loss given back; the small
+// products of two K tiles come before the large ones, as each step truncates at the size of what is there already.  With chunks of
+// two K tiles 1.4e-7 from fp64 at 602 and at 256 columns (the interleaved order and no correction: 5.2e-7, in one piece 4.4e-6 and
+// 1.8e-6), 232,965 x 602 -> 256 in 576 us against 297 in one piece and 1,235 of the library.  (A kernel of its own: its epilogue's
+// registers and code cost the unchunked product 5 %.)
 template <bool CHUNKED, bool PAIR>
 __global__ void __launch_bounds__(kLinThreads, 1)
 linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_a2,
@@ -215,10 +219,32 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       RingStage st;
       int t = 0;
       bool ok = true;
+      auto small_products = [&](uint32_t d, uint32_t at, bool first) {
+        const uint64_t ahi = umma_desc_sw128(at), alo = umma_desc_sw128(at + kLinHalf), bhi = umma_desc_sw128(at + kLinSlotBytes),
+                       blo = umma_desc_sw128(at + kLinSlotBytes + p.b_slot);
+#pragma unroll
+        for (int k4 = 0; k4 < kLinTileK / 8; k4++) {
+          const uint64_t o = (uint64_t)(k4 * 2);   // 8 tf32 = 32 bytes along K inside the swizzle atom
+          mma(d, alo + o, bhi + o, !first || k4 != 0);
+          mma(d, ahi + o, blo + o, 1);
+        }
+      };
+      auto head_products = [&](uint32_t d, uint32_t at) {
+        const uint64_t ahi = umma_desc_sw128(at), bhi = umma_desc_sw128(at + kLinSlotBytes);
+#pragma unroll
+        for (int k4 = 0; k4 < kLinTileK / 8; k4++) mma(d, ahi + (uint64_t)(k4 * 2), bhi + (uint64_t)(k4 * 2), 1);
+      };
+      // The next stage, when it is split and B is there.
+      auto ready = [&](uint32_t& at) {
+        if (!wait(smem_u32(&s_ready[st.s]), st.ph)) return false;
+        tc_fence_after();
+        at = ring + (uint32_t)st.s * p.stage_bytes;
+        return true;
+      };
       for (int tile = first; tile < tiles && ok; tile += step) {
         int buf = 0;
         uint32_t d_tmem = 0;
-        for (int kb = 0; kb < p.kblocks; kb++, st.next(p.stages)) {
+        for (int kb = 0; kb < p.kblocks;) {
           const bool opens = CHUNKED ? kb % p.chunk == 0 : kb == 0;
           if (opens) {
             buf = t & 1;
@@ -228,27 +254,46 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
             d_tmem = tmem_base + (uint32_t)(buf * p.Npad);
             t++;
           }
-          if (!wait(smem_u32(&s_ready[st.s]), st.ph)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t base = ring + (uint32_t)st.s * p.stage_bytes;
-          const uint64_t ahi = umma_desc_sw128(base);
-          const uint64_t alo = umma_desc_sw128(base + kLinHalf);
-          const uint64_t bhi = umma_desc_sw128(base + kLinSlotBytes);
-          const uint64_t blo = umma_desc_sw128(base + kLinSlotBytes + p.b_slot);
-          if (elected) {
+          uint32_t at0, at1 = 0;
+          if (!ready(at0)) { ok = false; break; }
+          const int s0 = st.s;
+          st.next(p.stages);
+          if (!CHUNKED) {
+            if (elected) {
+              const uint64_t ahi = umma_desc_sw128(at0), alo = umma_desc_sw128(at0 + kLinHalf), bhi = umma_desc_sw128(at0 + kLinSlotBytes),
+                             blo = umma_desc_sw128(at0 + kLinSlotBytes + p.b_slot);
 #pragma unroll
-            for (int k4 = 0; k4 < kLinTileK / 8; k4++) {
-              const uint64_t o = (uint64_t)(k4 * 2);   // 8 tf32 = 32 bytes along K inside the swizzle atom
-              mma(d_tmem, alo + o, bhi + o, !opens || k4 != 0);
-              mma(d_tmem, ahi + o, bhi + o, 1);
-            }
+              for (int k4 = 0; k4 < kLinTileK / 8; k4++) {
+                const uint64_t o = (uint64_t)(k4 * 2);
+                mma(d_tmem, alo + o, bhi + o, !opens || k4 != 0);
+                mma(d_tmem, ahi + o, bhi + o, 1);
+              }
 #pragma unroll
-            for (int k4 = 0; k4 < kLinTileK / 8; k4++) {
-              const uint64_t o = (uint64_t)(k4 * 2);
-              mma(d_tmem, ahi + o, blo + o, 1);
+              for (int k4 = 0; k4 < kLinTileK / 8; k4++) mma(d_tmem, ahi + (uint64_t)(k4 * 2), blo + (uint64_t)(k4 * 2), 1);
+              commit(smem_u32(&s_empty[s0]));
+              if (kb + 1 == p.kblocks) commit(smem_u32(&s_tfull[buf]));
             }
-            commit(smem_u32(&s_empty[st.s]));
-            if ((CHUNKED && (kb + 1) % p.chunk == 0) || kb + 1 == p.kblocks) commit(smem_u32(&s_tfull[buf]));
+            kb++;
+          } else {
+            // the small products of two K tiles before the large ones: the accumulator truncates at its own size
+            if (elected) small_products(d_tmem, at0, opens);
+            const bool two = kb + 1 < p.kblocks && (kb + 1) % p.chunk != 0;
+            const int s1 = st.s;
+            if (two) {
+              if (!ready(at1)) { ok = false; break; }
+              st.next(p.stages);
+            }
+            if (elected) {
+              if (two) small_products(d_tmem, at1, false);
+              head_products(d_tmem, at0);
+              commit(smem_u32(&s_empty[s0]));
+              if (two) {
+                head_products(d_tmem, at1);
+                commit(smem_u32(&s_empty[s1]));
+              }
+            }
+            kb += two ? 2 : 1;
+            if (elected && (kb % p.chunk == 0 || kb == p.kblocks)) commit(smem_u32(&s_tfull[buf]));
           }
           __syncwarp();
         }
@@ -339,6 +384,8 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 #pragma unroll
               for (int j = 0; j < 4; j++) {
                 float4 o = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                o.x = __fmaf_rn(o.x, kLinLoss, o.x); o.y = __fmaf_rn(o.y, kLinLoss, o.y);
+                o.z = __fmaf_rn(o.z, kLinLoss, o.z); o.w = __fmaf_rn(o.w, kLinLoss, o.w);
                 if (ch > 0) {
                   const float4 q = old[h * 4 + j];
                   o.x += q.x; o.y += q.y; o.z += q.z; o.w += q.w;
@@ -359,13 +406,15 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       const int buf = t & 1;
       const uint32_t ph = (uint32_t)(t >> 1) & 1u;
       t++;
-      float4 sum[8];         // the running sums of the next 32 columns
+      float4 sum[8];         // the running sums of the next 32 columns (zero where this chunk is the only one)
+#pragma unroll
+      for (int j = 0; j < 8; j++) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
       auto fetch = [&](int c0) {
 #pragma unroll
         for (int j = 0; j < 8; j++)
           if (c0 + j * 4 < p.Npad) sum[j] = __ldcg(part + (size_t)(c0 / 4 + j) * kLinTileM);
       };
-      if (CHUNKED) fetch(share * 32);
+      if (CHUNKED && chunks > 1) fetch(share * 32);
       if (!mbar_wait<kLinSleepNs>(smem_u32(&s_tfull[buf]), ph, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.Npad);
@@ -379,7 +428,10 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 #pragma unroll
             for (int j = 0; j < 4; j++) {
               const float4 q = h ? sum[4 + j] : sum[j];
-              v[4 * j] += q.x; v[4 * j + 1] += q.y; v[4 * j + 2] += q.z; v[4 * j + 3] += q.w;
+              v[4 * j] = __fmaf_rn(v[4 * j], kLinLoss, v[4 * j]) + q.x;
+              v[4 * j + 1] = __fmaf_rn(v[4 * j + 1], kLinLoss, v[4 * j + 1]) + q.y;
+              v[4 * j + 2] = __fmaf_rn(v[4 * j + 2], kLinLoss, v[4 * j + 2]) + q.z;
+              v[4 * j + 3] = __fmaf_rn(v[4 * j + 3], kLinLoss, v[4 * j + 3]) + q.w;
             }
           }
 #pragma unroll
@@ -391,7 +443,7 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                          : "memory");
           }
         }
-        if (CHUNKED && c0 + 32 * kLinEpiGroups < p.Npad) fetch(c0 + 32 * kLinEpiGroups);
+        if (CHUNKED && chunks > 1 && c0 + 32 * kLinEpiGroups < p.Npad) fetch(c0 + 32 * kLinEpiGroups);
         __syncwarp();
         const uint32_t ci = (uint32_t)lane & 7u;
         const int c = c0 + (int)ci * 4;
@@ -563,7 +615,7 @@ int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t l
   while (cols < (unsigned)(2 * Npad)) cols <<= 1;
   p.tmem_cols = cols;
   const size_t dyn = (size_t)kLinSlots * kLinSlotBytes + 4 * kLinEpiGroups * 4096 + 1024;
-  const bool chunked = p.chunk < p.kblocks;
+  const bool chunked = k_chunk > 0;
   auto* kern = pair ? (chunked ? linear_tf32x3_kernel<true, true> : linear_tf32x3_kernel<false, true>)
                     : (chunked ? linear_tf32x3_kernel<true, false> : linear_tf32x3_kernel<false, false>);
   EXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
