@@ -61,7 +61,8 @@ constexpr int kLinMaxStages = 4;
 constexpr uint32_t kLinSlotBytes = 32 * 1024;
 constexpr uint32_t kLinHalf = 16 * 1024;        // raw / tail halves of an A slot
 constexpr int kLinSleepNs = 200;                // back-off between polls of the epilogue, which waits long
-constexpr float kLinLoss = 1.1920929e-7f;       // 2^-23: what a chunk of two K tiles loses to the truncating accumulator on average
+constexpr float kLinGain = 1.00000011920929f;   // 1 + 2^-23: gives back what a chunk of two K tiles loses to the truncating accumulator on average
+constexpr int kLinChunkedCols = 128;             // columns of a launch in chunks
 constexpr int kLinPrefetch = 4;                 // K tiles of A requested into L2 ahead of their TMA load
 
 struct LinParams {
@@ -77,7 +78,6 @@ struct LinParams {
   const float* addend;     // [M, ldadd] added to the product (C itself: C += ...), or null
   long long ldadd;
   int chunk;               // K tiles that are accumulated in TMEM before their sum is taken over in fp32
-  float* partial;          // [grid, Npad / 4, 128, 4]: running sums of the chunks before the last, per CTA
   int stages;              // K tiles the ring holds
   unsigned b_slot;         // bytes of a B_hi / B_lo slot: 128 per row of B in this CTA
   unsigned stage_bytes;    // A slot (32 KB) + two B slots
@@ -100,8 +100,8 @@ __device__ __forceinline__ void fence_proxy_async_smem_lin() {
 
 // CHUNKED: the contraction is drained from TMEM every p.chunk K tiles, in fp32 and with a chunk's average loss given back; the small
 // products of two K tiles come before the large ones, as each step truncates at the size of what is there already.  With chunks of
-// two K tiles 1.4e-7 from fp64 at 602 and at 256 columns (the interleaved order and no correction: 5.2e-7, in one piece 4.4e-6 and
-// 1.8e-6), 232,965 x 602 -> 256 in 576 us against 297 in one piece and 1,235 of the library.  (A kernel of its own: its epilogue's
+// two K tiles 1.4e-7 and 1.3e-7 from fp64 at 602 and at 256 columns (the interleaved order and no correction: 5.2e-7, in one piece 4.4e-6 and
+// 1.8e-6).  (A kernel of its own: its epilogue's
 // registers and code cost the unchunked product 5 %.)
 template <bool CHUNKED, bool PAIR>
 __global__ void __launch_bounds__(kLinThreads, 1)
@@ -360,131 +360,116 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     int t = 0;
     bool ok = true;
     const int chunks = CHUNKED ? (p.kblocks + p.chunk - 1) / p.chunk : 1;
-    // this thread's row of the running sums: 16 bytes per four columns, adjacent lanes adjacent
-    float4* __restrict__ part = !CHUNKED ? nullptr : reinterpret_cast<float4*>(p.partial) + (size_t)blockIdx.x * (p.Npad / 4) * kLinTileM + quad * 32 + lane;
-    for (int tile = first; tile < tiles && ok; tile += step) {
-      for (int ch = 0; CHUNKED && ch + 1 < chunks && ok; ch++, t++) {
-        const int buf = t & 1;
-        if (!mbar_wait<kLinSleepNs>(smem_u32(&s_tfull[buf]), (uint32_t)(t >> 1) & 1u, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.Npad);
-        for (int c0 = share * 32; c0 < p.Npad; c0 += 32 * kLinEpiGroups) {
-          const int cols = p.Npad - c0 < 32 ? p.Npad - c0 : 32;
-          float4 old[8];
-          if (ch > 0) {
+    // 16 columns of this thread's row to the warp's staging tile
+    auto stage16 = [&](int h, const float* v) {
 #pragma unroll
-            for (int j = 0; j < 8; j++)
-              if (j * 4 < cols) old[j] = __ldcg(part + (size_t)(c0 / 4 + j) * kLinTileM);
-          }
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            if (h * 16 < cols) {
-              float v[16];
-              tmem_ld16(taddr + (uint32_t)(c0 + h * 16), v);
-#pragma unroll
-              for (int j = 0; j < 4; j++) {
-                float4 o = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                o.x = __fmaf_rn(o.x, kLinLoss, o.x); o.y = __fmaf_rn(o.y, kLinLoss, o.y);
-                o.z = __fmaf_rn(o.z, kLinLoss, o.z); o.w = __fmaf_rn(o.w, kLinLoss, o.w);
-                if (ch > 0) {
-                  const float4 q = old[h * 4 + j];
-                  o.x += q.x; o.y += q.y; o.z += q.z; o.w += q.w;
-                }
-                __stcg(part + (size_t)(c0 / 4 + h * 4 + j) * kLinTileM, o);
-              }
-            }
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-        if (PAIR) mbar_arrive_leader(smem_u32(&s_tempty[buf]));
-        else mbar_arrive(smem_u32(&s_tempty[buf]));
+      for (int j = 0; j < 4; j++) {
+        const uint32_t ci = (uint32_t)(h * 4 + j);
+        const uint32_t addr = stage_addr + (uint32_t)lane * 128u + ((ci ^ ((uint32_t)lane & 7u)) << 4);
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v[4 * j]), "f"(v[4 * j + 1]),
+                     "f"(v[4 * j + 2]), "f"(v[4 * j + 3])
+                     : "memory");
       }
+    };
+    // the staged columns c0 .. c0 + cols - 1 of the warp's 32 rows (+ bias, + addend) to C
+    auto write_out = [&](int c0, int cols, long long row_base) {
+      __syncwarp();
+      const uint32_t ci = (uint32_t)lane & 7u;
+      const int c = c0 + (int)ci * 4;
+      float bv[4] = {0.f, 0.f, 0.f, 0.f};
+      if (p.bias != nullptr) {
+#pragma unroll
+        for (int bb = 0; bb < 4; bb++)
+          if (c + bb < p.N) bv[bb] = __ldg(p.bias + c + bb);
       }
-      if (!ok) break;
-      const int buf = t & 1;
-      const uint32_t ph = (uint32_t)(t >> 1) & 1u;
-      t++;
-      float4 sum[8];         // the running sums of the next 32 columns (zero where this chunk is the only one)
 #pragma unroll
-      for (int j = 0; j < 8; j++) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      auto fetch = [&](int c0) {
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-          if (c0 + j * 4 < p.Npad) sum[j] = __ldcg(part + (size_t)(c0 / 4 + j) * kLinTileM);
-      };
-      if (CHUNKED && chunks > 1) fetch(share * 32);
-      if (!mbar_wait<kLinSleepNs>(smem_u32(&s_tfull[buf]), ph, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.Npad);
-      const long long row_base = (long long)tile * kLinTileM + quad * 32;
-      for (int c0 = share * 32; c0 < p.Npad; c0 += 32 * kLinEpiGroups) {
-        const int cols = (p.Npad - c0) < 32 ? (p.Npad - c0) : 32;   // 16 or 32
-        for (int h = 0; h * 16 < cols; h++) {
-          float v[16];
-          tmem_ld16(taddr + (uint32_t)(c0 + h * 16), v);
-          if (CHUNKED) {
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-              const float4 q = h ? sum[4 + j] : sum[j];
-              v[4 * j] = __fmaf_rn(v[4 * j], kLinLoss, v[4 * j]) + q.x;
-              v[4 * j + 1] = __fmaf_rn(v[4 * j + 1], kLinLoss, v[4 * j + 1]) + q.y;
-              v[4 * j + 2] = __fmaf_rn(v[4 * j + 2], kLinLoss, v[4 * j + 2]) + q.z;
-              v[4 * j + 3] = __fmaf_rn(v[4 * j + 3], kLinLoss, v[4 * j + 3]) + q.w;
+      for (int i = 0; i < 8; i++) {
+        const int rr = 4 * i + (lane >> 3);
+        const long long nn = row_base + rr;
+        float4 o;
+        const uint32_t addr = stage_addr + (uint32_t)rr * 128u + ((ci ^ ((uint32_t)rr & 7u)) << 4);
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(addr));
+        if (nn < p.M && (int)ci * 4 < cols && c < p.N) {
+          float* d = p.C + nn * p.ldc + c;
+          const float* add = p.addend ? p.addend + nn * p.ldadd + c : nullptr;
+          o.x += bv[0]; o.y += bv[1]; o.z += bv[2]; o.w += bv[3];
+          if (vec) {   // N % 4 == 0, so c + 4 <= N
+            if (add) {
+              const float4 old = *reinterpret_cast<const float4*>(add);
+              o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
             }
-          }
+            __stcs(reinterpret_cast<float4*>(d), o);
+          } else {
+            const float ov[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const uint32_t ci = (uint32_t)(h * 4 + j);
-            const uint32_t addr = stage_addr + (uint32_t)lane * 128u + ((ci ^ ((uint32_t)lane & 7u)) << 4);
-            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v[4 * j]), "f"(v[4 * j + 1]),
-                         "f"(v[4 * j + 2]), "f"(v[4 * j + 3])
-                         : "memory");
+            for (int bb = 0; bb < 4; bb++)
+              if (c + bb < p.N) d[bb] = add ? add[bb] + ov[bb] : ov[bb];
           }
         }
-        if (CHUNKED && chunks > 1 && c0 + 32 * kLinEpiGroups < p.Npad) fetch(c0 + 32 * kLinEpiGroups);
-        __syncwarp();
-        const uint32_t ci = (uint32_t)lane & 7u;
-        const int c = c0 + (int)ci * 4;
-        float bv[4] = {0.f, 0.f, 0.f, 0.f};
-        if (p.bias != nullptr) {
-#pragma unroll
-          for (int bb = 0; bb < 4; bb++)
-            if (c + bb < p.N) bv[bb] = __ldg(p.bias + c + bb);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const int rr = 4 * i + (lane >> 3);
-          const long long nn = row_base + rr;
-          float4 o;
-          const uint32_t addr = stage_addr + (uint32_t)rr * 128u + ((ci ^ ((uint32_t)rr & 7u)) << 4);
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(addr));
-          if (nn < p.M && (int)ci * 4 < cols && c < p.N) {
-            float* d = p.C + nn * p.ldc + c;
-            const float* add = p.addend ? p.addend + nn * p.ldadd + c : nullptr;
-            o.x += bv[0]; o.y += bv[1]; o.z += bv[2]; o.w += bv[3];
-            if (vec) {   // N % 4 == 0, so c + 4 <= N
-              if (add) {
-                const float4 old = *reinterpret_cast<const float4*>(add);
-                o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-              }
-              __stcs(reinterpret_cast<float4*>(d), o);
-            } else {
-              const float ov[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-              for (int bb = 0; bb < 4; bb++)
-                if (c + bb < p.N) d[bb] = add ? add[bb] + ov[bb] : ov[bb];
-            }
-          }
-        }
-        __syncwarp();
       }
+      __syncwarp();
+    };
+    auto release = [&](int buf) {
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
         if (PAIR) mbar_arrive_leader(smem_u32(&s_tempty[buf]));
         else mbar_arrive(smem_u32(&s_tempty[buf]));
+      }
+    };
+    for (int tile = first; tile < tiles && ok; tile += step) {
+      const long long row_base = (long long)tile * kLinTileM + quad * 32;
+      if constexpr (CHUNKED) {
+        // At most 128 columns, so that this thread's half of a row's sums stays in registers: kept in memory they were 16 TB/s of
+        // L2 traffic.  232,965 x 602 -> 256, two launches, chunks of 64: 576 -> 457 us; x 512 453 -> 377 (library: 1,235, 1,049).
+        static_assert(kLinEpiGroups == 2 && kLinChunkedCols == 128, "64 columns a thread");
+        float run[64];
+#pragma unroll
+        for (int i = 0; i < 64; i++) run[i] = 0.f;
+        for (int ch = 0; ch < chunks; ch++, t++) {
+          const int buf = t & 1;
+          if (!mbar_wait<kLinSleepNs>(smem_u32(&s_tfull[buf]), (uint32_t)(t >> 1) & 1u, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.Npad);
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const int c0 = (q >> 1) * 64 + share * 32 + (q & 1) * 16;
+            if (c0 < p.Npad) {
+              float v[16];
+              tmem_ld16(taddr + (uint32_t)c0, v);
+#pragma unroll
+              for (int e = 0; e < 16; e++) run[16 * q + e] = __fmaf_rn(v[e], kLinGain, run[16 * q + e]);
+            }
+          }
+          release(buf);
+        }
+        if (!ok) break;
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+          const int c0 = b * 64 + share * 32;
+          if (c0 < p.Npad) {
+            stage16(0, run + 32 * b);
+            stage16(1, run + 32 * b + 16);
+            write_out(c0, p.Npad - c0 < 32 ? p.Npad - c0 : 32, row_base);
+          }
+        }
+      } else {
+        const int buf = t & 1;
+        const uint32_t ph = (uint32_t)(t >> 1) & 1u;
+        t++;
+        if (!mbar_wait<kLinSleepNs>(smem_u32(&s_tfull[buf]), ph, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.Npad);
+        for (int c0 = share * 32; c0 < p.Npad; c0 += 32 * kLinEpiGroups) {
+          const int cols = (p.Npad - c0) < 32 ? (p.Npad - c0) : 32;   // 16 or 32
+          for (int h = 0; h * 16 < cols; h++) {
+            float v[16];
+            tmem_ld16(taddr + (uint32_t)(c0 + h * 16), v);
+            stage16(h, v);
+          }
+          write_out(c0, cols, row_base);
+        }
+        release(buf);
       }
     }
   }
@@ -507,13 +492,13 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 
 // Heads and tails of [B | B2] (rows = output features), zero padded to [Npad, Kpad1 + Kpad2], in the order and with the swizzle
 // of the shared-memory tiles: K tile by K tile, in it the share of each CTA of a pair (b_rows rows), in that the heads and then
-// the tails, so that a CTA's part of a K tile is one contiguous run.  Also clears the status word.
+// the tails, so that a CTA's part of a K tile is one contiguous run.  Also clears the status word, if given.
 __global__ void linear_prepare_kernel(const float* __restrict__ B, int K, long long ldb, long long incb,
                                       const float* __restrict__ B2, int K2, long long ldb2, long long incb2, int N, int Npad,
                                       int Kpad1, int Kpad,
                                       int b_rows, float* __restrict__ out, int* status) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) *status = 0;
+  if (i == 0 && status != nullptr) *status = 0;
   if (i >= Npad * Kpad) return;
   const int n = i / Kpad, kk = i - n * Kpad;
   float v = 0.f;
@@ -534,49 +519,10 @@ __global__ void linear_prepare_kernel(const float* __restrict__ B, int K, long l
 
 static inline int lin_kpad(long long K) { return (int)((K + kLinTileK - 1) / kLinTileK * kLinTileK); }
 
-}  // namespace exb
-
-using namespace exb;
-
-extern "C" {
-
-int64_t exact_linear_workspace_bytes(int64_t N, int64_t K, int64_t K2) {
-  if (N <= 0 || K <= 0 || K2 < 0) return 256;
-  const int64_t Npad = (N + 15) / 16 * 16;
-  return 256 + 2 * Npad * (int64_t)(lin_kpad(K) + lin_kpad(K2)) * 4;
-}
-
-int64_t exact_linear_partial_bytes(int64_t N) {
-  const int64_t Npad = (N + 15) / 16 * 16;
-  return N > 0 ? (int64_t)sm_count() * Npad * kLinTileM * 4 : 0;
-}
-
-int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb,
-                         const float* A2, int64_t K2, int64_t lda2, const float* B2, int64_t ldb2, int64_t N,
-                         const float* bias, int accumulate, void* workspace, float* C, int64_t ldc, void* stream) {
-  return exact_linear_forward_strided(A, M, K, lda, B, ldb, 1, A2, K2, lda2, B2, ldb2, 1, N, bias, accumulate ? C : nullptr,
-                                      accumulate ? ldc : 0, 0, nullptr, workspace, C, ldc, stream);
-}
-
-int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb, int64_t incb,
-                         const float* A2, int64_t K2, int64_t lda2, const float* B2, int64_t ldb2, int64_t incb2, int64_t N,
-                         const float* bias, const float* addend, int64_t ldadd, int64_t k_chunk, float* partial, void* workspace,
-                         float* C, int64_t ldc, void* stream) {
-  EXB_REQUIRE(k_chunk >= 0 && k_chunk % kLinTileK == 0 && (k_chunk == 0 || (partial && (reinterpret_cast<uintptr_t>(partial) & 15) == 0)),
-              "linear_forward: k_chunk must be a multiple of 32 and needs a 16-byte aligned buffer of partial sums");
-  EXB_REQUIRE(M >= 0 && K > 0 && N > 0 && K2 >= 0, "linear_forward: bad shape");
-  if (M == 0) return EXB_OK;
-  EXB_REQUIRE(A && B && C && workspace, "linear_forward: null pointer");
-  EXB_REQUIRE((A2 != nullptr) == (K2 > 0) && (B2 != nullptr) == (K2 > 0), "linear_forward: the second operand pair needs A2, B2 and K2 > 0");
-  EXB_REQUIRE(lda >= K && (incb != 1 || ldb >= K) && ldc >= N && (K2 == 0 || (lda2 >= K2 && (incb2 != 1 || ldb2 >= K2))), "linear_forward: leading dimension smaller than the row");
-  EXB_REQUIRE(addend == nullptr || ldadd >= N, "linear_forward: leading dimension of the addend smaller than the row");
-  if (N > 256) return fail(EXB_ERR_UNSUPPORTED, "linear_forward: N = %lld exceeds one MMA tile (256); call per 256-column block", (long long)N);
-  if (lda % 4 != 0 || (reinterpret_cast<uintptr_t>(A) & 15) != 0 ||
-      (K2 > 0 && (lda2 % 4 != 0 || (reinterpret_cast<uintptr_t>(A2) & 15) != 0)))
-    return fail(EXB_ERR_UNSUPPORTED, "linear_forward: the TMA path needs 16-byte aligned rows of A (lda %% 4 == 0)");
-  EXB_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "linear_forward: workspace must be 256-byte aligned");
-  EXB_REQUIRE((M + kLinTileM - 1) / kLinTileM < 2147483647LL / kLinTileM, "linear_forward: too many rows");
-  cudaStream_t st = (cudaStream_t)stream;
+// One launch over checked arguments: N <= 256 columns, <= 128 of them in chunks.  clears: whether it clears the workspace's status.
+static int lin_launch(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb, int64_t incb, const float* A2, int64_t K2,
+                      int64_t lda2, const float* B2, int64_t ldb2, int64_t incb2, int64_t N, const float* bias, const float* addend,
+                      int64_t ldadd, int64_t k_chunk, bool clears, void* workspace, float* C, int64_t ldc, cudaStream_t st) {
   const int Npad = (int)((N + 15) / 16 * 16);
   const int Kpad1 = lin_kpad(K), Kpad2 = lin_kpad(K2), Kpad = Kpad1 + Kpad2;
   int* status = reinterpret_cast<int*>(workspace);
@@ -587,7 +533,7 @@ int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t l
   const int b_rows = pair ? Npad / 2 : Npad;   // of B in one CTA
 
   linear_prepare_kernel<<<(Npad * Kpad + 255) / 256, 256, 0, st>>>(B, (int)K, ldb, incb, B2, (int)K2, ldb2, incb2, (int)N, Npad,
-                                                                   Kpad1, Kpad, b_rows, b, status);
+                                                                   Kpad1, Kpad, b_rows, b, clears ? status : nullptr);
   EXB_CUDA_OK(cudaGetLastError());
 
   CUtensorMap tm_a, tm_a2;
@@ -606,7 +552,6 @@ int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t l
   p.num_tiles = num_tiles;
   p.addend = addend; p.ldadd = ldadd;
   p.chunk = k_chunk > 0 ? (int)(k_chunk / kLinTileK) : p.kblocks;
-  p.partial = partial;
   p.b_slot = (unsigned)b_rows * kLinTileK * 4;
   p.stage_bytes = kLinSlotBytes + 2 * p.b_slot;
   p.stages = (int)((kLinSlots * kLinSlotBytes) / p.stage_bytes);
@@ -635,6 +580,56 @@ int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t l
   cfg.numAttrs = pair ? 1 : 0;
   EXB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tm_a, tm_a2, p));
   EXB_CUDA_OK(cudaGetLastError());
+  return EXB_OK;
+}
+
+}  // namespace exb
+
+using namespace exb;
+
+extern "C" {
+
+int64_t exact_linear_workspace_bytes(int64_t N, int64_t K, int64_t K2) {
+  if (N <= 0 || K <= 0 || K2 < 0) return 256;
+  const int64_t Npad = (N + 15) / 16 * 16;
+  return 256 + 2 * Npad * (int64_t)(lin_kpad(K) + lin_kpad(K2)) * 4;
+}
+
+int64_t exact_linear_partial_bytes(int64_t) { return 0; }   // the running sums of a contraction in chunks stay in registers
+
+int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb,
+                         const float* A2, int64_t K2, int64_t lda2, const float* B2, int64_t ldb2, int64_t N,
+                         const float* bias, int accumulate, void* workspace, float* C, int64_t ldc, void* stream) {
+  return exact_linear_forward_strided(A, M, K, lda, B, ldb, 1, A2, K2, lda2, B2, ldb2, 1, N, bias, accumulate ? C : nullptr,
+                                      accumulate ? ldc : 0, 0, nullptr, workspace, C, ldc, stream);
+}
+
+int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb, int64_t incb,
+                         const float* A2, int64_t K2, int64_t lda2, const float* B2, int64_t ldb2, int64_t incb2, int64_t N,
+                         const float* bias, const float* addend, int64_t ldadd, int64_t k_chunk, float* partial, void* workspace,
+                         float* C, int64_t ldc, void* stream) {
+  (void)partial;
+  EXB_REQUIRE(k_chunk >= 0 && k_chunk % kLinTileK == 0, "linear_forward: k_chunk must be a multiple of 32");
+  EXB_REQUIRE(M >= 0 && K > 0 && N > 0 && K2 >= 0, "linear_forward: bad shape");
+  if (M == 0) return EXB_OK;
+  EXB_REQUIRE(A && B && C && workspace, "linear_forward: null pointer");
+  EXB_REQUIRE((A2 != nullptr) == (K2 > 0) && (B2 != nullptr) == (K2 > 0), "linear_forward: the second operand pair needs A2, B2 and K2 > 0");
+  EXB_REQUIRE(lda >= K && (incb != 1 || ldb >= K) && ldc >= N && (K2 == 0 || (lda2 >= K2 && (incb2 != 1 || ldb2 >= K2))), "linear_forward: leading dimension smaller than the row");
+  EXB_REQUIRE(addend == nullptr || ldadd >= N, "linear_forward: leading dimension of the addend smaller than the row");
+  if (N > 256) return fail(EXB_ERR_UNSUPPORTED, "linear_forward: N = %lld exceeds one MMA tile (256); call per 256-column block", (long long)N);
+  if (lda % 4 != 0 || (reinterpret_cast<uintptr_t>(A) & 15) != 0 ||
+      (K2 > 0 && (lda2 % 4 != 0 || (reinterpret_cast<uintptr_t>(A2) & 15) != 0)))
+    return fail(EXB_ERR_UNSUPPORTED, "linear_forward: the TMA path needs 16-byte aligned rows of A (lda %% 4 == 0)");
+  EXB_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "linear_forward: workspace must be 256-byte aligned");
+  EXB_REQUIRE((M + kLinTileM - 1) / kLinTileM < 2147483647LL / kLinTileM, "linear_forward: too many rows");
+  cudaStream_t st = (cudaStream_t)stream;
+  if (k_chunk == 0) return lin_launch(A, M, K, lda, B, ldb, incb, A2, K2, lda2, B2, ldb2, incb2, N, bias, addend, ldadd, 0, true, workspace, C, ldc, st);
+  for (int64_t n0 = 0; n0 < N; n0 += kLinChunkedCols) {
+    const int rc = lin_launch(A, M, K, lda, B + n0 * ldb, ldb, incb, A2, K2, lda2, K2 ? B2 + n0 * ldb2 : nullptr, ldb2, incb2,
+                              N - n0 < kLinChunkedCols ? N - n0 : kLinChunkedCols, bias ? bias + n0 : nullptr, addend ? addend + n0 : nullptr,
+                              ldadd, k_chunk, n0 == 0, workspace, C + n0, ldc, st);
+    if (rc) return rc;
+  }
   return EXB_OK;
 }
 

@@ -418,9 +418,9 @@ Tensor aggregate_node(const Tensor& x, const OptTensor& value, const OptTensor& 
 
 // ---- evaluation -----------------------------------------------------------------------------------------
 // Evaluation is compared with the plain fp32 model, so its products are no further from the exact ones than the library's fp32 GEMM:
-// contractions in chunks of 64 columns, the small products first, 1.3e-7 to 1.5e-7 (Frobenius) at every width against 1.8e-7 at
+// contractions in chunks of 64 columns, the small products first, 1.3e-7 to 1.4e-7 (Frobenius) at every width against 1.8e-7 at
 // 100, 2.0e-7 at 256 and 4.4e-7 at 602 columns; in one piece the accumulator's truncation makes it 8e-7, 1.8e-6 and 4.4e-6.  Up to
-// 64 columns the library is the nearer one (9e-8 against 1.1e-7 at 48) and takes them, 200,000 x 48 -> 256 in 178 us against 83.
+// 64 columns the library is the nearer one (9e-8 against 1.1e-7 at 48) and takes them, 200,000 x 48 -> 256 in 173 us against 98.
 constexpr int64_t kEvalChunk = 64;
 
 // a w^T (+ a2 w2^T) (+ bias) (+ addend)

@@ -212,8 +212,6 @@ Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const 
   Tensor out = out_ ? *out_ : empty({M, N}, at::kFloat, a);
   const OptTensor addend = addend_ ? addend_ : out_ && accumulate ? OptTensor(out) : OptTensor();
   if (out.size(0) != M || out.size(1) != N || out.stride(1) != 1) throw std::runtime_error("linear: out does not fit");
-  Tensor partial;      // of a contraction in chunks (exact_linear_forward_chunked)
-  if (k_chunk > 0 && K + K2 > k_chunk) partial = empty({lib.exact_linear_partial_bytes(std::min<int64_t>(N, 256))}, at::kByte, a);
   for (int64_t n0 = 0; n0 < N; n0 += 256) {
     const int64_t n = std::min<int64_t>(N - n0, 256);
     Tensor ws = empty({lib.exact_linear_workspace_bytes(n, K, K2)}, at::kByte, a);
@@ -228,7 +226,7 @@ Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const 
                                       K2 ? a2.stride(0) : 0, w2b, K2 ? w2.stride(0) : 0, K2 ? w2.stride(1) : 1, n,
                                       bias.defined() ? ptr<float>(bias) + n0 : nullptr,
                                               addend ? ptr<float>(addend) + n0 : nullptr, addend ? addend->stride(0) : 0,
-                                              partial.defined() ? k_chunk : 0, partial.defined() ? ptr<float>(partial) : nullptr, ptr(ws),
+                                              k_chunk, nullptr, ptr(ws),
                                               cb, out.stride(0), st);
     });
   }

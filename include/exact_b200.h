@@ -467,7 +467,7 @@ EXACT_API int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t
  * multiple of 32; 0: one chunk).  The tensor core truncates its fp32 accumulator at every MMA, a bias of about 7e-9 of the
  * result per contracted column in one piece.  With chunks the small products of two K tiles come first, a chunk's sum has the
  * loss of a chunk of 64 given back and is added to the previous ones by an fp32 addition: 1.5e-7 (Frobenius, against fp64) with 64,
- * 6e-7 with 128, 1.5e-6 with 256, whatever K is.  partial: exact_linear_partial_bytes(N) bytes, 16-byte aligned. */
+ * 6e-7 with 128, 1.5e-6 with 256, whatever K is.  partial: exact_linear_partial_bytes(N) bytes (none: not used any more). */
 EXACT_API int64_t exact_linear_partial_bytes(int64_t N);
 EXACT_API int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb,
                                            int64_t incb, const float* A2, int64_t K2, int64_t lda2, const float* B2,
