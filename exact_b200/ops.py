@@ -212,11 +212,13 @@ def linear_backward_from_compressed(quantized, weight, bias, randmat, ori_input_
     """ops.py:152-178: (grad_input, grad_weight, grad_bias) of y = x W^T + b from the compressed x."""
     projected = config.kept_frac < 1.0 and rp and randmat is not None
     input = None
-    if (config.compress_activation and not config.simulate and not config.swap and quantized[1] is not None
+    if (config.compress_activation and not config.simulate and quantized[1] is not None
             and len(q_input_shape) == 2 and (not projected or config.grad_weight_in_projected_space)
             and ext_backward_func.grad_weight_takes(grad_output)):
         # g^T Xq on the tensor cores with the dequantisation in the operand path: the [N, k] fp32 activation is
         # never written; with a projection, (g^T Xq) R^T instead of g^T (Xq R^T)
+        if config.swap:   # the codes come back from pinned memory, as dequantize_activation fetches them
+            quantized = (quantized[0].to(grad_output.device, non_blocking=True), *quantized[1:])
         grad_weight, _ = ext_backward_func.grad_weight_from_packed(grad_output, quantized, q_input_shape[1])
         if projected:
             grad_weight = grad_weight.mm(randmat.t())
