@@ -32,7 +32,8 @@
 //   warps 20-27  add an accumulator to their sums in registers, 64 columns of 32 outputs a warp, while the other one fills.
 // Each of these chains is several hundred cycles of latency a stage, so each has its own warps, and short loops: with the
 // statistics, B and the sums in one chain 2,449,029 x 256 outputs x (32 + 32) columns took 939 us, with A's 64 values held in registers
-// (450 instructions in a row, evicting the other roles' code) 611 us.
+// (450 instructions in a row, evicting the other roles' code) 611 us, now 526 to 550; 48 outputs 265 us, 169,343 x 256 x 256 at INT2 109,
+// at INT8 197, 232,965 x 256 x 602 345 us (one tf32 product: 431, 406, 101, 179 and 995).  Three quarters of the issue slots are busy.
 // The CTAs that share a range of rows are neighbours in the grid, so g comes from HBM once.  Each CTA's sums go to the workspace
 // and a second kernel adds them in a fixed order, so the result does not depend on timing.
 //

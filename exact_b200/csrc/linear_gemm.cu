@@ -36,9 +36,9 @@
 //              parity are counted instead of divided out.  Accumulators are double-buffered in TMEM.
 //   warps 10-17 epilogue: tcgen05.ld -> per-warp staging tile in shared memory -> (+ bias, + addend)
 //              -> coalesced global stores; two groups of four take alternate blocks of 32 columns.
-// Measured (us, before -> now): 2,449,029 x 256 -> 256: 1,673 -> 1,400, with a second operand pair of 256 3,365 -> 2,460; 48 -> 256:
-// 1,046 -> 630; 256 -> 47: 1,305 -> 880; 232,965 x 604 -> 256: 368 -> 299; 169,343 x 128 -> 256: 100 -> 66.  With the pair alone and
-// the chains as they were it lost (1,710 -> 2,008).
+// Measured (us, single CTAs -> now; ranges over boxes and runs): 2,449,029 x 256 -> 256: 1,673 -> 1,335 - 1,365, with a second operand
+// pair of 256 3,365 -> 2,400 - 2,890; 48 -> 256: 1,046 -> 810 - 950; 256 -> 47: 1,305 -> 760 - 860; 232,965 x 604 -> 256: 368 ->
+// 298 - 321; 169,343 x 128 -> 256: 100 -> 71 - 83.  With the pair alone and the chains as they were it lost (1,710 -> 2,008).
 // The weight is split, padded and laid out as the tiles once per call by a preparation kernel.
 //
 // Every mbarrier wait is bounded; on expiry the CTA raises an abort flag, all roles leave their loops,
@@ -169,7 +169,7 @@ linear_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                     2 * p.b_slot, bfull);
           if (uses < p.stages) uses++;
           // A comes from HBM exactly once: pull the tile that will be loaded kLinPrefetch K tiles from
-          // now into L2, so that its TMA load later pays L2 latency only (the ring holds two or three K tiles)
+          // now into L2, so that its TMA load later pays L2 latency only (the ring holds three or four K tiles)
           int pk = kb + kLinPrefetch, pt = tile;
           if (pk >= p.kblocks) { pk -= p.kblocks; pt += step; }
           if (pt < p.num_tiles && pk < p.kblocks) {

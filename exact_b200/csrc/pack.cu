@@ -333,7 +333,7 @@ __device__ __forceinline__ void quantize_rows(const PackParams& p, const TileCtx
 // and -min(-a, -b) treats NaN and signed zeros as max does), folded: at each level a lane keeps the half of the values that
 // one bit of its index names and hands the other half over, so 16 reductions take 14 or 15 shuffles.  redux.sync takes one
 // value per instruction, once per tile of the warp: 64 columns (two tiles a warp) 179 us against 113 us for 128 columns and
-// the same 128 M elements; 125 us with the folded shuffles (which at one tile a warp lose to redux, 125 against 113 us).
+// the same 128 M elements; 130 us with the folded shuffles (which at one tile a warp lose to redux, 125 against 110 us).
 // tpt = 16: lane l of the tile ends with row l & 7 (maximum for l >= 8) in v0; 8: rows 2 (l & 3) in v0 and 2 (l & 3) + 1 in
 // v1 (l >= 4).  All lanes of the warp take part.
 __device__ __forceinline__ void reduce_rows(const float (&lo)[8], const float (&hi)[8], int tpt, int lane, float& v0, float& v1) {
