@@ -404,7 +404,7 @@ grad_weight_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_consta
       }
       __syncwarp();
     }
-    if (it > 0 && it < nst) {   // given up: the MMAs issued so far still read the tiles (bounded)
+    if (it > 0) {   // no MMA under way when the tensor memory is given back, also where another role has given up (bounded)
       const long long t0 = clock64();
       while (!mbar_try_wait(smem_u32(&s_done[(it - 1) & (kGwASlots - 1)]), (uint32_t)((it - 1) >> 2) & 1u) &&
              clock64() - t0 < kWaitLimitCycles) {}

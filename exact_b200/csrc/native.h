@@ -43,7 +43,7 @@ struct LibraryError : std::runtime_error {   // becomes exact_b200.ExactB200Erro
   X(exact_rows_scale_copy_colsum) X(exact_quantize_pack_rows) X(exact_rp_quantize_pack_rows)                          \
   X(exact_bn_backward_workspace_bytes) X(exact_bn_backward_from_packed)                                               \
   X(exact_rp_workspace_bytes) X(exact_rademacher) X(exact_grad_weight_workspace_bytes)      \
-  X(exact_grad_weight_from_packed) X(exact_linear_workspace_bytes) X(exact_linear_partial_bytes) X(exact_linear_forward_strided)                            \
+  X(exact_grad_weight_from_packed) X(exact_linear_workspace_bytes) X(exact_linear_forward_strided)                            \
   X(exact_spmm_minmax_scratch_bytes) X(exact_spmm_minmax_planned) X(exact_spmm_minmax_backward)                       \
   X(exact_spmm_value_bw) X(exact_status_peek)
 
