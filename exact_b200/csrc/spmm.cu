@@ -80,6 +80,20 @@ __device__ __forceinline__ void ldg_vec<2>(const float* p, float (&o)[2]) {
 template <>
 __device__ __forceinline__ void ldg_vec<1>(const float* p, float (&o)[1]) { o[0] = __ldg(p); }
 
+// Loads that see what other kernels may still have been writing when this one started.
+template <int VEC>
+__device__ __forceinline__ void ld_vec(const float* p, float (&o)[VEC]) {
+  if constexpr (VEC == 4) {
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(p));
+    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+  } else if constexpr (VEC == 2) {
+    const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+    o[0] = v.x; o[1] = v.y;
+  } else {
+    o[0] = __ldcg(p);
+  }
+}
+
 template <int VEC>
 __device__ __forceinline__ void st_vec(float* p, const float (&a)[VEC]) {
   if (VEC == 4) *reinterpret_cast<float4*>(p) = make_float4(a[0], a[1 % VEC], a[2 % VEC], a[3 % VEC]);
@@ -101,6 +115,39 @@ __device__ __forceinline__ void store_row(const SpmmParams& p, long long row, lo
     for (int x = 0; x < VEC; x++)
       if (c + x < p.Kout) d[x] = p.bias != nullptr ? __fadd_rn(acc[x], __ldg(p.bias + c + x)) : acc[x];
   }
+}
+
+// Columns c .. c + VEC - 1 of long row i: its pieces' partial sums, added in the order of the edges.  BATCH of them are on
+// their way at a time: with one, a hub row's few hundred pieces were a chain of as many memory latencies.
+template <typename IdxT, int VEC, int BATCH>
+__device__ __forceinline__ void sum_pieces(const SpmmParams& p, long long i, long long c) {
+  if (c >= p.K) return;
+  const IdxT* __restrict__ rowptr = reinterpret_cast<const IdxT*>(p.rowptr);
+  const long long row = p.long_row[i];
+  const int s0 = p.long_item_ptr[i], s1 = p.long_item_ptr[i + 1];
+  const float* src = p.scratch + (long long)s0 * p.K + c;
+  float acc[VEC];
+#pragma unroll
+  for (int x = 0; x < VEC; x++) acc[x] = 0.f;
+  for (int s = s0; s < s1; s += BATCH, src += BATCH * p.K) {
+    float m[BATCH][VEC];
+#pragma unroll
+    for (int u = 0; u < BATCH; u++)
+      if (s + u < s1) ld_vec<VEC>(src + u * p.K, m[u]);
+#pragma unroll
+    for (int u = 0; u < BATCH; u++)
+      if (s + u < s1) {
+#pragma unroll
+        for (int x = 0; x < VEC; x++) acc[x] = __fadd_rn(acc[x], m[u][x]);
+      }
+  }
+  if (p.mean) {
+    const long long cnt = (long long)rowptr[row + 1] - (long long)rowptr[row];
+    const float dv = (float)(cnt > 0 ? cnt : 1);
+#pragma unroll
+    for (int x = 0; x < VEC; x++) acc[x] = __fdiv_rn(acc[x], dv);
+  }
+  store_row<VEC>(p, row, c, acc);
 }
 
 // acc += sum over edges [begin, end) of val[e] * mat[col[e], column tile], in edge order.
@@ -187,6 +234,8 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_kernel(const __grid_
   const long long unit = (long long)blockIdx.x * kSpmmWarps + warp;
   const IdxT* __restrict__ rowptr = reinterpret_cast<const IdxT*>(p.rowptr);
   const long long K = p.K;
+  if (MODE == MODE_ITEMS) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  else if (p.n_items > 0 && blockIdx.x == gridDim.x - 1 && blockIdx.y == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 
   long long coff[KVT];
   bool cvalid[KVT];
@@ -356,25 +405,20 @@ __global__ void __launch_bounds__(kRowWarps * 32, kRowBlocks) spmm_rows_kernel(c
       row = row1; row1 = row2; row2 = row3;
     }
   }
+  if (p.n_items > 0) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const long long tiles = (K + 32 * VEC - 1) / (32 * VEC), units = p.n_long * tiles;
+    for (long long u = (long long)blockIdx.x * kRowWarps + warp; u < units; u += stride)
+      sum_pieces<IdxT, VEC, 8>(p, u / tiles, (u % tiles * 32 + lane) * VEC);
+  }
 }
 
-// Adds the partial sums of each long row in item order and writes the row of the output.
-template <typename IdxT>
-__global__ void __launch_bounds__(128) spmm_long_reduce_kernel(const __grid_constant__ SpmmParams p) {
-  const long long i = blockIdx.x;
-  if (i >= p.n_long) return;
-  const IdxT* __restrict__ rowptr = reinterpret_cast<const IdxT*>(p.rowptr);
-  const long long row = p.long_row[i];
-  const int s0 = p.long_item_ptr[i], s1 = p.long_item_ptr[i + 1];
-  const long long cnt = (long long)rowptr[row + 1] - (long long)rowptr[row];
-  const float dv = (float)(cnt > 0 ? cnt : 1);
-  float* __restrict__ dst = output_row(p, row);
-  for (long long c = threadIdx.x; c < p.Kout; c += blockDim.x) {
-    float a = 0.f;
-    for (int s = s0; s < s1; s++) a = __fadd_rn(a, p.scratch[(long long)s * p.K + c]);
-    if (p.mean) a = __fdiv_rn(a, dv);
-    dst[c] = p.bias != nullptr ? __fadd_rn(a, __ldg(p.bias + c)) : a;
-  }
+// Adds the partial sums of each long row in item order and writes the row of the output: a warp per long row and 32 * VEC columns.
+template <typename IdxT, int VEC>
+__global__ void __launch_bounds__(kSpmmWarps * 32) spmm_long_reduce_kernel(const __grid_constant__ SpmmParams p) {
+  const long long i = (long long)blockIdx.x * kSpmmWarps + (threadIdx.x >> 5);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (i < p.n_long) sum_pieces<IdxT, VEC, 16>(p, i, ((long long)blockIdx.y * 32 + (threadIdx.x & 31)) * VEC);
 }
 
 // Narrow operands (K <= 64): a group of LPE = 4, 8 or 16 lanes (LPE x float4 = the whole row of the operand) owns
@@ -486,12 +530,27 @@ __global__ void __launch_bounds__(kSpmmWarps * 32) spmm_csr_multi_kernel(const _
   }
 }
 
-template <typename IdxT>
+// A launch whose blocks may start before the kernel in front of it has finished (`early`: that kernel says from where on).
+template <typename... Args>
+static int launch_after(void (*kernel)(Args...), dim3 grid, int threads, cudaStream_t st, bool early, const SpmmParams& p) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
+  EXB_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, p));
+  return EXB_OK;
+}
+
+template <typename IdxT, int VEC>
 static int launch_long_reduce(const SpmmParams& p, cudaStream_t st) {
   if (p.n_items == 0) return EXB_OK;
-  spmm_long_reduce_kernel<IdxT><<<(unsigned)p.n_long, 128, 0, st>>>(p);
-  EXB_CUDA_OK(cudaGetLastError());
-  return EXB_OK;
+  const dim3 grid((unsigned)((p.n_long + kSpmmWarps - 1) / kSpmmWarps), (unsigned)((p.K + 32 * VEC - 1) / (32 * VEC)));
+  return launch_after(spmm_long_reduce_kernel<IdxT, VEC>, grid, kSpmmWarps * 32, st, true, p);
 }
 
 template <typename IdxT, bool HAS_VAL, int LPE>
@@ -501,7 +560,7 @@ static int launch_spmm_multi(const SpmmParams& p, cudaStream_t st) {
   dim3 grid((unsigned)((p.n_items + p.M + per_cta - 1) / per_cta), gy);
   spmm_csr_multi_kernel<IdxT, HAS_VAL, LPE><<<grid, kSpmmWarps * 32, 0, st>>>(p);
   EXB_CUDA_OK(cudaGetLastError());
-  return launch_long_reduce<IdxT>(p, st);
+  return launch_long_reduce<IdxT, 4>(p, st);
 }
 
 template <typename IdxT, bool HAS_VAL>
@@ -511,28 +570,32 @@ static int launch_spmm_pair(const SpmmParams& p, cudaStream_t st) {
   return launch_spmm_multi<IdxT, HAS_VAL, 16>(p, st);
 }
 
+// The pieces of long rows first; the rows' kernel does not wait for them (programmatic launch: its blocks take the places that the
+// pieces' last blocks leave free) but ends after them, and the persistent one then adds the pieces up as well.  Launched one
+// after the other, the three kernels each ended with a nearly empty GPU: 169,343 nodes / 2.54 M edges x 128 columns 148 us, now
+// 124, x 256 263 and 228; 60,000 / 1.2 M x 256 142 and 114; 232,965 / 23 M x 256 1,185 and 1,117.
+// (One persistent kernel for pieces and rows, in any mixture, costs the pieces their 48 warps per SM: 5 % faster than separate
+// launches at 2.54 M edges, 10 - 25 % slower from 20 M on.)
 template <typename IdxT, int VEC, int KVT, bool HAS_VAL, bool FULL>
 static int launch_spmm_mode(const SpmmParams& p, cudaStream_t st) {
   const long long C = p.K / VEC;
   const unsigned gy = (unsigned)((C + 32 * KVT - 1) / (32 * KVT));
-  // From 16 rows a warp on: with fewer the rows' own latency counts, and the other kernel keeps twice the gathers in flight
-  // (12,093 rows x 256 columns 66 us here, 58 there; 38,146 rows 93 and 89; 169,343 rows 241 and 276).
-  if (p.row_order != nullptr && p.M < 2147483647LL && p.M >= 16LL * sm_count() * kRowBlocks * kRowWarps) {
-    long long blocks = (p.M + kRowWarps - 1) / kRowWarps;
-    if (blocks > sm_count() * kRowBlocks) blocks = sm_count() * kRowBlocks;
-    spmm_rows_kernel<IdxT, VEC, HAS_VAL><<<(unsigned)blocks, kRowWarps * 32, 0, st>>>(p);
-    EXB_CUDA_OK(cudaGetLastError());
-  } else {
-    dim3 grid((unsigned)((p.M + kSpmmWarps - 1) / kSpmmWarps), gy);
-    spmm_csr_kernel<IdxT, VEC, KVT, HAS_VAL, FULL, MODE_ROWS><<<grid, kSpmmWarps * 32, 0, st>>>(p);
-    EXB_CUDA_OK(cudaGetLastError());
-  }
   if (p.n_items > 0) {
     dim3 grid((unsigned)((p.n_items + kSpmmWarps - 1) / kSpmmWarps), gy);
     spmm_csr_kernel<IdxT, VEC, KVT, HAS_VAL, FULL, MODE_ITEMS><<<grid, kSpmmWarps * 32, 0, st>>>(p);
     EXB_CUDA_OK(cudaGetLastError());
   }
-  return launch_long_reduce<IdxT>(p, st);
+  // From 16 rows a warp on: with fewer the rows' own latency counts, and the other kernel keeps twice the gathers in flight
+  // (12,093 rows x 256 columns 66 us here, 58 there; 38,146 rows 93 and 89; 169,343 rows 241 and 276).
+  if (p.row_order != nullptr && p.M < 2147483647LL && p.M >= 16LL * sm_count() * kRowBlocks * kRowWarps) {
+    long long blocks = (p.M + kRowWarps - 1) / kRowWarps;
+    if (blocks > sm_count() * kRowBlocks) blocks = sm_count() * kRowBlocks;
+    return launch_after(spmm_rows_kernel<IdxT, VEC, HAS_VAL>, dim3((unsigned)blocks), kRowWarps * 32, st, p.n_items > 0, p);
+  }
+  const dim3 grid((unsigned)((p.M + kSpmmWarps - 1) / kSpmmWarps), gy);
+  const int rc = launch_after(spmm_csr_kernel<IdxT, VEC, KVT, HAS_VAL, FULL, MODE_ROWS>, grid, kSpmmWarps * 32, st, p.n_items > 0, p);
+  if (rc) return rc;
+  return launch_long_reduce<IdxT, VEC>(p, st);
 }
 
 template <typename IdxT, int VEC, bool HAS_VAL>
