@@ -39,3 +39,26 @@ def test_pack_and_unpack(N, D, dtype, bits):
 @pytest.mark.parametrize("N,D", [(17, 256), (41, 260), (1027, 320), (8, 384), (63, 512), (25, 516)])
 def test_pack_at_the_edges_of_two_warps_a_tile(N, D, dtype, bits):
     test_pack_and_unpack(N, D, dtype, bits)
+
+
+# one warp a tile with three chunks of four columns (257 - 384), five in 16-bit types (513 - 640), their neighbours, in accesses of
+# four elements, two and one; 9,472 rows are where enough tiles for 148 SMs begin
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,D", [(9475, 257), (9480, 300), (9465, 300), (9473, 382), (9472, 385), (9477, 516), (9479, 602), (9473, 637),
+                                 (9474, 641), (9476, 33), (9478, 66)])
+def test_pack_one_warp_tiles(N, D, dtype):
+    test_pack_and_unpack(N, D, dtype, 4)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,D,first", [(41, 47, 1), (65, 301, 1), (19, 128, 1), (19, 128, 2), (33, 602, 1), (24, 1, 1), (16, 3, 3)])
+def test_pack_of_a_view_off_its_alignment(N, D, first, dtype):
+    x = torch.from_numpy(normal(N, D, 72)).to(dtype)
+    base = torch.full((N * D + 8,), 1e4, dtype=dtype, device="cuda")   # neighbours that would move every range
+    view = base[first:first + N * D].view(N, D)
+    view.copy_(x)
+    for bits in (1, 2, 4, 8):
+        for a, b in zip(Q.quantize_pack(view, bits, seed=5, offset=2), Q.quantize_pack(x.cuda().clone(), bits, seed=5, offset=2)):
+            a, b = (t.view(torch.int8 if t.element_size() == 1 else torch.int16) for t in (a, b))
+            n = a.numel() - (a.element_size() == 1)      # the stream's last byte is never written
+            assert torch.equal(a[:n], b[:n])
