@@ -81,6 +81,10 @@ SIGNATURES = {
     "exact_bn_backward_workspace_bytes": (c_i64, [c_i64]),
     "exact_bn_backward_from_packed": (c_int, [c_ptr, c_i64, c_i64, c_ptr, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_int,
                                               c_ptr, c_i64, c_ptr, c_ptr, c_ptr, c_ptr]),
+    "exact_bn_act_forward": (c_int, [c_ptr, c_i64, c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_f32, c_f32, c_f32, c_u64, c_u64, c_i64, c_ptr,
+                                     c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr]),
+    "exact_bn_act_backward_from_packed": (c_int, [c_ptr, c_ptr, c_f32, c_i64, c_i64, c_ptr, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
+                                                  c_ptr, c_i64, c_ptr, c_ptr, c_ptr, c_ptr]),
     "exact_crows_slot_bytes": (c_i64, [c_i64]),
     "exact_crows_pack": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_i64, ctypes.POINTER(c_ptr), c_int, c_ptr, c_ptr]),
     "exact_crows_unpack": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_i64, c_ptr]),

@@ -1,5 +1,6 @@
 // Shared device helpers of the exact_b200 CUDA library (sm_100a only).
 #pragma once
+#include <cmath>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -70,6 +71,44 @@ inline PhiloxKey make_philox_key(uint64_t seed) {
 }
 
 #ifdef __CUDACC__
+// Blocks of a kernel whose blocks walk over the data: as many as are resident at once, or fewer when there is less to do.  With
+// more, the last round of blocks leaves SMs idle (at 40 registers six blocks of 256 threads fit; eight per SM took two rounds, the
+// second a third full).
+template <typename K>
+inline int resident_blocks(K kernel, int threads, long long want) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
+  if (per_sm > 8) per_sm = 8;      // what the workspaces of partial sums are sized for
+  const long long most = (long long)sm_count() * per_sm;
+  return (int)(want < 1 ? 1 : want < most ? want : most);
+}
+#endif
+
+// What dropout multiplies kept values by, and divides their gradients by.
+struct DropoutScale {
+  float pinv;            // float(1 / (1 - p)), quantization_cuda_kernel.cu:455
+  float p1m;             // float(1 - p), quantization.cc:120
+  float p1m_inv_exact;   // 1 / p1m when p1m is a power of two (then g / p1m == g * that, bit for bit), else 0
+};
+inline DropoutScale dropout_scale(float prob) {
+  DropoutScale s;
+  s.pinv = (float)(1.0 / (1.0 - (double)prob));
+  s.p1m = (float)(1.0 - (double)prob);
+  int ex = 0;
+  const float mant = frexpf(s.p1m, &ex);   // p1m = mant * 2^ex, mant in [0.5, 1)
+  s.p1m_inv_exact = (s.p1m > 0.f && mant == 0.5f && ex > -120 && ex < 120) ? ldexpf(1.f, 1 - ex) : 0.f;
+  return s;
+}
+
+#ifdef __CUDACC__
+// A kept gradient: g / float(1 - p) (quantization_cuda_kernel.cu:565-569); a power-of-two divisor (p = 0.5, 0.75, ...) is an exact
+// scaling, done as one multiply.
+__device__ __forceinline__ float dropout_grad(float g, float p1m, float p1m_inv_exact) {
+  return p1m_inv_exact != 0.f ? __fmul_rn(g, p1m_inv_exact) : __fdiv_rn(g, p1m);
+}
+// 16-bit draw -> (h + 0.5) / 65536, exact.
+__device__ __forceinline__ float dropout_uniform(uint32_t h) { return __fmaf_rn((float)h, 1.52587890625e-05f, 7.62939453125e-06f); }
+
 // CTAs and kernels that give up at the same moment all leave their bit: an atomic on mapped host memory is one for all threads of
 // the device that maps it, and the host writes the word only to clear or set it, after the stream it was asked for.
 __device__ __forceinline__ void raise_status(int* word, int bit) {

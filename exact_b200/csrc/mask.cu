@@ -7,7 +7,6 @@
 // layout is private: the reference's mask never leaves its extension either (quantization.cc:71,92,119), only
 // outputs and gradients are observable.
 #include "common.cuh"
-#include <cmath>
 #include <cuda_fp16.h>
 
 #include "exact_b200.h"
@@ -134,7 +133,7 @@ __global__ void __launch_bounds__(256) mask_forward_kernel(const __grid_constant
 #pragma unroll
         for (int j = 0; j < 8; j++) {
           const uint32_t h = (w[j >> 1] >> (16 * (j & 1))) & 0xffffu;
-          u[j] = __fmaf_rn((float)h, 1.52587890625e-05f, 7.62939453125e-06f);   // (h + 0.5) / 65536, exact
+          u[j] = dropout_uniform(h);
         }
       }
 #pragma unroll
@@ -187,10 +186,7 @@ __global__ void __launch_bounds__(256) mask_backward_kernel(const __grid_constan
       } else if (OP == OP_LEAKY_RELU) {
         o[j] = keep ? g[j] : __fmul_rn(g[j], p.p);     // quantization_cuda_kernel.cu:408-412
       } else {
-        // quantization_cuda_kernel.cu:565-569: g / float(1 - p); a power-of-two divisor (p = 0.5, 0.75, ...)
-        // is an exact scaling, done as one multiply
-        const float q = p.p1m_inv_exact != 0.f ? __fmul_rn(g[j], p.p1m_inv_exact) : __fdiv_rn(g[j], p.p1m);
-        o[j] = keep ? q : 0.f;
+        o[j] = keep ? dropout_grad(g[j], p.p1m, p.p1m_inv_exact) : 0.f;
       }
     }
     const float a[4] = {o[0], o[1], o[2], o[3]}, b[4] = {o[4], o[5], o[6], o[7]};
@@ -211,27 +207,21 @@ static int launch_mask(bool forward, const MaskParams& p, cudaStream_t st) {
   const unsigned vb = 4 * sizeof(T);   // one 4-element vector access
   const bool al = aligned_to(p.x, vb) && aligned_to(p.out, vb) && (p.u == nullptr || aligned16(p.u));
   const long long nchunks = (p.n + 255) >> 8;
-  long long blocks = (nchunks + 7) / 8;
-  const long long cap = (long long)sm_count() * 8;
-  if (blocks > cap) blocks = cap;
-  if (forward) {
-    if (al) mask_forward_kernel<OP, true, T><<<(int)blocks, 256, 0, st>>>(p);
-    else mask_forward_kernel<OP, false, T><<<(int)blocks, 256, 0, st>>>(p);
-  } else {
-    if (al) mask_backward_kernel<OP, true, T><<<(int)blocks, 256, 0, st>>>(p);
-    else mask_backward_kernel<OP, false, T><<<(int)blocks, 256, 0, st>>>(p);
-  }
+  auto kernel = forward ? (al ? mask_forward_kernel<OP, true, T> : mask_forward_kernel<OP, false, T>)
+                        : (al ? mask_backward_kernel<OP, true, T> : mask_backward_kernel<OP, false, T>);
+  // more blocks than are resident: 2.45 M x 256, backward 848 us, with resident ones only 928 - 972
+  const long long want = (nchunks + 7) / 8, cap = (long long)sm_count() * 8;
+  kernel<<<(int)(want < cap ? want : cap), 256, 0, st>>>(p);
   EXB_CUDA_OK(cudaGetLastError());
   return EXB_OK;
 }
 
 static void dropout_constants(MaskParams& p, float prob) {
+  const DropoutScale s = dropout_scale(prob);
   p.p = prob;
-  p.pinv = (float)(1.0 / (1.0 - (double)prob));  // quantization_cuda_kernel.cu:455
-  p.p1m = (float)(1.0 - (double)prob);           // quantization.cc:120
-  int ex = 0;
-  const float mant = frexpf(p.p1m, &ex);   // p1m = mant * 2^ex, mant in [0.5, 1)
-  p.p1m_inv_exact = (p.p1m > 0.f && mant == 0.5f && ex > -120 && ex < 120) ? ldexpf(1.f, 1 - ex) : 0.f;
+  p.pinv = s.pinv;
+  p.p1m = s.p1m;
+  p.p1m_inv_exact = s.p1m_inv_exact;
 }
 
 }  // namespace exb
@@ -312,13 +302,7 @@ int exact_act_quantized_dropout_backward(const float* grad_out, const uint32_t* 
   EXB_REQUIRE(n >= 0, "dropout: negative size");
   MaskParams p{};
   p.x = grad_out; p.out = grad_in; p.mask = const_cast<uint32_t*>(mask); p.n = n;
-  p.p = prob;
-  p.p1m = (float)(1.0 - (double)prob);  // quantization.cc:120
-  {
-    int ex = 0;
-    const float mant = frexpf(p.p1m, &ex);   // p1m = mant * 2^ex, mant in [0.5, 1)
-    p.p1m_inv_exact = (p.p1m > 0.f && mant == 0.5f && ex > -120 && ex < 120) ? ldexpf(1.f, 1 - ex) : 0.f;
-  }
+  dropout_constants(p, prob);
   return launch_mask<OP_DROPOUT>(false, p, (cudaStream_t)stream);
 }
 

@@ -41,7 +41,8 @@ struct LibraryError : std::runtime_error {   // becomes exact_b200.ExactB200Erro
   X(exact_spmm_f16_planned) X(exact_rows_scale_colsum_workspace_bytes)                     \
   X(exact_rows_scale_colsum) X(exact_bn_forward_workspace_bytes) X(exact_bn_forward) X(exact_rows_half_colsum) \
   X(exact_rows_scale_copy_colsum) X(exact_quantize_pack_rows) X(exact_rp_quantize_pack_rows)                          \
-  X(exact_bn_backward_workspace_bytes) X(exact_bn_backward_from_packed)                                               \
+  X(exact_bn_backward_workspace_bytes) X(exact_bn_backward_from_packed) X(exact_bn_act_forward)                       \
+  X(exact_bn_act_backward_from_packed)                                                                                \
   X(exact_rp_workspace_bytes) X(exact_rademacher) X(exact_grad_weight_workspace_bytes)      \
   X(exact_grad_weight_from_packed) X(exact_linear_workspace_bytes) X(exact_linear_forward_strided)                            \
   X(exact_spmm_minmax_scratch_bytes) X(exact_spmm_minmax_planned) X(exact_spmm_minmax_backward)                       \
@@ -133,9 +134,15 @@ std::tuple<Tensor, Tensor> rows_half_colsum(const Tensor& g, bool want_colsum);
 std::tuple<Tensor, Tensor, Tensor> bn_forward(const Tensor& x, const OptTensor& weight, const OptTensor& bias,
                                               const OptTensor& running_mean, const OptTensor& running_var, double momentum,
                                               double eps);
+// (dropout(relu(y)), its mask, mean, invstd): act_forward on bn_forward's result, without that result
+std::tuple<Tensor, Tensor, Tensor, Tensor> bn_act_forward(const Tensor& x, const OptTensor& weight, const OptTensor& bias,
+                                                          const OptTensor& running_mean, const OptTensor& running_var,
+                                                          double momentum, double eps, double p, uint64_t seed, uint64_t offset,
+                                                          int64_t index_offset);
+// mask (with its p): g is the gradient of bn_act_forward's output
 std::tuple<Tensor, Tensor, Tensor> bn_backward(const Tensor& g, const Packed& q, int64_t bits, const OptTensor& weight,
                                                const Tensor& mean, const Tensor& invstd, bool train, bool want_input,
-                                               bool want_weight, bool want_bias);
+                                               bool want_weight, bool want_bias, const OptTensor& mask = {}, double p = 0.0);
 std::tuple<Tensor, Tensor> act_forward(int64_t op, const Tensor& x, double param, const OptTensor& uniforms, uint64_t seed,
                                        uint64_t offset, int64_t index_offset);
 Tensor act_backward(int64_t op, const Tensor& g, const Tensor& mask, double param);

@@ -321,6 +321,9 @@ struct BnState : torch::CustomClassHolder {
   Tensor mean, invstd;
   OptTensor weight;
   int64_t bits;
+  bool act = false;              // ReLU and dropout follow
+  double p = 0.0;
+  uint64_t drop_offset = 0;
 };
 
 struct BnNode : Function<BnNode> {
@@ -329,9 +332,16 @@ struct BnNode : Function<BnNode> {
                         const c10::intrusive_ptr<BnState>& s, const Saving& how) {
     const Tensor x = x_.contiguous();
     s->x = quantize_pack(x, how.bits, {}, how.seed, how.offset, how.row_offset);
-    auto [y, mean, invstd] = bn_forward(x, weight, bias, running_mean, running_var, momentum, eps);
-    s->mean = mean;
-    s->invstd = invstd;
+    Tensor y;
+    if (s->act) {
+      Tensor mask;
+      std::tie(y, mask, s->mean, s->invstd) =
+          bn_act_forward(x, weight, bias, running_mean, running_var, momentum, eps, s->p, how.seed, s->drop_offset,
+                         how.row_offset * x.size(1));
+      ctx->save_for_backward({mask});
+    } else {
+      std::tie(y, s->mean, s->invstd) = bn_forward(x, weight, bias, running_mean, running_var, momentum, eps);
+    }
     if (weight) s->weight = weight->detach();
     s->bits = how.bits;
     ctx->saved_data["s"] = c10::IValue::make_capsule(s);
@@ -340,8 +350,10 @@ struct BnNode : Function<BnNode> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     Plain plain;
     auto s = state_of<BnState>(ctx);
+    OptTensor mask;
+    if (s->act) mask = ctx->get_saved_variables()[0];
     auto [gx, gw, gb] = bn_backward(grads[0], s->x, s->bits, s->weight, s->mean, s->invstd, true, ctx->needs_input_grad(0),
-                                    s->weight && ctx->needs_input_grad(1), s->weight && ctx->needs_input_grad(2));
+                                    s->weight && ctx->needs_input_grad(1), s->weight && ctx->needs_input_grad(2), mask, s->p);
     return {gx, gw, gb, {}, {}, {}, {}, {}, {}};
   }
 };
@@ -349,6 +361,15 @@ struct BnNode : Function<BnNode> {
 Tensor bn_node(const Tensor& x, const OptTensor& weight, const OptTensor& bias, const OptTensor& running_mean,
                const OptTensor& running_var, double momentum, double eps, const Saving& how) {
   return BnNode::apply(x, weight, bias, running_mean, running_var, momentum, eps, c10::make_intrusive<BnState>(), how);
+}
+
+Tensor bn_act_node(const Tensor& x, const OptTensor& weight, const OptTensor& bias, const OptTensor& running_mean,
+                   const OptTensor& running_var, double momentum, double eps, const Saving& how, double p, uint64_t drop_offset) {
+  auto s = c10::make_intrusive<BnState>();
+  s->act = true;
+  s->p = p;
+  s->drop_offset = drop_offset;
+  return BnNode::apply(x, weight, bias, running_mean, running_var, momentum, eps, s, how);
 }
 
 // ---- aggregation: qspmm_sum / mean / max / min (ops.py:257-436) --------------------------------------------

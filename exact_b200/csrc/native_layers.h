@@ -31,6 +31,9 @@ Tensor sage_node(const Tensor& x, const Tensor& w_l, const OptTensor& b_l, const
 // Training batch norm with its input saved compressed (qbatch_norm, ops.py:206-254).
 Tensor bn_node(const Tensor& x, const OptTensor& weight, const OptTensor& bias, const OptTensor& running_mean,
                const OptTensor& running_var, double momentum, double eps, const Saving& how);
+// The same with the ReLU and dropout (probability p, noise at `drop_offset`) that follow it.
+Tensor bn_act_node(const Tensor& x, const OptTensor& weight, const OptTensor& bias, const OptTensor& running_mean,
+                   const OptTensor& running_var, double momentum, double eps, const Saving& how, double p, uint64_t drop_offset);
 
 // reduce(A, x) with gradients to x and, when they ask for one, the edge values (qspmm_sum / mean / max / min).
 // reduce: 0 sum, 1 mean, 2 max, 3 min; the graph's transpose carries the weights of the reduction.  row: the row of every edge

@@ -238,6 +238,12 @@ Tensor bn_op(const Tensor& x, const OptTensor& weight, const OptTensor& bias, co
              int64_t row_offset) {
   return bn_node(x, weight, bias, running_mean, running_var, momentum, eps, Saving{bits, 0, seed, offset, row_offset, true});
 }
+Tensor bn_act_op(const Tensor& x, const OptTensor& weight, const OptTensor& bias, const OptTensor& running_mean,
+                 const OptTensor& running_var, double momentum, double eps, int64_t bits, uint64_t seed, uint64_t offset,
+                 int64_t row_offset, double p, uint64_t drop_offset) {
+  return bn_act_node(x, weight, bias, running_mean, running_var, momentum, eps, Saving{bits, 0, seed, offset, row_offset, true}, p,
+                     drop_offset);
+}
 Tensor aggregate_op(const Tensor& x, const OptTensor& value, const OptTensor& row, const c10::intrusive_ptr<Graph>& graph,
                     int64_t reduce, bool keep_x, int64_t bits, int64_t kept, uint64_t seed, uint64_t offset, int64_t row_offset,
                     bool fused) {
@@ -283,7 +289,7 @@ PyMethodDef methods[] = {
     EXB_METHOD("quantize_pack", quantize_pack), EXB_METHOD("unpack", unpack), EXB_METHOD("rademacher", rademacher),
     EXB_METHOD("rp_quantize_pack", rp_quantize_pack_op), EXB_METHOD("bn_backward", bn_backward_op), EXB_METHOD("linear", linear_op), EXB_METHOD("grad_weight", grad_weight_op), EXB_METHOD("grad_weight_takes", grad_weight_takes),
     EXB_METHOD("rows_scale_colsum", rows_scale_colsum), EXB_METHOD("spmm", spmm_op), EXB_METHOD("act", act_node),
-    EXB_METHOD("batch_norm", bn_op), EXB_METHOD("aggregate", aggregate_op), EXB_METHOD("spmm_minmax", spmm_minmax_op),
+    EXB_METHOD("batch_norm", bn_op), EXB_METHOD("batch_norm_act", bn_act_op), EXB_METHOD("aggregate", aggregate_op), EXB_METHOD("spmm_minmax", spmm_minmax_op),
     EXB_METHOD("spmm_minmax_backward", spmm_minmax_backward), EXB_METHOD("spmm_value_backward", spmm_value_backward),
     EXB_METHOD("gcn", gcn_op), EXB_METHOD("sage", sage_op), EXB_METHOD("gcn_eval", gcn_eval), EXB_METHOD("sage_eval", sage_eval), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

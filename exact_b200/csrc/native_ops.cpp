@@ -345,9 +345,29 @@ std::tuple<Tensor, Tensor, Tensor> bn_forward(const Tensor& x, const OptTensor& 
   return {y, mean, invstd};
 }
 
+std::tuple<Tensor, Tensor, Tensor, Tensor> bn_act_forward(const Tensor& x, const OptTensor& weight_, const OptTensor& bias_,
+                                                          const OptTensor& running_mean, const OptTensor& running_var,
+                                                          double momentum, double eps, double p, uint64_t seed, uint64_t offset,
+                                                          int64_t index_offset) {
+  c10::cuda::CUDAGuard guard(x.device());
+  OptTensor weight, bias;
+  if (weight_) weight = weight_->detach().contiguous();
+  if (bias_) bias = bias_->detach().contiguous();
+  const int64_t N = x.size(0), D = x.size(1), ws_bytes = lib.exact_bn_forward_workspace_bytes(D);
+  Tensor ws = empty({ws_bytes}, at::kByte, x), out = empty({N, D}, at::kFloat, x), mean = empty({D}, at::kFloat, x),
+         invstd = empty({D}, at::kFloat, x), mask = empty({lib.exact_mask_words(N * D)}, at::kInt, x);
+  invoke("exact_bn_act_forward", {12 * N * D + N * D / 8}, [&](void* st) {
+    return lib.exact_bn_act_forward(ptr<float>(x), N, D, ptr<float>(weight), ptr<float>(bias), ptr<float>(running_mean),
+                                    ptr<float>(running_var), (float)momentum, (float)eps, (float)p, seed, offset, index_offset,
+                                    ptr(ws), ws_bytes, ptr<float>(out), ptr<uint32_t>(mask), ptr<float>(mean), ptr<float>(invstd),
+                                    st);
+  });
+  return {out, mask, mean, invstd};
+}
+
 std::tuple<Tensor, Tensor, Tensor> bn_backward(const Tensor& g_, const Packed& q, int64_t bits, const OptTensor& weight_,
                                                const Tensor& mean_, const Tensor& invstd_, bool train, bool want_input,
-                                               bool want_weight, bool want_bias) {
+                                               bool want_weight, bool want_bias, const OptTensor& mask, double p) {
   c10::cuda::CUDAGuard guard(g_.device());
   const Tensor g = g_.contiguous(), mean = mean_.to(at::kFloat).contiguous(), invstd = invstd_.to(at::kFloat).contiguous();
   OptTensor weight;
@@ -359,6 +379,16 @@ std::tuple<Tensor, Tensor, Tensor> bn_backward(const Tensor& g_, const Packed& q
   if (want_bias) gb = empty({D}, at::kFloat, g);
   const int64_t pass = N * D * 4 + lib.exact_packed_bytes(N, D, (int)bits) + 4 * N;
   const bool both = want_input && (train || want_weight || want_bias);
+  if (mask) {
+    invoke("exact_bn_act_backward_from_packed", {(both ? 2 : 1) * (pass + N * D / 8) + (want_input ? N * D * 4 : 0)}, [&](void* st) {
+      return lib.exact_bn_act_backward_from_packed(ptr<float>(g), ptr<uint32_t>(*mask), (float)p, N, D, ptr<uint8_t>(q.codes),
+                                                   (int)bits, ptr<uint16_t>(q.scale), ptr<uint16_t>(q.mn), ptr<float>(weight),
+                                                   ptr<float>(mean), ptr<float>(invstd), ptr(ws), ws_bytes,
+                                                   want_input ? ptr<float>(gi) : nullptr, want_weight ? ptr<float>(gw) : nullptr,
+                                                   want_bias ? ptr<float>(gb) : nullptr, st);
+    });
+    return {gi, gw, gb};
+  }
   invoke("exact_bn_backward_from_packed", {(both ? 2 : 1) * pass + (want_input ? N * D * 4 : 0)}, [&](void* st) {
     return lib.exact_bn_backward_from_packed(ptr<float>(g), N, D, ptr<uint8_t>(q.codes), (int)bits, ptr<uint16_t>(q.scale),
                                              ptr<uint16_t>(q.mn), ptr<float>(weight), ptr<float>(mean), ptr<float>(invstd),

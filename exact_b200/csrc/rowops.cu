@@ -199,10 +199,9 @@ static int rows_pass(const float* g, int64_t n, int64_t K, int64_t ldg, const fl
     const long long pieces = n * (Kout / 4);
     if (pieces == 0) return EXB_OK;
     const bool pairs = (reinterpret_cast<uintptr_t>(g) & 7) == 0 && ldg % 2 == 0;
-    long long blocks = (pieces + 4 * kRowOpsThreads - 1) / (4 * kRowOpsThreads);
-    if (blocks > (long long)sm_count() * 8) blocks = (long long)sm_count() * 8;
-    if (pairs) pad_rows_kernel<true><<<(int)blocks, kRowOpsThreads, 0, st>>>(g, rowscale, static_cast<float*>(out), pieces, (int)K, ldg, (int)(Kout / 4));
-    else pad_rows_kernel<false><<<(int)blocks, kRowOpsThreads, 0, st>>>(g, rowscale, static_cast<float*>(out), pieces, (int)K, ldg, (int)(Kout / 4));
+    auto kernel = pairs ? pad_rows_kernel<true> : pad_rows_kernel<false>;
+    const int blocks = resident_blocks(kernel, kRowOpsThreads, (pieces + 4 * kRowOpsThreads - 1) / (4 * kRowOpsThreads));
+    kernel<<<blocks, kRowOpsThreads, 0, st>>>(g, rowscale, static_cast<float*>(out), pieces, (int)K, ldg, (int)(Kout / 4));
     EXB_CUDA_OK(cudaGetLastError());
     return EXB_OK;
   }

@@ -188,6 +188,23 @@ class QReLUDropout(torch.nn.Module):
         return F.relu(input)
 
 
+def _watched(module):
+    """Whether a call of the module does more than its forward."""
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
+                or torch.nn.modules.module._has_any_global_hook())
+
+
+def norm_act(norm, act, input):
+    """act(norm(input)).  A quantised batch norm followed by QReLUDropout runs as one node, without the pass over the values in
+    between, which nothing else reads; a module that is hooked or replaced is called by itself."""
+    if norm is None:
+        return act(input)
+    if (type(norm) is QBatchNorm1d and type(act) is QReLUDropout and act.training and norm.takes_activation(input)
+            and not _watched(norm) and not _watched(act)):
+        return norm.forward(input, act.p)
+    return act(norm(input))
+
+
 class QDropout2(torch.nn.Module):
     """layers.py:328-337."""
 
@@ -208,7 +225,17 @@ class QBatchNorm1d(torch.nn.BatchNorm1d):
         super().__init__(num_features, eps, momentum, affine, track_running_stats)
         self.scheme = QScheme("batchnorm") if config.single_precision else None
 
-    def forward(self, input):
+    def _native_takes(self, input):
+        return (config.native_layers() and config.bn_backward_from_packed and input.is_cuda and input.dim() == 2
+                and input.dtype == torch.float32 and input.size(1) % 4 == 0 and input.size(0) >= 1024
+                and (self.weight is None or self.weight.dtype == torch.float32))
+
+    def takes_activation(self, input):
+        """Whether forward(input, dropout) can stand for the ReLU and dropout behind this module as well."""
+        return self.training and self._native_takes(input) and input.size(1) <= 4096
+
+    def forward(self, input, dropout=None):
+        """`dropout`: the probability of the ReLU + dropout to apply as well (only where takes_activation allows it)."""
         if not self.training:
             return super().forward(input)
         self._check_input_dim(input)
@@ -220,15 +247,15 @@ class QBatchNorm1d(torch.nn.BatchNorm1d):
             else:
                 exponential_average_factor = self.momentum
         bn_training = True
-        if (config.native_layers() and config.bn_backward_from_packed and input.is_cuda and input.dim() == 2
-                and input.dtype == torch.float32 and input.size(1) % 4 == 0 and input.size(0) >= 1024
-                and (self.weight is None or self.weight.dtype == torch.float32)):
+        if self._native_takes(input):
             # fewer rows: the framework's one-launch kernels are as fast
             track = self.track_running_stats
-            return _lib.native().batch_norm(input, self.weight, self.bias, self.running_mean if track else None,
-                                            self.running_var if track else None, exponential_average_factor, self.eps,
-                                            config.activation_compression_bits[0], config.seed, config.take_offsets(1),
-                                            config.row_offset)
+            args = (input, self.weight, self.bias, self.running_mean if track else None, self.running_var if track else None,
+                    exponential_average_factor, self.eps, config.activation_compression_bits[0], config.seed,
+                    config.take_offsets(1), config.row_offset)
+            if dropout is not None:
+                return _lib.native().batch_norm_act(*args, dropout, config.take_offsets(1))
+            return _lib.native().batch_norm(*args)
         return qbatch_norm.apply(
             input,
             self.running_mean if not self.training or self.track_running_stats else None,

@@ -4,7 +4,7 @@ layers of this package so that QModule can convert them."""
 import torch
 from torch.nn import BatchNorm1d, ModuleList
 
-from .layers import ActDropout, GCNConv, SAGEConv
+from .layers import ActDropout, GCNConv, SAGEConv, norm_act
 
 
 class GCN(torch.nn.Module):
@@ -39,11 +39,12 @@ class GCN(torch.nn.Module):
             x = self.input_dropout(x)
         for idx, conv in enumerate(self.convs[:-1]):
             h = conv(x, adj_t)
-            if self.batch_norm:
-                h = self.bns[idx](h)
+            norm = self.bns[idx] if self.batch_norm else None
             if self.residual and h.size(-1) == x.size(-1):
+                if norm is not None:
+                    h, norm = norm(h), None
                 h = h + x[:h.size(0)]
-            x = self.act_drop(h)
+            x = norm_act(norm, self.act_drop, h)
         return self.convs[-1](x, adj_t)
 
 
@@ -84,11 +85,12 @@ class SAGE(torch.nn.Module):
             h = conv(x, adj_t)
             if self.use_linear:
                 h = h + self.lins[idx](x)
-            if self.batch_norm:
-                h = self.bns[idx](h)
+            norm = self.bns[idx] if self.batch_norm else None
             if self.residual and h.size(-1) == x.size(-1):
+                if norm is not None:
+                    h, norm = norm(h), None
                 h = h + x[:h.size(0)]
-            x = self.act_drop(h)
+            x = norm_act(norm, self.act_drop, h)
         h = self.convs[-1](x, adj_t)
         if self.use_linear:
             h = h + self.lins[-1](x)

@@ -314,6 +314,14 @@ EXACT_API int exact_bn_backward_from_packed(const float* grad_out, int64_t N, in
                                             int64_t workspace_bytes, float* grad_input, float* grad_weight,
                                             float* grad_bias, void* stream);
 
+/* The same with the ReLU and dropout behind the batch norm: grad_out is the gradient of their output, mask and prob as
+ * exact_bn_act_forward left and took them (mask 16-byte aligned); always the training form. */
+EXACT_API int exact_bn_act_backward_from_packed(const float* grad_out, const uint32_t* mask, float prob, int64_t N, int64_t D,
+                                                const uint8_t* packed, int bits, const uint16_t* scale_bf16,
+                                                const uint16_t* min_bf16, const float* weight, const float* mean,
+                                                const float* invstd, void* workspace, int64_t workspace_bytes, float* grad_input,
+                                                float* grad_weight, float* grad_bias, void* stream);
+
 /* Batch norm of a training step, forward (native_batch_norm of ops.py:222-229): batch statistics of x [N, D] (fp32, D % 4 == 0,
  * 16-byte aligned; other widths return code 3), y, the saved mean and 1 / sqrt(var + eps), and the running statistics (both or
  * neither may be NULL) moved by `momentum`.  workspace: exact_bn_forward_workspace_bytes(D) bytes. */
@@ -321,6 +329,13 @@ EXACT_API int64_t exact_bn_forward_workspace_bytes(int64_t D);
 EXACT_API int exact_bn_forward(const float* x, int64_t N, int64_t D, const float* weight, const float* bias, float* running_mean,
                                float* running_var, float momentum, float eps, void* workspace, int64_t workspace_bytes,
                                float* y, float* save_mean, float* save_invstd, void* stream);
+
+/* exact_bn_forward followed by exact_act_quantized_relu_dropout_forward on its result, without the result in between: out =
+ * dropout(relu(y)) and the mask of that call, bit for bit.  out and mask 16-byte aligned; widths without a kernel return code 3. */
+EXACT_API int exact_bn_act_forward(const float* x, int64_t N, int64_t D, const float* weight, const float* bias,
+                                   float* running_mean, float* running_var, float momentum, float eps, float prob, uint64_t seed,
+                                   uint64_t offset, int64_t index_offset, void* workspace, int64_t workspace_bytes, float* out,
+                                   uint32_t* mask, float* save_mean, float* save_invstd, void* stream);
 
 /* CSR SpMM on fp16 operands with the arithmetic of the reference's half instantiation (spmm_cuda.cu:142; AMP runs
  * cast the operands to fp16, exact/exact/ops.py:260, 313): term = half(value[e] * mat[col[e], c]) (the bare operand
