@@ -85,6 +85,8 @@ SIGNATURES = {
                                      c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr]),
     "exact_bn_act_backward_from_packed": (c_int, [c_ptr, c_ptr, c_f32, c_i64, c_i64, c_ptr, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
                                                   c_ptr, c_i64, c_ptr, c_ptr, c_ptr, c_ptr]),
+    "exact_spmm_weighted_backward": (c_int, [c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_i64, c_i64, c_i64, c_ptr, c_ptr,
+                                             c_ptr, c_ptr, c_i64, c_ptr, c_ptr, c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr]),
     "exact_crows_slot_bytes": (c_i64, [c_i64]),
     "exact_crows_pack": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_i64, ctypes.POINTER(c_ptr), c_int, c_ptr, c_ptr]),
     "exact_crows_unpack": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_ptr, c_i64, c_ptr]),

@@ -46,7 +46,7 @@ struct LibraryError : std::runtime_error {   // becomes exact_b200.ExactB200Erro
   X(exact_rp_workspace_bytes) X(exact_rademacher) X(exact_grad_weight_workspace_bytes)      \
   X(exact_grad_weight_from_packed) X(exact_linear_workspace_bytes) X(exact_linear_forward_strided)                            \
   X(exact_spmm_minmax_scratch_bytes) X(exact_spmm_minmax_planned) X(exact_spmm_minmax_backward)                       \
-  X(exact_spmm_value_bw) X(exact_status_peek)
+  X(exact_spmm_value_bw) X(exact_spmm_weighted_backward) X(exact_status_peek)
 
 struct Library {
 #define EXB_POINTER(name) decltype(&::name) name = nullptr;
@@ -191,5 +191,10 @@ struct Csr {
 inline Tensor spmm(const Csr& a, const OptTensor& value, const Tensor& mat, bool mean, const OptTensor& bias = {}) {
   return spmm(a.rowptr, a.col, *a.plan, value, mat, mean, bias);
 }
+
+// (grad of mat, grad of the values) of a weighted sum or mean; t: the transpose with its weights, perm as its edges' forward
+// positions, fw_rowptr: the forward rows of a mean
+std::tuple<Tensor, Tensor> spmm_weighted_backward(const Csr& t, const Tensor& perm, const OptTensor& fw_rowptr, const Tensor& mat,
+                                                  const Tensor& grad);
 
 }  // namespace exb

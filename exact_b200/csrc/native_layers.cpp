@@ -376,7 +376,7 @@ Tensor bn_act_node(const Tensor& x, const OptTensor& weight, const OptTensor& bi
 struct AggregateState : torch::CustomClassHolder {
   c10::intrusive_ptr<Graph> graph;
   Saving how;
-  OptTensor value, row;
+  OptTensor value, row, perm;
   Compressed x;        // only when the edge values get a gradient: nothing else reads it
   Tensor arg;
   int64_t reduce, rows;
@@ -412,7 +412,11 @@ struct AggregateNode : Function<AggregateNode> {
       x = unpack(s->x.q.codes, s->how.bits, s->x.q.scale, s->x.q.mn, s->rows, s->x.width);
       if (s->x.R.defined()) x = linear_supported(x) ? linear(x, s->x.R, {}, {}, {}, {}, false) : at::matmul(x, s->x.R.t());
     }
-    if (s->reduce <= 1) {
+    if (s->reduce <= 1 && need_v && need_x && s->perm && gr.bw.value && g.size(1) <= 256 && gr.fw.col.size(0) > 0) {
+      OptTensor rows;
+      if (s->reduce == 1) rows = gr.fw.rowptr;
+      std::tie(gx, gv) = spmm_weighted_backward(gr.bw, *s->perm, rows, x, g);
+    } else if (s->reduce <= 1) {
       if (need_v) gv = spmm_value_backward(*s->row, gr.fw.rowptr, gr.fw.col, x, g, s->reduce == 1);
       if (need_x) gx = spmm(gr.bw, gr.bw.value, g, false);
     } else {
@@ -426,13 +430,14 @@ struct AggregateNode : Function<AggregateNode> {
   }
 };
 
-Tensor aggregate_node(const Tensor& x, const OptTensor& value, const OptTensor& row, const c10::intrusive_ptr<Graph>& graph,
-                      int64_t reduce, bool keep_x, const Saving& how) {
+Tensor aggregate_node(const Tensor& x, const OptTensor& value, const OptTensor& row, const OptTensor& perm,
+                      const c10::intrusive_ptr<Graph>& graph, int64_t reduce, bool keep_x, const Saving& how) {
   auto s = c10::make_intrusive<AggregateState>();
   s->keep_x = keep_x;
   s->graph = graph;
   s->how = how;
   s->row = row;
+  s->perm = perm;
   s->reduce = reduce;
   return AggregateNode::apply(x, value, s);
 }

@@ -38,8 +38,9 @@ Tensor bn_act_node(const Tensor& x, const OptTensor& weight, const OptTensor& bi
 // reduce(A, x) with gradients to x and, when they ask for one, the edge values (qspmm_sum / mean / max / min).
 // reduce: 0 sum, 1 mean, 2 max, 3 min; the graph's transpose carries the weights of the reduction.  row: the row of every edge
 // (needed for the values' gradient of a sum or mean).  keep_x: the values' gradient will be asked for, x is saved compressed.
-Tensor aggregate_node(const Tensor& x, const OptTensor& value, const OptTensor& row, const c10::intrusive_ptr<Graph>& graph,
-                      int64_t reduce, bool keep_x, const Saving& how);
+// perm: the forward position of the transpose's edges, when both gradients of a weighted sum or mean may be asked for.
+Tensor aggregate_node(const Tensor& x, const OptTensor& value, const OptTensor& row, const OptTensor& perm,
+                      const c10::intrusive_ptr<Graph>& graph, int64_t reduce, bool keep_x, const Saving& how);
 
 // The same layers without anything saved (evaluation).
 Tensor gcn_eval(const Tensor& x, const Tensor& w, const OptTensor& b, const c10::intrusive_ptr<Graph>& graph, bool half);

@@ -244,10 +244,11 @@ Tensor bn_act_op(const Tensor& x, const OptTensor& weight, const OptTensor& bias
   return bn_act_node(x, weight, bias, running_mean, running_var, momentum, eps, Saving{bits, 0, seed, offset, row_offset, true}, p,
                      drop_offset);
 }
-Tensor aggregate_op(const Tensor& x, const OptTensor& value, const OptTensor& row, const c10::intrusive_ptr<Graph>& graph,
+Tensor aggregate_op(const Tensor& x, const OptTensor& value, const OptTensor& row, const OptTensor& perm,
+                    const c10::intrusive_ptr<Graph>& graph,
                     int64_t reduce, bool keep_x, int64_t bits, int64_t kept, uint64_t seed, uint64_t offset, int64_t row_offset,
                     bool fused) {
-  return aggregate_node(x, value, row, graph, reduce, keep_x, Saving{bits, kept, seed, offset, row_offset, fused});
+  return aggregate_node(x, value, row, perm, graph, reduce, keep_x, Saving{bits, kept, seed, offset, row_offset, fused});
 }
 std::tuple<Tensor, Tensor> spmm_minmax_op(const Tensor& rowptr, const Tensor& col, const PlanPtr& plan, const OptTensor& value,
                                           const Tensor& mat, bool is_max) {

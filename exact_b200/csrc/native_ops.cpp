@@ -630,6 +630,36 @@ std::tuple<Tensor, Tensor> spmm_minmax_backward(const Tensor& col, const OptTens
   return {gv, gm};
 }
 
+std::tuple<Tensor, Tensor> spmm_weighted_backward(const Csr& t, const Tensor& perm, const OptTensor& fw_rowptr, const Tensor& mat_,
+                                                  const Tensor& grad_) {
+  const Tensor mat = mat_.contiguous(), grad = grad_.contiguous();
+  check_type(mat.scalar_type() == at::kFloat && grad.scalar_type() == at::kFloat, "mat or grad");
+  check_type(perm.scalar_type() == t.col.scalar_type() && (!fw_rowptr || fw_rowptr->scalar_type() == t.col.scalar_type()), "perm or rowptr");
+  same_device(t.rowptr, mat);
+  same_device(t.col, grad);
+  same_device(perm, grad);
+  c10::cuda::CUDAGuard guard(mat.device());
+  const int64_t M = t.rowptr.size(0) - 1, K = mat.size(1), nnz = t.col.size(0);
+  const int ib = t.col.scalar_type() == at::kInt ? 4 : 8;
+  const RowPlan::Pieces& pc = t.plan->pieces(t.rowptr, t.col);
+  Tensor gm = empty({M, K}, at::kFloat, mat), gv = empty({nnz}, at::kFloat, mat), scratch;
+  if (pc.n) scratch = empty({pc.n, K}, at::kFloat, mat);
+  CallInfo info;
+  info.bytes = 4 * K * (2 * M + grad.size(0)) + nnz * (2 * ib + 8) + (M + 1) * ib;
+  info.l2_bytes = nnz * K * 4 + info.bytes;
+  info.edge_columns = nnz * K;
+  const int32_t* order = M > 0 ? ptr<int32_t>(t.plan->row_order(t.rowptr)) : nullptr;
+  invoke("exact_spmm_weighted_backward", info, [&](void* st) {
+    return lib.exact_spmm_weighted_backward(
+        ptr(t.rowptr), ptr(t.col), ptr<float>(*t.value), ptr(perm), ptr(fw_rowptr), ib, ptr<float>(mat), ptr<float>(grad), M, K,
+        pc.n ? t.plan->threshold : 0, pc.n ? ptr<int32_t>(pc.row) : nullptr, pc.n ? ptr<int64_t>(pc.begin) : nullptr,
+        pc.n ? ptr<int64_t>(pc.end) : nullptr, pc.n ? ptr<int32_t>(pc.slot) : nullptr, pc.n, pc.n ? ptr<int32_t>(pc.long_row) : nullptr,
+        pc.n ? ptr<int32_t>(pc.long_ptr) : nullptr, pc.n_long, pc.n ? ptr<float>(scratch) : nullptr, order, ptr<float>(gm), ptr<float>(gv),
+        st);
+  });
+  return {gm, gv};
+}
+
 Tensor spmm_value_backward(const Tensor& row, const Tensor& rowptr, const Tensor& col, const Tensor& mat_, const Tensor& grad_,
                            bool mean) {
   const Tensor mat = mat_.contiguous(), grad = grad_.contiguous();

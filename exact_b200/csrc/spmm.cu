@@ -17,6 +17,7 @@
 // scratch, and a last small kernel adds each long row's partials in order.  Only those rows differ
 // from the reference's summation order (by regrouping, within fp32 rounding).
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -720,6 +721,210 @@ __global__ void __launch_bounds__(128) spmm_value_bw_kernel(const IdxT* __restri
   }
 }
 
+// Both gradients of a weighted sum or mean in one walk of the transposed structure: for row j of it (a row of the operand) and its
+// edges e to rows i of grad,
+//     grad_mat[j] = sum_e w[e] * grad[i]   (edge order, one FMA an edge, as spmm_rows_kernel)
+//     grad_value[perm[e]] = dot(mat[j], grad[i])   (/ max(length of row i, 1) for mean; as spmm_value_bw_kernel, bit for bit:
+//                           lane l takes columns l, l + 32, ..., the lanes are added by the same tree)
+// A row of grad is gathered once for both and the row of mat stays in registers, where the separate kernels gathered a row per edge
+// each.  Bound by the gathers' latency: persistent warps take pieces of long rows, then rows, longest first, as spmm_rows_kernel
+// does, eight edges in flight.  The eight dots of a step are folded together (9 shuffles).
+// 169,343 nodes / 2.2 M edges x 128 columns: 158 + 115 us in two walks, now 224.  (The next eight gathers before the dots are folded
+// need registers that spill: 356 us.)
+struct WeightedBwParams {
+  SpmmParams s;            // the transposed structure, its weights, mat = grad, out = grad_mat
+  const void* perm;        // [nnz] position of the transposed structure's edges in the forward one
+  const void* fw_rowptr;   // forward rows, for mean, or null
+  const float* x;          // [M, K] the operand
+  float* grad_value;
+};
+
+template <int B>
+__device__ __forceinline__ float fold_dots(float (&d)[B], int lane) {
+  int h = 16;
+#pragma unroll
+  for (int n = B; n > 1; n >>= 1, h >>= 1) {
+    const bool upper = (lane & h) != 0;
+#pragma unroll
+    for (int u = 0; u < n / 2; u++)
+      d[u] = __fadd_rn(upper ? d[u + n / 2] : d[u], __shfl_xor_sync(0xffffffffu, upper ? d[u] : d[u + n / 2], h));
+  }
+#pragma unroll
+  for (; h > 0; h >>= 1) d[0] = __fadd_rn(d[0], __shfl_xor_sync(0xffffffffu, d[0], h));
+  return d[0];
+}
+
+// What a lane needs of the matrices: grad0 / grad_last at its first and last column (lanes past K: a column of the row, dropped).
+struct WeightedBwLane {
+  const float* g0;
+  const float* g_last;
+  unsigned long long K;
+  bool last_valid;
+  int lane;
+};
+
+template <int B, int NC>
+__device__ __forceinline__ void weighted_bw_load(const WeightedBwLane& l, const uint32_t* idx, float (&m)[B][NC]) {
+#pragma unroll
+  for (int u = 0; u < B; u++) {
+    const unsigned long long at = (unsigned long long)idx[u] * l.K;
+#pragma unroll
+    for (int c = 0; c < NC - 1; c++) m[u][c] = __ldg(l.g0 + at + 32 * c);
+    m[u][NC - 1] = __ldg(l.g_last + at);
+  }
+}
+
+template <int B, int NC>
+__device__ __forceinline__ void weighted_bw_add(const WeightedBwLane& l, const float* val, float (&m)[B][NC], const float (&xr)[NC],
+                                                float (&acc)[NC], float (&d)[B]) {
+#pragma unroll
+  for (int u = 0; u < B; u++) {
+    const float w = val[u];
+    if (!l.last_valid) m[u][NC - 1] = 0.f;
+    d[u] = 0.f;
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      d[u] = __fmaf_rn(xr[c], m[u][c], d[u]);
+      acc[c] = __fmaf_rn(w, m[u][c], acc[c]);
+    }
+  }
+}
+
+template <int B, typename IdxT>
+__device__ __forceinline__ void weighted_bw_values(const WeightedBwParams& p, const uint32_t* idx, const IdxT* perm, int lane, float (&d)[B]) {
+  float v = fold_dots<B>(d, lane);
+  constexpr int kLanes = 32 / B;                // the edge of lane l is l / kLanes
+  if (lane % kLanes == 0) {
+    const int e = lane / kLanes;
+    if (p.fw_rowptr) {
+      const IdxT* rp = static_cast<const IdxT*>(p.fw_rowptr) + idx[e];
+      const long long deg = (long long)rp[1] - (long long)rp[0];
+      v = __fdiv_rn(v, (float)(deg > 1 ? deg : 1));
+    }
+    p.grad_value[perm[e]] = v;
+  }
+}
+
+template <typename IdxT, int NC>
+__global__ void __launch_bounds__(kRowWarps * 32, NC <= 4 ? 3 : 2) spmm_weighted_bw_kernel(const __grid_constant__ WeightedBwParams p) {
+  __shared__ uint32_t s_idx[kRowWarps][32];
+  __shared__ float s_val[kRowWarps][32];
+  __shared__ IdxT s_perm[kRowWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const IdxT* __restrict__ rowptr = static_cast<const IdxT*>(p.s.rowptr);
+  const IdxT* __restrict__ col = static_cast<const IdxT*>(p.s.col);
+  const IdxT* __restrict__ perm = static_cast<const IdxT*>(p.perm);
+  const long long K = p.s.K, units = p.s.n_items + p.s.M, stride = (long long)gridDim.x * kRowWarps;
+  const int last = 32 * (NC - 1) + lane;
+  const bool last_valid = last < K;
+  const WeightedBwLane l{p.s.mat + lane, p.s.mat + (last_valid ? last : 32 * (NC - 1)), (unsigned long long)K, last_valid, lane};
+  uint32_t* const my_idx = s_idx[warp];
+  float* const my_val = s_val[warp];
+  IdxT* const my_perm = s_perm[warp];
+
+  struct Unit {
+    long long row, slot;     // slot: of a piece, -1 for a row
+    IdxT b, e;
+  };
+  auto unit_at = [&](long long q) {
+    Unit u{0, -1, 0, 0};
+    if (q < p.s.n_items) {
+      u.row = p.s.item_row[q];
+      u.slot = p.s.item_slot ? p.s.item_slot[q] : q;
+      u.b = (IdxT)p.s.item_begin[q];
+      u.e = (IdxT)p.s.item_end[q];
+    } else if (q < units) {
+      u.row = p.s.row_order ? (long long)p.s.row_order[q - p.s.n_items] : q - p.s.n_items;
+      u.b = rowptr[u.row];
+      u.e = rowptr[u.row + 1];
+    }
+    return u;
+  };
+  uint32_t idx;
+  float val;
+  IdxT pos;
+  auto edges = [&](long long at, long long end) {
+    idx = 0;
+    val = 0.f;
+    pos = 0;
+    if (at < end) {
+      idx = (uint32_t)col[at];
+      val = __ldg(p.s.val + at);
+      pos = perm[at];
+    }
+  };
+  long long q = (long long)blockIdx.x * kRowWarps + warp;
+  Unit cur = unit_at(q), nxt = unit_at(q + stride);
+  edges((long long)cur.b + lane, (long long)cur.e);
+  for (; q < units; q += stride) {
+    const long long len = (long long)(cur.e - cur.b);
+    const bool skip = cur.slot < 0 && p.s.long_threshold > 0 && len > p.s.long_threshold;   // done by its pieces
+    const Unit after = unit_at(q + 2 * stride);
+    float xr[NC], acc[NC];
+    if (!skip) {
+      const float* __restrict__ x = p.x + cur.row * K;
+#pragma unroll
+      for (int c = 0; c < NC; c++) {
+        acc[c] = 0.f;
+        xr[c] = c < NC - 1 || last_valid ? __ldg(x + lane + 32 * c) : 0.f;
+      }
+    }
+    for (long long base = 0; base == 0 || (base < len && !skip); base += 32) {
+      __syncwarp();
+      my_idx[lane] = idx;
+      my_val[lane] = val;
+      my_perm[lane] = pos;
+      __syncwarp();
+      // the next edges of this unit, or the first ones of the next
+      if (!skip && base + 32 < len) edges((long long)cur.b + base + 32 + lane, (long long)cur.e);
+      else edges((long long)nxt.b + lane, (long long)nxt.e);
+      if (skip) break;
+      const int cnt = len - base < 32 ? (int)(len - base) : 32;
+      int t = 0;
+      auto few = [&](auto n) {
+        constexpr int B = decltype(n)::value;
+        float m[B][NC], d[B];
+        weighted_bw_load<B, NC>(l, my_idx + t, m);
+        weighted_bw_add<B, NC>(l, my_val + t, m, xr, acc, d);
+        weighted_bw_values<B, IdxT>(p, my_idx + t, my_perm + t, lane, d);
+        t += B;
+      };
+#pragma unroll 1
+      while (t + 8 <= cnt) few(std::integral_constant<int, 8>());
+      if (cnt & 4) few(std::integral_constant<int, 4>());
+      if (cnt & 2) few(std::integral_constant<int, 2>());
+      if (cnt & 1) few(std::integral_constant<int, 1>());
+    }
+    if (!skip) {
+      float* dst = cur.slot >= 0 ? p.s.scratch + cur.slot * K : p.s.out + cur.row * K;
+#pragma unroll
+      for (int c = 0; c < NC; c++)
+        if (c < NC - 1 || last_valid) dst[lane + 32 * c] = acc[c];
+    }
+    cur = nxt;
+    nxt = after;
+  }
+}
+
+template <typename IdxT>
+static int launch_weighted_bw(const WeightedBwParams& p, cudaStream_t st) {
+  const int nc = (int)((p.s.K + 31) / 32);
+#define EXB_WBW(NC_)                                                                                                       \
+  case NC_: {                                                                                                              \
+    const int grid = resident_blocks(spmm_weighted_bw_kernel<IdxT, NC_>, kRowWarps * 32, (p.s.n_items + p.s.M + kRowWarps - 1) / kRowWarps); \
+    spmm_weighted_bw_kernel<IdxT, NC_><<<grid, kRowWarps * 32, 0, st>>>(p);                                                \
+    break;                                                                                                                 \
+  }
+  switch (nc) {
+    EXB_WBW(1) EXB_WBW(2) EXB_WBW(3) EXB_WBW(4) EXB_WBW(5) EXB_WBW(6) EXB_WBW(7) EXB_WBW(8)
+    default: return fail(EXB_ERR_UNSUPPORTED, "spmm_weighted_backward: more than 256 columns");
+  }
+#undef EXB_WBW
+  EXB_CUDA_OK(cudaGetLastError());
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p.s.out) | reinterpret_cast<uintptr_t>(p.s.scratch);
+  return p.s.K % 4 == 0 && a % 16 == 0 ? launch_long_reduce<IdxT, 4>(p.s, st) : launch_long_reduce<IdxT, 1>(p.s, st);
+}
+
 // max / min aggregation with the position of the winning edge (spmm_cuda.cu:27-104 with REDUCE = MAX / MIN;
 // reducer.cuh:43-85): out[r, c] = max_e value[e] * mat[col[e], c], arg[r, c] = the first edge that attains it
 // (a later edge replaces the current one only when strictly greater / smaller), rows without edges give 0 and
@@ -977,6 +1182,31 @@ int exact_spmm_value_bw(const void* row, const void* rowptr, const void* col, in
         K, mean, out);
   EXB_CUDA_OK(cudaGetLastError());
   return EXB_OK;
+}
+
+int exact_spmm_weighted_backward(const void* t_rowptr, const void* t_col, const float* t_value, const void* perm,
+                                 const void* fw_rowptr, int idx_bytes, const float* mat, const float* grad, int64_t M, int64_t K,
+                                 int64_t long_threshold, const int32_t* item_row, const int64_t* item_begin,
+                                 const int64_t* item_end, const int32_t* item_slot, int64_t n_items, const int32_t* long_row,
+                                 const int32_t* long_item_ptr, int64_t n_long, float* scratch, const int32_t* row_order,
+                                 float* grad_mat, float* grad_value, void* stream) {
+  EXB_REQUIRE(idx_bytes == 4 || idx_bytes == 8, "spmm_weighted_backward: idx_bytes must be 4 or 8 (got %d)", idx_bytes);
+  EXB_REQUIRE(M >= 0 && K >= 0 && n_items >= 0 && n_long >= 0, "spmm_weighted_backward: negative size");
+  if (K > 256) return fail(EXB_ERR_UNSUPPORTED, "spmm_weighted_backward: more than 256 columns");
+  if (M == 0 || K == 0) return EXB_OK;
+  EXB_REQUIRE(M < (1LL << 32) && n_items <= 2147483647LL && n_long <= 2147483647LL, "spmm_weighted_backward: too many rows");
+  EXB_REQUIRE(t_rowptr && t_col && t_value && perm && mat && grad && grad_mat && grad_value, "spmm_weighted_backward: null pointer");
+  if (n_items > 0)
+    EXB_REQUIRE(long_threshold > 0 && item_row && item_begin && item_end && long_row && long_item_ptr && scratch && n_long > 0,
+                "spmm_weighted_backward: null plan array or scratch");
+  WeightedBwParams p{};
+  p.s.rowptr = t_rowptr; p.s.col = t_col; p.s.val = t_value; p.s.mat = grad; p.s.out = grad_mat; p.s.M = M; p.s.K = p.s.Kout = K;
+  p.s.long_threshold = n_items > 0 ? long_threshold : 0;
+  p.s.item_row = item_row; p.s.item_begin = reinterpret_cast<const long long*>(item_begin);
+  p.s.item_end = reinterpret_cast<const long long*>(item_end); p.s.item_slot = item_slot; p.s.n_items = n_items;
+  p.s.long_row = long_row; p.s.long_item_ptr = long_item_ptr; p.s.n_long = n_long; p.s.scratch = scratch; p.s.row_order = row_order;
+  p.perm = perm; p.fw_rowptr = fw_rowptr; p.x = mat; p.grad_value = grad_value;
+  return idx_bytes == 4 ? launch_weighted_bw<int32_t>(p, (cudaStream_t)stream) : launch_weighted_bw<int64_t>(p, (cudaStream_t)stream);
 }
 
 int exact_spmm(const void* rowptr, const void* col, int idx_bytes, const float* value, const float* mat,

@@ -50,6 +50,13 @@ class SparseStorage:
             self._csr2csc = torch.argsort(key, stable=True)
         return self._csr2csc
 
+    def transposed_edges(self):
+        """csr2csc in the width of the other indices, cached."""
+        hit = self._t_cache.get("edges")
+        if hit is None:
+            hit = self._t_cache["edges"] = self.csr2csc().to(self._col.dtype).contiguous()
+        return hit
+
     def colptr(self):
         if self._colptr is None:
             N = self._sparse_sizes[1]

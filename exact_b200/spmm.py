@@ -41,6 +41,7 @@ def qmatmul(src, other, reduce="sum", quantized=None, randmat=None, scheme=None)
         kept = config.kept_columns(other.size(1)) if code < 2 else 0
         draws = (2 if kept else 1) if value_rg or code >= 2 else 0
         return _lib.native().aggregate(other, value, st.row() if value_rg and code < 2 else None,
+                                       st.transposed_edges() if value_rg and need_t else None,
                                        st.native_graph(("sum", "mean")[code] if need_t else None, weighted=need_t and code == 1),
                                        code, value_rg, config.activation_compression_bits[0], kept, config.seed, config.take_offsets(draws),
                                        config.row_offset, config.fused_rp)

@@ -1,0 +1,77 @@
+"""Both gradients of a weighted aggregation from one walk of the transposed structure, against the oracle's separate ones."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from exact_b200 import SparseTensor, config, qmatmul
+from helpers import normal
+
+pytestmark = pytest.mark.gpu
+
+
+def hub_graph(n, seed):
+    """Rows and columns of up to 300 - 900 edges (pieces), of every small length, and empty ones."""
+    rng = np.random.default_rng(seed)
+    r = np.concatenate([np.full(900, 7), rng.integers(0, n, 700), rng.integers(0, n // 2, 9 * n)])
+    c = np.concatenate([rng.integers(0, n, 900), np.full(700, 11), rng.integers(0, n // 3, 9 * n)])
+    key = np.unique(r * n + c)
+    return key // n, key % n
+
+
+# columns: every number of 32-column groups with and without a remainder, and one width beyond the kernel's range
+@pytest.mark.parametrize("idx", [torch.int32, torch.int64])
+@pytest.mark.parametrize("K", [1, 31, 32, 33, 64, 100, 128, 160, 192, 200, 224, 250, 256, 260])
+@pytest.mark.parametrize("reduce", ["sum", "mean"])
+def test_both_gradients(K, reduce, idx):
+    n = 2000
+    row, col = hub_graph(n, K)
+    rowptr = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(row, minlength=n), out=rowptr[1:])
+    val = np.random.default_rng(1).standard_normal(col.size).astype(np.float32)
+    t = torch.from_numpy
+    v = t(val).cuda().requires_grad_()
+    adj = SparseTensor(row=t(row).cuda(), col=t(col).cuda(), value=v, sparse_sizes=(n, n), is_sorted=True)
+    adj.fill_cache_()
+    if idx == torch.int32:
+        adj.to_int32_()
+    mat, g = normal(n, K, 6), normal(n, K, 7)
+    if K > 1:
+        g[5, K - 1] = np.inf                   # stays in its row's edges and its column
+    x = t(mat).cuda().requires_grad_()
+    config.compress_activation = False
+    try:
+        qmatmul(adj, x, reduce).backward(t(g).cuda())
+    finally:
+        config.compress_activation = True
+    assert np.array_equal(v.grad.cpu().numpy(), oracle.spmm_value_bw(rowptr, col, mat, g, reduce), equal_nan=True)
+    perm = np.argsort(col * n + row, kind="stable")
+    w = val[perm]
+    if reduce == "mean":
+        w = w / np.maximum(np.diff(rowptr), 1)[row[perm]].astype(np.float32)
+    colptr = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(col, minlength=n), out=colptr[1:])
+    ref = oracle.spmm(colptr, row[perm], w, g, "sum")
+    got, long = x.grad.cpu().numpy(), np.diff(colptr) > int(config.spmm_long_row)
+    assert long.any() and np.array_equal(got[~long], ref[~long], equal_nan=True)
+    ok = np.isfinite(ref[long])
+    # pieces of 256 edges: a regrouped sum of fp32 terms, 1e-5 of the row's largest entry as elsewhere
+    assert np.abs((got[long] - ref[long])[ok]).max() <= 1e-5 * np.abs(ref[long][ok]).max()
+
+
+def test_one_gradient_at_a_time_takes_the_separate_kernels():
+    n, K = 2000, 64
+    row, col = (torch.from_numpy(a).cuda() for a in hub_graph(n, 3))
+    val = torch.rand(col.numel(), device="cuda")
+    mat, g = (torch.from_numpy(normal(n, K, s)).cuda() for s in (6, 7))
+
+    def grads(x_rg, v_rg):
+        v, x = val.clone().requires_grad_(v_rg), mat.clone().requires_grad_(x_rg)
+        adj = SparseTensor(row=row, col=col, value=v, sparse_sizes=(n, n), is_sorted=True)
+        config.compress_activation = True
+        config.manual_seed(1)
+        qmatmul(adj, x, "sum").backward(g)
+        return x.grad, v.grad
+
+    both, only_x, only_v = grads(True, True), grads(True, False), grads(False, True)
+    assert torch.equal(both[0], only_x[0]) and torch.equal(both[1], only_v[1])
