@@ -421,6 +421,11 @@ int make_tensor_map_2d_f32(CUtensorMap* map, const void* base, unsigned long lon
                            unsigned long long pitch_bytes, unsigned box_inner, unsigned box_outer, bool swizzle128) {
   auto enc = get_encode();
   if (enc == nullptr) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  // A driver call: it finds no context in a thread that has not used the device through the runtime yet (the backward thread of a
+  // framework, when this is the first thing it does).
+  int dev = 0;
+  EXB_CUDA_OK(cudaGetDevice(&dev));
+  EXB_CUDA_OK(cudaSetDevice(dev));
   cuuint64_t dims[2] = {inner, outer};
   cuuint64_t strides[1] = {pitch_bytes};
   cuuint32_t box[2] = {box_inner, box_outer};
