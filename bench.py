@@ -389,8 +389,8 @@ def roofline_of_dominant_kernel(ksum, ms_total, steps, hbm_peak, peak_kind):
     HBM-bound kernels: `achieved` = bytes that must cross HBM at least once (the operand in the form the kernel
     reads it, the indices, the output) / mean launch time, so that `frac` cannot exceed 1 by counting cache hits;
     for the gathers `l2_side_GB/s` gives the bytes requested from L2 when no source row is reused (the
-    reference's kernel moves exactly those).  The dense-layer GEMM is tensor-bound: tf32 flop issued (three
-    MMAs per product) against half the measured bf16 peak."""
+    reference's kernel moves exactly those).  The dense-layer GEMM: fp16 flop issued (three MMAs per product) against the
+    measured bf16 peak, which is also fp16's."""
     if not ksum:
         return None
     name, r = max(ksum.items(), key=lambda kv: kv[1]["ms"])
@@ -402,14 +402,14 @@ def roofline_of_dominant_kernel(ksum, ms_total, steps, hbm_peak, peak_kind):
         peak = None
         try:
             with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
-                peak = float(json.load(f)["bf16_tflops_sustained"]) / 2.0
-            kind = "measured bf16 sustained / 2 (tf32 runs at half the bf16 rate)"
+                peak = float(json.load(f)["bf16_tflops_sustained"])
+            kind = "measured bf16 sustained (fp16 runs at the bf16 rate)"
         except Exception:
-            peak, kind = 1400.0 / 2.0, "fallback bf16 sustained / 2"
+            peak, kind = 1400.0, "fallback bf16 sustained"
         achieved = r["flops"] / r["launches"] / sec / 1e12
         return dict(common, bound="tensor", achieved=round(achieved, 1), peak=peak, peak_kind=kind, unit="TFLOP/s",
                     frac=round(achieved / peak, 4), traffic=None,
-                    flops_model="6*M*K*N tf32 flop per call: every fp32 product is three tf32 MMAs (head*head, "
+                    flops_model="6*M*K*N fp16 flop per call: every fp32 product is three fp16 MMAs (head*head, "
                                 "tail*head, head*tail)")
     achieved = r["bytes"] / r["launches"] / sec / 1e9
     out = dict(common, bound="hbm", achieved=round(achieved, 1), peak=hbm_peak, peak_kind=peak_kind, unit="GB/s",
@@ -547,7 +547,7 @@ def kernel_bandwidths(torch, Q, _lib, dev, hbm_peak, N=1_000_000, D=128, reps=20
     ref = reference_kernel_times(torch, dev, hbm_peak, reps)
     if ref is not None:
         out["ref_cuda"] = ref
-    # the dense-layer GEMM (tf32 head/tail split, three MMAs per tile) against the library's fp32 GEMM
+    # the dense-layer GEMM (fp16 head/tail split, three MMAs per tile) against the library's fp32 GEMM
     from exact_b200.cpp_extension import backward_func as B
     M3, K3, N3 = 1_000_000, 256, 256
     a3 = torch.randn(M3, K3, device=dev, generator=gen)
@@ -564,7 +564,7 @@ def kernel_bandwidths(torch, Q, _lib, dev, hbm_peak, N=1_000_000, D=128, reps=20
         b.record()
         torch.cuda.synchronize()
         times[name] = a.elapsed_time(b) * 1e-3 / reps
-    out["linear_tf32x3_1Mx256x256"] = {"ms": round(times["tc"] * 1e3, 4), "library_fp32_ms": round(times["lib"] * 1e3, 4),
+    out["linear_f16x3_1Mx256x256"] = {"ms": round(times["tc"] * 1e3, 4), "library_fp32_ms": round(times["lib"] * 1e3, 4),
                                        "fp32_equiv_TFLOP/s": round(2.0 * M3 * K3 * N3 / times["tc"] / 1e12, 1),
                                        "tensor_TFLOP/s": round(6.0 * M3 * K3 * N3 / times["tc"] / 1e12, 1)}
     return out

@@ -110,10 +110,6 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc)
       : "memory");
 }
-// fp32 accumulator, fp16 A and B, both K-major
-__host__ __device__ inline uint32_t umma_idesc_f16(int M, int N) {
-  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
                "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
@@ -125,11 +121,6 @@ __device__ __forceinline__ void bulk_prefetch(const void* src, uint32_t bytes) {
 }
 __device__ __forceinline__ void copy16(uint32_t dst, const void* src, uint32_t bytes) {   // the rest of 16 is zero-filled
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-template <int REGS, bool MORE>
-__device__ __forceinline__ void set_registers() {
-  if (MORE) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS));
-  else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
 }
 // Shared memory by 32-bit address, in program order.
 __device__ __forceinline__ uint32_t lds_u8(uint32_t addr) {

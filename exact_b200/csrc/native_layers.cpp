@@ -232,7 +232,7 @@ struct SageNode : Function<SageNode> {
       const Tensor t = spmm(g.fw, g.fw.value, linear(x, wcat, {}, {}, {}, {}, false), s->mean);
       s->agg.q = quantize_pack_rows(t.narrow(1, 0, k), s->how.bits, s->how.seed, offset + 1, s->how.row_offset);
       const Tensor part = t.narrow(1, kp, out_f);
-      if (w_r) out = linear(x, *w_r, b, {}, {}, {}, false, 0, part);
+      if (w_r) out = linear(x, *w_r, b, {}, {}, {}, false, part);
       else out = b ? part.add(*b) : part.contiguous();
     } else {
       const Tensor agg = spmm(g.fw, g.fw.value, x, s->mean);
@@ -444,15 +444,14 @@ Tensor aggregate_node(const Tensor& x, const OptTensor& value, const OptTensor& 
 
 // ---- evaluation -----------------------------------------------------------------------------------------
 // Evaluation is compared with the plain fp32 model, so its products are no further from the exact ones than the library's fp32 GEMM:
-// contractions in chunks of 64 columns, the small products first, 1.3e-7 to 1.4e-7 (Frobenius) at every width against 1.8e-7 at
-// 100, 2.0e-7 at 256 and 4.4e-7 at 602 columns; in one piece the accumulator's truncation makes it 8e-7, 1.8e-6 and 4.4e-6.  Up to
-// 64 columns the library is the nearer one (9e-8 against 1.1e-7 at 48) and takes them, 200,000 x 48 -> 256 in 173 us against 98.
-constexpr int64_t kEvalChunk = 64;
+// 1.06e-7 to 1.2e-7 (Frobenius) from 100 columns on against 1.8e-7 at 100, 2.0e-7 at 256 and 4.4e-7 at 602.  Up to 64 columns the
+// library is the nearer one (9e-8 against 1.04e-7 at 48) and takes them, 200,000 x 48 -> 256 in 173 us against 58.
+constexpr int64_t kEvalLibrary = 64;
 
 // a w^T (+ a2 w2^T) (+ bias) (+ addend)
 Tensor eval_product(const Tensor& a, const Tensor& w, const OptTensor& bias = {}, const OptTensor& a2 = {}, const OptTensor& w2 = {},
                     const OptTensor& addend = {}) {
-  if (a.size(1) + (a2 ? a2->size(1) : 0) > kEvalChunk) return linear(a, w, bias, a2, w2, {}, false, kEvalChunk, addend);
+  if (a.size(1) + (a2 ? a2->size(1) : 0) > kEvalLibrary) return linear(a, w, bias, a2, w2, {}, false, addend);
   Tensor out = at::linear(a, w, bias);
   if (a2) out.addmm_(*a2, w2->t());
   return addend ? out.add_(*addend) : out;

@@ -1,4 +1,4 @@
-"""Dense-layer GEMM on the tensor cores with operands split into tf32 head and tail
+"""Dense-layer GEMM on the tensor cores with operands split into head and tail
 (exact_linear_forward) against an fp64 product, over every shape class the layers use (ragged K and N,
 second operand pair, accumulation into C, outputs wider than one MMA tile).
 
