@@ -547,7 +547,7 @@ def kernel_bandwidths(torch, Q, _lib, dev, hbm_peak, N=1_000_000, D=128, reps=20
     ref = reference_kernel_times(torch, dev, hbm_peak, reps)
     if ref is not None:
         out["ref_cuda"] = ref
-    # the dense-layer GEMM (fp16 head/tail split, three MMAs per tile) against the library's fp32 GEMM
+    # the dense-layer GEMM (tf32 head/tail split, three MMAs per tile) against the library's fp32 GEMM
     from exact_b200.cpp_extension import backward_func as B
     M3, K3, N3 = 1_000_000, 256, 256
     a3 = torch.randn(M3, K3, device=dev, generator=gen)
@@ -564,7 +564,7 @@ def kernel_bandwidths(torch, Q, _lib, dev, hbm_peak, N=1_000_000, D=128, reps=20
         b.record()
         torch.cuda.synchronize()
         times[name] = a.elapsed_time(b) * 1e-3 / reps
-    out["linear_f16x3_1Mx256x256"] = {"ms": round(times["tc"] * 1e3, 4), "library_fp32_ms": round(times["lib"] * 1e3, 4),
+    out["linear_tf32x3_1Mx256x256"] = {"ms": round(times["tc"] * 1e3, 4), "library_fp32_ms": round(times["lib"] * 1e3, 4),
                                        "fp32_equiv_TFLOP/s": round(2.0 * M3 * K3 * N3 / times["tc"] / 1e12, 1),
                                        "tensor_TFLOP/s": round(6.0 * M3 * K3 * N3 / times["tc"] / 1e12, 1)}
     return out

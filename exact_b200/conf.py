@@ -46,7 +46,7 @@ class QuantizationConfig:
         # Do not produce compressed copies that no backward formula reads (the SpMM's dense operand
         # when edge values need no gradient).  Outputs and gradients are unaffected.
         self.skip_dead_saves = True
-        # Dense-layer GEMMs over node rows on the tensor cores with operands split into fp16 head and tail
+        # Dense-layer GEMMs over node rows on the tensor cores with operands split into head and tail
         # (fp32-equivalent accuracy); False: the library's fp32 GEMM.
         self.linear_tensor_core = True
         # Weight gradients of the quantised linear layers straight from the packed activation on the tensor

@@ -7,14 +7,16 @@
 // (exact/exact/cpp_extension/backward_func.cc:86).  M is the number of node rows (millions), K and N are
 // feature widths (<= 256 per call for N).
 //
+// The interface, and the kernel of the contractions that are summed in chunks (k_chunk > 0); linear_tf32.cu has the other one.
+//
 // Arithmetic.  A row of A is scaled by a power of two per K tile (64 columns), a row of B by one for all of them, so that the
 // largest element lies in [2^14, 2^15); then every operand is split into an fp16 head and an fp16 tail,
 //     a = a_hi + a_lo,   a_hi = rn_f16(a),   a_lo = rn_f16(a - a_hi)      (22 bits),
 // and a K tile's product is a_lo b_hi + a_hi b_lo + a_hi b_hi, accumulated in TMEM in this order: the tensor core truncates its
 // fp32 accumulator, at the size of what is there already.  The K tile's sum is read back, gets its average loss (2^-23) and its
 // scales back, and is added to the others in fp32 registers.  Against fp64 (Frobenius; M = 100,000 rows of the layers' operands):
-// 1.04e-7 .. 1.2e-7 at 33 to 602 columns.  tf32 heads and tails in one chain, the former kernel of training, 3e-7 .. 4.4e-6; in
-// chains of 64 columns, the former one of evaluation, 1.04e-7 .. 1.39e-7; the library's fp32 GEMM 9e-8 (48) .. 4.4e-7 (602).  The
+// 1.04e-7 .. 1.2e-7 at 33 to 602 columns.  tf32 heads and tails in one chain, 3e-7 .. 4.4e-6; in
+// chains of 64 columns, the former kernel of evaluation, 1.04e-7 .. 1.39e-7; the library's fp32 GEMM 9e-8 (48) .. 4.4e-7 (602).  The
 // tail of an element is exact to 2^-39 of its row's largest one in the K tile.  Non-finite inputs stay non-finite and confined to
 // their rows, but an infinite element turns its output row into NaN where an fp32 GEMM gives +-inf (its tail is inf - inf).
 //
@@ -558,6 +560,12 @@ __global__ void __launch_bounds__(kLinPrepThreads) linear_prepare_kernel(
   }
 }
 
+namespace tf32 {   // linear_tf32.cu
+int launch_linear(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb, int64_t incb, const float* A2, int64_t K2,
+                  int64_t lda2, const float* B2, int64_t ldb2, int64_t incb2, int64_t N, const float* bias, const float* addend,
+                  int64_t ldadd, void* workspace, float* C, int64_t ldc, cudaStream_t st);
+}
+
 static inline int lin_kpad(long long K) { return (int)((K + kLinTileK - 1) / kLinTileK * kLinTileK); }
 
 // One launch over checked arguments: N <= 256 columns.
@@ -640,7 +648,7 @@ extern "C" {
 int64_t exact_linear_workspace_bytes(int64_t N, int64_t K, int64_t K2) {
   if (N <= 0 || K <= 0 || K2 < 0) return 256;
   const int64_t Npad = (N + 15) / 16 * 16;
-  // what the call's tiles and scales take, and not less than two fp32 copies in rows of 32 columns, as it was
+  // the tiles and scales of this file's kernel, and the two fp32 copies in rows of 32 columns of the other's
   const int64_t tiles = 256 + 2 * kLinMaxCols * 4 + 2 * Npad * (int64_t)(lin_kpad(K) + lin_kpad(K2)) * 2;
   const int64_t copies = 256 + 2 * Npad * ((K + 31) / 32 * 32 + (K2 + 31) / 32 * 32) * 4;
   return tiles > copies ? tiles : copies;
@@ -674,7 +682,8 @@ int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t l
   EXB_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "linear_forward: workspace must be 256-byte aligned");
   EXB_REQUIRE((M + kLinTileM - 1) / kLinTileM < 2147483647LL / kLinTileM, "linear_forward: too many rows");
   cudaStream_t st = (cudaStream_t)stream;
-  return lin_launch(A, M, K, lda, B, ldb, incb, A2, K2, lda2, B2, ldb2, incb2, N, bias, addend, ldadd, workspace, C, ldc, st);
+  return (k_chunk > 0 ? lin_launch : tf32::launch_linear)(A, M, K, lda, B, ldb, incb, A2, K2, lda2, B2, ldb2, incb2, N, bias, addend, ldadd,
+                                                          workspace, C, ldc, st);
 }
 
 }  // extern "C"

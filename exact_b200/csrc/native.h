@@ -121,7 +121,7 @@ bool linear_supported(const Tensor& a);
 Tensor rows16(const Tensor& a);
 // fp32 operands; w may be a transposed view (its rows are read through both strides); addend: rows of any pitch
 Tensor linear(const Tensor& a, const Tensor& w, const OptTensor& bias, const OptTensor& a2, const OptTensor& w2,
-              const OptTensor& out, bool accumulate, const OptTensor& addend = {});
+              const OptTensor& out, bool accumulate, int64_t k_chunk = 0, const OptTensor& addend = {});
 bool grad_weight_takes(const Tensor& g);
 Tensor rows_reduce_mm(const Tensor& g, const Tensor& x, int64_t batches = 512);
 Tensor grad_weight(const Tensor& g, int64_t bits, const Packed& q0, int64_t k0, const Packed* q1, int64_t k1);

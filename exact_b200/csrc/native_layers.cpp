@@ -71,13 +71,19 @@ Tensor weight_grad(const Tensor& g, const Compressed& c, int64_t bits, int64_t N
   return c.R.defined() ? at::mm(G, c.R.t()) : G.contiguous();
 }
 
+// Products by the kernel that adds sums of 64 columns up in fp32 (exact_linear_forward_strided): the gradients, evaluation, and the
+// forward pass of layers that project what they save.  Without a projection the next layer quantises the product itself, whose codes
+// follow its last bits, and the kernel that it always came from stays (csrc/linear_tf32.cu).
+constexpr int64_t kSumChunk = 64;
+int64_t forward_chunk(const Saving& how) { return how.kept ? kSumChunk : 0; }
+
 // A (x W^T) + b with fewer columns in than out: (A x) W^T gathers the narrower operand.
 bool aggregates_first(const Tensor& x, const Tensor& w) { return x.size(1) < w.size(0) && x.size(1) % 4 == 0; }
 
 // A (x W^T) + b
-Tensor gcn_product(const Graph& g, const Tensor& x, const Tensor& w, const OptTensor& b) {
-  if (aggregates_first(x, w)) return linear(spmm(g.fw, g.fw.value, x, false), w, b, {}, {}, {}, false);
-  return spmm(g.fw, g.fw.value, linear(x, w, {}, {}, {}, {}, false), false, b);
+Tensor gcn_product(const Graph& g, const Tensor& x, const Tensor& w, const OptTensor& b, int64_t chunk) {
+  if (aggregates_first(x, w)) return linear(spmm(g.fw, g.fw.value, x, false), w, b, {}, {}, {}, false, chunk);
+  return spmm(g.fw, g.fw.value, linear(x, w, {}, {}, {}, {}, false, chunk), false, b);
 }
 
 }  // namespace
@@ -130,7 +136,7 @@ struct GcnNode : Function<GcnNode> {
       out = spmm(g.fw, g.fw.value, at::linear(x, w), false, b);   // with a bias: half + float is a float
     } else {
       s->x = compress(x, s->how, s->how.offset);
-      out = gcn_product(g, x, w, b);
+      out = gcn_product(g, x, w, b, forward_chunk(s->how));
     }
     s->w = w;
     s->rows = x.size(0);
@@ -173,7 +179,7 @@ struct GcnNode : Function<GcnNode> {
         gw = weight_grad(gh, s->x, s->how.bits, s->rows);
         if (O % 4) gw = gw.narrow(0, 0, O);
       }
-      if (need_x) gx = linear(gh.narrow(1, 0, O), s->w.t(), {}, {}, {}, {}, false);
+      if (need_x) gx = linear(gh.narrow(1, 0, O), s->w.t(), {}, {}, {}, {}, false, kSumChunk);
     }
     return {gx, gw, gb, {}};
   }
@@ -229,17 +235,17 @@ struct SageNode : Function<SageNode> {
       Tensor wcat = at::zeros({kp + op, in_f}, w_l.options());
       wcat.narrow(0, 0, k).copy_(s->agg.R.t());
       wcat.narrow(0, kp, out_f).copy_(w_l);
-      const Tensor t = spmm(g.fw, g.fw.value, linear(x, wcat, {}, {}, {}, {}, false), s->mean);
+      const Tensor t = spmm(g.fw, g.fw.value, linear(x, wcat, {}, {}, {}, {}, false, forward_chunk(s->how)), s->mean);
       s->agg.q = quantize_pack_rows(t.narrow(1, 0, k), s->how.bits, s->how.seed, offset + 1, s->how.row_offset);
       const Tensor part = t.narrow(1, kp, out_f);
-      if (w_r) out = linear(x, *w_r, b, {}, {}, {}, false, part);
+      if (w_r) out = linear(x, *w_r, b, {}, {}, {}, false, forward_chunk(s->how), part);
       else out = b ? part.add(*b) : part.contiguous();
     } else {
       const Tensor agg = spmm(g.fw, g.fw.value, x, s->mean);
       s->agg = compress(agg, s->how, offset);
       OptTensor a2;
       if (w_r) a2 = x;
-      out = linear(agg, w_l, b, a2, w_r, {}, false);
+      out = linear(agg, w_l, b, a2, w_r, {}, false, forward_chunk(s->how));
     }
     ctx->saved_data["s"] = c10::IValue::make_capsule(s);
     return out;
@@ -291,12 +297,12 @@ struct SageNode : Function<SageNode> {
       if (aggregate_g) {
         // A^T (D^-1 g) reads no edge weights; with edge values, or a sum, the transposed structure's weights apply
         const Tensor t = spmm(gr.bw, by_degree ? OptTensor() : gr.bw.value, scaled.defined() ? scaled : g, false);
-        gx = linear(t.narrow(1, 0, O), s->w_l.t(), {}, a2, w2, {}, false);
+        gx = linear(t.narrow(1, 0, O), s->w_l.t(), {}, a2, w2, {}, false, kSumChunk);
       } else {
-        Tensor y = linear(g_true, s->w_l.t(), {}, {}, {}, {}, false);
+        Tensor y = linear(g_true, s->w_l.t(), {}, {}, {}, {}, false, kSumChunk);
         if (by_degree) y.mul_(gr.inv_degree->unsqueeze(1));   // the transposed structure carries no weights of the mean
         gx = spmm(gr.bw, gr.bw.value, y, false);
-        if (has_r) linear(g_true, s->w_r.t(), {}, {}, {}, gx, true);
+        if (has_r) linear(g_true, s->w_r.t(), {}, {}, {}, gx, true, kSumChunk);
       }
     }
     return {gx, gl, gb, gwr, {}};
@@ -451,7 +457,7 @@ constexpr int64_t kEvalLibrary = 64;
 // a w^T (+ a2 w2^T) (+ bias) (+ addend)
 Tensor eval_product(const Tensor& a, const Tensor& w, const OptTensor& bias = {}, const OptTensor& a2 = {}, const OptTensor& w2 = {},
                     const OptTensor& addend = {}) {
-  if (a.size(1) + (a2 ? a2->size(1) : 0) > kEvalLibrary) return linear(a, w, bias, a2, w2, {}, false, addend);
+  if (a.size(1) + (a2 ? a2->size(1) : 0) > kEvalLibrary) return linear(a, w, bias, a2, w2, {}, false, kSumChunk, addend);
   Tensor out = at::linear(a, w, bias);
   if (a2) out.addmm_(*a2, w2->t());
   return addend ? out.add_(*addend) : out;

@@ -197,7 +197,7 @@ Tensor rows16(const Tensor& a) {
 }
 
 Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const OptTensor& a2_, const OptTensor& w2_,
-              const OptTensor& out_, bool accumulate, const OptTensor& addend_) {
+              const OptTensor& out_, bool accumulate, int64_t k_chunk, const OptTensor& addend_) {
   c10::cuda::CUDAGuard guard(a_.device());
   const int64_t M = a_.size(0), K = a_.size(1), N = w_.size(0);
   const Tensor a = rows16(a_), w = w_;
@@ -226,7 +226,7 @@ Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const 
                                       K2 ? a2.stride(0) : 0, w2b, K2 ? w2.stride(0) : 0, K2 ? w2.stride(1) : 1, n,
                                       bias.defined() ? ptr<float>(bias) + n0 : nullptr,
                                               addend ? ptr<float>(addend) + n0 : nullptr, addend ? addend->stride(0) : 0,
-                                              0, nullptr, ptr(ws),
+                                              k_chunk, nullptr, ptr(ws),
                                               cb, out.stride(0), st);
     });
   }

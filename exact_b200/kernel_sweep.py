@@ -120,7 +120,7 @@ def run_unpack_rp(N, D, kept_frac, bits, reps):
 
 
 def run_linear(M, K, N, reps):
-    """Dense-layer GEMM (fp16 head/tail split, tcgen05) against the library fp32 GEMM: ms, TFLOP/s, error vs fp64."""
+    """Dense-layer GEMM (tf32 head/tail split, tcgen05) against the library fp32 GEMM: ms, TFLOP/s, error vs fp64."""
     from .cpp_extension import backward_func as B
     dev = torch.device("cuda")
     g = torch.Generator(device=dev).manual_seed(0)

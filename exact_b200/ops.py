@@ -125,7 +125,7 @@ def input2rp(input, kept_acts):
     assert len(input.size()) == 2
     rand_matrix = _rademacher(input.shape[1], kept_acts, input.device, input.dtype)
     if ext_backward_func._tc_ok(input):
-        # the dense product on this library's tensor-core GEMM (fp32 operands split into fp16 head and tail)
+        # the dense product on this library's tensor-core GEMM (fp32 operands split into tf32 head and tail)
         dim_reduced_input = ext_backward_func.linear_forward(input, rand_matrix.t().contiguous())
     else:
         _lib.note_library_call("input2rp as torch.matmul (fewer than 1024 rows, not fp32 or not CUDA)")

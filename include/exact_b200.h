@@ -470,8 +470,8 @@ EXACT_API int exact_unpack_dequant_rp(const uint8_t* packed, int bits, const uin
                                       const uint16_t* min_bf16, int64_t N, int64_t k, const float* R, int64_t D,
                                       void* workspace, float* out, void* stream);
 
-/* Dense layer GEMM with fp32-equivalent accuracy on the tensor cores (each operand scaled by powers of two and split into an fp16
- * head and tail, three tcgen05 MMAs per tile, sums of 64 columns added in fp32; 1.2e-7 Frobenius against fp64):
+/* Dense layer GEMM with fp32-equivalent accuracy on the tensor cores (each operand split into a tf32
+ * head and tail, three tcgen05 MMAs per tile, fp32 accumulation):
  *     C[M, N] (+)= A[M, K] B[N, K]^T  (+ A2[M, K2] B2[N, K2]^T)  (+ bias[N])
  * Replaces the fp32 cuBLAS GEMMs of the quantised linear layer: F.linear(input, weight, bias) in
  * qlinear.forward (exact/exact/ops.py:150) with A = input, B = weight [out, in]; and
@@ -490,8 +490,11 @@ EXACT_API int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t
                                    int64_t ldc, void* stream);
 /* exact_linear_forward with three more choices.  addend: [M, N] with pitch ldadd, added to the product in place of what C held
  * (NULL: nothing; it may be C).  incb, incb2: distance between the elements of a row of B, B2 (ldb = 1 and incb =
- * the pitch: the transposed weight, without a copy).  k_chunk (a multiple of 32) and partial (exact_linear_partial_bytes(N)
- * bytes, none) are not used any more: every contraction is summed in chunks of 64 columns. */
+ * the pitch: the transposed weight, without a copy).  k_chunk (a multiple of 32): 0: the contraction is one chain of tf32 products
+ * in the tensor core's accumulator, which truncates at every MMA, a bias of about 7e-9 of the result per contracted column.  Else
+ * it is cut into chunks of 64 columns, whose operands are scaled by powers of two and split into fp16 head and tail; a chunk's sum
+ * has its average loss given back and is added to the others in fp32: 1.04e-7 .. 1.2e-7 (Frobenius, against fp64) whatever K is, and
+ * faster but for rows of C that are no multiple of 16 bytes.  partial: exact_linear_partial_bytes(N) bytes (none: not used any more). */
 EXACT_API int64_t exact_linear_partial_bytes(int64_t N);
 EXACT_API int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb,
                                            int64_t incb, const float* A2, int64_t K2, int64_t lda2, const float* B2,

@@ -1,4 +1,4 @@
-"""exact_linear_forward where its scales, K tiles and ways of storing can go wrong: rows of very different magnitudes, zero and
+"""The chunked dense GEMM where its scales, K tiles and ways of storing can go wrong: rows of very different magnitudes, zero and
 non-finite rows, contractions around a multiple of 64, results of any pitch, with and without an addend."""
 import numpy as np
 import pytest
@@ -25,7 +25,7 @@ def product(a, w, bias=None, addend=None, ldc=None, a2=None, w2=None):
     ws = torch.empty(lib.exact_linear_workspace_bytes(N, K, K2), dtype=torch.uint8, device="cuda")
     _lib.invoke("exact_linear_forward_strided", 0, _lib.ptr(a), M, K, a.shape[1], _lib.ptr(w), K, 1, _lib.ptr(a2), K2,
                 a2.shape[1] if K2 else 0, _lib.ptr(w2), K2, 1, N, _lib.ptr(bias), _lib.ptr(addend), addend.shape[1] if addend is not None else 0,
-                0, None, _lib.ptr(ws), _lib.ptr(out), ldc, _lib.stream_ptr())
+                64, None, _lib.ptr(ws), _lib.ptr(out), ldc, _lib.stream_ptr())
     check_status()
     assert bool((out[:, N:] == 7.0).all())
     return out[:, :N]
