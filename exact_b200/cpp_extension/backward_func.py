@@ -23,7 +23,15 @@ def _rows16(a):
     return out[:, :K]
 
 
-def linear_forward(a, weight, bias=None, a2=None, weight2=None, out=None, accumulate=False):
+SUM_CHUNK = 64   # sums of 64 columns added in fp32: the gradients' products (exact_linear_forward_strided)
+
+
+def forward_chunk():
+    """How the layers' forward products are summed: as the C++ nodes do it (forward_chunk, csrc/native_layers.cpp)."""
+    return SUM_CHUNK if config.kept_frac < 1.0 else 0
+
+
+def linear_forward(a, weight, bias=None, a2=None, weight2=None, out=None, accumulate=False, k_chunk=0):
     """a @ weight.T (+ a2 @ weight2.T) (+ bias), optionally added to `out`: F.linear of ops.py:150 and the
     g W product of backward_func.cc:86 (pass weight.t()).  fp32 in and out."""
     if not _tc_ok(a) or (a2 is not None and not _tc_ok(a2)):
@@ -34,7 +42,7 @@ def linear_forward(a, weight, bias=None, a2=None, weight2=None, out=None, accumu
         if out is not None:
             return out.add_(r) if accumulate else out.copy_(r)
         return r
-    out = _lib.native().linear(a, weight, bias, a2, weight2, out, accumulate)
+    out = _lib.native().linear(a, weight, bias, a2, weight2, out, accumulate, k_chunk)
     if config.check_device_status:
         _lib.check_status(a.device, force=True)
     return out
@@ -89,7 +97,7 @@ def grad_weight_from_packed(g, q0, k0, q1=None, k1=0):
 
 def linear_backward(grad_output, input, weight, bias=None, need_grad_input=True):
     """backward_func.cc:83-93.  The input gradient is left out (None) when the caller has no use for it."""
-    grad_input = linear_forward(grad_output, weight.t()) if need_grad_input else None
+    grad_input = linear_forward(grad_output, weight.t(), k_chunk=SUM_CHUNK) if need_grad_input else None
     grad_weight = rows_reduce_mm(grad_output, input)
     grad_bias = rows_scale_colsum(grad_output)[1] if bias is not None else None
     return grad_input, grad_weight, grad_bias

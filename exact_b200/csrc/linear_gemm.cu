@@ -294,7 +294,7 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     }
   }
   } else if (warp < kLinFirstEpi) {
-    // ---------------- converters ----------------
+    // ---------------- converter: warps 4 .. 11 ----------------
     set_registers<kLinRegsConv, false>();
     // A row of the K tile is 64 elements in two boxes; its heads replace it in the first, its tails in the second.  Four lanes
     // of a warp own a row (eight rows a pass, four passes), read all of it and write only then, so no row is overwritten early;

@@ -198,8 +198,8 @@ PyObject* make_graph(const Tensor& rowptr, const Tensor& col, const OptTensor& v
   return make_capsule(std::move(g));
 }
 Tensor linear_op(const Tensor& a, const Tensor& w, const OptTensor& bias, const OptTensor& a2, const OptTensor& w2,
-                 const OptTensor& out, bool accumulate) {
-  return linear(a, w, bias, a2, w2, out, accumulate);
+                 const OptTensor& out, bool accumulate, int64_t k_chunk) {
+  return linear(a, w, bias, a2, w2, out, accumulate, k_chunk);
 }
 Tensor spmm_op(const Tensor& rowptr, const Tensor& col, const PlanPtr& plan, const OptTensor& value, const Tensor& mat, bool mean) {
   return spmm(rowptr, col, *plan, value, mat, mean);

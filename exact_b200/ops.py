@@ -192,7 +192,7 @@ class qlinear(Function):
         ctx.saved = quantized, weight, bias, randmat
         ctx.other_args = ori_input_shape, proj_input_shape, rp
         if input.dim() == 2:
-            return ext_backward_func.linear_forward(input, weight, bias)
+            return ext_backward_func.linear_forward(input, weight, bias, k_chunk=ext_backward_func.forward_chunk())
         return F.linear(input, weight, bias)
 
     @staticmethod
@@ -224,7 +224,9 @@ def linear_backward_from_compressed(quantized, weight, bias, randmat, ori_input_
             grad_weight = grad_weight.mm(randmat.t())
         else:
             grad_weight = grad_weight.contiguous()
-        grad_input = ext_backward_func.linear_forward(grad_output, weight.t()) if need_grad_input else None
+        grad_input = None
+        if need_grad_input:
+            grad_input = ext_backward_func.linear_forward(grad_output, weight.t(), k_chunk=ext_backward_func.SUM_CHUNK)
         grad_bias = ext_backward_func.rows_scale_colsum(grad_output)[1] if bias is not None else None
         return grad_input, grad_weight, grad_bias
     if (projected and not config.grad_weight_in_projected_space and config.fused_rp and config.compress_activation
@@ -242,7 +244,9 @@ def linear_backward_from_compressed(quantized, weight, bias, randmat, ori_input_
         # grad_W = g^T (Xq R^T) = (g^T Xq) R^T: the [N, D] reconstruction of ops.py:165-166 is never
         # materialised and the large GEMM shrinks from 2*N*out*D to 2*N*out*k flops.
         grad_weight = ext_backward_func.rows_reduce_mm(grad_output, input).mm(randmat.t())
-        grad_input = ext_backward_func.linear_forward(grad_output, weight.t()) if need_grad_input else None
+        grad_input = None
+        if need_grad_input:
+            grad_input = ext_backward_func.linear_forward(grad_output, weight.t(), k_chunk=ext_backward_func.SUM_CHUNK)
         grad_bias = ext_backward_func.rows_scale_colsum(grad_output)[1] if bias is not None else None
     else:
         if projected:

@@ -83,6 +83,9 @@ class QMatmul(torch.nn.Module):
         return qmatmul(src, other, self.reduce, quantized, randmat, self.scheme)
 
 
+_SUM_CHUNK, _forward_chunk = ext_backward_func.SUM_CHUNK, ext_backward_func.forward_chunk
+
+
 def _operand(src, x, tag, rowscale=None):
     """The dense operand x (times rowscale[:, None]) of an aggregation over `src`, with every row the local
     adjacency rows reference in local HBM."""
@@ -171,7 +174,7 @@ class qsage_layer(Function):
 
         def lin_r_early():
             if w_r is not None:
-                early["y"] = ext_backward_func.linear_forward(x, w_r, b_l)
+                early["y"] = ext_backward_func.linear_forward(x, w_r, b_l, k_chunk=_forward_chunk())
 
         def compress_x_and_lin_r():
             early["q"] = project_and_quantize(x, scheme_x, True)
@@ -193,8 +196,8 @@ class qsage_layer(Function):
             ctx.saved = q_x, randmat_x, q_agg, randmat_agg, w_l, b_l, w_r
             ctx.other_args = x.shape, proj_x, proj_agg
             if w_r is None:
-                return ext_backward_func.linear_forward(agg, w_l, b_l)
-            return ext_backward_func.linear_forward(agg, w_l, None, out=early["y"], accumulate=True)
+                return ext_backward_func.linear_forward(agg, w_l, b_l, k_chunk=_forward_chunk())
+            return ext_backward_func.linear_forward(agg, w_l, None, out=early["y"], accumulate=True, k_chunk=_forward_chunk())
         # the input, compressed once (layers.py:153-159)
         q_x, randmat_x, proj_x = project_and_quantize(x, scheme_x, True)
         if w_r is None:
@@ -211,7 +214,8 @@ class qsage_layer(Function):
                 wcat = x.new_zeros((kp + op, in_f))
                 wcat[:k_agg].copy_(randmat_agg.t())
                 wcat[kp:kp + out_f].copy_(w_l)
-                t = _aggregate(src, ext_backward_func.linear_forward(x, wcat), reduce, tag="fw%d" % (kp + op),
+                t = _aggregate(src, ext_backward_func.linear_forward(x, wcat, k_chunk=_forward_chunk()), reduce,
+                               tag="fw%d" % (kp + op),
                                meanwhile=lin_r_early if overlap else None)
                 q_bits = config.activation_compression_bits[0]
                 q_in, q_scale, q_min = ext_quantization.quantize_pack(t[:, :k_agg].contiguous(), q_bits, offset=off_n)
@@ -225,7 +229,7 @@ class qsage_layer(Function):
                     if b_l is not None:
                         y += b_l
                     if w_r is not None:
-                        y = ext_backward_func.linear_forward(x, w_r, None, out=y, accumulate=True)
+                        y = ext_backward_func.linear_forward(x, w_r, None, out=y, accumulate=True, k_chunk=_forward_chunk())
             empty_cache(config.empty_cache_threshold)
             ctx.src, ctx.reduce = src, reduce
             ctx.saved = q_x, randmat_x, q_agg, randmat_agg, w_l, b_l, w_r
@@ -237,7 +241,8 @@ class qsage_layer(Function):
         ctx.src, ctx.reduce = src, reduce
         ctx.saved = q_x, randmat_x, q_agg, randmat_agg, w_l, b_l, w_r
         ctx.other_args = x.shape, proj_x, proj_agg
-        return ext_backward_func.linear_forward(agg, w_l, b_l, a2=x if w_r is not None else None, weight2=w_r)
+        return ext_backward_func.linear_forward(agg, w_l, b_l, a2=x if w_r is not None else None, weight2=w_r,
+                                                k_chunk=_forward_chunk())
 
     @staticmethod
     @custom_bwd(device_type="cuda")
@@ -318,11 +323,11 @@ class qsage_layer(Function):
                 t = _aggregate_transposed(ctx.src, gp, ctx.reduce, rowscale=inv, prescaled=prescaled,
                                           tag="bw%d" % gp.size(1), meanwhile=weight_grads)
                 grad_x = ext_backward_func.linear_forward(t, wp.t(), None, a2=g if w_r is not None else None,
-                                                          weight2=w_r.t() if w_r is not None else None)
+                                                          weight2=w_r.t() if w_r is not None else None, k_chunk=_SUM_CHUNK)
             else:
-                grad_x = _aggregate_transposed(ctx.src, ext_backward_func.linear_forward(g, w_l.t()), ctx.reduce)
+                grad_x = _aggregate_transposed(ctx.src, ext_backward_func.linear_forward(g, w_l.t(), k_chunk=_SUM_CHUNK), ctx.reduce)
                 if w_r is not None:
-                    grad_x = ext_backward_func.linear_forward(g, w_r.t(), None, out=grad_x, accumulate=True)
+                    grad_x = ext_backward_func.linear_forward(g, w_r.t(), None, out=grad_x, accumulate=True, k_chunk=_SUM_CHUNK)
         return None, grad_x, wg["l"], wg["b"], wg["r"], None, None, None
 
 
