@@ -403,34 +403,44 @@ __global__ void rp_prepare_kernel(const float* __restrict__ R, int D, int k, int
   rt[i] = v;
 }
 
-static PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
+struct DriverCalls {
+  PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+  PFN_cuCtxGetCurrent_v4000 context = nullptr;
+};
+
+static void* driver_entry(const char* name) {
+  void* p = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  return cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? p : nullptr;
+}
+
+static DriverCalls driver_calls() {
+  static DriverCalls calls;
   static std::mutex mu;
   std::lock_guard<std::mutex> lock(mu);
-  if (fn == nullptr) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-  }
-  return fn;
+  if (calls.encode == nullptr) calls.encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(driver_entry("cuTensorMapEncodeTiled"));
+  if (calls.context == nullptr) calls.context = reinterpret_cast<PFN_cuCtxGetCurrent_v4000>(driver_entry("cuCtxGetCurrent"));
+  return calls;
 }
 
 int make_tensor_map_2d_f32(CUtensorMap* map, const void* base, unsigned long long inner, unsigned long long outer,
                            unsigned long long pitch_bytes, unsigned box_inner, unsigned box_outer, bool swizzle128) {
-  auto enc = get_encode();
-  if (enc == nullptr) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  const DriverCalls driver = driver_calls();
+  if (driver.encode == nullptr) return fail(EXB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   // A driver call: it finds no context in a thread that has not used the device through the runtime yet (the backward thread of a
-  // framework, when this is the first thing it does).
-  int dev = 0;
-  EXB_CUDA_OK(cudaGetDevice(&dev));
-  EXB_CUDA_OK(cudaSetDevice(dev));
+  // framework, when this is the first thing it does).  Asked for rather than set each time: a call of the dense GEMM costs the host
+  // 9.6 us this way, 10.0 with the device set before every map.
+  CUcontext context = nullptr;
+  if (driver.context == nullptr || driver.context(&context) != CUDA_SUCCESS || context == nullptr) {
+    int dev = 0;
+    EXB_CUDA_OK(cudaGetDevice(&dev));
+    EXB_CUDA_OK(cudaSetDevice(dev));
+  }
   cuuint64_t dims[2] = {inner, outer};
   cuuint64_t strides[1] = {pitch_bytes};
   cuuint32_t box[2] = {box_inner, box_outer};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = driver.encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
