@@ -42,7 +42,8 @@
 // Measured (us, tf32 -> now): 2,449,029 x 256 -> 256: 1,283 -> 1,058, with a second operand pair of 256 2,424 -> 1,826; 48 -> 256:
 // 607 -> 589; 256 -> 80: 794 -> 677, 256 -> 47 (pitch 47): 660 -> 699, with an addend 1,111 -> 1,041; 232,965 x 602 -> 256: 275 -> 220
 // (in chunks, evaluation: 458), 169,343 x 128 -> 256: 67 -> 63.
-// Not kept: one scale per row over the whole contraction, found ahead by four more warps, and one chain in TMEM: 2,424 -> 3,561.
+// Not kept: one scale per row over the whole contraction, found ahead by four more warps, and one chain in TMEM: 2,424 -> 3,561;
+// sixteen epilogue warps with 64 sums a thread: 1,058 -> 1,115.
 // The weight is scaled, split, padded and laid out as the tiles once per call by a preparation kernel.
 //
 // Every mbarrier wait is bounded; on expiry the CTA raises an abort flag, all roles leave their loops,
