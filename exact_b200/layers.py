@@ -189,9 +189,12 @@ class QReLUDropout(torch.nn.Module):
 
 
 def _watched(module):
-    """Whether a call of the module does more than its forward."""
+    """Whether a call of the module does anything but run the forward that its class has here: hooks, a forward replaced on the
+    instance or the class (offloading and profiling wrappers), a compiled call, a replaced Module.__call__ (tracers)."""
     return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
-                or torch.nn.modules.module._has_any_global_hook())
+                or torch.nn.modules.module._has_any_global_hook()
+                or getattr(module.forward, "__func__", None) is not _FORWARDS[type(module)]
+                or getattr(module, "_compiled_call_impl", None) is not None or type(module).__call__ is not _MODULE_CALL)
 
 
 def norm_act(norm, act, input):
@@ -199,9 +202,9 @@ def norm_act(norm, act, input):
     between, which nothing else reads; a module that is hooked or replaced is called by itself."""
     if norm is None:
         return act(input)
-    if (type(norm) is QBatchNorm1d and type(act) is QReLUDropout and act.training and norm.takes_activation(input)
-            and not _watched(norm) and not _watched(act)):
-        return norm.forward(input, act.p)
+    if (type(norm) is QBatchNorm1d and type(act) is QReLUDropout and not _watched(norm) and not _watched(act)
+            and act.training and norm.takes_activation(input)):
+        return norm._normalise(input, act.p)
     return act(norm(input))
 
 
@@ -231,13 +234,16 @@ class QBatchNorm1d(torch.nn.BatchNorm1d):
                 and (self.weight is None or self.weight.dtype == torch.float32))
 
     def takes_activation(self, input):
-        """Whether forward(input, dropout) can stand for the ReLU and dropout behind this module as well."""
+        """Whether the ReLU and dropout behind this module can run in its node."""
         return self.training and self._native_takes(input) and input.size(1) <= 4096
 
-    def forward(self, input, dropout=None):
-        """`dropout`: the probability of the ReLU + dropout to apply as well (only where takes_activation allows it)."""
+    def forward(self, input):
         if not self.training:
             return super().forward(input)
+        return self._normalise(input)
+
+    def _normalise(self, input, dropout=None):
+        """The training forward; `dropout`: the probability of the ReLU + dropout to apply as well, where takes_activation allows it."""
         self._check_input_dim(input)
         exponential_average_factor = 0.0 if self.momentum is None else self.momentum
         if self.training and self.track_running_stats and self.num_batches_tracked is not None:
@@ -261,6 +267,10 @@ class QBatchNorm1d(torch.nn.BatchNorm1d):
             self.running_mean if not self.training or self.track_running_stats else None,
             self.running_var if not self.training or self.track_running_stats else None,
             self.weight, self.bias, bn_training, exponential_average_factor, self.eps, self.scheme)
+
+
+_MODULE_CALL = torch.nn.Module.__call__
+_FORWARDS = {cls: cls.forward for cls in (QBatchNorm1d, QReLUDropout)}
 
 
 class QGCNConv(GCNConv):
