@@ -431,6 +431,13 @@ static int pack_common(const void* x, int dtype, long long N, long long D, long 
   if (!choose_pack_shape(N, D, D % 4 == 0 ? max_vec : D % 2 == 0 && max_vec >= 2 ? 2 : 1, dtype == EXACT_DTYPE_F32, &s))
     return fail(EXB_ERR_UNSUPPORTED, "pack: D=%lld is beyond the register-tiled kernels (max 4096 when D%%4==0, 2048 when D%%2==0, 1024 otherwise)", D);
   p.tpt = s.tpt;
+  // Single accesses of 16-bit rows: a run of odd rows that starts on a pair is read in pairs whose halves are known (ACC 1); rows
+  // that are pitched or start elsewhere in pairs too, whose halves depend on pitch and base (ACC 0).  80 M elements of bf16, INT2,
+  // us, element by element | so: 101 columns in rows of 104 321 | 118, 301 of 305 471 | 109, 600 of 605 265 | 101; the run's form
+  // takes 109 for 101 columns of 101, one form for both 111 and, at 47 columns, 158 instead of 123 (registers).
+  if (s.vec == 1 && eb == 2 && noise == nullptr &&
+      ((ldx & 1) == 0 || ldx != D || (reinterpret_cast<uintptr_t>(x) & 3) != 0))
+    s.vec = 0;
   if (dtype == kDtypeHalf) return launch_pack_bits<HalfBits>(p, bits, s, st);
   if (dtype == EXACT_DTYPE_F32) return launch_pack_bits<float>(p, bits, s, st);
   return launch_pack_bits<uint16_t>(p, bits, s, st);

@@ -51,7 +51,8 @@ struct HalfBits { uint16_t bits; };   // fp16 activations: the half arithmetic o
 // and 188, 47 182 and 137, 101 176 and 109, 601 135 and 103, 1,023 127 and 87; bf16 322 and 180, 183 and 128, 177 and 114, 160 and
 // 98, 185 and 80).
 // The elements are kept as loaded; 16-bit types stay packed in pairs: half the registers of the widened tile, and
-// their minimum and maximum are taken two at a time.  ACC: elements per access (4, 2 or 1, what the rows' alignment allows);
+// their minimum and maximum are taken two at a time.  ACC: elements per access (4, 2 or 1, what the rows' alignment allows; 0: one
+// element too, of 16-bit rows that are pitched or start off a pair, see load_unaligned_tile);
 // `have` of the four exist (always 4 with ACC == 4); the others repeat the first, by the address: with
 // a predicate on each access the loads of a tile waited for one another (30 columns 204 us, 47 columns 248).
 template <typename InT>
@@ -93,6 +94,20 @@ struct Raw {
       w[0] = __byte_perm(m[0], 0u, have > 1 ? 0x3210u : 0x1010u);
       w[1] = __byte_perm(m[1], 0u, have > 3 ? 0x3210u : 0x1010u);
     }
+  }
+  // The four elements at p, which need not start on a pair (odd: they start on the second half of one), from the pairs they lie in.
+  static __device__ __forceinline__ void load_around(const InT* p, int odd, int have, uint32_t (&m)[3]) {
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(p - odd);
+    const int last = (odd + (have > 0 ? have < 4 ? have : 4 : 1) - 1) >> 1;   // the pair of the last one that exists
+    m[0] = __ldcs(q);
+    m[1] = __ldcs(q + (last > 0 ? 1 : 0));
+    m[2] = __ldcs(q + last);
+  }
+  __device__ __forceinline__ void from_around(const uint32_t (&m)[3], int odd, int have) {
+    const uint32_t first = have == 1 ? 0x1010u : 0x3210u, second = have & 1 && have < 4 ? 0x1010u : 0x3210u;
+    const uint32_t first_odd = have == 1 ? 0x3232u : 0x5432u, second_odd = have >= 4 ? 0x5432u : have == 2 ? 0x1010u : 0x3232u;
+    w[0] = __byte_perm(m[0], m[1], odd ? first_odd : first);
+    w[1] = __byte_perm(m[1], m[2], odd ? second_odd : second);
   }
   __device__ __forceinline__ void clear() { w[0] = w[1] = 0u; }
   static __device__ __forceinline__ float low(uint32_t v) {
@@ -179,6 +194,22 @@ __device__ __forceinline__ void load_odd_tile(const InT* __restrict__ x, const T
     for (int r = 0; r < 8; r++) Raw<InT>::load_pairs(base + r * (unsigned)c.ldx, r, have[v], m[r]);
 #pragma unroll
     for (int r = 0; r < 8; r++) xv[r][v].from_pairs(m[r], r, have[v]);
+  }
+}
+// The same of 16-bit rows that start anywhere (of any pitch and base).  The pairs that hold a row's ends may reach one element past
+// either of them, so the tile has a row in front of it and one behind.
+template <typename InT, int V>
+__device__ __forceinline__ void load_unaligned_tile(const InT* __restrict__ x, const TileCtx& c, long long tile,
+                                                    const long long (&col)[V], const int (&have)[V], Raw<InT> (&xv)[8][V]) {
+  const int base_odd = (int)(reinterpret_cast<uintptr_t>(x) >> 1) & 1, pitch_odd = (int)(c.ldx & 1);
+#pragma unroll
+  for (int v = 0; v < V; v++) {
+    const InT* __restrict__ base = x + (tile << 3) * c.ldx + (have[v] > 0 ? col[v] : 0);
+    uint32_t m[8][3];
+#pragma unroll
+    for (int r = 0; r < 8; r++) Raw<InT>::load_around(base + r * (unsigned)c.ldx, (base_odd + r * pitch_odd) & 1, have[v], m[r]);
+#pragma unroll
+    for (int r = 0; r < 8; r++) xv[r][v].from_around(m[r], (base_odd + r * pitch_odd) & 1, have[v]);
   }
 }
 
@@ -569,7 +600,7 @@ quantize_pack_kernel(const __grid_constant__ PackParams p) {
   // find their lines on chip.
   const long long tile_bytes = 8 * p.D * (long long)sizeof(InT);
   const bool can_prefetch = p.ldx == p.D && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 && (tile_bytes & 15) == 0;
-  constexpr bool ODD16 = ACC == 1 && sizeof(InT) == 2;
+  constexpr bool ODD16 = ACC == 1 && sizeof(InT) == 2, UNALIGNED16 = ACC == 0;   // ODD16: one run that starts on a pair
   const bool fast = p.noise == nullptr &&
                     (!ODD16 || ((p.ldx & 1) != 0 && p.ldx == p.D && (reinterpret_cast<uintptr_t>(p.x) & 3) == 0));
   Raw<InT> xv[8][V];
@@ -584,8 +615,10 @@ quantize_pack_kernel(const __grid_constant__ PackParams p) {
                    : "memory");
     }
     bool done = false;
-    if (fast && tile - in_warp + last_in_warp < full_tiles) {
-      if constexpr (ODD16) load_odd_tile<InT, V>(x, c, tile, col, have, xv);
+    // an unaligned tile's neighbours: none in front of the first, none certain behind the last
+    if (fast && tile - in_warp + last_in_warp < (UNALIGNED16 ? num_tiles - 1 : full_tiles) && (!UNALIGNED16 || tile - in_warp > 0)) {
+      if constexpr (UNALIGNED16) load_unaligned_tile<InT, V>(x, c, tile, col, have, xv);
+      else if constexpr (ODD16) load_odd_tile<InT, V>(x, c, tile, col, have, xv);
       else load_tile<InT, ACC, V, true>(x, c, tile, col, have, xv);
       done = process_tile<InT, BITS, ACC, V, KIND, true>(p, c, tile, it, col, have, xv, s_part, s_fin);
       if (!done) ++it;  // the redo below exchanges its statistics through the other shared-memory buffer
@@ -637,6 +670,7 @@ static int launch_pack(const PackParams& p, const TileShape& s, cudaStream_t st)
   EXB_PACK_CASES(4) EXB_PACK_CASES(2) EXB_PACK_CASES(1)
   EXB_PACK_CASE(4, 4, TILE_MULTI)
   if constexpr (sizeof(InT) == 2) {
+    EXB_PACK_CASES(0)
     EXB_PACK_CASE(4, 5, TILE_WARP) EXB_PACK_CASE(2, 5, TILE_WARP)
   }
 #undef EXB_PACK_CASES

@@ -29,6 +29,22 @@ def test_quantize_pack_rows(N, D, ldx, at, bits):
         assert torch.equal(a.view(torch.int16), b.view(torch.int16))
 
 
+# odd rows of 16-bit values: pitched to an odd and an even number, off a pair, one tile to a warp and several warps to a tile
+@pytest.mark.parametrize("bits", [1, 2, 4, 8])
+@pytest.mark.parametrize("N,D,ldx,at", [(1003, 47, 48, 0), (2049, 101, 105, 1), (9477, 301, 304, 0), (77, 601, 605, 2), (66, 1023, 1024, 1),
+                                        (65, 100, 205, 1), (24, 1, 3, 1), (9, 5, 6, 0), (16, 7, 9, 1)])
+def test_quantize_pack_rows_bf16(N, D, ldx, at, bits):
+    x = torch.randn(N, ldx, device="cuda", generator=torch.Generator(device="cuda").manual_seed(N + D)).bfloat16()[:, at:at + D]
+    x[N // 2] = 1.5                                   # a constant row: its tile takes the general path
+    want = Q.quantize_pack(x.contiguous(), bits, seed=7, offset=3, row_offset=8)
+    got = [torch.zeros_like(t) for t in want[:3]]
+    got[0].copy_(want[0]).bitwise_not_()
+    _lib.invoke("exact_quantize_pack_rows", 0, _lib.ptr(x), 1, N, D, ldx, bits, 7, 3, 8, *(_lib.ptr(t) for t in got), _lib.stream_ptr())
+    assert torch.equal(got[0][:-1], want[0][:-1])
+    for a, b in zip(got[1:], want[1:]):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
 @pytest.mark.parametrize("N,D,ldx,k", [(1000, 602, 604, 76), (1537, 100, 104, 13), (300, 47, 49, 8), (4096, 128, 256, 32)])
 def test_projection_of_pitched_rows(N, D, ldx, k):
     x = _wide(N, D, ldx)
