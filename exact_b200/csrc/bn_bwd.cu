@@ -338,8 +338,9 @@ static int launch_bn_bwd(BnBwdParams p, cudaStream_t st) {
   p.ry = kBnThreads / p.cg;
   const long long units = wide && BITS == 1 ? 2 * p.groups : p.groups;
   // one grid with a mask and without: the order of the sums, and with it their last bits, does not depend on it
-  auto sized_for = wide ? bn_bwd8_kernel<BITS, APPLY, true> : bn_bwd_kernel<BITS, APPLY, true>;
-  const int grid = resident_blocks(sized_for, kBnThreads, (units + p.ry - 1) / p.ry);
+  const long long want = (units + p.ry - 1) / p.ry;
+  const int grid = wide ? resident_blocks<bn_bwd8_kernel<BITS, APPLY, true>>(kBnThreads, want)
+                        : resident_blocks<bn_bwd_kernel<BITS, APPLY, true>>(kBnThreads, want);
   kernel<<<grid, kBnThreads, 0, st>>>(p);
   return grid;
 }

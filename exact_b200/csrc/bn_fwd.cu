@@ -253,7 +253,7 @@ static int bn_statistics(BnFwdParams& p, cudaStream_t st, int* grid) {
   p.cg_total = p.D / 4;
   p.cg = p.cg_total < 64 ? p.cg_total : 64;
   p.ry = kBnFwdThreads / p.cg;
-  *grid = resident_blocks(bn_fwd_stats_kernel, kBnFwdThreads, (p.N + p.ry - 1) / p.ry);
+  *grid = resident_blocks<bn_fwd_stats_kernel>(kBnFwdThreads, (p.N + p.ry - 1) / p.ry);
   bn_fwd_stats_kernel<<<*grid, kBnFwdThreads, 0, st>>>(p);
   EXB_CUDA_OK(cudaGetLastError());
   bn_fwd_finish_kernel<<<(unsigned)((p.D + 31) / 32), dim3(32, kBnSlices), 0, st>>>(p, *grid);
@@ -286,7 +286,7 @@ int exact_bn_forward(const float* x, int64_t N, int64_t D, const float* weight, 
   int grid = 0;
   const int rc = bn_statistics(p, st, &grid);
   if (rc) return rc;
-  bn_fwd_apply_kernel<<<resident_blocks(bn_fwd_apply_kernel, kBnFwdThreads, (N + p.ry - 1) / p.ry), kBnFwdThreads, 0, st>>>(p);
+  bn_fwd_apply_kernel<<<resident_blocks<bn_fwd_apply_kernel>(kBnFwdThreads, (N + p.ry - 1) / p.ry), kBnFwdThreads, 0, st>>>(p);
   EXB_CUDA_OK(cudaGetLastError());
   return EXB_OK;
 }
@@ -301,7 +301,7 @@ int exact_bn_act_forward(const float* x, int64_t N, int64_t D, const float* weig
   long long period = D;                       // D / gcd(D, 256) runs of 256 elements later a lane is at the same columns
   for (int i = 0; i < 8 && period % 2 == 0; i++) period /= 2;
   const long long nchunks = (N * D + 255) / 256;
-  long long warps = 16LL * resident_blocks(bn_act_apply_kernel, 256, 1LL << 40);   // two rounds of blocks: 69 us with one, 67, 69 with four
+  long long warps = 16LL * resident_blocks<bn_act_apply_kernel>(256, 1LL << 40);   // two rounds of blocks: 69 us with one, 67, 69 with four
   if (warps > (nchunks + period) / period * period) warps = (nchunks + period) / period * period;
   if (D % 4 != 0 || D > (1 << 20) || period > warps)
     return fail(EXB_ERR_UNSUPPORTED, "bn_act_forward: no kernel for D = %lld", (long long)D);

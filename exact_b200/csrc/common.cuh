@@ -1,5 +1,6 @@
 // Shared device helpers of the exact_b200 CUDA library (sm_100a only).
 #pragma once
+#include <atomic>
 #include <cmath>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -71,13 +72,27 @@ inline PhiloxKey make_philox_key(uint64_t seed) {
 }
 
 #ifdef __CUDACC__
+// Blocks of a kernel without dynamic shared memory that fit on an SM of the current device, at least one.  A property of the
+// compiled kernel, so the latest answer is kept per kernel, with its device and block size in the same word, which any thread may
+// replace.
+template <auto KERNEL>
+inline int blocks_per_sm(int threads) {
+  static std::atomic<uint64_t> latest{0};
+  int dev = 0, blocks = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  const uint64_t key = (uint64_t)(uint32_t)(dev + 1) << 32 | (uint64_t)(uint32_t)threads << 16;
+  const uint64_t kept = latest.load(std::memory_order_relaxed);
+  if ((kept & ~(uint64_t)0xffff) == key) return (int)(kept & 0xffff);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, KERNEL, threads, 0) != cudaSuccess || blocks < 1) return 1;
+  latest.store(key | (uint64_t)blocks, std::memory_order_relaxed);
+  return blocks;
+}
 // Blocks of a kernel whose blocks walk over the data: as many as are resident at once, or fewer when there is less to do.  With
 // more, the last round of blocks leaves SMs idle (at 40 registers six blocks of 256 threads fit; eight per SM took two rounds, the
 // second a third full).
-template <typename K>
-inline int resident_blocks(K kernel, int threads, long long want) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
+template <auto KERNEL>
+inline int resident_blocks(int threads, long long want) {
+  int per_sm = blocks_per_sm<KERNEL>(threads);
   if (per_sm > 8) per_sm = 8;      // what the workspaces of partial sums are sized for
   const long long most = (long long)sm_count() * per_sm;
   return (int)(want < 1 ? 1 : want < most ? want : most);

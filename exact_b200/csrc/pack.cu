@@ -455,13 +455,10 @@ static int launch_unpack(const UnpackParams& p, const TileShape& s, cudaStream_t
   const long long tiles = (p.N + 7) / 8;
   const int tiles_per_cta = s.block / s.tpt;
   const long long ctas = (tiles + tiles_per_cta - 1) / tiles_per_cta;
-  int grid = 1;
 #define EXB_UNPACK_CASE(VEC_, V_)                                                      \
   if (s.vec == VEC_ && s.v == V_) {                                                    \
-    auto k = unpack_dequant_kernel<BITS, VEC_, V_, STATS>;                                \
-    int rc = persistent_grid(k, s.block, ctas, &grid);                                 \
-    if (rc) return rc;                                                                 \
-    k<<<grid, s.block, 0, st>>>(p);                                                    \
+    constexpr auto k = unpack_dequant_kernel<BITS, VEC_, V_, STATS>;                   \
+    k<<<persistent_grid<k>(s.block, ctas), s.block, 0, st>>>(p);                       \
     EXB_CUDA_OK(cudaGetLastError());                                                   \
     return EXB_OK;                                                                     \
   }

@@ -636,16 +636,10 @@ struct TileShape {
   int vec, v, tpt, block;
 };
 
-template <typename K>
-static int persistent_grid(K kernel, int block, long long work_ctas, int* grid) {
-  int per_sm = 0;
-  EXB_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0));
-  if (per_sm < 1) per_sm = 1;
-  long long g = (long long)sm_count() * per_sm;
-  if (g > work_ctas) g = work_ctas;
-  if (g < 1) g = 1;
-  *grid = (int)g;
-  return EXB_OK;
+template <auto KERNEL>
+static int persistent_grid(int block, long long work_ctas) {
+  const long long most = (long long)sm_count() * blocks_per_sm<KERNEL>(block);
+  return (int)(work_ctas < 1 ? 1 : work_ctas < most ? work_ctas : most);
 }
 
 template <typename InT, int BITS>
@@ -653,14 +647,11 @@ static int launch_pack(const PackParams& p, const TileShape& s, cudaStream_t st)
   const long long tiles = (p.N + 7) / 8;
   const int tiles_per_cta = s.block / s.tpt;
   const long long ctas = (tiles + tiles_per_cta - 1) / tiles_per_cta;
-  int grid = 1;
   const int kind = s.tpt < 32 ? TILE_SUB : s.tpt == 32 ? TILE_WARP : s.tpt == 64 ? TILE_PAIR : TILE_MULTI;
 #define EXB_PACK_CASE(ACC_, V_, KIND_)                                                 \
   if (s.vec == ACC_ && s.v == V_ && kind == KIND_) {                                   \
-    auto k = quantize_pack_kernel<InT, BITS, ACC_, V_, KIND_>;                         \
-    int rc = persistent_grid(k, s.block, ctas, &grid);                                 \
-    if (rc) return rc;                                                                 \
-    k<<<grid, s.block, 0, st>>>(p);                                                    \
+    constexpr auto k = quantize_pack_kernel<InT, BITS, ACC_, V_, KIND_>;               \
+    k<<<persistent_grid<k>(s.block, ctas), s.block, 0, st>>>(p);                       \
     EXB_CUDA_OK(cudaGetLastError());                                                   \
     return EXB_OK;                                                                     \
   }

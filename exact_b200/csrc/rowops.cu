@@ -200,7 +200,9 @@ static int rows_pass(const float* g, int64_t n, int64_t K, int64_t ldg, const fl
     if (pieces == 0) return EXB_OK;
     const bool pairs = (reinterpret_cast<uintptr_t>(g) & 7) == 0 && ldg % 2 == 0;
     auto kernel = pairs ? pad_rows_kernel<true> : pad_rows_kernel<false>;
-    const int blocks = resident_blocks(kernel, kRowOpsThreads, (pieces + 4 * kRowOpsThreads - 1) / (4 * kRowOpsThreads));
+    const long long want = (pieces + 4 * kRowOpsThreads - 1) / (4 * kRowOpsThreads);
+    const int blocks = pairs ? resident_blocks<pad_rows_kernel<true>>(kRowOpsThreads, want)
+                             : resident_blocks<pad_rows_kernel<false>>(kRowOpsThreads, want);
     kernel<<<blocks, kRowOpsThreads, 0, st>>>(g, rowscale, static_cast<float*>(out), pieces, (int)K, ldg, (int)(Kout / 4));
     EXB_CUDA_OK(cudaGetLastError());
     return EXB_OK;

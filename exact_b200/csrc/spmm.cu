@@ -911,7 +911,7 @@ static int launch_weighted_bw(const WeightedBwParams& p, cudaStream_t st) {
   const int nc = (int)((p.s.K + 31) / 32);
 #define EXB_WBW(NC_)                                                                                                       \
   case NC_: {                                                                                                              \
-    const int grid = resident_blocks(spmm_weighted_bw_kernel<IdxT, NC_>, kRowWarps * 32, (p.s.n_items + p.s.M + kRowWarps - 1) / kRowWarps); \
+    const int grid = resident_blocks<spmm_weighted_bw_kernel<IdxT, NC_>>(kRowWarps * 32, (p.s.n_items + p.s.M + kRowWarps - 1) / kRowWarps); \
     spmm_weighted_bw_kernel<IdxT, NC_><<<grid, kRowWarps * 32, 0, st>>>(p);                                                \
     break;                                                                                                                 \
   }
