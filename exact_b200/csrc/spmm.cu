@@ -906,6 +906,13 @@ __global__ void __launch_bounds__(kRowWarps * 32, NC <= 4 ? 3 : 2) spmm_weighted
   }
 }
 
+// No columns: the dots are empty sums.
+template <typename IdxT>
+__global__ void __launch_bounds__(256) zero_edge_values_kernel(const IdxT* __restrict__ rowptr, long long M, float* __restrict__ out) {
+  const long long nnz = (long long)rowptr[M];
+  for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < nnz; e += (long long)gridDim.x * 256) out[e] = 0.f;
+}
+
 template <typename IdxT>
 static int launch_weighted_bw(const WeightedBwParams& p, cudaStream_t st) {
   const int nc = (int)((p.s.K + 31) / 32);
@@ -1193,7 +1200,14 @@ int exact_spmm_weighted_backward(const void* t_rowptr, const void* t_col, const 
   EXB_REQUIRE(idx_bytes == 4 || idx_bytes == 8, "spmm_weighted_backward: idx_bytes must be 4 or 8 (got %d)", idx_bytes);
   EXB_REQUIRE(M >= 0 && K >= 0 && n_items >= 0 && n_long >= 0, "spmm_weighted_backward: negative size");
   if (K > 256) return fail(EXB_ERR_UNSUPPORTED, "spmm_weighted_backward: more than 256 columns");
-  if (M == 0 || K == 0) return EXB_OK;
+  if (M == 0) return EXB_OK;
+  if (K == 0) {
+    EXB_REQUIRE(t_rowptr && grad_value, "spmm_weighted_backward: null pointer");
+    if (idx_bytes == 4) zero_edge_values_kernel<<<sm_count(), 256, 0, (cudaStream_t)stream>>>(static_cast<const int32_t*>(t_rowptr), M, grad_value);
+    else zero_edge_values_kernel<<<sm_count(), 256, 0, (cudaStream_t)stream>>>(static_cast<const int64_t*>(t_rowptr), M, grad_value);
+    EXB_CUDA_OK(cudaGetLastError());
+    return EXB_OK;
+  }
   EXB_REQUIRE(M < (1LL << 32) && n_items <= 2147483647LL && n_long <= 2147483647LL, "spmm_weighted_backward: too many rows");
   EXB_REQUIRE(t_rowptr && t_col && t_value && perm && mat && grad && grad_mat && grad_value, "spmm_weighted_backward: null pointer");
   if (n_items > 0)

@@ -215,7 +215,8 @@ EXACT_API int exact_spmm_value_bw(const void* row, const void* rowptr, const voi
  * structure: t_rowptr [M + 1], t_col, t_value (with a mean's 1 / row length in it) and perm [nnz], the forward position of the
  * transpose's edges, idx_bytes wide like the rest; fw_rowptr: the forward rows for a mean, NULL for a sum; mat [M, K] the operand,
  * grad the output's gradient; plan arrays and scratch [n_items, K] of the transpose as in exact_spmm_planned.  grad_mat [M, K] and
- * grad_value [nnz] (every edge of the transpose writes its own) have the values of the separate calls.  K <= 256, else code 3. */
+ * grad_value [nnz] (every edge of the transpose writes its own; zeros with K = 0) have the values of the separate calls.  K <= 256,
+ * else code 3. */
 EXACT_API int exact_spmm_weighted_backward(const void* t_rowptr, const void* t_col, const float* t_value, const void* perm,
                                            const void* fw_rowptr, int idx_bytes, const float* mat, const float* grad, int64_t M,
                                            int64_t K, int64_t long_threshold, const int32_t* item_row, const int64_t* item_begin,

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import oracle
-from exact_b200 import SparseTensor, config, qmatmul
+from exact_b200 import SparseTensor, _lib, config, qmatmul
 from helpers import normal
 
 pytestmark = pytest.mark.gpu
@@ -75,3 +75,24 @@ def test_one_gradient_at_a_time_takes_the_separate_kernels():
 
     both, only_x, only_v = grads(True, True), grads(True, False), grads(False, True)
     assert torch.equal(both[0], only_x[0]) and torch.equal(both[1], only_v[1])
+
+
+@pytest.mark.parametrize("idx", [torch.int32, torch.int64])
+def test_no_columns_give_zero_gradients_of_the_values(idx):
+    rowptr = torch.tensor([0, 2, 2, 5], dtype=idx, device="cuda")
+    col, perm = torch.tensor([0, 1, 1, 2, 3], dtype=idx, device="cuda"), torch.tensor([3, 0, 1, 4, 2], dtype=idx, device="cuda")
+    val, out = torch.ones(5, device="cuda"), torch.full((6,), 7.0, device="cuda")
+    p = _lib.ptr
+    _lib.invoke("exact_spmm_weighted_backward", 0, p(rowptr), p(col), p(val), p(perm), None, rowptr.element_size(), None, None, 3, 0, 0,
+                None, None, None, None, 0, None, None, 0, None, None, None, p(out), _lib.stream_ptr())
+    assert out.tolist() == [0, 0, 0, 0, 0, 7]
+    n = 500
+    poison = torch.full((3 * n,), float("nan"), device="cuda")   # what the allocator hands out next
+    v = torch.rand(3 * n, device="cuda").requires_grad_()
+    row = torch.arange(3 * n, device="cuda") // 3
+    adj = SparseTensor(row=row, col=(row * 7 + torch.arange(3 * n, device="cuda")) % n, value=v, sparse_sizes=(n, n))
+    x = torch.empty(n, 0, device="cuda").requires_grad_()
+    y = qmatmul(adj, x, "sum")
+    del poison
+    y.backward(torch.empty_like(y))
+    assert not bool(v.grad.any()) and x.grad.shape == x.shape
