@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import oracle
-from exact_b200 import SparseTensor, _lib, config, qmatmul
+from exact_b200 import SparseTensor, _lib, config, dequantize_activation, qmatmul, quantize_activation
 from helpers import normal
 
 pytestmark = pytest.mark.gpu
@@ -19,7 +19,94 @@ def hub_graph(n, seed):
     return key // n, key % n
 
 
+def calls_of(run):
+    """Library calls of run() by name."""
+    native = _lib.native()
+    native.set_timing(True)
+    try:
+        run()
+        return [c[0] for c in native.take_calls()]
+    finally:
+        native.set_timing(False)
+
+
+def graph_of(row, col, val, shape, idx):
+    t = torch.from_numpy
+    v = t(val).cuda().requires_grad_()
+    adj = SparseTensor(row=t(row).cuda(), col=t(col).cuda(), value=v, sparse_sizes=shape, is_sorted=True)
+    adj.fill_cache_()
+    return v, adj.to_int32_() if idx == torch.int32 else adj
+
+
+def check_both_gradients(row, col, shape, K, reduce, idx, g):
+    """Against the oracle's gradients from the operand as it is saved (8 bits); g: numpy, or a torch tensor on the GPU."""
+    n_rows, n_cols = shape
+    rowptr, colptr = np.zeros(n_rows + 1, np.int64), np.zeros(n_cols + 1, np.int64)
+    np.cumsum(np.bincount(row, minlength=n_rows), out=rowptr[1:])
+    np.cumsum(np.bincount(col, minlength=n_cols), out=colptr[1:])
+    val = np.random.default_rng(1).standard_normal(col.size).astype(np.float32)
+    v, adj = graph_of(row, col, val, shape, idx)
+    x = torch.from_numpy(normal(n_cols, K, 6)).cuda().requires_grad_()
+    config.compress_activation, config.kept_frac = True, 1.0
+    saved, config.activation_compression_bits = config.activation_compression_bits, [8]
+    try:
+        config.manual_seed(4)
+        q = quantize_activation(x.detach(), None)
+        mat = dequantize_activation(q, tuple(x.shape)).cpu().numpy()
+        config.manual_seed(4)
+        names = calls_of(lambda: qmatmul(adj, x, reduce).backward(g if isinstance(g, torch.Tensor) else torch.from_numpy(g).cuda()))
+    finally:
+        config.activation_compression_bits = saved
+    assert ("exact_spmm_weighted_backward" in names) == (K <= 256) and ("exact_spmm_value_bw" in names) == (K > 256)
+    g = g.cpu().numpy() if isinstance(g, torch.Tensor) else g
+    assert np.array_equal(v.grad.cpu().numpy(), oracle.spmm_value_bw(rowptr, col, mat, g, reduce), equal_nan=True)
+    perm = np.argsort(col * n_rows + row, kind="stable")
+    w = val[perm]
+    if reduce == "mean":
+        w = w / np.maximum(np.diff(rowptr), 1)[row[perm]].astype(np.float32)
+    ref = oracle.spmm(colptr, row[perm], w, g, "sum")
+    got, long = x.grad.cpu().numpy(), np.diff(colptr) > int(config.spmm_long_row)
+    assert np.array_equal(got[~long], ref[~long], equal_nan=True)
+    # long rows are summed in pieces of 256 edges: two orders of n fp32 multiply-adds, each within n * 2^-24 of the sum of magnitudes
+    size = oracle.spmm(colptr, row[perm], np.abs(w), np.abs(np.nan_to_num(g, posinf=0)), "sum")[long]
+    ok = np.isfinite(ref[long])
+    assert (np.abs(got[long] - ref[long])[ok] <= (2 * np.diff(colptr)[long, None] * 2.0 ** -24 * size)[ok]).all()
+    return long.any()
+
+
 # columns: every number of 32-column groups with and without a remainder, and one width beyond the kernel's range
+@pytest.mark.parametrize("idx", [torch.int32, torch.int64])
+@pytest.mark.parametrize("K", [1, 31, 32, 33, 64, 100, 128, 160, 192, 200, 224, 250, 256, 260])
+@pytest.mark.parametrize("reduce", ["sum", "mean"])
+def test_both_gradients_in_one_walk(K, reduce, idx):
+    n = 2000
+    row, col = hub_graph(n, K)
+    g = normal(n, K, 7)
+    if K > 1:
+        g[5, K - 1] = np.inf                   # stays in its row's edges and its column
+    assert check_both_gradients(row, col, (n, n), K, reduce, idx, g)
+
+
+# adjacencies that are not square, with empty rows and columns, and gradients that are transposed, sliced or expanded
+@pytest.mark.parametrize("shape", [(2000, 700), (700, 2000), (2000, 2000)])
+@pytest.mark.parametrize("K,layout", [(40, "transposed"), (97, "sliced"), (128, "expanded"), (5, "transposed")])
+@pytest.mark.parametrize("reduce", ["sum", "mean"])
+def test_rectangular_and_strided(shape, K, layout, reduce):
+    row, col = hub_graph(2000, K)
+    keep = (row < shape[0]) & (col < shape[1])
+    row, col = row[keep], col[keep]
+    base = torch.from_numpy(normal(shape[0], K, 7)).cuda()
+    if layout == "transposed":
+        g = base.t().contiguous().t()
+    elif layout == "sliced":
+        g = torch.cat([base, base], 1)[:, 3:3 + K]
+    else:
+        g = base[0].expand(shape[0], K)
+    assert not g.is_contiguous()
+    check_both_gradients(row, col, shape, K, reduce, torch.int64, g)
+
+
+# nothing saved compressed: the Python nodes and their separate kernels
 @pytest.mark.parametrize("idx", [torch.int32, torch.int64])
 @pytest.mark.parametrize("K", [1, 31, 32, 33, 64, 100, 128, 160, 192, 200, 224, 250, 256, 260])
 @pytest.mark.parametrize("reduce", ["sum", "mean"])
