@@ -389,6 +389,28 @@ struct AggregateState : torch::CustomClassHolder {
   bool keep_x;
 };
 
+// Whether both gradients of a weighted sum or mean come from one walk (exact_spmm_weighted_backward, up to 256 columns).  It gives
+// a row of the transpose a warp, of which few columns use few lanes, where the separate kernels take several short rows, or 32
+// edges, a warp.  So many rows of few edges and columns stay with those: below (56 - columns) / 5 edges a row, from 65,536 rows on
+// (one to three columns, whose rows are no whole 16-byte pieces: from 2^20).  With long rows, whose pieces the separate kernels wait
+// for twice, from 2^18 rows on, and up to 2^20 at half as many edges.  Both gradients, one walk over separate, random graphs of
+// 3 | 7 | 11 | 21 edges a row:
+//     columns      4                          16                         24                    32                    64
+//     40,000       1.09 | 0.96 | 0.79         1.00 | 0.94 | 0.79         0.97 | 0.92 | 0.79    0.94 | 0.93 | 0.86    0.88 | 0.89 | 0.80
+//     170,000      1.58 | 1.16 | 0.96 | 0.75  1.50 | 1.09 | 0.93 | 0.74  1.21 | 0.99 | 0.86    1.14 | 0.94 | 0.82    0.95 | 0.88 | 0.80
+//     500,000      1.86 | 1.26 | 1.00 | 0.77  1.49 | 1.18 | 0.98 | 0.81  1.32 | 1.08 | 0.93    1.19 | 0.97 | 0.85    1.01 | 0.84 | 0.75
+//     2,000,000    2.12 | 1.43                1.55 | 1.10                1.33 | 1.01           1.25 | 0.97           1.04 | 0.86
+//     power-law graphs: 170,000 at most 0.98 anywhere, 500,000 with 4 and 16 columns 1.29 | 1.05 | 0.92 and 1.09 | 0.89 | 0.85,
+//     2,000,000 of 3 | 7 edges 1.98 | 1.33 and 1.45 | 1.08.
+// What the lines leave: 1.22 for two columns of 500,000 x 7, 1.13 at worst elsewhere.
+bool one_walk(const Graph& g, int64_t K, int64_t nnz) {
+  if (K > 256 || nnz == 0) return false;
+  const int64_t M = g.bw.rowptr.size(0) - 1;
+  if (M < (1 << 16) || 5 * nnz >= (56 - K) * M) return true;
+  if (g.bw.plan->pieces(g.bw.rowptr, g.bw.col).n * 4096 > M && M < (1 << 20)) return M < (1 << 18) || K < 4 || 10 * nnz >= (56 - K) * M;
+  return K < 4 && M < (1 << 20);
+}
+
 struct AggregateNode : Function<AggregateNode> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x_, const OptTensor& value, const c10::intrusive_ptr<AggregateState>& s) {
     const Graph& g = *s->graph;
@@ -418,7 +440,7 @@ struct AggregateNode : Function<AggregateNode> {
       x = unpack(s->x.q.codes, s->how.bits, s->x.q.scale, s->x.q.mn, s->rows, s->x.width);
       if (s->x.R.defined()) x = linear_supported(x) ? linear(x, s->x.R, {}, {}, {}, {}, false) : at::matmul(x, s->x.R.t());
     }
-    if (s->reduce <= 1 && need_v && need_x && s->perm && gr.bw.value && g.size(1) <= 256 && gr.fw.col.size(0) > 0) {
+    if (s->reduce <= 1 && need_v && need_x && s->perm && gr.bw.value && one_walk(gr, g.size(1), gr.fw.col.size(0))) {
       OptTensor rows;
       if (s->reduce == 1) rows = gr.fw.rowptr;
       std::tie(gx, gv) = spmm_weighted_backward(gr.bw, *s->perm, rows, x, g);

@@ -183,3 +183,33 @@ def test_no_columns_give_zero_gradients_of_the_values(idx):
     del poison
     y.backward(torch.empty_like(y))
     assert not bool(v.grad.any()) and x.grad.shape == x.shape
+
+
+def short_rows(n, per_row, hubs, seed):
+    """n rows of per_row edges each way (a few less: duplicates), and `hubs` columns of 300 edges."""
+    rng = np.random.default_rng(seed)
+    r = np.concatenate([np.tile(np.arange(n), per_row), rng.integers(0, n, 300 * hubs)])
+    c = np.concatenate([np.concatenate([rng.permutation(n) for _ in range(per_row)]), np.repeat(rng.integers(0, n, hubs), 300)])
+    key = np.unique(r * n + c)
+    return key // n, key % n
+
+
+# either side of every line of the rule, and the same bits on both
+@pytest.mark.parametrize("n,per_row,hubs,K,joint", [(65536, 3, 0, 16, False), (65535, 3, 0, 16, True), (70000, 3, 0, 64, True), (70000, 9, 0, 16, True),
+                                                    (70000, 3, 0, 3, True), (70000, 3, 30, 16, True), (70000, 3, 8, 16, False),
+                                                    (1 << 20, 2, 0, 3, False), (1 << 18, 3, 40, 8, False), (1 << 18, 6, 40, 8, True)])
+def test_short_narrow_rows_keep_the_separate_kernels(n, per_row, hubs, K, joint):
+    row, col = short_rows(n, per_row, hubs, K)
+    val = np.random.default_rng(1).random(col.size, dtype=np.float32)
+    g, mat = torch.from_numpy(normal(n, K, 7)).cuda(), torch.from_numpy(normal(n, K, 6)).cuda()
+    config.compress_activation = True
+    grads = []
+    for x_rg, v_rg in ((True, True), (True, False), (False, True)):
+        v, adj = graph_of(row, col, val, (n, n), torch.int64)
+        v.requires_grad_(v_rg)
+        x = mat.clone().requires_grad_(x_rg)
+        config.manual_seed(2)
+        names = calls_of(lambda: qmatmul(adj, x, "sum").backward(g))
+        assert ("exact_spmm_weighted_backward" in names) == (joint and x_rg and v_rg)
+        grads.append((x.grad, v.grad))
+    assert torch.equal(grads[0][0], grads[1][0]) and torch.equal(grads[0][1], grads[2][1])
