@@ -16,9 +16,15 @@
 // fp32 accumulator, at the size of what is there already.  The K tile's sum is read back, gets its average loss (2^-23) and its
 // scales back, and is added to the others in fp32 registers.  Against fp64 (Frobenius; M = 100,000 rows of the layers' operands):
 // 1.04e-7 .. 1.2e-7 at 33 to 602 columns.  tf32 heads and tails in one chain, 3e-7 .. 4.4e-6; in
-// chains of 64 columns, the former kernel of evaluation, 1.04e-7 .. 1.39e-7; the library's fp32 GEMM 9e-8 (48) .. 4.4e-7 (602).  The
-// tail of an element is exact to 2^-39 of its row's largest one in the K tile.  Non-finite inputs stay non-finite and confined to
-// their rows, but an infinite element turns its output row into NaN where an fp32 GEMM gives +-inf (its tail is inf - inf).
+// chains of 64 columns, the former kernel of evaluation, 1.04e-7 .. 1.39e-7; the library's fp32 GEMM 9e-8 (48) .. 4.4e-7 (602).
+// Elements that share a power of two share its range: below 2^-17 of the largest one an element has fewer than those 22 bits, and
+// beside one of 2^39 times its size none.  A tile of A in which that is more than a rare element (kLinLost), or that has rows from 2^96
+// on, whose sums could overflow under B's scale, is therefore done again from its fp32 values in tf32 (kind::tf32, heads and tails of 11
+// bits each with an exponent of their own, K tiles of 32 columns), and a weight of which it is true makes all tiles tf32:
+// 1.1e-7 .. 1.35e-7 whatever the range.  The first way's result of such a tile is not stored.  2,449,029 x 256 -> 256, plain 1,170 -
+// 1,230 us (the look for such elements is 20 - 30 of them), all tiles twice 2,550, wide weight 2,070; 169,343 x 256 -> 256: 93, 189, 140.
+// Non-finite inputs stay non-finite and confined to their rows, but an infinite element turns its output row into NaN where an fp32
+// GEMM gives +-inf (its tail is inf - inf).
 //
 // Structure (one CTA per SM, persistent over 128-row tiles of A, 20 warps).  Two CTAs of a cluster work as a pair on two
 // neighbouring tiles (tcgen05.mma.cta_group::2, M = 256): each holds its rows of A and half of the rows of B, so a CTA fetches and
@@ -33,7 +39,7 @@
 //   warps 4-11 converters: find a row's largest magnitude in the K tile (four lanes own it), scale, split, write the heads and
 //              tails in place, fence.proxy.async, signal.  Two groups of four take alternate K tiles: a K tile is a chain of
 //              wait, reads, conversions, stores, fence and arrival.  The first warp of a group also waits for B, so that the
-//              issuing thread has one wait per K tile.
+//              issuing thread has one wait per K tile.  They also look for elements that fp16 cannot hold.
 //   warps 12-19 epilogue: add every K tile up, 128 sums a thread (registers moved to them by setmaxnreg); then the scales of the
 //              columns and the bias, a staging tile per warp and a TMA store of 32 x 32 boxes: with plain stores from the
 //              staging tiles the write-out was what narrow operands were bound by (2,449,029 x 48 -> 256: 904 us, boxes 589).
@@ -44,7 +50,8 @@
 // (in chunks, evaluation: 458), 169,343 x 128 -> 256: 67 -> 63.
 // Not kept: one scale per row over the whole contraction, found ahead by four more warps, and one chain in TMEM: 2,424 -> 3,561;
 // sixteen epilogue warps with 64 sums a thread: 1,058 -> 1,115.
-// The weight is scaled, split, padded and laid out as the tiles once per call by a preparation kernel.
+// The weight is scaled, split, padded and laid out as the tiles (both ways) once per call by a preparation kernel; the product's CTAs
+// start while it runs and wait for it once they are set up (4,096 x 128 -> 64: 17.4 us one after the other, 15.4 so).
 //
 // Every mbarrier wait is bounded; on expiry the CTA raises an abort flag, all roles leave their loops,
 // bulk copies in flight are waited for (bounded), TMEM is freed and the status word is set.
@@ -75,21 +82,34 @@ constexpr float kLinGain = 1.00000011920929f;   // 1 + 2^-23: gives back what a 
 constexpr int kLinPrefetch = 2;                 // K tiles of A requested into L2 ahead of their TMA load
 constexpr int kLinScales = 8;                   // K tiles whose row scales are kept
 constexpr int kLinHeadExp = 14;                 // the largest element of a row of a K tile is scaled to [2^14, 2^15)
+// Tiles whose elements fp16 cannot hold are done again in tf32 (kind::tf32, K = 8): a K tile is 32 columns, 128 bytes as well.
+constexpr int kLinWideK = 32;
+constexpr int kLinWideExp = -8;                 // there the row's largest goes to [2^-8, 2^-7): no product with an fp32 number overflows
+// What makes a tile wide: so many hits.  Of the 128 pieces of 16 columns of a row in a K tile's 32 rows: those with an element with lost
+// bits, looking at half of a piece's columns, in eight rows at one and in eight rows at the other half.  (Normally
+// distributed values: 0.015 hits; a column that is small beside the others: 16; a row in which most are small beside one: 4.)  Of a
+// row of B: elements with lost bits.  And a row of either whose largest is 2^96 or more: sums, which carry B's scale, could overflow.
+constexpr int kLinLost = 3;
+constexpr int kLinFlagWords = 32;               // tiles of a CTA in a launch: one bit each
 
 constexpr int kLinMaxCols = 256;                // of a launch
 
 struct LinParams {
   const __half* b;         // heads and tails of the weight, as linear_prepare_kernel lays them out
+  const float* b_wide;     // the same in tf32, not scaled
   const float* col_inv;   // [Npad] what the columns were scaled by, inverted
+  const float* unit;       // [Npad] ones: the same for tf32
+  const int* b_lost;       // [Npad] elements of a row of B with lost bits
   float* C;
-  const float* bias;
   const float* bias_pad;   // [Npad], with zeros behind, or null
   int* status;
   int* lib_status;    // library-wide status word of this device (capi.cu), or null
   long long M, ldc;
   int N, Npad;
   int kblocks1, kblocks;   // K tiles of the first operand pair, and of both pairs together
+  int wide_kblocks1, wide_kblocks;   // the same in tf32
   int num_tiles;
+  int after_prepare;       // this launch started while the preparation was running
   int bulk_out;            // C is stored by TMA: rows on 16-byte boundaries and nothing to add
   const float* addend;     // [M, ldadd] added to the product (C itself: C += ...), or null
   long long ldadd;
@@ -99,23 +119,34 @@ struct LinParams {
   unsigned tmem_cols;
 };
 
-// The exponent (biased) of the power of two that brings a largest magnitude (its bits) to [2^14, 2^15); of 1 for zero and for inf
-// and NaN, which stay what they are.
+// The exponent (biased) of the power of two that brings a largest magnitude (its bits) to [2^HEAD, 2^(HEAD + 1)), between 2^-120 and
+// 2^120; of 1 for zero.  (Under an infinite one any will do: its NaN tail makes the result NaN.)
+template <int HEAD>
 __device__ __forceinline__ uint32_t lin_scale_exp(uint32_t magnitude) {
   const int e = (int)(magnitude >> 23);
-  if (magnitude == 0 || e == 255) return 127u;
-  const int up = kLinHeadExp + 127 - e;
-  return (uint32_t)((up > 120 ? 120 : up) + 127);
+  if (magnitude == 0) return 127u;
+  const int up = e == 255 ? 120 : min(HEAD + 127 - e, 120);
+  return (uint32_t)((HEAD < 7 ? max(up, -120) : up) + 127);
 }
+// An fp16 head and tail hold fewer than 22 bits of a scaled element other than zero when it is below 2^-3, 2^-17 of the largest one
+// that shares the scale.  In this form zero is the largest number and the sign drops out.
+constexpr uint32_t kLinLostBelow = 2u * 0x3e000000u - 1u;
+__device__ __forceinline__ uint32_t lin_twice_minus_one(float x) { return 2u * __float_as_uint(x) - 1u; }
+// Whether the largest magnitude that was brought to [2^14, 2^15) by this is 2^96 or more.
+__device__ __forceinline__ bool lin_huge(uint32_t exponent) { return exponent <= 127u + kLinHeadExp - 96u; }
 __device__ __forceinline__ float lin_scale(uint32_t exponent) { return __uint_as_float(exponent << 23); }
 __device__ __forceinline__ float lin_inverse(uint32_t exponent) { return __uint_as_float((254u - exponent) << 23); }
-// Four scaled elements -> heads and tails, two to a word.  A non-finite element has a NaN tail (inf - inf), so its output row is NaN.
-__device__ __forceinline__ void split_f16(const float (&a)[4], f32x2 scale, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
+// Four scaled elements -> heads and tails, two to a word, and the lesser lin_twice_minus_one of the first and the last (ODD: of the
+// two between).  A non-finite element has a NaN tail (inf - inf), so its output row is NaN.
+template <bool ODD>
+__device__ __forceinline__ uint32_t split_f16(const float (&a)[4], f32x2 scale, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
+  uint32_t least[2];
 #pragma unroll
   for (int e = 0; e < 2; e++) {
     const f32x2 x = f2_mul(f2_pack(a[2 * e], a[2 * e + 1]), scale);
     float x0, x1;
     f2_unpack(x, x0, x1);
+    least[e] = lin_twice_minus_one((e != 0) != ODD ? x1 : x0);
     const __half2 h = __floats2half2_rn(x0, x1);
     const float2 back = __half22float2(h);
     f2_unpack(f2_sub(x, f2_pack(back.x, back.y)), x0, x1);
@@ -123,6 +154,12 @@ __device__ __forceinline__ void split_f16(const float (&a)[4], f32x2 scale, uint
     hi[e] = *reinterpret_cast<const uint32_t*>(&h);
     lo[e] = *reinterpret_cast<const uint32_t*>(&t);
   }
+  return min(least[0], least[1]);
+}
+__device__ __forceinline__ float lin_rna_tf32(float x) {
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return __uint_as_float(r);
 }
 __device__ __forceinline__ void fence_proxy_async_smem_lin() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -141,6 +178,8 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   __shared__ __align__(8) unsigned long long s_tempty[2];
   __shared__ __align__(8) unsigned long long s_sfull[kLinScales];    // a K tile's row scales are there
   __shared__ uint8_t s_scale[kLinScales][kLinTileM];    // exponents: the ring leaves little room
+  __shared__ __align__(8) unsigned long long s_narrow;               // all tiles have been through the first pass
+  __shared__ uint32_t s_lost[kLinFlagWords + 1];   // a bit per tile of this CTA: to be done in tf32; the last word: whether there is any
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
 
@@ -149,7 +188,6 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t stage_base = ring + kLinSlots * kLinSlotBytes;   // 4 KB of staging per epilogue warp
   volatile int* abort_flag = &s_abort;
-
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int s = 0; s < kLinMaxStages; s++) {
@@ -161,6 +199,8 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     for (int b = 0; b < kLinScales; b++) {
       mbar_init(smem_u32(&s_sfull[b]), kLinConvGroup);
     }
+    mbar_init(smem_u32(&s_narrow), (PAIR ? 4 : 2) * kLinConvGroup);
+    for (int w = 0; w <= kLinFlagWords; w++) s_lost[w] = 0u;
     for (int b = 0; b < 2; b++) {
       mbar_init(smem_u32(&s_tfull[b]), 1);
       mbar_init(smem_u32(&s_tempty[b]), (PAIR ? 8 : 4) * kLinEpiGroups);
@@ -171,14 +211,45 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     if (PAIR) tmem_alloc_pair(smem_u32(&s_tmem_base), p.tmem_cols);
     else tmem_alloc(smem_u32(&s_tmem_base), p.tmem_cols);
   }
+  // Nothing that the preparation wrote is read by __ldg: a read-only load could be moved up past this.
+  if (p.after_prepare) asm volatile("griddepcontrol.wait;" ::: "memory");
+  // A weight with a row of a wide range, or with small elements in every fourth row (a column of it beside larger ones): tf32 for
+  // all.  Each warp reads the counts.
+  int4 b_lost[kLinMaxCols / 128];
+#pragma unroll
+  for (int h = 0; h < kLinMaxCols / 128; h++) {
+    b_lost[h] = make_int4(0, 0, 0, 0);
+    if (128 * h + 4 * lane < p.Npad) b_lost[h] = __ldcg(reinterpret_cast<const int4*>(p.b_lost) + 32 * h + lane);
+  }
   tc_fence_before();
   __syncthreads();
   if (PAIR) cluster_sync();     // the other CTA arrives on these barriers
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
+  int b_many = 0, b_rows = 0;
+#pragma unroll
+  for (int h = 0; h < kLinMaxCols / 128; h++) {
+    b_many = max(max(b_many, max(b_lost[h].x, b_lost[h].y)), max(b_lost[h].z, b_lost[h].w));
+    b_rows += (b_lost[h].x > 0) + (b_lost[h].y > 0) + (b_lost[h].z > 0) + (b_lost[h].w > 0);
+  }
+  const bool wide = __any_sync(0xffffffffu, b_many >= kLinLost) || 4 * __reduce_add_sync(0xffffffffu, b_rows) >= p.N;
 
   // the tiles of a pair are neighbours; one past the last (an odd number of tiles) reads zeros and stores nothing
   const int first = blockIdx.x, step = gridDim.x, tiles = PAIR ? (p.num_tiles + 1) / 2 * 2 : p.num_tiles;
+
+  // The tiles are walked twice: in fp16 (pass 0, not with a wide weight), and then those in tf32 that fp16 could not hold.  Every
+  // role goes from one pass to the next when the converters of both CTAs are through the first; a pair walks a tile again for either.
+  auto lost_here = [&](int i) { return (*(volatile const uint32_t*)(s_lost + (i >> 5)) >> (i & 31) & 1u) != 0; };
+  auto walks = [&](int pass, int i) {
+    return pass == 0 || wide || lost_here(i) || (PAIR && (smem_of_rank(smem_u32(s_lost + (i >> 5)), rank ^ 1) >> (i & 31) & 1u) != 0);
+  };
+  auto second_pass = [&](bool& ok) {     // whether there is one
+    if (wide) return true;
+    ok = PAIR ? mbar_wait_pair(smem_u32(&s_narrow), 0u, abort_flag) : mbar_wait(smem_u32(&s_narrow), 0u, abort_flag);
+    if (!ok) return false;
+    return *(volatile const uint32_t*)(s_lost + kLinFlagWords) != 0 ||
+           (PAIR && smem_of_rank(smem_u32(s_lost + kLinFlagWords), rank ^ 1) != 0);
+  };
 
   if (warp < kLinFirstConv) {
   set_registers<kLinRegsIssue, false>();
@@ -188,20 +259,25 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       RingStage st;
       int uses = 0;   // K tiles requested so far, at most p.stages
       bool ok = true;
-      for (int tile = first; tile < tiles && ok; tile += step) {
-        for (int kb = 0; kb < p.kblocks; kb++, st.next(p.stages)) {
+      for (int pass = wide ? 1 : 0; pass < 2 && ok; pass++) {
+      if (pass == 1 && !second_pass(ok)) break;
+      const int kblocks = pass ? p.wide_kblocks : p.kblocks, kblocks1 = pass ? p.wide_kblocks1 : p.kblocks1;
+      const char* b = pass ? reinterpret_cast<const char*>(p.b_wide) : reinterpret_cast<const char*>(p.b);
+      for (int tile = first, nth = 0; tile < tiles && ok; tile += step, nth++) {
+        if (!walks(pass, nth)) continue;
+        for (int kb = 0; kb < kblocks; kb++, st.next(p.stages)) {
           if (!mbar_wait(smem_u32(&s_empty[st.s]), st.ph ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t full = smem_u32(&s_full[st.s]), bfull = smem_u32(&s_bfull[st.s]);
           const uint32_t dst = ring + (uint32_t)st.s * p.stage_bytes;
-          mbar_arrive_expect_tx(full, 2 * kLinHalf);      // a box past the row's end is zeros
-          const CUtensorMap* map = kb < p.kblocks1 ? &tm_a : &tm_a2;
-          const int x = (kb < p.kblocks1 ? kb : kb - p.kblocks1) * kLinTileK;
+          const CUtensorMap* map = kb < kblocks1 ? &tm_a : &tm_a2;
+          const int x = (kb < kblocks1 ? kb : kb - kblocks1) * (pass ? kLinWideK : kLinTileK);
+          mbar_arrive_expect_tx(full, pass ? kLinHalf : 2 * kLinHalf);      // a box past the row's end is zeros
           tma_load_2d(dst, map, x, tile * kLinTileM, full);
-          tma_load_2d(dst + kLinHalf, map, x + kLinBoxK, tile * kLinTileM, full);
+          if (pass == 0) tma_load_2d(dst + kLinHalf, map, x + kLinBoxK, tile * kLinTileM, full);
           mbar_arrive_expect_tx(bfull, 2 * p.b_slot);
-          bulk_load(dst + kLinSlotBytes, reinterpret_cast<const char*>(p.b) + (size_t)(PAIR ? 2 * kb + rank : kb) * (2 * p.b_slot),
-                    2 * p.b_slot, bfull);
+          bulk_load(dst + kLinSlotBytes, b + (size_t)(PAIR ? 2 * kb + rank : kb) * (2 * p.b_slot), 2 * p.b_slot, bfull);
           if (uses < p.stages) uses++;
+          if (pass) continue;
           // A comes from HBM exactly once: pull the tile that will be loaded kLinPrefetch K tiles from now into L2, so that its
           // TMA load later pays L2 latency only
           int pk = kb + kLinPrefetch, pt = tile;
@@ -213,6 +289,7 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             tma_prefetch_2d(pmap, px + kLinBoxK, pt * kLinTileM);
           }
         }
+      }
       }
       // the latest round of every stage that was used: the stage before `st` and those before it
       const long long t0 = clock64();
@@ -239,10 +316,20 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     // MMAs first moved its operands there.
     if (rank == 0) {
       const bool elected = elect_one();
-      const uint32_t idesc = umma_idesc_f16(PAIR ? 2 * kLinTileM : kLinTileM, p.Npad);
-      auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
-        if (PAIR) umma_f16_pair(d, a, b, idesc, acc);
-        else umma_f16(d, a, b, idesc, acc);
+      constexpr int M = PAIR ? 2 * kLinTileM : kLinTileM;
+      // A K tile's products, 16 halves or 8 tf32 = 32 bytes along K inside the swizzle atom at a time.  The small ones come before the
+      // large ones: the accumulator truncates at its own size.
+      auto products = [&](auto mma, uint32_t at) {
+        const uint64_t ahi = umma_desc_sw128(at), alo = umma_desc_sw128(at + kLinHalf), bhi = umma_desc_sw128(at + kLinSlotBytes),
+                       blo = umma_desc_sw128(at + kLinSlotBytes + p.b_slot);
+#pragma unroll
+        for (int k = 0; k < kLinTileK / 16; k++) {
+          const uint64_t o = (uint64_t)(k * 2);
+          mma(alo + o, bhi + o, (uint32_t)(k != 0));
+          mma(ahi + o, blo + o, 1u);
+        }
+#pragma unroll
+        for (int k = 0; k < kLinTileK / 16; k++) mma(ahi + (uint64_t)(k * 2), bhi + (uint64_t)(k * 2), 1u);
       };
       auto wait = [&](uint32_t bar, uint32_t parity) {
         const bool there = PAIR ? mbar_wait_pair(bar, parity, abort_flag) : mbar_wait(bar, parity, abort_flag);
@@ -262,8 +349,16 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         at = ring + (uint32_t)st.s * p.stage_bytes;
         return true;
       };
-      for (int tile = first; tile < tiles && ok; tile += step) {
-        for (int kb = 0; kb < p.kblocks; kb++) {
+      for (int pass = wide ? 1 : 0; pass < 2 && ok; pass++) {
+      if (pass == 1) {
+        const bool second = second_pass(ok);
+        ok = __all_sync(0xffffffffu, ok) != 0;
+        if (!__all_sync(0xffffffffu, second)) break;
+      }
+      const int kblocks = pass ? p.wide_kblocks : p.kblocks;
+      for (int tile = first, nth = 0; tile < tiles && ok; tile += step, nth++) {
+        if (!__any_sync(0xffffffffu, walks(pass, nth))) continue;
+        for (int kb = 0; kb < kblocks; kb++) {
           const int buf = t & 1;
           if (!wait(smem_u32(&s_tempty[buf]), ((uint32_t)(t >> 1) & 1u) ^ 1u)) { ok = false; break; }
           tc_fence_after();
@@ -274,23 +369,23 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           const int s0 = st.s;
           st.next(p.stages);
           if (elected) {
-            const uint64_t ahi = umma_desc_sw128(at), alo = umma_desc_sw128(at + kLinHalf), bhi = umma_desc_sw128(at + kLinSlotBytes),
-                           blo = umma_desc_sw128(at + kLinSlotBytes + p.b_slot);
-            // 16 halves = 32 bytes along K inside the swizzle atom.  The small products come before the large ones: the accumulator
-            // truncates at its own size.
-#pragma unroll
-            for (int k = 0; k < kLinTileK / 16; k++) {
-              const uint64_t o = (uint64_t)(k * 2);
-              mma(d_tmem, alo + o, bhi + o, k != 0);
-              mma(d_tmem, ahi + o, blo + o, 1);
+            if (pass == 0) {
+              products([&](uint64_t a, uint64_t b, uint32_t acc) {
+                if (PAIR) umma_f16_pair(d_tmem, a, b, umma_idesc_f16(M, p.Npad), acc);
+                else umma_f16(d_tmem, a, b, umma_idesc_f16(M, p.Npad), acc);
+              }, at);
+            } else {
+              products([&](uint64_t a, uint64_t b, uint32_t acc) {
+                if (PAIR) umma_tf32_pair(d_tmem, a, b, umma_idesc_tf32(M, p.Npad), acc);
+                else umma_tf32(d_tmem, a, b, umma_idesc_tf32(M, p.Npad), acc);
+              }, at);
             }
-#pragma unroll
-            for (int k = 0; k < kLinTileK / 16; k++) mma(d_tmem, ahi + (uint64_t)(k * 2), bhi + (uint64_t)(k * 2), 1);
             commit(smem_u32(&s_empty[s0]));
             commit(smem_u32(&s_tfull[buf]));
           }
           __syncwarp();
         }
+      }
       }
     }
   }
@@ -308,8 +403,18 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     int turn = group, seen = 0;   // seen: K tiles so far, up to a full ring
     int n = 0;                    // K tiles so far
     bool ok = true;
-    for (int tile = first; tile < tiles && ok; tile += step) {
-      for (int kb = 0; kb < p.kblocks; kb++, st.next(p.stages), turn ^= 1, n++) {
+    for (int pass = wide ? 1 : 0; pass < 2 && ok; pass++) {
+    if (pass == 1) {
+      if (!wide && lane == 0) {
+        if (PAIR) mbar_arrive_pair(smem_u32(&s_narrow));
+        else mbar_arrive(smem_u32(&s_narrow));
+      }
+      if (!second_pass(ok)) break;
+    }
+    const int kblocks = pass ? p.wide_kblocks : p.kblocks;
+    for (int tile = first, nth = 0; tile < tiles && ok; tile += step, nth++) {
+      if (!walks(pass, nth)) continue;
+      for (int kb = 0; kb < kblocks; kb++, st.next(p.stages), turn ^= 1, n++) {
         const bool again = seen >= p.stages;
         if (!again) seen++;
         if (turn) continue;
@@ -318,6 +423,39 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         if (again && !mbar_wait(smem_u32(&s_empty[st.s]), st.ph ^ 1u, abort_flag)) { ok = false; break; }
         if (!mbar_wait(smem_u32(&s_full[st.s]), st.ph, abort_flag)) { ok = false; break; }
         const uint32_t base = ring + (uint32_t)st.s * p.stage_bytes + (uint32_t)(row0 + r8) * 128u;
+        int lost = 0;
+        if (pass == 1) {
+          // Eight elements of a row a lane, which its heads replace; the tails go to the slot's other half.
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            float v[2][4], m = 0.f;
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[j][0]), "=f"(v[j][1]), "=f"(v[j][2]), "=f"(v[j][3])
+                           : "r"(base + (uint32_t)q * 1024u + (uint32_t)(((part + 4 * j) ^ r8) << 4)) : "memory");
+#pragma unroll
+              for (int e = 0; e < 4; e++) m = fmaxf(m, fabsf(v[j][e]));
+            }
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            const uint32_t exponent = lin_scale_exp<kLinWideExp>(__float_as_uint(m));
+            const float scale = lin_scale(exponent);
+            if (part == 0) s_scale[n & (kLinScales - 1)][row0 + q * 8 + r8] = (uint8_t)exponent;
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+              float hi[4], lo[4];
+#pragma unroll
+              for (int e = 0; e < 4; e++) {
+                const float x = __fmul_rn(v[j][e], scale);
+                hi[e] = lin_rna_tf32(x);
+                lo[e] = lin_rna_tf32(__fsub_rn(x, hi[e]));
+              }
+              const uint32_t to = base + (uint32_t)q * 1024u + (uint32_t)(((part + 4 * j) ^ r8) << 4);
+              asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(hi[0]), "f"(hi[1]), "f"(hi[2]), "f"(hi[3]) : "memory");
+              asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + kLinHalf), "f"(lo[0]), "f"(lo[1]), "f"(lo[2]), "f"(lo[3]) : "memory");
+            }
+          }
+        } else {
         float a[2][4][4];
         auto read = [&](int pass, float (&v)[4][4]) {
 #pragma unroll
@@ -332,35 +470,46 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         for (int pass = 0; pass < 4; pass++) {
           float(&v)[4][4] = a[pass & 1];
           if (pass < 3) read(pass + 1, a[(pass + 1) & 1]);
-          // inf reaches the maximum and leaves the row as it is; NaN does not and stays NaN under any scale
+          // inf reaches the maximum, NaN does not; both stay what they are under any scale
           float m = 0.f;
 #pragma unroll
           for (int j = 0; j < 4; j++) m = fmaxf(fmaxf(m, fmaxf(fabsf(v[j][0]), fabsf(v[j][1]))), fmaxf(fabsf(v[j][2]), fabsf(v[j][3])));
           m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
           m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));    // the four lanes of a row have read it
-          const uint32_t exponent = lin_scale_exp(__float_as_uint(m));
+          const uint32_t exponent = lin_scale_exp<kLinHeadExp>(__float_as_uint(m));
           const float scale = lin_scale(exponent);
           if (part == 0) s_scale[n & (kLinScales - 1)][row0 + pass * 8 + r8] = (uint8_t)exponent;
           const f32x2 s2 = f2_pack(scale, scale);
+          uint32_t least[4];
 #pragma unroll
           for (int j = 0; j < 4; j++) {
             const int box = (j >> 1) ^ (r8 >> 1 & 1), c = part + 4 * ((j & 1) ^ (r8 & 1));
             uint32_t hi[2], lo[2];
-            split_f16(v[j], s2, hi, lo);
+            least[j] = pass & 1 ? split_f16<true>(v[j], s2, hi, lo) : split_f16<false>(v[j], s2, hi, lo);
             const uint32_t to = base + (uint32_t)pass * 1024u + (uint32_t)(((box * 4 + (c >> 1)) ^ r8) << 4) + (uint32_t)(c & 1) * 8u;
             asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(to), "r"(hi[0]), "r"(hi[1]) : "memory");
             asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(to + kLinHalf), "r"(lo[0]), "r"(lo[1]) : "memory");
           }
+          lost += lin_huge(exponent) ? kLinLost : min(min(least[0], least[1]), min(least[2], least[3])) < kLinLostBelow ? 1 : 0;
+        }
         }
         fence_proxy_async_smem_lin();  // generic-proxy stores -> visible to the tensor core's reads
         __syncwarp();
         if (first_warp && !mbar_wait(smem_u32(&s_bfull[st.s]), st.ph, abort_flag)) { ok = false; break; }   // for the MMA's one wait
         if (lane == 0) {
-          mbar_arrive(smem_u32(&s_sfull[n & (kLinScales - 1)]));
           if (PAIR) mbar_arrive_leader(smem_u32(&s_ready[st.s]));
           else mbar_arrive(smem_u32(&s_ready[st.s]));
         }
+        lost = __reduce_add_sync(0xffffffffu, lost);
+        if (lane == 0) {
+          if (lost >= kLinLost) {
+            atomicOr(&s_lost[nth >> 5], 1u << (nth & 31));
+            s_lost[kLinFlagWords] = 1u;
+          }
+          mbar_arrive(smem_u32(&s_sfull[n & (kLinScales - 1)]));
+        }
       }
+    }
     }
   } else {
     // ---------------- epilogue ----------------
@@ -383,13 +532,13 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     };
     // The staged columns c0 .. c0 + cols - 1 of the warp's 32 rows, scaled (+ bias), to C: where it cannot be stored as a box, and
     // nothing is added.  Four rows at a time, four columns a lane.
-    auto write_out = [&](int c0, int cols, long long row_base) {
+    auto write_out = [&](int c0, int cols, long long row_base, const float* col_inv) {
       __syncwarp();
       const uint32_t ci = (uint32_t)lane & 7u;
       const int c = c0 + (int)ci * 4;
       const bool inside = (int)ci * 4 < cols && c < p.N;
-      const float4 inv = inside ? __ldg(reinterpret_cast<const float4*>(p.col_inv + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 bias = inside && p.bias_pad != nullptr ? __ldg(reinterpret_cast<const float4*>(p.bias_pad + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 inv = inside ? *reinterpret_cast<const float4*>(col_inv + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 bias = inside && p.bias_pad != nullptr ? *reinterpret_cast<const float4*>(p.bias_pad + c) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < 8; i++) {
         const int rr = 4 * i + (lane >> 3);
@@ -409,11 +558,11 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     };
     // The same with an addend.  A lane is a column here, and 16 rows of the addend are read before they are written (C may be the
     // addend): with four at a time 2,449,029 x 256 -> 47 took 1,440 us, 1,000 this way.
-    auto add_out = [&](int c0, int cols, long long row_base) {
+    auto add_out = [&](int c0, int cols, long long row_base, const float* col_inv) {
       __syncwarp();
       const int c = c0 + lane;
       const bool inside = lane < cols && c < p.N;
-      const float inv = inside ? __ldg(p.col_inv + c) : 0.f, bias = inside && p.bias_pad != nullptr ? __ldg(p.bias_pad + c) : 0.f;
+      const float inv = inside ? col_inv[c] : 0.f, bias = inside && p.bias_pad != nullptr ? p.bias_pad[c] : 0.f;
       const int rows = p.M - row_base < 32 ? (int)(p.M - row_base) : 32;
       float* d = p.C + row_base * p.ldc + c;
       const float* add = p.addend + row_base * p.ldadd + c;
@@ -440,14 +589,19 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         else mbar_arrive(smem_u32(&s_tempty[buf]));
       }
     };
-    for (int tile = first; tile < tiles && ok; tile += step) {
+    for (int pass = wide ? 1 : 0; pass < 2 && ok; pass++) {
+    if (pass == 1 && !second_pass(ok)) break;
+    const int kblocks = pass ? p.wide_kblocks : p.kblocks;
+    const float* const col_inv = pass ? p.unit : p.col_inv;
+    for (int tile = first, nth = 0; tile < tiles && ok; tile += step, nth++) {
+      if (!walks(pass, nth)) continue;
       const long long row_base = (long long)tile * kLinTileM + quad * 32;
       // Every K tile is drained and added up here in fp32, with its scales and its average loss given back: half of a row's 256
       // columns a thread.  (Kept in memory the sums were 16 TB/s of L2 traffic.)
       float run[kLinMaxCols / kLinEpiGroups];
 #pragma unroll
       for (int i = 0; i < kLinMaxCols / kLinEpiGroups; i++) run[i] = 0.f;
-      for (int kb = 0; kb < p.kblocks; kb++, t++) {
+      for (int kb = 0; kb < kblocks; kb++, t++) {
         const int buf = t & 1;
         if (!mbar_wait(smem_u32(&s_tfull[buf]), (uint32_t)(t >> 1) & 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
@@ -469,6 +623,7 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         release(buf);
       }
       if (!ok) break;
+      if ((wide || lost_here(nth)) != (pass == 1)) continue;   // the other pass stores it (all converters of the tile's rows have been here)
 #pragma unroll
       for (int b = 0; b < kLinMaxCols / kLinEpiGroups / 32; b++) {
         const int c0 = b * 64 + share * 32;
@@ -481,8 +636,8 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           for (int j = 0; j < 8; j++) {
             const int c = c0 + 4 * j;
             float4 inv = make_float4(0.f, 0.f, 0.f, 0.f), bias = inv;
-            if (c < p.Npad) inv = __ldg(reinterpret_cast<const float4*>(p.col_inv + c));
-            if (p.bias_pad != nullptr && c < p.Npad) bias = __ldg(reinterpret_cast<const float4*>(p.bias_pad + c));
+            if (c < p.Npad) inv = *reinterpret_cast<const float4*>(col_inv + c);
+            if (p.bias_pad != nullptr && c < p.Npad) bias = *reinterpret_cast<const float4*>(p.bias_pad + c);
             const float* v = run + 32 * b + 4 * j;
             const uint32_t addr = stage_addr + (uint32_t)lane * 128u + (((uint32_t)j ^ ((uint32_t)lane & 7u)) << 4);
             asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(__fmaf_rn(v[0], inv.x, bias.x)),
@@ -497,10 +652,11 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           stage16(0, run + 32 * b);
           stage16(1, run + 32 * b + 16);
           const int cols = p.Npad - c0 < 32 ? p.Npad - c0 : 32;
-          if (p.addend != nullptr) add_out(c0, cols, row_base);
-          else write_out(c0, cols, row_base);
+          if (p.addend != nullptr) add_out(c0, cols, row_base, col_inv);
+          else write_out(c0, cols, row_base, col_inv);
         }
       }
+    }
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // before the staging tile goes away
   }
@@ -523,41 +679,67 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
 
 // Heads and tails of [B | B2] (rows = output features), each row scaled by a power of two, zero padded to [Npad, Kpad1 + Kpad2], in
 // the order and with the swizzle of the shared-memory tiles: K tile by K tile, in it the share of each CTA of a pair (b_rows rows),
-// in that the heads and then the tails, so that a CTA's part of a K tile is one contiguous run.  A block per row; also writes the
-// inverse scales and clears the status word, if given.
+// in that the heads and then the tails, so that a CTA's part of a K tile is one contiguous run.  Once in fp16 and once, not scaled, in
+// tf32 with its K tiles of 32 columns.  A block per row; also writes the inverse scales, counts the elements that fp16 cannot
+// hold and clears the status word, if given.
 constexpr int kLinPrepThreads = 128;
-__global__ void __launch_bounds__(kLinPrepThreads) linear_prepare_kernel(
-    const float* __restrict__ B, int K, long long ldb, long long incb, const float* __restrict__ B2, int K2, long long ldb2,
-    long long incb2, int N, int Npad, int Kpad1, int Kpad, int b_rows, __half* __restrict__ out, float* __restrict__ col_inv,
-    const float* __restrict__ bias, float* __restrict__ bias_pad, int* status) {
-  __shared__ uint32_t s_max[kLinPrepThreads / 32];
+struct LinPrep {
+  const float *B, *B2, *bias;
+  long long ldb, incb, ldb2, incb2;
+  int K, K2, N, Npad, Kpad1, Kpad, b_rows;
+  int wide1;               // K tiles of B in tf32
+  __half* out;
+  float *wide, *col_inv, *bias_pad, *unit;
+  int *lost, *status;
+};
+__global__ void __launch_bounds__(kLinPrepThreads) linear_prepare_kernel(const __grid_constant__ LinPrep p) {
+  __shared__ uint32_t s_max[kLinPrepThreads / 32], s_lost[kLinPrepThreads / 32];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the product's CTAs set up their barriers and TMEM meanwhile
   const int n = blockIdx.x;
-  if (n == 0 && threadIdx.x == 0 && status != nullptr) *status = 0;
+  if (n == 0 && threadIdx.x == 0 && p.status != nullptr) *p.status = 0;
   auto element = [&](int kk) {
-    if (n >= N) return 0.f;
-    if (kk < Kpad1) return kk < K ? __ldg(B + (long long)n * ldb + kk * incb) : 0.f;
-    return kk - Kpad1 < K2 ? __ldg(B2 + (long long)n * ldb2 + (kk - Kpad1) * incb2) : 0.f;
+    if (n >= p.N) return 0.f;
+    if (kk < p.Kpad1) return kk < p.K ? __ldg(p.B + (long long)n * p.ldb + kk * p.incb) : 0.f;
+    return kk - p.Kpad1 < p.K2 ? __ldg(p.B2 + (long long)n * p.ldb2 + (kk - p.Kpad1) * p.incb2) : 0.f;
   };
-  uint32_t m = 0;
-  for (int kk = threadIdx.x; kk < Kpad; kk += kLinPrepThreads) m = max(m, __float_as_uint(element(kk)) & 0x7fffffffu);
+  uint32_t m = 0, lost = 0;
+  for (int kk = threadIdx.x; kk < p.Kpad; kk += kLinPrepThreads) m = max(m, __float_as_uint(element(kk)) & 0x7fffffffu);
   m = __reduce_max_sync(0xffffffffu, m);
   if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < kLinPrepThreads / 32; w++) m = max(m, s_max[w]);
-  const float scale = lin_scale(lin_scale_exp(m));
-  if (threadIdx.x == 0) {
-    col_inv[n] = lin_inverse(lin_scale_exp(m));
-    bias_pad[n] = bias != nullptr && n < N ? bias[n] : 0.f;
-  }
-  const int share = n / b_rows, r = n - share * b_rows;
-  for (int kk = threadIdx.x; kk < Kpad; kk += kLinPrepThreads) {
-    const float v = element(kk) * scale;
+  const uint32_t exponent = lin_scale_exp<kLinHeadExp>(m);
+  const float scale = lin_scale(exponent);
+  const int share = n / p.b_rows, r = n - share * p.b_rows, shares = p.Npad / p.b_rows;
+  for (int kk = threadIdx.x; kk < p.Kpad; kk += kLinPrepThreads) {
+    const float x = element(kk), v = x * scale;
+    lost += lin_twice_minus_one(v) < kLinLostBelow ? 1u : 0u;
     const __half hi = __float2half_rn(v), lo = __float2half_rn(v - __half2float(hi));
     const int kb = kk / kLinTileK, e = kk - kb * kLinTileK;
-    const size_t at = (size_t)(kb * (Npad / b_rows) + share) * 2 * b_rows * kLinTileK + r * kLinTileK + (((e >> 3) ^ (r & 7)) << 3) + (e & 7);
-    out[at] = hi;
-    out[at + (size_t)b_rows * kLinTileK] = lo;
+    const size_t at = (size_t)(kb * shares + share) * 2 * p.b_rows * kLinTileK + r * kLinTileK + (((e >> 3) ^ (r & 7)) << 3) + (e & 7);
+    p.out[at] = hi;
+    p.out[at + (size_t)p.b_rows * kLinTileK] = lo;
+    const int k = kk < p.Kpad1 ? kk : kk - p.Kpad1, of = kk < p.Kpad1 ? p.K : p.K2;
+    if (k / kLinWideK * kLinWideK < of) {      // the last K tile in tf32 may end sooner
+      const int kw = (kk < p.Kpad1 ? 0 : p.wide1) + k / kLinWideK, f = k % kLinWideK;
+      const size_t to = (size_t)(kw * shares + share) * 2 * p.b_rows * kLinWideK + r * kLinWideK + (((f >> 2) ^ (r & 7)) << 2) + (f & 3);
+      const float head = lin_rna_tf32(x);
+      p.wide[to] = head;
+      p.wide[to + (size_t)p.b_rows * kLinWideK] = lin_rna_tf32(__fsub_rn(x, head));
+    }
+  }
+  lost = __reduce_add_sync(0xffffffffu, lost);
+  if ((threadIdx.x & 31) == 0) s_lost[threadIdx.x >> 5] = lost;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    lost = lin_huge(exponent) ? kLinLost : 0;
+#pragma unroll
+    for (int w = 0; w < kLinPrepThreads / 32; w++) lost += s_lost[w];
+    p.lost[n] = (int)lost;
+    p.col_inv[n] = lin_inverse(exponent);
+    p.unit[n] = 1.f;
+    p.bias_pad[n] = p.bias != nullptr && n < p.N ? p.bias[n] : 0.f;
   }
 }
 
@@ -568,26 +750,11 @@ int launch_linear(const float* A, int64_t M, int64_t K, int64_t lda, const float
 }
 
 static inline int lin_kpad(long long K) { return (int)((K + kLinTileK - 1) / kLinTileK * kLinTileK); }
+static inline int lin_wide_tiles(long long K) { return (int)((K + kLinWideK - 1) / kLinWideK); }
 
-// One launch over checked arguments: N <= 256 columns.
-static int lin_launch(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb, int64_t incb, const float* A2, int64_t K2,
-                      int64_t lda2, const float* B2, int64_t ldb2, int64_t incb2, int64_t N, const float* bias, const float* addend,
-                      int64_t ldadd, void* workspace, float* C, int64_t ldc, cudaStream_t st) {
-  const int Npad = (int)((N + 15) / 16 * 16);
-  const int Kpad1 = lin_kpad(K), Kpad2 = lin_kpad(K2), Kpad = Kpad1 + Kpad2;
-  int* status = reinterpret_cast<int*>(workspace);
-  float* col_inv = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + 256);
-  float* bias_pad = col_inv + kLinMaxCols;
-  __half* b = reinterpret_cast<__half*>(bias_pad + kLinMaxCols);
-  const int num_tiles = (int)((M + kLinTileM - 1) / kLinTileM);
-  // Pairs need whole 16-row groups of B in each half; a single tile has no partner.
-  const bool pair = num_tiles >= 2 && Npad % 32 == 0;
-  const int b_rows = pair ? Npad / 2 : Npad;   // of B in one CTA
-
-  linear_prepare_kernel<<<Npad, kLinPrepThreads, 0, st>>>(B, (int)K, ldb, incb, B2, (int)K2, ldb2, incb2, (int)N, Npad, Kpad1, Kpad,
-                                                          b_rows, b, col_inv, bias, bias_pad, status);
-  EXB_CUDA_OK(cudaGetLastError());
-
+// One launch; the rest of its parameters is the same for all rows.
+static int lin_launch_rows(const float* A, int64_t M, int64_t K, int64_t lda, const float* A2, int64_t K2, int64_t lda2, int64_t N,
+                           const float* addend, int64_t ldadd, float* C, int64_t ldc, LinParams p, bool pair, bool after_prepare, cudaStream_t st) {
   CUtensorMap tm_a, tm_a2;
   int rc = make_tensor_map_2d_f32(&tm_a, A, (unsigned long long)K, (unsigned long long)M, (unsigned long long)lda * 4, kLinBoxK, kLinTileM);
   if (rc) return rc;
@@ -605,19 +772,9 @@ static int lin_launch(const float* A, int64_t M, int64_t K, int64_t lda, const f
     if (rc) return rc;
   }
 
-  LinParams p{};
-  p.b = b; p.C = C; p.bias = bias; p.status = status; p.lib_status = status_word_ptr(); p.M = M; p.ldc = ldc; p.N = (int)N; p.Npad = Npad;
-  p.kblocks1 = Kpad1 / kLinTileK; p.kblocks = Kpad / kLinTileK;
-  p.num_tiles = num_tiles;
-  p.addend = addend; p.ldadd = ldadd;
-  p.col_inv = col_inv; p.bias_pad = bias ? bias_pad : nullptr; p.bulk_out = bulk_out ? 1 : 0;
-  p.b_slot = (unsigned)b_rows * kLinTileK * 2;
-  p.stage_bytes = kLinSlotBytes + 2 * p.b_slot;
-  p.stages = (int)((kLinSlots * kLinSlotBytes) / p.stage_bytes);
-  if (p.stages > kLinMaxStages) p.stages = kLinMaxStages;
-  unsigned cols = 32;
-  while (cols < (unsigned)(2 * Npad)) cols <<= 1;
-  p.tmem_cols = cols;
+  p.after_prepare = after_prepare ? 1 : 0;
+  p.C = C; p.M = M; p.ldc = ldc; p.addend = addend; p.ldadd = ldadd; p.bulk_out = bulk_out ? 1 : 0;
+  p.num_tiles = (int)((M + kLinTileM - 1) / kLinTileM);
   const size_t dyn = (size_t)kLinSlots * kLinSlotBytes + 4 * kLinEpiGroups * 4096 + 1024;
   auto* kern = pair ? linear_f16x3_kernel<true> : linear_f16x3_kernel<false>;
   EXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
@@ -629,14 +786,65 @@ static int lin_launch(const float* A, int64_t M, int64_t K, int64_t lda, const f
   cfg.blockDim = dim3(kLinThreads);
   cfg.dynamicSmemBytes = dyn;
   cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 2;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = pair ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  if (pair) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = 2;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    cfg.numAttrs++;
+  }
+  if (after_prepare) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs++;
+  }
   EXB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tm_a, tm_a2, tm_c, p));
   EXB_CUDA_OK(cudaGetLastError());
+  return EXB_OK;
+}
+
+// One preparation and its launches over checked arguments: N <= 256 columns.
+static int lin_launch(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb, int64_t incb, const float* A2, int64_t K2,
+                      int64_t lda2, const float* B2, int64_t ldb2, int64_t incb2, int64_t N, const float* bias, const float* addend,
+                      int64_t ldadd, void* workspace, float* C, int64_t ldc, cudaStream_t st) {
+  const int Npad = (int)((N + 15) / 16 * 16);
+  // Pairs need whole 16-row groups of B in each half; a single tile has no partner.
+  const bool pair = M > kLinTileM && Npad % 32 == 0;
+  LinPrep b{};
+  b.B = B; b.B2 = B2; b.bias = bias; b.ldb = ldb; b.incb = incb; b.ldb2 = ldb2; b.incb2 = incb2;
+  b.K = (int)K; b.K2 = (int)K2; b.N = (int)N; b.Npad = Npad; b.Kpad1 = lin_kpad(K); b.Kpad = b.Kpad1 + lin_kpad(K2);
+  b.b_rows = pair ? Npad / 2 : Npad;   // of B in one CTA
+  b.wide1 = lin_wide_tiles(K);
+  b.status = reinterpret_cast<int*>(workspace);
+  b.col_inv = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + 256);
+  b.bias_pad = b.col_inv + kLinMaxCols;
+  b.unit = b.bias_pad + kLinMaxCols;
+  b.lost = reinterpret_cast<int*>(b.unit + kLinMaxCols);
+  b.out = reinterpret_cast<__half*>(b.lost + kLinMaxCols);
+  b.wide = reinterpret_cast<float*>(b.out + (size_t)2 * Npad * b.Kpad);
+  linear_prepare_kernel<<<Npad, kLinPrepThreads, 0, st>>>(b);
+  EXB_CUDA_OK(cudaGetLastError());
+
+  LinParams p{};
+  p.b = b.out; p.b_wide = b.wide; p.col_inv = b.col_inv; p.unit = b.unit; p.b_lost = b.lost; p.bias_pad = bias ? b.bias_pad : nullptr;
+  p.status = b.status; p.lib_status = status_word_ptr(); p.N = (int)N; p.Npad = Npad;
+  p.kblocks1 = b.Kpad1 / kLinTileK; p.kblocks = b.Kpad / kLinTileK;
+  p.wide_kblocks1 = b.wide1; p.wide_kblocks = b.wide1 + lin_wide_tiles(K2);
+  p.b_slot = (unsigned)b.b_rows * kLinTileK * 2;
+  p.stage_bytes = kLinSlotBytes + 2 * p.b_slot;
+  p.stages = (int)((kLinSlots * kLinSlotBytes) / p.stage_bytes);
+  if (p.stages > kLinMaxStages) p.stages = kLinMaxStages;
+  unsigned cols = 32;
+  while (cols < (unsigned)(2 * Npad)) cols <<= 1;
+  p.tmem_cols = cols;
+  // as many rows at a time as the CTAs have bits for (19.4 million on 148 SMs)
+  const int64_t most = (int64_t)(sm_count() / 2 * 2) * kLinFlagWords * 32 * kLinTileM;
+  for (int64_t r = 0; r < M; r += most) {
+    const int rc = lin_launch_rows(A + r * lda, M - r < most ? M - r : most, K, lda, A2 ? A2 + r * lda2 : nullptr, K2, lda2, N,
+                                   addend ? addend + r * ldadd : nullptr, ldadd, C + r * ldc, ldc, p, pair, r == 0, st);
+    if (rc) return rc;
+  }
   return EXB_OK;
 }
 
@@ -649,10 +857,9 @@ extern "C" {
 int64_t exact_linear_workspace_bytes(int64_t N, int64_t K, int64_t K2) {
   if (N <= 0 || K <= 0 || K2 < 0) return 256;
   const int64_t Npad = (N + 15) / 16 * 16;
-  // the tiles and scales of this file's kernel, and the two fp32 copies in rows of 32 columns of the other's
-  const int64_t tiles = 256 + 2 * kLinMaxCols * 4 + 2 * Npad * (int64_t)(lin_kpad(K) + lin_kpad(K2)) * 2;
-  const int64_t copies = 256 + 2 * Npad * ((K + 31) / 32 * 32 + (K2 + 31) / 32 * 32) * 4;
-  return tiles > copies ? tiles : copies;
+  // this file's scales, and its tiles in fp16 and in tf32; linear_tf32.cu needs less
+  return 256 + 4 * kLinMaxCols * 4 + 2 * Npad * (int64_t)(lin_kpad(K) + lin_kpad(K2)) * 2 +
+         2 * Npad * (int64_t)(lin_wide_tiles(K) + lin_wide_tiles(K2)) * kLinWideK * 4;
 }
 
 int64_t exact_linear_partial_bytes(int64_t) { return 0; }   // the running sums of a contraction in chunks stay in registers

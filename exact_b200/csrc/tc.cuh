@@ -178,6 +178,25 @@ __device__ __forceinline__ bool mbar_wait_pair(uint32_t bar, uint32_t parity, vo
   asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
   return true;
 }
+// An arrival on the barriers at `bar` in both CTAs, which announces this CTA's shared memory to threads that wait by mbar_wait_pair,
+// and the word at this CTA's address `word` in the CTA `rank`.
+__device__ __forceinline__ void mbar_arrive_pair(uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\t"
+      "fence.release.sync_restrict::shared::cta.cluster;\n\t"
+      "mapa.shared::cluster.u32 ra, %0, 0;\n\tmbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [ra];\n\t"
+      "mapa.shared::cluster.u32 ra, %0, 1;\n\tmbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t smem_of_rank(uint32_t word, int rank) {
+  uint32_t v;
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.relaxed.cluster.shared::cluster.u32 %0, [ra];\n\t}"
+      : "=r"(v)
+      : "r"(word), "r"(rank)
+      : "memory");
+  return v;
+}
 // Both CTAs of the pair call these; the columns are the same in both.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
