@@ -531,28 +531,19 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       }
     };
     // The staged columns c0 .. c0 + cols - 1 of the warp's 32 rows, scaled (+ bias), to C: where it cannot be stored as a box, and
-    // nothing is added.  Four rows at a time, four columns a lane.
+    // nothing is added.  A lane is a column: a store is one run of a row, whatever the row's pitch.
     auto write_out = [&](int c0, int cols, long long row_base, const float* col_inv) {
       __syncwarp();
-      const uint32_t ci = (uint32_t)lane & 7u;
-      const int c = c0 + (int)ci * 4;
-      const bool inside = (int)ci * 4 < cols && c < p.N;
-      const float4 inv = inside ? *reinterpret_cast<const float4*>(col_inv + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 bias = inside && p.bias_pad != nullptr ? *reinterpret_cast<const float4*>(p.bias_pad + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const int c = c0 + lane;
+      const bool inside = lane < cols && c < p.N;
+      const float inv = inside ? col_inv[c] : 0.f, bias = inside && p.bias_pad != nullptr ? p.bias_pad[c] : 0.f;
+      const int rows = !inside ? 0 : p.M - row_base < 32 ? (int)(p.M - row_base) : 32;
+      float* d = p.C + row_base * p.ldc + c;
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const int rr = 4 * i + (lane >> 3);
-        float4 o;
-        const uint32_t addr = stage_addr + (uint32_t)rr * 128u + ((ci ^ ((uint32_t)rr & 7u)) << 4);
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(addr));
-        if (row_base + rr < p.M && inside) {
-          float* d = p.C + (row_base + rr) * p.ldc + c;
-          const float v[4] = {__fmaf_rn(o.x, inv.x, bias.x), __fmaf_rn(o.y, inv.y, bias.y), __fmaf_rn(o.z, inv.z, bias.z),
-                              __fmaf_rn(o.w, inv.w, bias.w)};   // the products are exact
-#pragma unroll
-          for (int e = 0; e < 4; e++)
-            if (c + e < p.N) d[e] = v[e];
-        }
+      for (int r = 0; r < 32; r++, d += p.ldc) {
+        float o;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(o) : "r"(stage_addr + (uint32_t)r * 128u + ((((uint32_t)lane >> 2) ^ ((uint32_t)r & 7u)) << 4) + ((uint32_t)lane & 3u) * 4u));
+        if (r < rows) *d = __fmaf_rn(o, inv, bias);      // the product is exact
       }
       __syncwarp();
     };
