@@ -587,6 +587,13 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     for (int tile = first, nth = 0; tile < tiles && ok; tile += step, nth++) {
       if (!walks(pass, nth)) continue;
       const long long row_base = (long long)tile * kLinTileM + quad * 32;
+      if (p.addend != nullptr && row_base + lane < p.M) {     // on its way to L2 while the tile is summed
+        const float* add = p.addend + (row_base + lane) * p.ldadd;
+        for (int c0 = share * 32; c0 < p.N; c0 += 64) {
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(add + c0));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(add + (c0 + 31 < p.N ? c0 + 31 : p.N - 1)));
+        }
+      }
       // Every K tile is drained and added up here in fp32, with its scales and its average loss given back: half of a row's 256
       // columns a thread.  (Kept in memory the sums were 16 TB/s of L2 traffic.)
       float run[kLinMaxCols / kLinEpiGroups];
