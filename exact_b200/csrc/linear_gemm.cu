@@ -33,6 +33,7 @@
 //              [128 x 32] by TMA, which the heads and tails replace) and B_hi and B_lo (the CTA's rows x 64, one contiguous
 //              run): three stages at Npad = 256, four for narrow outputs.  128-byte swizzle, no multicast.  The boxes of two K
 //              tiles ahead are requested into L2: A is read from HBM exactly once and the ring is only a few K tiles deep.
+//              Products of one K tile do without, a stage is a tile there (600,000 x 48 -> 256: 150 us, 157 with).
 //   warp 1     MMA issuer (of the pair's first CTA): kind::f16, N = Npad, K = 16; 12 MMAs per K tile (with tf32, K = 8, it was as
 //              many per 32 columns, and the tensor pipe was what wide products were bound by), then two commits: one frees the
 //              stage (in both CTAs), one hands the accumulator over.  Accumulators are double-buffered in TMEM.
@@ -46,7 +47,7 @@
 //              Rows whose width or pitch is no multiple of 16 bytes, and an addend, take plain stores.
 // Bound by the chains of the roles: 2,250 cycles a K tile against 1,400 for its bytes (one launch of 128 columns, evaluation).
 // Measured (us, tf32 -> now): 2,449,029 x 256 -> 256: 1,283 -> 1,058, with a second operand pair of 256 2,424 -> 1,826; 48 -> 256:
-// 607 -> 589; 256 -> 80: 794 -> 677, 256 -> 47 (pitch 47): 660 -> 699, with an addend 1,111 -> 1,041; 232,965 x 602 -> 256: 275 -> 220
+// 607 -> 589; 256 -> 80: 794 -> 677, 256 -> 47 (pitch 47): 668 -> 625, with an addend 1,720 -> 1,040; 232,965 x 602 -> 256: 275 -> 220
 // (in chunks, evaluation: 458), 169,343 x 128 -> 256: 67 -> 63.
 // Not kept: one scale per row over the whole contraction, found ahead by four more warps, and one chain in TMEM: 2,424 -> 3,561;
 // sixteen epilogue warps with 64 sums a thread: 1,058 -> 1,115.
@@ -282,7 +283,7 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           // TMA load later pays L2 latency only
           int pk = kb + kLinPrefetch, pt = tile;
           if (pk >= p.kblocks) { pk -= p.kblocks; pt += step; }
-          if (pt < p.num_tiles && pk < p.kblocks) {
+          if (pt < p.num_tiles && pk < p.kblocks) {       // not with one K tile
             const CUtensorMap* pmap = pk < p.kblocks1 ? &tm_a : &tm_a2;
             const int px = (pk < p.kblocks1 ? pk : pk - p.kblocks1) * kLinTileK;
             tma_prefetch_2d(pmap, px, pt * kLinTileM);

@@ -7,9 +7,9 @@
 // Arithmetic.  Every fp32 operand is split into a tf32 head and a tf32 tail,
 //     a = a_hi + a_lo,   a_hi = rna_tf32(a),   a_lo = rna_tf32(a - a_hi)      (|a_lo| <= 2^-11 |a|),
 // and the product is accumulated in fp32 as  a_hi b_hi + a_lo b_hi + a_hi b_lo.  The dropped terms
-// (a_lo b_lo and the rounding of the tails) are below 2^-21 |a b|, the size of the fp32 rounding of a
-// plain fp32 dot product, so the result is as accurate as an fp32 SIMT GEMM at three tensor-core MMAs
-// per tile instead of one fp32 FMA per product.  Non-finite inputs stay non-finite and confined to their
+// (a_lo b_lo and the rounding of the tails) are below 2^-21 |a b|, the size of the rounding of an fp32 product; the error is that of the
+// accumulator, which truncates at every MMA: 3e-7 .. 4.4e-6 (Frobenius, against fp64) at 33 to 602 columns, where a plain
+// fp32 GEMM has 9e-8 .. 4.4e-7.  Non-finite inputs stay non-finite and confined to their
 // rows, but an infinite element turns its output row into NaN where an fp32 GEMM gives +-inf (its tail is
 // inf - inf).
 //
@@ -33,7 +33,7 @@
 //              parity are counted instead of divided out.  Accumulators are double-buffered in TMEM.
 //   warps 10-17 epilogue: tcgen05.ld -> per-warp staging tile in shared memory -> (+ bias, + addend)
 //              -> coalesced global stores; two groups of four take alternate blocks of 32 columns.
-// Measured (us, here | the other kernel): 169,343 x 128 -> 256: 67 | 63, 256 -> 256: 95 | 85, 256 -> 40: 58 | 52; 2,449,029 x 256 -> 47: 660 | 699.
+// Measured (us, here | the other kernel): 169,343 x 128 -> 256: 67 | 66, 256 -> 256: 95 | 93, 256 -> 40: 58 | 56; 2,449,029 x 256 -> 47: 668 | 625.
 // The weight is split, padded and laid out as the tiles once per call by a preparation kernel.
 //
 // Every mbarrier wait is bounded; on expiry the CTA raises an abort flag, all roles leave their loops,

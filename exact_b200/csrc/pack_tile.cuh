@@ -420,7 +420,6 @@ constexpr int resident_ctas(int acc, int v, int kind) {
   if (v != 2) return 1;
   if (acc < 4 && kind >= TILE_MULTI) return 2;
   return kind == TILE_PAIR || (kind == TILE_WARP && std::is_same<InT, uint16_t>::value) ? 2 : 1;
-  return kind >= TILE_MULTI ? 3 : 1;
 }
 
 // FAST: the tile has all 8 rows and the noise is drawn from Philox.  Then there is no per-row
