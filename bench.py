@@ -389,8 +389,8 @@ def roofline_of_dominant_kernel(ksum, ms_total, steps, hbm_peak, peak_kind):
     HBM-bound kernels: `achieved` = bytes that must cross HBM at least once (the operand in the form the kernel
     reads it, the indices, the output) / mean launch time, so that `frac` cannot exceed 1 by counting cache hits;
     for the gathers `l2_side_GB/s` gives the bytes requested from L2 when no source row is reused (the
-    reference's kernel moves exactly those).  The dense-layer GEMM: fp16 flop issued (three MMAs per product) against the
-    measured bf16 peak, which is also fp16's."""
+    reference's kernel moves exactly those).  The dense-layer GEMMs: flop issued (three MMAs per product) against the
+    measured bf16 peak, which is also fp16's, or half of it for the tf32 one."""
     if not ksum:
         return None
     name, r = max(ksum.items(), key=lambda kv: kv[1]["ms"])
@@ -398,19 +398,21 @@ def roofline_of_dominant_kernel(ksum, ms_total, steps, hbm_peak, peak_kind):
     sec = per_ms * 1e-3
     common = {"kernel": name, "launches_per_step": r["launches"] / steps, "ms_per_launch": round(per_ms, 4),
               "share_of_step": round(r["ms"] / ms_total, 4)}
-    if name == "exact_linear_forward":
-        peak = None
+    if name in ("exact_linear_forward", "exact_linear_forward_tf32"):
+        kind_of, rate, of = ("tf32", 0.5, "half the") if name.endswith("tf32") else ("fp16", 1.0, "the")
         try:
             with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
                 peak = float(json.load(f)["bf16_tflops_sustained"])
-            kind = "measured bf16 sustained (fp16 runs at the bf16 rate)"
+            kind = "measured bf16 sustained"
         except Exception:
             peak, kind = 1400.0, "fallback bf16 sustained"
+        peak *= rate
+        kind += " (%s runs at %s bf16 rate)" % (kind_of, of)
         achieved = r["flops"] / r["launches"] / sec / 1e12
         return dict(common, bound="tensor", achieved=round(achieved, 1), peak=peak, peak_kind=kind, unit="TFLOP/s",
                     frac=round(achieved / peak, 4), traffic=None,
-                    flops_model="6*M*K*N fp16 flop per call: every fp32 product is three fp16 MMAs (head*head, "
-                                "tail*head, head*tail)")
+                    flops_model="6*M*K*N %s flop per call: every fp32 product is three MMAs (head*head, "
+                                "tail*head, head*tail)" % kind_of)
     achieved = r["bytes"] / r["launches"] / sec / 1e9
     out = dict(common, bound="hbm", achieved=round(achieved, 1), peak=hbm_peak, peak_kind=peak_kind, unit="GB/s",
                frac=round(achieved / hbm_peak, 4))
@@ -547,13 +549,14 @@ def kernel_bandwidths(torch, Q, _lib, dev, hbm_peak, N=1_000_000, D=128, reps=20
     ref = reference_kernel_times(torch, dev, hbm_peak, reps)
     if ref is not None:
         out["ref_cuda"] = ref
-    # the dense-layer GEMM (tf32 head/tail split, three MMAs per tile) against the library's fp32 GEMM
+    # the dense-layer GEMMs (tf32 or fp16 heads and tails, three MMAs per tile) against the library's fp32 GEMM
     from exact_b200.cpp_extension import backward_func as B
     M3, K3, N3 = 1_000_000, 256, 256
     a3 = torch.randn(M3, K3, device=dev, generator=gen)
     w3 = torch.randn(N3, K3, device=dev, generator=gen)
     times = {}
-    for name, call in (("tc", lambda: B.linear_forward(a3, w3)), ("lib", lambda: torch.nn.functional.linear(a3, w3))):
+    for name, call in (("tf32x3", lambda: B.linear_forward(a3, w3)), ("f16x3", lambda: B.linear_forward(a3, w3, k_chunk=B.SUM_CHUNK)),
+                       ("lib", lambda: torch.nn.functional.linear(a3, w3))):
         for _ in range(3):
             call()
         torch.cuda.synchronize()
@@ -564,9 +567,10 @@ def kernel_bandwidths(torch, Q, _lib, dev, hbm_peak, N=1_000_000, D=128, reps=20
         b.record()
         torch.cuda.synchronize()
         times[name] = a.elapsed_time(b) * 1e-3 / reps
-    out["linear_tf32x3_1Mx256x256"] = {"ms": round(times["tc"] * 1e3, 4), "library_fp32_ms": round(times["lib"] * 1e3, 4),
-                                       "fp32_equiv_TFLOP/s": round(2.0 * M3 * K3 * N3 / times["tc"] / 1e12, 1),
-                                       "tensor_TFLOP/s": round(6.0 * M3 * K3 * N3 / times["tc"] / 1e12, 1)}
+    for name in ("tf32x3", "f16x3"):
+        out["linear_%s_1Mx256x256" % name] = {"ms": round(times[name] * 1e3, 4), "library_fp32_ms": round(times["lib"] * 1e3, 4),
+                                              "fp32_equiv_TFLOP/s": round(2.0 * M3 * K3 * N3 / times[name] / 1e12, 1),
+                                              "tensor_TFLOP/s": round(6.0 * M3 * K3 * N3 / times[name] / 1e12, 1)}
     return out
 
 

@@ -221,7 +221,8 @@ Tensor linear(const Tensor& a_, const Tensor& w_, const OptTensor& bias_, const 
     CallInfo info;
     info.bytes = 4 * (M * (K + K2) + n * (K + K2) + M * n * (addend ? 2 : 1));
     info.flops = 6.0 * (double)M * (double)(K + K2) * (double)n;
-    invoke("exact_linear_forward", info, [&](void* st) {
+    // two kernels with different rates: timed under two names
+    invoke(k_chunk > 0 ? "exact_linear_forward" : "exact_linear_forward_tf32", info, [&](void* st) {
       return lib.exact_linear_forward_strided(ptr<float>(a), M, K, a.stride(0), wb, w.stride(0), w.stride(1), K2 ? ptr<float>(a2) : nullptr, K2,
                                       K2 ? a2.stride(0) : 0, w2b, K2 ? w2.stride(0) : 0, K2 ? w2.stride(1) : 1, n,
                                       bias.defined() ? ptr<float>(bias) + n0 : nullptr,

@@ -119,8 +119,8 @@ def run_unpack_rp(N, D, kept_frac, bits, reps):
             "peak_kind": kind}
 
 
-def run_linear(M, K, N, reps):
-    """Dense-layer GEMM (tf32 head/tail split, tcgen05) against the library fp32 GEMM: ms, TFLOP/s, error vs fp64."""
+def run_linear(M, K, N, reps, chunk=0):
+    """Dense-layer GEMM (tcgen05; tf32 heads and tails in one chain, or with a chunk fp16 ones and sums in fp32) against the library fp32 GEMM: ms, TFLOP/s, error vs fp64."""
     from .cpp_extension import backward_func as B
     dev = torch.device("cuda")
     g = torch.Generator(device=dev).manual_seed(0)
@@ -128,15 +128,15 @@ def run_linear(M, K, N, reps):
     w = torch.randn(N, K, device=dev, generator=g)
     b = torch.randn(N, device=dev, generator=g)
     flush = torch.empty(64 * 1024 * 1024, device=dev) if M * (K + N) * 4 < 256e6 else None
-    ms = _time(lambda: B.linear_forward(a, w, b), reps, flush)
+    ms = _time(lambda: B.linear_forward(a, w, b, k_chunk=chunk), reps, flush)
     ms_lib = _time(lambda: torch.nn.functional.linear(a, w, b), reps, flush)
     rows = min(M, 20000)
     ref = a[:rows].double() @ w.double().t() + b.double()
-    err = float((B.linear_forward(a, w, b)[:rows].double() - ref).norm() / ref.norm())
+    err = float((B.linear_forward(a, w, b, k_chunk=chunk)[:rows].double() - ref).norm() / ref.norm())
     err_lib = float((torch.nn.functional.linear(a, w, b)[:rows].double() - ref).norm() / ref.norm())
     nbytes = 4 * (M * K + N * K + M * N)
     peak, kind = _peak()
-    return {"op": "linear", "M": M, "K": K, "N": N, "ms": round(ms, 4), "library_fp32_ms": round(ms_lib, 4),
+    return {"op": "linear", "M": M, "K": K, "N": N, "k_chunk": chunk, "ms": round(ms, 4), "library_fp32_ms": round(ms_lib, 4),
             "TFLOP/s": round(2.0 * M * K * N / (ms * 1e-3) / 1e12, 1),
             "tensor_TFLOP/s": round(6.0 * M * K * N / (ms * 1e-3) / 1e12, 1),
             "GB/s": round(nbytes / (ms * 1e-3) / 1e9, 1), "frac_hbm": round(nbytes / (ms * 1e-3) / 1e9 / peak, 4),
@@ -427,7 +427,8 @@ def main():
         for M in a.N:
             for K in a.D:
                 for N in a.K:
-                    print(json.dumps(run_linear(M, K, N, a.reps)), flush=True)
+                    for chunk in (0, 64):
+                        print(json.dumps(run_linear(M, K, N, a.reps, chunk)), flush=True)
         return
     if a.op == "unpack_rp":
         for N in a.N:
