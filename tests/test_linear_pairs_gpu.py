@@ -32,14 +32,46 @@ def test_tiles_and_widths(M, K, K2, N, chunk):
     _lib.check_status(force=True)
 
 
-@pytest.mark.parametrize("N", [256, 128, 47])
-def test_same_result_whatever_the_timing_of_the_loads(N):
+# rings of two (240 columns and a single CTA), three (256) and four stages; results stored as boxes and (47, and the addend) plainly;
+# more than 256 columns; the weight transposed; fp16, tf32 beside it (a range too wide for fp16) and tf32 in one chain
+@pytest.mark.parametrize("chunk,wide", [(0, False), (64, False), (64, True)])
+@pytest.mark.parametrize("N,addend,transposed", [(256, False, False), (256, True, True), (240, False, True), (128, False, False), (47, False, False),
+                                                 (47, True, False), (300, True, False)])
+def test_same_result_whatever_the_timing_of_the_loads(N, addend, transposed, chunk, wide):
     """Cold and warm operands: the groups of warps that take alternate K tiles must not meet a stage a round early."""
     from exact_b200.cpp_extension import backward_func as B
-    a, w = torch.randn(128 * 700, 256, device="cuda"), torch.randn(N, 256, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    a, w = torch.randn(128 * 700, 256, device="cuda", generator=gen), torch.randn(N, 256, device="cuda", generator=gen)
+    if wide:
+        a[128 * 100:128 * 400, 7] *= 1e8
+        w[:, 7] = 0
+    if transposed:
+        w = w.t().contiguous().t()
+    c = torch.randn(128 * 700, N, device="cuda", generator=gen) if addend else None
     flush = torch.empty(64 << 20, device="cuda")
-    want = B.linear_forward(a, w)
+
+    def product():
+        return B.linear_forward(a, w, k_chunk=chunk, out=c.clone() if addend else None, accumulate=addend)
+    want, ref = product(), a.double() @ w.double().t()
+    if addend:
+        ref += c.double()
+    assert (want.double() - ref).norm() <= (2e-7 if chunk else 3e-6) * ref.norm()
     for i in range(20):
         if i % 2:
             flush.fill_(float(i))
-        assert torch.equal(B.linear_forward(a, w), want)
+        assert torch.equal(product(), want)
+    _lib.check_status(force=True)
+
+
+def test_lone_tile_of_256_columns():
+    """One CTA with a ring of two stages."""
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    a, w = torch.randn(128, 512, device="cuda", generator=gen), torch.randn(256, 512, device="cuda", generator=gen)
+    ws = torch.empty(_lib.load().exact_linear_workspace_bytes(256, 512, 0), dtype=torch.uint8, device="cuda")
+    ref = a.double() @ w.double().t()
+    for chunk in (0, 64) * 10:
+        out = torch.empty(128, 256, device="cuda")
+        _lib.invoke("exact_linear_forward_strided", 0, _lib.ptr(a), 128, 512, 512, _lib.ptr(w), 512, 1, None, 0, 0, None, 0, 1, 256, None, None,
+                    0, chunk, None, _lib.ptr(ws), _lib.ptr(out), 256, _lib.stream_ptr())
+        assert (out.double() - ref).norm() <= (2e-7 if chunk else 5e-6) * ref.norm()
+    _lib.check_status(force=True)
