@@ -18,11 +18,13 @@
 // 1.04e-7 .. 1.2e-7 at 33 to 602 columns.  tf32 heads and tails in one chain, 3e-7 .. 4.4e-6; in
 // chains of 64 columns, the former kernel of evaluation, 1.04e-7 .. 1.39e-7; the library's fp32 GEMM 9e-8 (48) .. 4.4e-7 (602).
 // Elements that share a power of two share its range: below 2^-17 of the largest one an element has fewer than those 22 bits, and
-// beside one of 2^39 times its size none.  A tile of A in which that is more than a rare element (kLinLost), or that has rows from 2^96
-// on, whose sums could overflow under B's scale, is therefore done again from its fp32 values in tf32 (kind::tf32, heads and tails of 11
-// bits each with an exponent of their own, K tiles of 32 columns), and a weight of which it is true makes all tiles tf32:
-// 1.1e-7 .. 1.35e-7 whatever the range.  The first way's result of such a tile is not stored.  2,449,029 x 256 -> 256, plain 1,170 -
-// 1,230 us (the look for such elements is 20 - 30 of them), all tiles twice 2,550, wide weight 2,070; 169,343 x 256 -> 256: 93, 189, 140.
+// beside one of 2^39 times its size none.  That shows where the large ones are not in the sum: where the weight has a wide range itself
+// (all tiles are then done in tf32: kind::tf32, heads and tails of 11 bits each with an exponent of their own, K tiles of 32 columns), and
+// in a tile of A in which it is more than a rare element (kLinLost) while the weight has zeros or small elements to go with large ones
+// (such tiles are done again in tf32, and the first way's result is not stored).  So are tiles with rows from 2^96 on, whose sums could
+// overflow under B's scale.  1.1e-7 .. 1.35e-7 whatever the range.  2,449,029 x 256 -> 256: plain 1,170 us, all tiles twice
+// 3,240, wide weight 2,710; 169,343 x 256 -> 256: 91, 245, 199.  (Tiles of gradients, whose magnitudes often differ that much, are
+// looked through under weak weights only: done again without that rule they cost a 169,343-node GCN step 42 of 2,330 us.)
 // Non-finite inputs stay non-finite and confined to their rows, but an infinite element turns its output row into NaN where an fp32
 // GEMM gives +-inf (its tail is inf - inf).
 //
@@ -40,14 +42,15 @@
 //   warps 4-11 converters: find a row's largest magnitude in the K tile (four lanes own it), scale, split, write the heads and
 //              tails in place, fence.proxy.async, signal.  Two groups of four take alternate K tiles: a K tile is a chain of
 //              wait, reads, conversions, stores, fence and arrival.  The first warp of a group also waits for B, so that the
-//              issuing thread has one wait per K tile.  They also look for elements that fp16 cannot hold.
+//              issuing thread has one wait per K tile.  They also look for elements that fp16 cannot hold, and
+//              make the tiles of B for those of A in tf32, from the weight itself.
 //   warps 12-19 epilogue: add every K tile up, 128 sums a thread (registers moved to them by setmaxnreg); then the scales of the
 //              columns and the bias, a staging tile per warp and a TMA store of 32 x 32 boxes: with plain stores from the
 //              staging tiles the write-out was what narrow operands were bound by (2,449,029 x 48 -> 256: 904 us, boxes 589).
 //              Rows whose width or pitch is no multiple of 16 bytes, and an addend, take plain stores.
 // Bound by the chains of the roles: 2,250 cycles a K tile against 1,400 for its bytes (one launch of 128 columns, evaluation).
 // Measured (us, tf32 -> now): 2,449,029 x 256 -> 256: 1,283 -> 1,058, with a second operand pair of 256 2,424 -> 1,826; 48 -> 256:
-// 607 -> 589; 256 -> 80: 794 -> 677, 256 -> 47 (pitch 47): 668 -> 625, with an addend 1,720 -> 1,040; 232,965 x 602 -> 256: 275 -> 220
+// 607 -> 589; 256 -> 80: 794 -> 677, 256 -> 47 (pitch 47): 683 -> 574, with an addend 1,750 -> 1,110; 232,965 x 602 -> 256: 275 -> 220
 // (in chunks, evaluation: 458), 169,343 x 128 -> 256: 67 -> 63.
 // Not kept: one scale per row over the whole contraction, found ahead by four more warps, and one chain in TMEM: 2,424 -> 3,561;
 // sixteen epilogue warps with 64 sums a thread: 1,058 -> 1,115.
@@ -59,6 +62,7 @@
 #include <cuda_fp16.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "exact_b200.h"
 #include "tc.cuh"
@@ -86,8 +90,8 @@ constexpr int kLinHeadExp = 14;                 // the largest element of a row 
 // Tiles whose elements fp16 cannot hold are done again in tf32 (kind::tf32, K = 8): a K tile is 32 columns, 128 bytes as well.
 constexpr int kLinWideK = 32;
 constexpr int kLinWideExp = -8;                 // there the row's largest goes to [2^-8, 2^-7): no product with an fp32 number overflows
-// What makes a tile wide: so many hits.  Of the 128 pieces of 16 columns of a row in a K tile's 32 rows: those with an element with lost
-// bits, looking at half of a piece's columns, in eight rows at one and in eight rows at the other half.  (Normally
+// What makes a tile of A wide: so many hits.  Of the 128 pieces of 16 columns of a row in a K tile's 32 rows: those with an element with
+// lost bits, looking at half of a piece's columns, in eight rows at one and in eight rows at the other half.  (Normally
 // distributed values: 0.015 hits; a column that is small beside the others: 16; a row in which most are small beside one: 4.)  Of a
 // row of B: elements with lost bits.  And a row of either whose largest is 2^96 or more: sums, which carry B's scale, could overflow.
 constexpr int kLinLost = 3;
@@ -97,10 +101,11 @@ constexpr int kLinMaxCols = 256;                // of a launch
 
 struct LinParams {
   const __half* b;         // heads and tails of the weight, as linear_prepare_kernel lays them out
-  const float* b_wide;     // the same in tf32, not scaled
   const float* col_inv;   // [Npad] what the columns were scaled by, inverted
-  const float* unit;       // [Npad] ones: the same for tf32
-  const int* b_lost;       // [Npad] elements of a row of B with lost bits
+  const int* b_range;      // [Npad] what linear_prepare_kernel says about the rows of B
+  const float *B, *B2;     // the weight itself, for tiles in tf32: B[n * ldb + k * incb]
+  long long ldb, incb, ldb2, incb2;
+  int K, K2;
   float* C;
   const float* bias_pad;   // [Npad], with zeros behind, or null
   int* status;
@@ -132,6 +137,7 @@ __device__ __forceinline__ uint32_t lin_scale_exp(uint32_t magnitude) {
 // An fp16 head and tail hold fewer than 22 bits of a scaled element other than zero when it is below 2^-3, 2^-17 of the largest one
 // that shares the scale.  In this form zero is the largest number and the sign drops out.
 constexpr uint32_t kLinLostBelow = 2u * 0x3e000000u - 1u;
+constexpr float kLinWeakBelow = 0.5f;            // scaled: 2^-15 of a row's largest
 __device__ __forceinline__ uint32_t lin_twice_minus_one(float x) { return 2u * __float_as_uint(x) - 1u; }
 // Whether the largest magnitude that was brought to [2^14, 2^15) by this is 2^96 or more.
 __device__ __forceinline__ bool lin_huge(uint32_t exponent) { return exponent <= 127u + kLinHeadExp - 96u; }
@@ -139,7 +145,7 @@ __device__ __forceinline__ float lin_scale(uint32_t exponent) { return __uint_as
 __device__ __forceinline__ float lin_inverse(uint32_t exponent) { return __uint_as_float((254u - exponent) << 23); }
 // Four scaled elements -> heads and tails, two to a word, and the lesser lin_twice_minus_one of the first and the last (ODD: of the
 // two between).  A non-finite element has a NaN tail (inf - inf), so its output row is NaN.
-template <bool ODD>
+template <bool LOOK, bool ODD>
 __device__ __forceinline__ uint32_t split_f16(const float (&a)[4], f32x2 scale, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
   uint32_t least[2];
 #pragma unroll
@@ -147,7 +153,7 @@ __device__ __forceinline__ uint32_t split_f16(const float (&a)[4], f32x2 scale, 
     const f32x2 x = f2_mul(f2_pack(a[2 * e], a[2 * e + 1]), scale);
     float x0, x1;
     f2_unpack(x, x0, x1);
-    least[e] = lin_twice_minus_one((e != 0) != ODD ? x1 : x0);
+    if (LOOK) least[e] = lin_twice_minus_one((e != 0) != ODD ? x1 : x0);
     const __half2 h = __floats2half2_rn(x0, x1);
     const float2 back = __half22float2(h);
     f2_unpack(f2_sub(x, f2_pack(back.x, back.y)), x0, x1);
@@ -155,7 +161,7 @@ __device__ __forceinline__ uint32_t split_f16(const float (&a)[4], f32x2 scale, 
     hi[e] = *reinterpret_cast<const uint32_t*>(&h);
     lo[e] = *reinterpret_cast<const uint32_t*>(&t);
   }
-  return min(least[0], least[1]);
+  return LOOK ? min(least[0], least[1]) : 0xffffffffu;
 }
 __device__ __forceinline__ float lin_rna_tf32(float x) {
   uint32_t r;
@@ -182,7 +188,7 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   __shared__ __align__(8) unsigned long long s_narrow;               // all tiles have been through the first pass
   __shared__ uint32_t s_lost[kLinFlagWords + 1];   // a bit per tile of this CTA: to be done in tf32; the last word: whether there is any
   __shared__ uint32_t s_tmem_base;
-  __shared__ int s_abort;
+  __shared__ int s_abort, s_range;
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // known to be uniform
   const int rank = PAIR ? (int)cluster_rank() : 0;
@@ -214,26 +220,29 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   }
   // Nothing that the preparation wrote is read by __ldg: a read-only load could be moved up past this.
   if (p.after_prepare) asm volatile("griddepcontrol.wait;" ::: "memory");
-  // A weight with a row of a wide range, or with small elements in every fourth row (a column of it beside larger ones): tf32 for
-  // all.  Each warp reads the counts.
-  int4 b_lost[kLinMaxCols / 128];
+  // What the weight's range asks for.  1: a row of B has a wide range, or one row in sixteen has elements with lost bits (a column of B
+  // that is small beside others), or a row is huge: tf32 for all tiles.  2: one row in sixteen has elements below 2^-15 of its
+  // largest, or zeros.  (Of uniformly or normally distributed rows of 256 elements one in 200 and one in 50.)  One warp reads it: with
+  // all of them at the same few lines of L2 the kernel took 2 us longer.
+  if (warp == 2) {
+    int many = 0, rows = 0, weak = 0;
 #pragma unroll
-  for (int h = 0; h < kLinMaxCols / 128; h++) {
-    b_lost[h] = make_int4(0, 0, 0, 0);
-    if (128 * h + 4 * lane < p.Npad) b_lost[h] = __ldcg(reinterpret_cast<const int4*>(p.b_lost) + 32 * h + lane);
+    for (int h = 0; h < kLinMaxCols / 32; h++) {
+      const int r = 32 * h + lane < p.Npad ? __ldcg(p.b_range + 32 * h + lane) : 0;
+      many = max(many, r >> 1);
+      rows += r > 1;
+      weak += r & 1;
+    }
+    const bool all = __any_sync(0xffffffffu, many >= kLinLost) || 16 * __reduce_add_sync(0xffffffffu, rows) >= p.N;
+    weak = __reduce_add_sync(0xffffffffu, weak);
+    if (lane == 0) s_range = (all ? 1 : 0) | (16 * weak >= p.N ? 2 : 0);
   }
   tc_fence_before();
   __syncthreads();
   if (PAIR) cluster_sync();     // the other CTA arrives on these barriers
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
-  int b_many = 0, b_rows = 0;
-#pragma unroll
-  for (int h = 0; h < kLinMaxCols / 128; h++) {
-    b_many = max(max(b_many, max(b_lost[h].x, b_lost[h].y)), max(b_lost[h].z, b_lost[h].w));
-    b_rows += (b_lost[h].x > 0) + (b_lost[h].y > 0) + (b_lost[h].z > 0) + (b_lost[h].w > 0);
-  }
-  const bool wide = __any_sync(0xffffffffu, b_many >= kLinLost) || 4 * __reduce_add_sync(0xffffffffu, b_rows) >= p.N;
+  const bool wide = __any_sync(0xffffffffu, s_range & 1) != 0, weak = (s_range & 2) != 0;     // wide is known to be uniform
 
   // the tiles of a pair are neighbours; one past the last (an odd number of tiles) reads zeros and stores nothing
   const int first = blockIdx.x, step = gridDim.x, tiles = PAIR ? (p.num_tiles + 1) / 2 * 2 : p.num_tiles;
@@ -263,7 +272,6 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       for (int pass = wide ? 1 : 0; pass < 2 && ok; pass++) {
       if (pass == 1 && !second_pass(ok)) break;
       const int kblocks = pass ? p.wide_kblocks : p.kblocks, kblocks1 = pass ? p.wide_kblocks1 : p.kblocks1;
-      const char* b = pass ? reinterpret_cast<const char*>(p.b_wide) : reinterpret_cast<const char*>(p.b);
       for (int tile = first, nth = 0; tile < tiles && ok; tile += step, nth++) {
         if (!walks(pass, nth)) continue;
         for (int kb = 0; kb < kblocks; kb++, st.next(p.stages)) {
@@ -275,10 +283,14 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           mbar_arrive_expect_tx(full, pass ? kLinHalf : 2 * kLinHalf);      // a box past the row's end is zeros
           tma_load_2d(dst, map, x, tile * kLinTileM, full);
           if (pass == 0) tma_load_2d(dst + kLinHalf, map, x + kLinBoxK, tile * kLinTileM, full);
-          mbar_arrive_expect_tx(bfull, 2 * p.b_slot);
-          bulk_load(dst + kLinSlotBytes, b + (size_t)(PAIR ? 2 * kb + rank : kb) * (2 * p.b_slot), 2 * p.b_slot, bfull);
           if (uses < p.stages) uses++;
-          if (pass) continue;
+          if (pass) {
+            mbar_arrive(bfull);       // the converters make these tiles of B
+            continue;
+          }
+          mbar_arrive_expect_tx(bfull, 2 * p.b_slot);
+          bulk_load(dst + kLinSlotBytes, reinterpret_cast<const char*>(p.b) + (size_t)(PAIR ? 2 * kb + rank : kb) * (2 * p.b_slot),
+                    2 * p.b_slot, bfull);
           // A comes from HBM exactly once: pull the tile that will be loaded kLinPrefetch K tiles from now into L2, so that its
           // TMA load later pays L2 latency only
           int pk = kb + kLinPrefetch, pt = tile;
@@ -456,6 +468,29 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
               asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + kLinHalf), "f"(lo[0]), "f"(lo[1]), "f"(lo[2]), "f"(lo[3]) : "memory");
             }
           }
+          // This CTA's rows of B, from memory (L2): a lane is a column, or a row where columns are the contiguous direction.
+          const bool second = kb >= p.wide_kblocks1;
+          const float* B = second ? p.B2 : p.B;
+          const long long ldb = second ? p.ldb2 : p.ldb, incb = second ? p.incb2 : p.incb;
+          const int k0 = (second ? kb - p.wide_kblocks1 : kb) * kLinWideK, K = second ? p.K2 : p.K;
+          const int rows = (int)(p.b_slot / 128), n0 = rank * rows, w4 = (warp - kLinFirstConv) % kLinConvGroup;
+          const uint32_t bdst = ring + (uint32_t)st.s * p.stage_bytes + kLinSlotBytes;
+          auto put = [&](int r, int k) {
+            const float x = n0 + r < p.N && k0 + k < K ? __ldg(B + (long long)(n0 + r) * ldb + (long long)(k0 + k) * incb) : 0.f;
+            const float head = lin_rna_tf32(x), tail = lin_rna_tf32(__fsub_rn(x, head));
+            const uint32_t to = bdst + (uint32_t)r * 128u + (uint32_t)(((k >> 2) ^ (r & 7)) << 4) + (uint32_t)(k & 3) * 4u;
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(to), "f"(head) : "memory");
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(to + p.b_slot), "f"(tail) : "memory");
+          };
+          if (incb == 1) {
+#pragma unroll 4
+            for (int r = w4; r < rows; r += kLinConvGroup) put(r, lane);
+          } else {
+            for (int r = w4 * 32 + lane; r < rows; r += kLinConvGroup * 32) {
+#pragma unroll 4
+              for (int k = 0; k < kLinWideK; k++) put(r, k);
+            }
+          }
         } else {
         float a[2][4][4];
         auto read = [&](int pass, float (&v)[4][4]) {
@@ -466,6 +501,8 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                          : "r"(base + (uint32_t)pass * 1024u + (uint32_t)box * kLinHalf + (uint32_t)((c ^ r8) << 4)) : "memory");
           }
         };
+        auto convert = [&](auto look) {
+        constexpr bool LOOK = decltype(look)::value;
         read(0, a[0]);
 #pragma unroll
         for (int pass = 0; pass < 4; pass++) {
@@ -486,17 +523,22 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           for (int j = 0; j < 4; j++) {
             const int box = (j >> 1) ^ (r8 >> 1 & 1), c = part + 4 * ((j & 1) ^ (r8 & 1));
             uint32_t hi[2], lo[2];
-            least[j] = pass & 1 ? split_f16<true>(v[j], s2, hi, lo) : split_f16<false>(v[j], s2, hi, lo);
+            least[j] = pass & 1 ? split_f16<LOOK, true>(v[j], s2, hi, lo) : split_f16<LOOK, false>(v[j], s2, hi, lo);
             const uint32_t to = base + (uint32_t)pass * 1024u + (uint32_t)(((box * 4 + (c >> 1)) ^ r8) << 4) + (uint32_t)(c & 1) * 8u;
             asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(to), "r"(hi[0]), "r"(hi[1]) : "memory");
             asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(to + kLinHalf), "r"(lo[0]), "r"(lo[1]) : "memory");
           }
-          lost += lin_huge(exponent) ? kLinLost : min(min(least[0], least[1]), min(least[2], least[3])) < kLinLostBelow ? 1 : 0;
+          lost += lin_huge(exponent) ? kLinLost : LOOK && min(min(least[0], least[1]), min(least[2], least[3])) < kLinLostBelow ? 1 : 0;
         }
+        };
+        // Elements with lost bits are looked for only under a weak weight.  Else the row's largest element meets at least 2^-15 of the
+        // largest weight, and what another one lost is below 2^-24 of that product.
+        if (weak) convert(std::true_type());
+        else convert(std::false_type());
         }
         fence_proxy_async_smem_lin();  // generic-proxy stores -> visible to the tensor core's reads
         __syncwarp();
-        if (first_warp && !mbar_wait(smem_u32(&s_bfull[st.s]), st.ph, abort_flag)) { ok = false; break; }   // for the MMA's one wait
+        if (pass == 0 && first_warp && !mbar_wait(smem_u32(&s_bfull[st.s]), st.ph, abort_flag)) { ok = false; break; }   // for the MMA's one wait
         if (lane == 0) {
           if (PAIR) mbar_arrive_leader(smem_u32(&s_ready[st.s]));
           else mbar_arrive(smem_u32(&s_ready[st.s]));
@@ -537,7 +579,7 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       __syncwarp();
       const int c = c0 + lane;
       const bool inside = lane < cols && c < p.N;
-      const float inv = inside ? col_inv[c] : 0.f, bias = inside && p.bias_pad != nullptr ? p.bias_pad[c] : 0.f;
+      const float inv = inside && col_inv != nullptr ? col_inv[c] : 1.f, bias = inside && p.bias_pad != nullptr ? p.bias_pad[c] : 0.f;
       const int rows = !inside ? 0 : p.M - row_base < 32 ? (int)(p.M - row_base) : 32;
       float* d = p.C + row_base * p.ldc + c;
 #pragma unroll
@@ -554,7 +596,7 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       __syncwarp();
       const int c = c0 + lane;
       const bool inside = lane < cols && c < p.N;
-      const float inv = inside ? col_inv[c] : 0.f, bias = inside && p.bias_pad != nullptr ? p.bias_pad[c] : 0.f;
+      const float inv = inside && col_inv != nullptr ? col_inv[c] : 1.f, bias = inside && p.bias_pad != nullptr ? p.bias_pad[c] : 0.f;
       const int rows = p.M - row_base < 32 ? (int)(p.M - row_base) : 32;
       float* d = p.C + row_base * p.ldc + c;
       const float* add = p.addend + row_base * p.ldadd + c;
@@ -584,17 +626,10 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     for (int pass = wide ? 1 : 0; pass < 2 && ok; pass++) {
     if (pass == 1 && !second_pass(ok)) break;
     const int kblocks = pass ? p.wide_kblocks : p.kblocks;
-    const float* const col_inv = pass ? p.unit : p.col_inv;
+    const float* const col_inv = pass ? nullptr : p.col_inv;      // tf32: not scaled
     for (int tile = first, nth = 0; tile < tiles && ok; tile += step, nth++) {
       if (!walks(pass, nth)) continue;
       const long long row_base = (long long)tile * kLinTileM + quad * 32;
-      if (p.addend != nullptr && row_base + lane < p.M) {     // on its way to L2 while the tile is summed
-        const float* add = p.addend + (row_base + lane) * p.ldadd;
-        for (int c0 = share * 32; c0 < p.N; c0 += 64) {
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(add + c0));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(add + (c0 + 31 < p.N ? c0 + 31 : p.N - 1)));
-        }
-      }
       // Every K tile is drained and added up here in fp32, with its scales and its average loss given back: half of a row's 256
       // columns a thread.  (Kept in memory the sums were 16 TB/s of L2 traffic.)
       float run[kLinMaxCols / kLinEpiGroups];
@@ -634,8 +669,8 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
 #pragma unroll
           for (int j = 0; j < 8; j++) {
             const int c = c0 + 4 * j;
-            float4 inv = make_float4(0.f, 0.f, 0.f, 0.f), bias = inv;
-            if (c < p.Npad) inv = *reinterpret_cast<const float4*>(col_inv + c);
+            float4 inv = make_float4(1.f, 1.f, 1.f, 1.f), bias = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (col_inv != nullptr && c < p.Npad) inv = *reinterpret_cast<const float4*>(col_inv + c);
             if (p.bias_pad != nullptr && c < p.Npad) bias = *reinterpret_cast<const float4*>(p.bias_pad + c);
             const float* v = run + 32 * b + 4 * j;
             const uint32_t addr = stage_addr + (uint32_t)lane * 128u + (((uint32_t)j ^ ((uint32_t)lane & 7u)) << 4);
@@ -678,18 +713,17 @@ linear_f16x3_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
 
 // Heads and tails of [B | B2] (rows = output features), each row scaled by a power of two, zero padded to [Npad, Kpad1 + Kpad2], in
 // the order and with the swizzle of the shared-memory tiles: K tile by K tile, in it the share of each CTA of a pair (b_rows rows),
-// in that the heads and then the tails, so that a CTA's part of a K tile is one contiguous run.  Once in fp16 and once, not scaled, in
-// tf32 with its K tiles of 32 columns.  A block per row; also writes the inverse scales, counts the elements that fp16 cannot
-// hold and clears the status word, if given.
+// in that the heads and then the tails, so that a CTA's part of a K tile is one contiguous run.  A block per row; also writes the
+// inverse scales, what the row's range is (twice the number of elements with lost bits, kLinLost for a huge row, + 1 with an
+// element that is weak), and clears the status word, if given.
 constexpr int kLinPrepThreads = 128;
 struct LinPrep {
   const float *B, *B2, *bias;
   long long ldb, incb, ldb2, incb2;
   int K, K2, N, Npad, Kpad1, Kpad, b_rows;
-  int wide1;               // K tiles of B in tf32
   __half* out;
-  float *wide, *col_inv, *bias_pad, *unit;
-  int *lost, *status;
+  float *col_inv, *bias_pad;
+  int *range, *status;
 };
 __global__ void __launch_bounds__(kLinPrepThreads) linear_prepare_kernel(const __grid_constant__ LinPrep p) {
   __shared__ uint32_t s_max[kLinPrepThreads / 32], s_lost[kLinPrepThreads / 32];
@@ -702,6 +736,7 @@ __global__ void __launch_bounds__(kLinPrepThreads) linear_prepare_kernel(const _
     return kk - p.Kpad1 < p.K2 ? __ldg(p.B2 + (long long)n * p.ldb2 + (kk - p.Kpad1) * p.incb2) : 0.f;
   };
   uint32_t m = 0, lost = 0;
+  bool weak = false;
   for (int kk = threadIdx.x; kk < p.Kpad; kk += kLinPrepThreads) m = max(m, __float_as_uint(element(kk)) & 0x7fffffffu);
   m = __reduce_max_sync(0xffffffffu, m);
   if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
@@ -714,30 +749,22 @@ __global__ void __launch_bounds__(kLinPrepThreads) linear_prepare_kernel(const _
   for (int kk = threadIdx.x; kk < p.Kpad; kk += kLinPrepThreads) {
     const float x = element(kk), v = x * scale;
     lost += lin_twice_minus_one(v) < kLinLostBelow ? 1u : 0u;
+    weak |= fabsf(v) < kLinWeakBelow && (kk < p.Kpad1 ? kk < p.K : kk - p.Kpad1 < p.K2);
     const __half hi = __float2half_rn(v), lo = __float2half_rn(v - __half2float(hi));
     const int kb = kk / kLinTileK, e = kk - kb * kLinTileK;
     const size_t at = (size_t)(kb * shares + share) * 2 * p.b_rows * kLinTileK + r * kLinTileK + (((e >> 3) ^ (r & 7)) << 3) + (e & 7);
     p.out[at] = hi;
     p.out[at + (size_t)p.b_rows * kLinTileK] = lo;
-    const int k = kk < p.Kpad1 ? kk : kk - p.Kpad1, of = kk < p.Kpad1 ? p.K : p.K2;
-    if (k / kLinWideK * kLinWideK < of) {      // the last K tile in tf32 may end sooner
-      const int kw = (kk < p.Kpad1 ? 0 : p.wide1) + k / kLinWideK, f = k % kLinWideK;
-      const size_t to = (size_t)(kw * shares + share) * 2 * p.b_rows * kLinWideK + r * kLinWideK + (((f >> 2) ^ (r & 7)) << 2) + (f & 3);
-      const float head = lin_rna_tf32(x);
-      p.wide[to] = head;
-      p.wide[to + (size_t)p.b_rows * kLinWideK] = lin_rna_tf32(__fsub_rn(x, head));
-    }
   }
   lost = __reduce_add_sync(0xffffffffu, lost);
   if ((threadIdx.x & 31) == 0) s_lost[threadIdx.x >> 5] = lost;
-  __syncthreads();
+  weak = __syncthreads_or(weak && m != 0) != 0;
   if (threadIdx.x == 0) {
     lost = lin_huge(exponent) ? kLinLost : 0;
 #pragma unroll
     for (int w = 0; w < kLinPrepThreads / 32; w++) lost += s_lost[w];
-    p.lost[n] = (int)lost;
+    p.range[n] = (int)(2 * lost + (weak ? 1 : 0));
     p.col_inv[n] = lin_inverse(exponent);
-    p.unit[n] = 1.f;
     p.bias_pad[n] = p.bias != nullptr && n < p.N ? p.bias[n] : 0.f;
   }
 }
@@ -814,22 +841,20 @@ static int lin_launch(const float* A, int64_t M, int64_t K, int64_t lda, const f
   b.B = B; b.B2 = B2; b.bias = bias; b.ldb = ldb; b.incb = incb; b.ldb2 = ldb2; b.incb2 = incb2;
   b.K = (int)K; b.K2 = (int)K2; b.N = (int)N; b.Npad = Npad; b.Kpad1 = lin_kpad(K); b.Kpad = b.Kpad1 + lin_kpad(K2);
   b.b_rows = pair ? Npad / 2 : Npad;   // of B in one CTA
-  b.wide1 = lin_wide_tiles(K);
   b.status = reinterpret_cast<int*>(workspace);
   b.col_inv = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + 256);
   b.bias_pad = b.col_inv + kLinMaxCols;
-  b.unit = b.bias_pad + kLinMaxCols;
-  b.lost = reinterpret_cast<int*>(b.unit + kLinMaxCols);
-  b.out = reinterpret_cast<__half*>(b.lost + kLinMaxCols);
-  b.wide = reinterpret_cast<float*>(b.out + (size_t)2 * Npad * b.Kpad);
+  b.range = reinterpret_cast<int*>(b.bias_pad + kLinMaxCols);
+  b.out = reinterpret_cast<__half*>(b.range + kLinMaxCols);
   linear_prepare_kernel<<<Npad, kLinPrepThreads, 0, st>>>(b);
   EXB_CUDA_OK(cudaGetLastError());
 
   LinParams p{};
-  p.b = b.out; p.b_wide = b.wide; p.col_inv = b.col_inv; p.unit = b.unit; p.b_lost = b.lost; p.bias_pad = bias ? b.bias_pad : nullptr;
+  p.b = b.out; p.col_inv = b.col_inv; p.b_range = b.range; p.bias_pad = bias ? b.bias_pad : nullptr;
   p.status = b.status; p.lib_status = status_word_ptr(); p.N = (int)N; p.Npad = Npad;
   p.kblocks1 = b.Kpad1 / kLinTileK; p.kblocks = b.Kpad / kLinTileK;
-  p.wide_kblocks1 = b.wide1; p.wide_kblocks = b.wide1 + lin_wide_tiles(K2);
+  p.wide_kblocks1 = lin_wide_tiles(K); p.wide_kblocks = p.wide_kblocks1 + lin_wide_tiles(K2);
+  p.B = B; p.B2 = B2; p.ldb = ldb; p.incb = incb; p.ldb2 = ldb2; p.incb2 = incb2; p.K = (int)K; p.K2 = (int)K2;
   p.b_slot = (unsigned)b.b_rows * kLinTileK * 2;
   p.stage_bytes = kLinSlotBytes + 2 * p.b_slot;
   p.stages = (int)((kLinSlots * kLinSlotBytes) / p.stage_bytes);
@@ -856,9 +881,10 @@ extern "C" {
 int64_t exact_linear_workspace_bytes(int64_t N, int64_t K, int64_t K2) {
   if (N <= 0 || K <= 0 || K2 < 0) return 256;
   const int64_t Npad = (N + 15) / 16 * 16;
-  // this file's scales, and its tiles in fp16 and in tf32; linear_tf32.cu needs less
-  return 256 + 4 * kLinMaxCols * 4 + 2 * Npad * (int64_t)(lin_kpad(K) + lin_kpad(K2)) * 2 +
-         2 * Npad * (int64_t)(lin_wide_tiles(K) + lin_wide_tiles(K2)) * kLinWideK * 4;
+  // the tiles, scales and ranges of this file's kernel, and the two fp32 copies in rows of 32 columns of the other's
+  const int64_t tiles = 256 + 3 * kLinMaxCols * 4 + 2 * Npad * (int64_t)(lin_kpad(K) + lin_kpad(K2)) * 2;
+  const int64_t copies = 256 + 2 * Npad * (int64_t)(lin_wide_tiles(K) + lin_wide_tiles(K2)) * kLinWideK * 4;
+  return tiles > copies ? tiles : copies;
 }
 
 int64_t exact_linear_partial_bytes(int64_t) { return 0; }   // the running sums of a contraction in chunks stay in registers

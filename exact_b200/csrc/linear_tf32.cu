@@ -33,7 +33,7 @@
 //              parity are counted instead of divided out.  Accumulators are double-buffered in TMEM.
 //   warps 10-17 epilogue: tcgen05.ld -> per-warp staging tile in shared memory -> (+ bias, + addend)
 //              -> coalesced global stores; two groups of four take alternate blocks of 32 columns.
-// Measured (us, here | the other kernel): 169,343 x 128 -> 256: 67 | 66, 256 -> 256: 95 | 93, 256 -> 40: 58 | 56; 2,449,029 x 256 -> 47: 668 | 625.
+// Measured (us, here | the other kernel): 169,343 x 128 -> 256: 67 | 66, 256 -> 256: 95 | 93, 256 -> 40: 58 | 56; 2,449,029 x 256 -> 47: 683 | 574.
 // The weight is split, padded and laid out as the tiles once per call by a preparation kernel.
 //
 // Every mbarrier wait is bounded; on expiry the CTA raises an abort flag, all roles leave their loops,

@@ -493,12 +493,12 @@ EXACT_API int exact_linear_forward(const float* A, int64_t M, int64_t K, int64_t
  * (NULL: nothing; it may be C).  incb, incb2: distance between the elements of a row of B, B2 (ldb = 1 and incb =
  * the pitch: the transposed weight, without a copy).  k_chunk (a multiple of 32): 0: the contraction is one chain of tf32 products
  * in the tensor core's accumulator, which truncates at every MMA, a bias of about 7e-9 of the result per contracted column.  Else
- * it is cut into chunks of 64 columns, whose operands are scaled by powers of two and split into fp16 head and tail, or, where their
- * magnitudes differ too much for that (by more than 2^17 in a row's 64 columns, in more than a few elements of a tile of 128 rows;
- * for a weight, all rows), of 32 columns split into tf32 head and tail.  A chunk's sum has its average loss given back and is added to
- * the others in fp32: 1.04e-7 .. 1.35e-7 (Frobenius, against fp64) whatever K and the range are, and faster than one chain but for rows
- * of C that are no multiple of 16 bytes and for tf32 tiles (up to twice its time).  partial: exact_linear_partial_bytes(N)
- * bytes (none: not used any more). */
+ * it is cut into chunks of 64 columns, whose operands are scaled by powers of two and split into fp16 head and tail.  Where
+ * magnitudes differ so much that it would show (an element holds fewer than 22 bits below 2^-17 of the largest of a row's 64 columns,
+ * or of the weight's row) the tile's rows, or for a weight all rows, go in chunks of 32 columns split into tf32 head and tail.  A chunk's
+ * sum has its average loss given back and is added to the others in fp32: 1.04e-7 .. 1.35e-7 (Frobenius, against fp64) whatever
+ * K and the range are, and faster than one chain but for those tiles (up to 2.7 times the plain time).  partial:
+ * exact_linear_partial_bytes(N) bytes (none: not used any more). */
 EXACT_API int64_t exact_linear_partial_bytes(int64_t N);
 EXACT_API int exact_linear_forward_strided(const float* A, int64_t M, int64_t K, int64_t lda, const float* B, int64_t ldb,
                                            int64_t incb, const float* A2, int64_t K2, int64_t lda2, const float* B2,
