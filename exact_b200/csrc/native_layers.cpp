@@ -472,7 +472,8 @@ Tensor aggregate_node(const Tensor& x, const OptTensor& value, const OptTensor& 
 
 // ---- evaluation -----------------------------------------------------------------------------------------
 // Evaluation is compared with the plain fp32 model, so its products are no further from the exact ones than the library's fp32 GEMM:
-// 1.06e-7 to 1.2e-7 (Frobenius) from 100 columns on against 1.8e-7 at 100, 2.0e-7 at 256 and 4.4e-7 at 602.  Up to 64 columns the
+// 1.06e-7 to 1.2e-7 (Frobenius) from 100 columns on against 1.8e-7 at 100, 2.0e-7 at 256 and 4.4e-7 at 602.  (Where one feature outweighs
+// the others: 1.1e-7 .. 1.35e-7 against 1.0e-7 .. 1.3e-7, sums of few terms round less.)  Up to 64 columns the
 // library is the nearer one (9e-8 against 1.04e-7 at 48) and takes them, 200,000 x 48 -> 256 in 173 us against 58.
 constexpr int64_t kEvalLibrary = 64;
 
