@@ -177,3 +177,21 @@ def test_workspace_holds_anything_before(M, K, N):
                         None, 0, 64, None, _lib.ptr(ws), _lib.ptr(out), N, _lib.stream_ptr())
             assert torch.equal(out, result)
     check_status()
+
+
+# a layer whose two weights, and their operands the other way round, differ more and more; rows of one or both weights zero
+@pytest.mark.parametrize("shift", [-30, -21, -13, 0, 13, 16, 21, 30])
+@pytest.mark.parametrize("M,K,K2,N", [(1300, 100, 64, 256), (2000, 7, 130, 47)])
+def test_operand_pairs_of_different_magnitudes(M, K, K2, N, shift):
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    a, a2 = torch.randn(M, K, device="cuda", generator=gen) * 2.0 ** shift, torch.randn(M, K2, device="cuda", generator=gen)
+    w, w2 = torch.randn(N, K, device="cuda", generator=gen) * 2.0 ** -shift, torch.randn(N, K2, device="cuda", generator=gen)
+    w[1], w2[2] = 0.0, 0.0
+    w[3], w2[3] = 0.0, 0.0
+    bias = torch.randn(N, device="cuda", generator=gen)
+    got = product(a, w, bias, a2=a2, w2=w2).double()
+    A, W = torch.cat([a, a2], 1).double(), torch.cat([w, w2], 1).double()
+    ref = A @ W.t()
+    assert bool(((got - ref - bias.double()).abs() <= wide_bound(A, W, K + K2) + 2.0 ** -23 * (ref + bias).abs()).all())
+    assert torch.equal(got[:, 3].float(), bias[3].expand(M))
+    assert (got - ref - bias.double()).norm() <= 2e-7 * ref.norm()
